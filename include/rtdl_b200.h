@@ -631,16 +631,11 @@ RTDL_B200_API int rtdl_b200_get_last_query_stats(unsigned long long* values_out,
  * devices).  Benchmarks read it before and after a timed region. */
 RTDL_B200_API int rtdl_b200_get_launch_count(unsigned long long* count_out);
 
-/* Tuning knobs; the autotuner sets these.  leaf_size: points per LBVH leaf
- * bucket (1..32, applies to scenes built afterwards; 0, the default: 32);
- * block_threads: 64, 128
- * or 256; traversal: 0 = one warp walks the tree for 32 neighbouring queries
- * (packet), 1 = one thread per query, 2 = packet with the query's bounding
- * cube tested at internal nodes, 3 = packet whose leaf buckets are tested
- * point-major (a lane per point, the reaching queries in turn), 4 (the
- * default) = packet choosing lane- or point-major per bucket (point-major when
- * at most half as many of the packet's queries reach it as it holds points).
- * Every setting returns the same rows.  Returns 0 on success. */
+/* Tuning knobs: leaf_size 0..32, block_threads 64, 128 or 256, traversal 0..4.
+ * The walks have one form now (eight points per bucket, packets of 32
+ * neighbouring queries or a warp per query, chosen per call and per packet), so
+ * every setting runs the same kernels and returns the same rows; the call stays
+ * for callers that make it, with its checks.  Returns 0 on success. */
 RTDL_B200_API int rtdl_b200_set_tuning(int leaf_size, int block_threads, int traversal);
 
 #ifdef __cplusplus

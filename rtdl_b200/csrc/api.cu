@@ -421,10 +421,6 @@ struct PreparedHandle {
 
 }  // namespace
 
-int scene_leaf_size() {
-  if (tuning().leaf_size > 0) return tuning().leaf_size;
-  return 32;
-}
 
 cudaStream_t aux_stream(int which) {
   static thread_local std::map<std::pair<int, int>, cudaStream_t> streams;
@@ -648,7 +644,7 @@ int scene_create_impl(const void* points, size_t count, int dimension, int point
     }
     Scene* sc = nullptr;
     try {
-      sc = build_scene(d_points, (uint32_t)count, dimension, s, scene_leaf_size());
+      sc = build_scene(d_points, (uint32_t)count, dimension, s);
       unsigned int bad = 0;
       RTDL_CUDA_CHECK(cudaMemcpyAsync(&bad, &sc->stats->bad, sizeof(bad), cudaMemcpyDeviceToHost, s));
       RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
@@ -771,7 +767,7 @@ int rtdl_b200_batch_create(const void* points, const unsigned long long* point_o
         owned = upload(points, record_size(dimension) * count, s);
         d_points = owned;
       }
-      sc = build_scene_batch(d_points, point_offsets, problems, dimension, s, scene_leaf_size());
+      sc = build_scene_batch(d_points, point_offsets, problems, dimension, s);
       unsigned int bad = 0;
       RTDL_CUDA_CHECK(cudaMemcpyAsync(&bad, &sc->stats->bad, sizeof(bad), cudaMemcpyDeviceToHost, s));
       RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
@@ -1384,7 +1380,7 @@ int rtdl_b200_run_fixed_radius_count_threshold(const RtdlPoint* query_points, si
     void* d_query = nullptr;
     Scene* sc = nullptr;
     try {
-      sc = build_scene(d_search, (uint32_t)search_count, 2, s, scene_leaf_size());
+      sc = build_scene(d_search, (uint32_t)search_count, 2, s);
       d_query = upload(query_points, sizeof(RtdlPoint) * query_count, s);
       count_rows_to_host(sc, d_query, (uint32_t)query_count, radius, (uint32_t)threshold, rows_out, row_count_out, s);
     } catch (...) {
@@ -1676,7 +1672,7 @@ int rtdl_b200_prepare_point_group_nearest_witness_2d(const RtdlPoint* search_poi
     RTDL_CUDA_CHECK(cudaGetDevice(&dev));
     ensure_pool_configured(dev);
     *prepared_out = point_group_create(search_points, search_count, groups, group_count, max_radius,
-                                       scene_leaf_size(), library_stream());
+                                       library_stream());
   }, error_out, error_size);
 }
 

@@ -43,8 +43,7 @@ inline void sync_quietly(cudaStream_t s) {
 }
 
 constexpr int kSmCount = 148;          // B200: 2 dies x 74 SMs
-constexpr int kMaxList = 64;           // per-query list capacity held in shared memory
-constexpr int kStackDepth = 64;        // traversal stack; Karras depth <= 30 code bits + 32 index bits
+constexpr int kMaxList = 64;           // largest k of a nearest search that is not brute force
 constexpr uint32_t kNone = 0xFFFFFFFFu;
 
 // ---- reductions over an input point set ------------------------------------
@@ -88,30 +87,41 @@ __host__ __device__ inline float ordered_to_float(unsigned int o) {
 #endif
 }
 
-// ---- a built scene (LBVH over the search points) ---------------------------
-// Node layout: the collapsed tree in depth-first pre-order, 2 x float4 = 32 B
-// per node, traversed without a stack:
-//   n[0] = {lo.xyz, ref}   ref == kInternalNode: an internal node, its left
-//                          child is the next record (descend on overlap);
-//                          ref < 0: leaf bucket, see leaf_first / leaf_count
-//   n[1] = {hi.xyz, rope}  next record when the subtree is done or missed;
-//                          kRopeEnd ends the traversal
-// The root is record 0.
-constexpr int kRopeEnd = -1;
-constexpr int kInternalNode = 0;
-constexpr uint32_t kMaxScenePoints = 1u << 26;  // leaf references keep 26 bits for the first point
-__host__ __device__ inline int leaf_ref(int first, int count) { return ~((first << 5) | (count - 1)); }
-__host__ __device__ inline int leaf_first(int hit) { return (~hit) >> 5; }
-__host__ __device__ inline int leaf_count(int hit) { return ((~hit) & 31) + 1; }
+// ---- a built scene -----------------------------------------------------------
+constexpr uint32_t kMaxScenePoints = 1u << 26;
+
+// Wide tree over the points in curve order, what the fixed-radius walks read.
+// Eight consecutive points make a bucket (the last one of a problem is filled
+// up with points at infinity, which no radius reaches), 32 consecutive buckets
+// a level-1 node, 32 of those a level-2 node, and so on until a level has at
+// most 32 nodes: no links, no splits.  A warp tests a node's 32 children in
+// one step, one per lane, with coalesced loads; 1M points take four levels
+// where a binary walk visited about 200 dependent nodes per packet of queries.
+constexpr int kBucketPoints = 8;
+constexpr int kFan = 32;
+constexpr int kTreeLevels = 5;  // 2^26 points: 2^23 buckets, 2^18, 2^13, 2^8, 8 nodes
+struct TreeShape {
+  uint32_t base[kTreeLevels];  // first node of each level; level 0 are the buckets
+  uint32_t buckets;
+  uint32_t top;                // the level a walk starts at (at most kFan nodes)
+  uint32_t points;
+};
+__host__ __device__ inline uint32_t tree_level_nodes(uint32_t buckets, uint32_t level) {
+  return (buckets + ((1u << (5 * level)) - 1u)) >> (5 * level);
+}
 
 struct SceneView {
-  const float4* pts;      // n sorted points: x, y, z (0 for 2D), w = record id bits
+  const float4* pts;      // sorted points: x, y, z (0 for 2D), w = record id bits; whole buckets
   const uint32_t* perm;   // sorted index -> search input index
   const double* pts64;    // 3 doubles per sorted point (exact coordinates), used when inexact
-  const float4* nodes;    // 2 float4 per node, collapsed tree in pre-order
+  const float4* bucket_pts;     // 2 float4 per axis and bucket: x of points 0..3, 4..7, then y, then z;
+                                // one bucket of points at infinity follows the last (id slots / 8)
+  const float4* wide;           // 2 float4 per wide node: lo, hi
+  const TreeShape* trees;       // one per problem (one in all for a plain scene)
+  uint32_t tree_stride;         // 1: problem p walks trees[p]; 0: every problem walks trees[0]
   uint32_t n;
+  uint32_t slots;               // entries of pts (n and the buckets' filling)
   const unsigned int* inexact;  // device flag: scene coordinates are not all FP32-exact
-  const int* prob_root;   // problem batch: pre-order index of each problem's subtree (nullptr: one problem)
 };
 
 struct Scene {
@@ -120,46 +130,47 @@ struct Scene {
   uint32_t n = 0;
   double max_radius = 0.0;  // prepared-FRN contract only
   bool device_columns = false;  // built from partner-owned device columns (count-threshold contract)
-  int leaf_size = 8;
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   float4* pts = nullptr;
   uint32_t* perm = nullptr;
   double* pts64 = nullptr;
-  float4* nodes = nullptr;
-  uint32_t* codes = nullptr;    // Morton codes of the sorted points (seed nearest searches)
+  uint32_t* codes = nullptr;    // curve codes of the sorted points (seed nearest searches)
   PointStats* stats = nullptr;  // device copy of the build statistics
-  // A batch of independent problems (problems > 0) is built as one tree: the
-  // sort key is (problem << code_bits) | Morton code in the problem's own box,
-  // so every problem is one subtree; prob_root holds its pre-order index
-  // (kRopeEnd for a problem without points) and the subtree ends at that
-  // node's rope.
+  float4* bucket_pts = nullptr;
+  float4* wide = nullptr;
+  TreeShape* trees = nullptr;   // device
+  uint32_t slots = 0;           // entries of pts / perm / pts64
+  // A batch of independent problems (problems > 0) is sorted by (problem <<
+  // code_bits) | curve code in the problem's own box, and every problem's
+  // points make a wide tree of their own (trees[p], whole buckets each).
   uint32_t problems = 0;
   int code_bits = 0;
-  PointStats* prob_stats = nullptr;  // device, per problem: the box of its Morton codes
-  int* prob_root = nullptr;          // device, per problem
+  PointStats* prob_stats = nullptr;  // device, per problem: the box of its curve codes
   std::vector<unsigned long long> prob_offsets;  // host, problems + 1: input offsets of each problem's points
   SceneView view() const {
     SceneView v;
     v.pts = pts;
     v.perm = perm;
     v.pts64 = pts64;
-    v.nodes = nodes;
+    v.bucket_pts = bucket_pts;
+    v.wide = wide;
+    v.trees = trees;
+    v.tree_stride = problems ? 1u : 0u;
     v.n = n;
+    v.slots = slots;
     v.inexact = stats ? &stats->inexact : nullptr;
-    v.prob_root = prob_root;
     return v;
   }
 };
 
 // ---- tuning ---------------------------------------------------------------
+// Settings of rtdl_b200_set_tuning.  The walks have one form, so every setting
+// runs the same kernels; they stay for callers that set them.
 struct Tuning {
-  int leaf_size = 0;  // 0: automatic (scene_leaf_size)
+  int leaf_size = 0;
   int block_threads = 128;
-  int traversal = 4;  // fixed-radius collect: 0 = one warp per 32 queries (packet), 1 = one thread per
-                      // query, 2 = packet with cube tests at internal nodes, 3 = packet with
-                      // point-major leaf tests, 4 (default) = packet choosing lane- or point-major
-                      // per leaf
+  int traversal = 4;
 };
 // The tuning a call runs with: a copy of the process-wide setting taken when
 // the entry point starts (rtdl_b200_set_tuning from another thread changes the
@@ -208,16 +219,16 @@ void iota_u32(uint32_t* out, uint32_t n, cudaStream_t s);
 
 // ---- scene build (lbvh.cu) -------------------------------------------------
 // `points` is a device AoS of RtdlPoint (dim 2) or RtdlPoint3D (dim 3).
-Scene* build_scene(const void* points_dev, uint32_t n, int dim, cudaStream_t s, int leaf_size);
+Scene* build_scene(const void* points_dev, uint32_t n, int dim, cudaStream_t s);
 // Problem batch: points_dev holds the problems' points back to back, problem
 // p at [offsets[p], offsets[p + 1]) (host array of problems + 1 entries).
 Scene* build_scene_batch(const void* points_dev, const unsigned long long* offsets, uint32_t problems, int dim,
-                         cudaStream_t s, int leaf_size);
-// Bits of the problem id in a batch's sort keys, and the Morton bits below it.
+                         cudaStream_t s);
+// Bits of the problem id in a batch's sort keys, and the code bits below it.
 int batch_problem_bits(uint32_t problems);
 int batch_code_bits(uint32_t problems, int dim);
 // Per-point problem ids and per-problem boxes for points laid out by offsets_dev
-// (problems + 1 entries), then composite codes (p << code_bits) | Morton.
+// (problems + 1 entries), then composite codes (p << code_bits) | curve code.
 void batch_problem_ids(const unsigned long long* offsets_dev, uint32_t problems, uint32_t n, uint32_t* pid,
                        cudaStream_t s);
 void batch_boxes(const float4* pts, const uint32_t* pid, uint32_t n, PointStats* prob_stats, uint32_t problems,
@@ -228,8 +239,8 @@ void destroy_scene(Scene* sc);
 // Converts AoS points to float4 (w = id bits) and accumulates statistics.
 void prep_points(const void* points_dev, uint32_t n, int dim, float4* out, PointStats* stats, cudaStream_t s);
 void reset_stats(PointStats* stats, cudaStream_t s);
-// 32-bit Morton codes relative to the box held in `box_stats` (clamped).
-void morton_codes(const float4* pts, uint32_t n, int dim, const PointStats* box_stats, uint32_t* codes,
+// Hilbert codes relative to the box held in `box_stats` (clamped).
+void curve_codes(const float4* pts, uint32_t n, int dim, const PointStats* box_stats, uint32_t* codes,
                   cudaStream_t s);
 
 // ---- queries (query.cu) -----------------------------------------------------
@@ -254,7 +265,7 @@ struct BatchSpec {
   unsigned long long* row_offsets = nullptr; // host out, problems + 1: first row of each problem, then the total
 };
 // A query set prepared once for repeated fixed-radius calls: device records,
-// FP32 points, Morton processing order (in the set's own box) and output
+// FP32 points, curve processing order (in the set's own box) and output
 // order, so a call only computes its bands.
 struct PreparedQueries {
   int dim = 3;
@@ -305,7 +316,7 @@ struct PointGroupScene {
   double max_radius = 0.0;
 };
 PointGroupScene* point_group_create(const RtdlPoint* points, size_t count, const RtdlPointGroupBounds2D* groups,
-                                    size_t group_count, double max_radius, int leaf_size, cudaStream_t s);
+                                    size_t group_count, double max_radius, cudaStream_t s);
 void point_group_destroy(PointGroupScene* pg);
 void point_group_count(PointGroupScene* pg, const void* queries_dev, uint32_t nq, double radius, uint32_t threshold,
                        const CountOutputs& out, cudaStream_t s);
@@ -328,7 +339,7 @@ QueryResult run_nearest_witness(Scene* sc, const void* queries_dev, uint32_t nq,
 // The plain per-call form: builds the scene of the search records and answers
 // the query records (device, or host when query_host is set: uploaded inside).
 // fixed_radius_neighbors / bounded_knn_rows with k_max <= 64 prepare the query
-// set (statistics, own-box Morton order, output order) on `aux` while the scene
+// set (statistics, own-box curve order, output order) on `aux` while the scene
 // builds on `s`; the coordinates of both sets are checked at the query's first
 // read-back.  *scene_out and *query_owned (an uploaded copy) are the caller's to
 // release on `s` once the rows are used.
@@ -371,15 +382,6 @@ QueryResult run_build_and_query_chunked(const BuildQueryInputs& in, int predicat
 // run_build_and_query and the row copies, 1 the heavy queries' refinement
 // beside the emit kernels and the query ranges' preparation one range ahead.
 cudaStream_t aux_stream(int which = 0);
-// Leaf-bucket size of a scene build: the tuning's when set, else 32, the
-// largest a leaf reference holds.  Larger buckets shorten the walks: the
-// fixed-radius collect tests a bucket's points with four loads in flight
-// (0.69 ms at 32 points, 0.73 at 24, 0.76 at 20 on the clustered 1M x 1M
-// sets), and the nearest walks visit a bucket few lanes need a lane per point
-// (k = 16 walk 3.44 ms at 32 or 24 points against 3.65 ms at 8, the 4M x 4M
-// Hausdorff nearest 1.21 against 1.39 ms).
-int scene_leaf_size();
-
 // Ranked-summary aggregates of several (radius, k_max) requests over one
 // prepared query set and one plain scene, captured once as a CUDA graph over
 // buffers allocated at creation (worst-case sizes) and replayed on the graph's

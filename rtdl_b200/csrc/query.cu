@@ -8,47 +8,59 @@
 // (or k) are kept; rows are grouped by query_id in query input order.
 //
 // How the device reaches that exactly:
-//   * Traversal and candidate tests run in FP32 on float4 points.  A candidate
-//     is accepted without further work when its FP32 d2 is below lo2, dropped
-//     above hi2, and re-decided in FP64 in between.  lo2/hi2 bracket r^2 by a
-//     relative band (1e-5) plus, for inputs that are not FP32-exact, an
-//     absolute band of 8 * 2^-24 * max|coordinate| (the FP32 rounding of the
-//     inputs); see k_bands.
-//   * The per-query list keeps the best L candidates in shared memory, one
-//     column per lane ([slot][lane], bank-conflict free), sorted by insertion.
-//     Two keys whose FP32 values are closer than the same band are compared
-//     exactly: FP64 sqrt(d2), then neighbor id, then search input index.
-//   * Once a query provably has more than k_max in-radius neighbors (or its
-//     KNN list is full), subtrees whose box is definitely beyond the current
-//     k-th key are skipped.
-//   * Rows are written by a warp per query in output order, computing the FP64
-//     distance without fused multiply-adds, so distances are bit-identical to
+//   * Traversal and candidate tests run in FP32.  A candidate is accepted
+//     without further work when its FP32 d2 is below lo2, dropped above hi2, and
+//     re-decided in FP64 in between.  lo2/hi2 bracket r^2 by a relative band
+//     (1e-5) plus, for inputs that are not FP32-exact, an absolute band of
+//     8 * 2^-24 * max|coordinate| (the FP32 rounding of the inputs); see
+//     k_bands.
+//   * A warp walks the wide tree for a packet of 32 neighbouring queries and
+//     keeps every query's candidates (collect); a warp per query then sorts them
+//     by FP32 keys, re-decides near ties exactly (FP64 sqrt(d2), then neighbor
+//     id, then search input index) and writes the rows (emit).  The distance is
+//     computed in FP64 without fused multiply-adds, so it is bit-identical to
 //     the reference.
-//   * Queries needing more than 64 rows with more than 64 candidates (large
-//     k_max, or k > 64) go to a generic block-per-query path (gather, bitonic
-//     sort in global memory, emit).
+//   * k nearest (k <= 64) is the same with a radius per query that holds its k
+//     nearest.
+//   * Queries with more candidates than a slab row are collected again at a
+//     smaller radius; what that does not resolve, and k or k_max above 64 with
+//     more than 256 candidates, goes to a generic block-per-query path (gather,
+//     bitonic sort in global memory, emit).
 #include <cstdlib>
 #include <cstring>
 #include <functional>
 #include <mutex>
 
 #include "internal.cuh"
+#include "walk.cuh"
 
 namespace rtdl_b200 {
 
 namespace {
 
-constexpr float kU = 5.9604644775390625e-08f;  // 2^-24, FP32 unit roundoff
 constexpr int kExpandThreads = 256;
 constexpr int kHeavyThreads = 256;
 
 struct DevBands {
   float hi2, lo2, box_hi2;
+  float top, width;  // the bucket test's form of [lo2, hi2], see set_band_top
   float rho, e_abs, floor2;
   double r2;
   unsigned int ids_sorted;
   unsigned int any_inexact;
 };
+
+// The bucket test's form of [lo2, hi2].  It computes d2 - top as one fma chain
+// and looks at the sign, so top lies above hi2 and top - width below lo2 by
+// more than the chain's rounding near the boundary (a few units of hi2; eight
+// are added on either side): a point with a positive difference is outside,
+// one with a difference below -width inside, and FP64 decides the rest.
+__device__ __forceinline__ void set_band_top(DevBands& b) {
+  const double u = 5.9604644775390625e-08;  // 2^-24
+  const double lo = fminf(b.lo2, FLT_MAX), hi = fminf(b.hi2, FLT_MAX);
+  b.top = fminf(__double2float_ru(hi * (1.0 + 8.0 * u)), FLT_MAX);
+  b.width = __double2float_ru((double)b.top - lo * (1.0 - 8.0 * u));
+}
 
 // Band constants from the statistics of both point sets.  Error model (FP32
 // d2 from FP32-rounded coordinates vs the exact distance d):
@@ -83,6 +95,7 @@ __device__ DevBands make_bands(const PointStats* scene, const PointStats* querie
     b.box_hi2 = INFINITY;
     b.r2 = INFINITY;
   }
+  set_band_top(b);
   return b;
 }
 
@@ -166,445 +179,34 @@ __device__ __noinline__ bool exact_before(double ex, double ey, double ez, const
   return __ldg(&perm[ia]) < __ldg(&perm[ib]);
 }
 
-// True when candidate a orders strictly before candidate b.  FP32 keys decide
-// whenever they are further apart than the error band; otherwise FP64 does.
-__device__ __forceinline__ bool before(const Ctx& c, float ka, uint32_t ia, float kb, uint32_t ib) {
-  const float d = kb - ka;
-  const float t = key_tol(c, fmaxf(ka, kb));
-  if (d > t) return true;
-  if (-d > t) return false;
-  return exact_before(c.ex, c.ey, c.ez, c.pts, c.pts64, c.perm, c.scene_inexact, ia, ib);
-}
-
-// Every point in a box whose FP32 key lower bound is kbox orders after the
-// candidate with key klast.
-__device__ __forceinline__ bool box_beyond(const Ctx& c, float kbox, float klast) {
-  const float k = kbox * (1.f - 8.f * kU);
-  return (k - klast) > key_tol(c, k);
-}
-
-__device__ __forceinline__ float box_d2(float qx, float qy, float qz, const float4& lo, const float4& hi) {
-  const float dx = fmaxf(fmaxf(lo.x - qx, qx - hi.x), 0.f);
-  const float dy = fmaxf(fmaxf(lo.y - qy, qy - hi.y), 0.f);
-  const float dz = fmaxf(fmaxf(lo.z - qz, qz - hi.z), 0.f);
-  return fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-}
-
-struct Pass1Params {
-  SceneView S;
-  const float4* qpts;
-  const double* qraw;
-  int qstride;
-  const uint32_t* qorder;
-  uint32_t nq;
-  uint32_t kmax;
-  int L;
-  const DevBands* bands;
-  uint32_t* temp;
-  uint32_t* counts;
-  uint8_t* flags;
-  uint32_t* heavy_list;
-  uint32_t* heavy_m;
-  unsigned int* heavy_count;
-  unsigned int* error;
-  unsigned long long* stats;  // kStatCount counters, only with STATS
-  const uint32_t* qcodes;     // KNN: query Morton codes in processing order (seeds the list)
-  const uint32_t* scodes;     // KNN: the scene's sorted Morton codes
-};
-
 // Traversal counters gathered by the STATS instantiation (diagnostics).
 enum Stat { kStatNodes, kStatLeafPoints, kStatInRadius, kStatInserts, kStatShifts, kStatBand, kStatMaxLeafPoints,
             kStatGenericQueries, kStatLargeQueries, kStatLeafPairs, kStatEmitFixups, kStatRefined, kStatCount };
 
-// One thread per query, queries in Morton order so a warp walks neighbouring
-// subtrees.  KNN == false: radius-limited (fixed_radius_neighbors and
-// bounded_knn_rows); KNN == true: k nearest.  Every lane keeps its own list.
-// WALK: kWalkLane -- each lane walks the rope-linked records alone;
-// kWalkRope -- the warp walks them together in pre-order, entering a node
-// when any lane's current k-th bound reaches it; kWalkNear -- the warp walks
-// nearer child first with a stack (fewer nodes for longer lists, a dearer
-// step: 14% faster than kWalkRope at k = 16, 10% slower at k = 1 on the
-// benchmark's clustered 1M x 1M sets).  In the packet forms each lane tests a
-// leaf only when its own bound reaches it, so lists and rows are the
-// per-lane walk's.
-constexpr int kWalkLane = 0, kWalkRope = 1, kWalkNear = 2;
-// Half-width of the Morton window that seeds a nearest list of length L
-// before its walk (2w points, inserted by every lane at once): a wider window
-// tightens the k-th bound the divergent walk starts from, at the cost of the
-// window's own tests.  Measured on the clustered 1M x 1M sets (packets in
-// Morton order): k = 16 walk 3.69 / 3.69 / 3.71 / 3.84 ms at w = 2L / 3L /
-// 4L / 6L; k = 1 0.82 / 0.79 / 0.82 / 0.90 ms at w = 8 / 16 / 32 / 64 (the
-// 4M x 4M uniform 2D Hausdorff nearest: 1.48 / 1.52 / 1.68 / 2.08 ms).
-__host__ __device__ constexpr int seed_half_width(int L) { return L * 2 < 16 ? 16 : L * 2; }
-// Lists at least this long take kWalkNear (k = 4: 1.40 ms pre-order against
-// 1.46 ms nearer first).
-constexpr int kNearFirstMinList = 5;
-// A leaf at most this many lanes need is visited point-major (visit_leaf_pm).
-// With 24-point buckets: k = 1 walk 0.56 ms with 8 (0.60 with 4), the 4M x 4M
-// Hausdorff nearest 1.21 ms (1.23), k = 16 3.44 ms with 4 (3.48 with 2); with
-// 8-point buckets lane-major visits of every leaf took 0.79, 1.52 and 3.69 ms.
-__host__ __device__ constexpr int point_major_max(int L) { return L <= 4 ? 8 : 4; }
-// Held to 64 registers (32 resident warps at 128 threads per block): the
-// k = 16 walk ran 2.8% faster than at its natural 72 (28 warps); at 48
-// registers the spills cost more than the occupancy gained.
-template <bool KNN, bool STATS, int WALK = kWalkLane>
-__global__ void __launch_bounds__(256, 4) k_pass1(Pass1Params P) {
-  extern __shared__ uint32_t smem[];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int L = P.L;
-  uint32_t* lkey = smem + (size_t)warp * 64 * L;
-  uint32_t* lidx = lkey + 32 * L;
-  const uint32_t t0 = blockIdx.x * blockDim.x + threadIdx.x;
-  constexpr bool PACKET = WALK != kWalkLane;
-  if (PACKET ? !__any_sync(0xffffffffu, t0 < P.nq) : t0 >= P.nq) return;
-  const bool active = t0 < P.nq;  // PACKET: lanes past the end take part in the warp's walk only
-  const uint32_t t = active ? t0 : P.nq - 1;
-  const uint32_t qin = P.qorder[t];
-  const float4 q = P.qpts[qin];
-  const DevBands B = *P.bands;
-  const SceneView& S = P.S;
-  Ctx c;
-  c.qx = q.x;
-  c.qy = q.y;
-  c.qz = q.z;
-  {
-    const double* r = P.qraw + (size_t)qin * P.qstride;
-    c.ex = r[1];
-    c.ey = r[2];
-    c.ez = P.qstride == 4 ? r[3] : 0.0;
-  }
-  c.pts = S.pts;
-  c.pts64 = S.pts64;
-  c.perm = S.perm;
-  c.scene_inexact = *S.inexact;
-  c.rho = B.rho;
-  c.e_abs = B.e_abs;
-  c.floor2 = B.floor2;
-
-  const uint32_t kmax = P.kmax;
-  uint32_t count = 0;
-  int len = 0;
-  bool heavy = false;
-  bool prune = false;  // the list is complete: only candidates ordering before its last entry matter
-  float klast = INFINITY;
-  uint32_t ilast = kNone;
-  unsigned long long st_nodes = 0, st_points = 0, st_inserts = 0, st_shifts = 0, st_band = 0;
-  int win_lo = 0, win_hi = 0;  // seeded window (already in the list)
-
-  auto insert = [&](float key, uint32_t idx) {
-    int pos;
-    if (len < L) {
-      pos = len++;
-    } else {
-      pos = L - 1;
-    }
-    while (pos > 0) {
-      const float pk = __uint_as_float(lkey[(pos - 1) * 32 + lane]);
-      const uint32_t pi = lidx[(pos - 1) * 32 + lane];
-      if (!before(c, key, idx, pk, pi)) break;
-      lkey[pos * 32 + lane] = __float_as_uint(pk);
-      lidx[pos * 32 + lane] = pi;
-      --pos;
-      if (STATS) ++st_shifts;
-    }
-    if (STATS) ++st_inserts;
-    lkey[pos * 32 + lane] = __float_as_uint(key);
-    lidx[pos * 32 + lane] = idx;
-    if (len == L) {
-      klast = __uint_as_float(lkey[(L - 1) * 32 + lane]);
-      ilast = lidx[(L - 1) * 32 + lane];
-    }
-  };
-
-  auto visit_leaf = [&](int first, int cnt) {
-    if (STATS) st_points += cnt;
-    for (int i = first; i < first + cnt; ++i) {
-      if (KNN && i >= win_lo && i < win_hi) continue;
-      const float4 p = __ldg(&S.pts[i]);
-      const float dx = p.x - c.qx, dy = p.y - c.qy, dz = p.z - c.qz;
-      const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-      if (!KNN) {
-        if (d2 > B.hi2) continue;
-        if (prune && !before(c, d2, (uint32_t)i, klast, ilast)) continue;
-        if (d2 >= B.lo2) {
-          if (STATS) ++st_band;
-          if (exact_d2(c, (uint32_t)i) > B.r2) continue;
-        }
-        ++count;
-        if (heavy) continue;
-        if (len < L) {
-          insert(d2, (uint32_t)i);
-        } else if ((uint32_t)L == kmax) {
-          // more than k_max neighbors: keep the k_max nearest, then prune
-          prune = true;
-          if (before(c, d2, (uint32_t)i, klast, ilast)) insert(d2, (uint32_t)i);
-        } else {
-          heavy = true;  // needs more rows than the shared-memory list holds
-        }
-      } else {
-        if (len == L && !before(c, d2, (uint32_t)i, klast, ilast)) continue;
-        insert(d2, (uint32_t)i);
-        ++count;
-      }
-    }
-  };
-
-  // Point-major visit of a leaf few lanes need (nearest lists): lane j holds
-  // point first + j and the needing lanes are taken in turn; a point passes
-  // when it may order before that lane's current last entry (the FP32 side
-  // of `before`, a superset of what it accepts), and the owning lane then
-  // inserts the passing points one by one, exactly as visit_leaf would.
-  auto visit_leaf_pm = [&](int first, int cnt, unsigned int needers) {
-    const bool has = lane < cnt;
-    const uint32_t pi = (uint32_t)(first + (has ? lane : 0));
-    const float4 p = __ldg(&S.pts[pi]);
-    while (needers) {
-      const int q = __ffs(needers) - 1;
-      needers &= needers - 1u;
-      const float qx = __shfl_sync(0xffffffffu, c.qx, q), qy = __shfl_sync(0xffffffffu, c.qy, q),
-                  qz = __shfl_sync(0xffffffffu, c.qz, q);
-      const float kl = __shfl_sync(0xffffffffu, klast, q);
-      const bool full_list = __shfl_sync(0xffffffffu, (int)(len == L), q) != 0;
-      const int wlo = __shfl_sync(0xffffffffu, win_lo, q), whi = __shfl_sync(0xffffffffu, win_hi, q);
-      const float dx = p.x - qx, dy = p.y - qy, dz = p.z - qz;
-      const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-      bool pass = has && !((int)pi >= wlo && (int)pi < whi);
-      if (full_list) pass = pass && d2 - kl <= key_tol(c, fmaxf(d2, kl));
-      unsigned int passing = __ballot_sync(0xffffffffu, pass);
-      if (STATS && lane == q) st_points += cnt;
-      while (passing) {
-        const int j = __ffs(passing) - 1;
-        passing &= passing - 1u;
-        const float key = __shfl_sync(0xffffffffu, d2, j);
-        if (lane == q) {
-          const uint32_t idx = (uint32_t)(first + j);
-          if (!(len == L && !before(c, key, idx, klast, ilast))) {
-            insert(key, idx);
-            ++count;
-          }
-        }
-      }
-    }
-  };
-
-  auto box_ok = [&](float kb) -> bool {
-    if (!KNN && kb > B.box_hi2) return false;
-    const bool full = KNN ? (len == L) : prune;
-    if (full && box_beyond(c, kb, klast)) return false;
-    return true;
-  };
-
-  // KNN: seed the list with the scene points around the query's Morton code
-  // (a window in the sorted order), so the walk starts with a tight k-th
-  // bound; the walk skips the window's points.
-  if (KNN && S.n > 0 && P.scodes != nullptr) {
-    const uint32_t code = P.qcodes[t];
-    uint32_t lo = 0, hi = S.n;
-    while (lo < hi) {
-      const uint32_t mid = (lo + hi) >> 1;
-      if (__ldg(&P.scodes[mid]) < code) lo = mid + 1;
-      else hi = mid;
-    }
-    const int w = seed_half_width(L);
-    int a = (int)lo - w;
-    if (a < 0) a = 0;
-    int b = a + 2 * w;
-    if (b > (int)S.n) {
-      b = (int)S.n;
-      a = b - 2 * w < 0 ? 0 : b - 2 * w;
-    }
-    if (L >= kNearFirstMinList) {
-      // outward from the query's position (lo, lo - 1, lo + 1, ...): points
-      // nearer in the curve tend to be nearer in space, so more inserts land
-      // at the list's end instead of shifting it (k = 16: 178 shifts per
-      // query instead of 249); the list is the same
-      int right = (int)lo < a ? a : (int)lo < b ? (int)lo : b - 1, left = right - 1;
-      for (int j = a; j < b; ++j) {
-        const bool take_right = right < b && (((j - a) & 1) == 0 || left < a);
-        visit_leaf(take_right ? right : left, 1);
-        if (take_right) ++right;
-        else --left;
-      }
-    } else {
-      visit_leaf(a, b - a);
-    }
-    win_lo = a;
-    win_hi = b;
-  }
-  // depth-first walk over the pre-order records
-  int cur = S.n > 0 ? 0 : kRopeEnd;
-  if constexpr (WALK == kWalkRope) {
-    while (cur != kRopeEnd) {
-      const float4 a = __ldg(&S.nodes[2 * cur]), b = __ldg(&S.nodes[2 * cur + 1]);
-      if (STATS) ++st_nodes;
-      const int hit = __float_as_int(a.w);
-      const bool need = active && box_ok(box_d2(c.qx, c.qy, c.qz, a, b));
-      if (__ballot_sync(0xffffffffu, need)) {
-        if (hit >= 0) {
-          ++cur;  // internal node: its left child is the next record
-          continue;
-        }
-        const unsigned int nm = __ballot_sync(0xffffffffu, need);
-        if (KNN && __popc(nm) <= point_major_max(L)) visit_leaf_pm(leaf_first(hit), leaf_count(hit), nm);
-        else if (need) visit_leaf(leaf_first(hit), leaf_count(hit));
-      }
-      cur = __float_as_int(b.w);
-    }
-    if (!active) return;
-  } else if constexpr (WALK == kWalkNear) {
-    // Nearer child first.  A node's two children are tested together, by the
-    // lanes that needed the node; the packet enters the child that most of
-    // those lanes find nearer and keeps the other, if any lane needs it, on a
-    // warp-uniform stack in shared memory.  A kept child is tested again when
-    // it comes off the stack, against bounds that have shrunk meanwhile (a
-    // child's box lies inside its parent's, so a lane that did not need the
-    // parent never needs the child).  The right child of an internal record
-    // is its left child's rope; the depth, and so the stack, stays below
-    // kStackDepth (30 code bits plus 32 index bits).
-    __shared__ int stack_all[256 / 32][kStackDepth];
-    int* stack = stack_all[warp];
-    int sp = 0;
-    float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
-    bool need = false;
-    if (cur != kRopeEnd) {
-      a = __ldg(&S.nodes[0]);
-      b = __ldg(&S.nodes[1]);
-      if (STATS) ++st_nodes;
-      need = active && box_ok(box_d2(c.qx, c.qy, c.qz, a, b));
-      if (!__any_sync(0xffffffffu, need)) cur = kRopeEnd;
-    }
-    // at the loop top (a, b) is cur's record, `need` this lane's test of it,
-    // and some lane needs it
-    while (cur != kRopeEnd) {
-      const int hit = __float_as_int(a.w);
-      bool descended = false;
-      if (hit < 0) {
-        const unsigned int nm = __ballot_sync(0xffffffffu, need);
-        if (KNN && __popc(nm) <= point_major_max(L)) visit_leaf_pm(leaf_first(hit), leaf_count(hit), nm);
-        else if (need) visit_leaf(leaf_first(hit), leaf_count(hit));
-      } else {
-        const int left = cur + 1;
-        const float4 la = __ldg(&S.nodes[2 * left]), lb = __ldg(&S.nodes[2 * left + 1]);
-        const int right = __float_as_int(lb.w);
-        const float4 ra = __ldg(&S.nodes[2 * right]), rb = __ldg(&S.nodes[2 * right + 1]);
-        if (STATS) st_nodes += 2;
-        const float dl = box_d2(c.qx, c.qy, c.qz, la, lb), dr = box_d2(c.qx, c.qy, c.qz, ra, rb);
-        const bool nl = need && box_ok(dl), nr = need && box_ok(dr);
-        const unsigned int bl = __ballot_sync(0xffffffffu, nl), br = __ballot_sync(0xffffffffu, nr);
-        if (bl | br) {
-          bool right_first = br != 0;
-          if (bl && br) {
-            const unsigned int vote_r = __ballot_sync(0xffffffffu, nr && (!nl || dr < dl));
-            right_first = 2 * __popc(vote_r) > __popc(bl | br);
-            if (sp == kStackDepth) {  // cannot happen for a valid tree; the call reports it
-              if (lane == 0) atomicOr(P.error, 8u);
-              break;
-            }
-            if (lane == 0) stack[sp] = right_first ? left : right;
-            ++sp;
-          }
-          cur = right_first ? right : left;
-          a = right_first ? ra : la;
-          b = right_first ? rb : lb;
-          need = right_first ? nr : nl;
-          descended = true;
-        }
-      }
-      if (!descended) {  // the next kept node some lane still needs
-        cur = kRopeEnd;
-        while (sp > 0) {
-          __syncwarp();
-          const int k = stack[--sp];
-          __syncwarp();
-          a = __ldg(&S.nodes[2 * k]);
-          b = __ldg(&S.nodes[2 * k + 1]);
-          if (STATS) ++st_nodes;
-          need = active && box_ok(box_d2(c.qx, c.qy, c.qz, a, b));
-          if (__any_sync(0xffffffffu, need)) {
-            cur = k;
-            break;
-          }
-        }
-      }
-    }
-    if (!active) return;
-  } else {
-    while (cur != kRopeEnd) {
-      const float4 a = __ldg(&S.nodes[2 * cur]), b = __ldg(&S.nodes[2 * cur + 1]);
-      if (STATS) ++st_nodes;
-      const int hit = __float_as_int(a.w);
-      if (box_ok(box_d2(c.qx, c.qy, c.qz, a, b))) {
-        if (hit >= 0) {
-          ++cur;  // internal node: its left child is the next record
-          continue;
-        }
-        visit_leaf(leaf_first(hit), leaf_count(hit));
-      }
-      cur = __float_as_int(b.w);
-    }
-  }
-
-  if (STATS) {
-    atomicAdd(&P.stats[kStatNodes], st_nodes);
-    atomicAdd(&P.stats[kStatLeafPoints], st_points);
-    atomicAdd(&P.stats[kStatInRadius], (unsigned long long)count);
-    atomicAdd(&P.stats[kStatInserts], st_inserts);
-    atomicAdd(&P.stats[kStatShifts], st_shifts);
-    atomicAdd(&P.stats[kStatBand], st_band);
-    atomicMax(&P.stats[kStatMaxLeafPoints], st_points);
-  }
-  uint8_t fl = 0;
-  if (!KNN) {
-    P.counts[qin] = count < kmax ? count : kmax;
-    if (count > kmax) fl |= 1;
-  } else {
-    P.counts[qin] = (uint32_t)len;
-  }
-  if (heavy) {
-    fl |= 2;
-    const unsigned int h = atomicAdd(P.heavy_count, 1u);
-    P.heavy_list[h] = qin;
-    P.heavy_m[h] = count;
-    P.temp[(size_t)qin * L] = h;
-  } else {
-    uint32_t* dst = P.temp + (size_t)qin * L;
-    for (int j = 0; j < len; ++j) dst[j] = lidx[j * 32 + lane];
-  }
-  P.flags[qin] = fl;
-}
-
 // ---- fixed-radius collect pass ----------------------------------------------
-// One thread per query in Morton order.  In-radius candidates are appended
-// unsorted to the query's slab (capacity kSlab) as one 8-byte entry each; the
-// exact in-radius count is kept, so the overflow flag and the row offsets are
-// exact without any per-query list.
+// Queries in curve order, a packet of 32 per warp.  A query's in-radius points
+// go to its row of the candidate slab; the exact in-radius count is kept, so
+// the overflow flag and the row offsets are exact without any per-query list.
 constexpr int kSlab = 256;  // candidates kept per query
 constexpr unsigned int kStrideBlocks = kSmCount * 8;  // grid of the kernels that stride over device counts
 
-// Candidate slab: query-major, kSlab entries for the query at processing rank
-// t starting at t * kSlab.  An entry is (FP32 sort key bits << 32) | sorted
-// point index, so a lane appends one candidate with one 8-byte store and a
-// warp reads a query's candidates with contiguous loads.
+// Candidate slab: kSlab sorted point indices per processing rank, so a warp
+// reads a query's candidates with contiguous loads.
 __host__ __device__ __forceinline__ size_t slab_base(uint32_t t) { return (size_t)t * kSlab; }
-
-__device__ __forceinline__ unsigned long long slab_entry(float key, uint32_t i) {
-  return ((unsigned long long)__float_as_uint(key) << 32) | i;
-}
 
 // Per-query record written by the collect pass at the query's processing rank
 // and read by the emit kernels, so they find the query's exact coordinates,
 // id and candidate count with one load.
-struct QueryInfo {
+struct __align__(16) QueryInfo {
   double ex, ey, ez;  // exact query coordinates (z = 0 in 2D)
   uint32_t qid;
-  uint32_t meta;      // candidate count (<= kSlab), the kQuery* bits and the query's kmax (<= 64)
+  uint32_t meta;      // candidates (9 bits), the kQuery* bits, kmax (9 bits); 0: nothing to emit
 };
-constexpr uint32_t kQueryCountMask = 0xFFFFu;
-constexpr uint32_t kQueryGeneric = 1u << 16;   // more than kSlab candidates: generic path
-constexpr uint32_t kQueryBig = 1u << 17;       // 65..kSlab candidates, or refined: k_emit_list
-constexpr uint32_t kQueryOverflow = 1u << 18;  // more in-radius points than kmax
-constexpr int kQueryKmaxShift = 19;            // bits 19..25: kmax
-__device__ __forceinline__ int query_kmax(uint32_t meta) { return (int)((meta >> kQueryKmaxShift) & 127u); }
+constexpr uint32_t kQueryCountMask = 511u;
+constexpr uint32_t kQueryGeneric = 1u << 18;  // candidates not kept: generic path
+constexpr uint32_t kQueryBig = 1u << 19;      // 65..kSlab candidates: k_emit_list
+constexpr int kQueryKmaxShift = 20;           // kmax, at most kSlab
+__device__ __forceinline__ int query_kmax(uint32_t meta) { return (int)((meta >> kQueryKmaxShift) & 511u); }
 
 struct CollectParams {
   SceneView S;
@@ -613,329 +215,30 @@ struct CollectParams {
   int qstride;
   const uint32_t* qorder;    // processing rank -> query input index (kNone: padding of a problem batch)
   uint32_t nq;               // processing ranks (a batch pads every problem to whole warps)
+  uint32_t width;            // queries per packet, at most 32 (see launch_collect)
   uint32_t kmax;
+  double radius;             // of a single problem
   const DevBands* bands;     // one per problem (one in all for a single problem)
   const uint32_t* warp_prob; // problem batch: the problem of each warp of processing ranks (nullptr: single)
   const uint32_t* prob_kmax; // problem batch: kmax per problem
-  unsigned long long* slab;  // kSlab entries per query, see slab_base()
-  uint32_t* counts;          // min(count, kmax), query input order
+  const double* prob_radius; // problem batch: radius per problem
+  const double* rank_radius; // KNN: the radius of each processing rank (holds its kmax nearest); else nullptr
+  uint32_t* slab;            // slab_base(nq) entries
+  uint32_t* counts;          // min(in-radius count, kmax), query input order
   QueryInfo* qinfo;          // by processing rank
-  uint8_t* flags;            // bit0: count > kmax, bit1: count > kSlab (generic path), bit2: count > 64
-  uint32_t* heavy_list;
-  uint32_t* heavy_m;
-  uint32_t* heavy_t;         // processing rank of each heavy_list entry (optional)
-  uint32_t* mid_list;        // processing ranks of the queries with 65..128 candidates (or refined, <= 128)
+  uint8_t* flags;            // bit0: count > kmax, bit1: generic path (query input order)
+  uint32_t* heavy_list;      // generic path: query input index,
+  uint32_t* heavy_m;         // in-radius count at heavy_rad,
+  double* heavy_rad;         // a radius that holds the query's kmax nearest,
+  uint32_t* heavy_t;         // and processing rank
+  uint32_t* mid_list;        // processing ranks of the queries with 65..128 candidates
   uint32_t* big_list;        // processing ranks of the queries with 129..kSlab candidates
+  uint32_t* single_list;     // processing ranks the packets leave to k_collect_single
   unsigned int* small;       // [0] generic-path query count, [1] error bits, [2] mid_list length,
-                             // [3] big_list length, [4] emit fixup queue length
+                             // [3] big_list length, [4] emit fixup queue length, [6] single_list length
   uint8_t* overflow_out;     // optional: 1 per query (input order) when count > kmax
   unsigned long long* stats;
 };
-
-// Per-query state of the collect pass and its accept / finish steps, shared by
-// the per-lane and the per-warp (packet) traversals.
-struct CollectLane {
-  uint32_t t, qin;
-  float4 q;
-  uint32_t count;
-  unsigned long long* out;  // this query's slab entries
-  unsigned long long st_nodes, st_points, st_band, st_pairs;
-};
-
-// The query's exact coordinates, read when needed (the band's FP64 test and
-// the query record) rather than held in registers through the walk.
-__device__ __forceinline__ void query_exact(const CollectParams& P, uint32_t qin, double& ex, double& ey,
-                                            double& ez) {
-  const double* r = P.qraw + (size_t)qin * P.qstride;
-  ex = r[1];
-  ey = r[2];
-  ez = P.qstride == 4 ? r[3] : 0.0;
-}
-
-// Tests sorted point i against the lane's query and appends it when it is in
-// radius: FP32 decides outside the band, FP64 inside.  The stored key is the
-// FP32 d2 for FP32-exact inputs, else the exact FP64 d2 rounded to FP32.
-template <bool STATS>
-__device__ __forceinline__ void collect_point(const CollectParams& P, const DevBands& B, int scene_inexact,
-                                              CollectLane& L, uint32_t i, const float4& p) {
-  const float dx = p.x - L.q.x, dy = p.y - L.q.y, dz = p.z - L.q.z;
-  float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-  if (d2 > B.hi2) return;
-  if (d2 >= B.lo2 || B.any_inexact) {
-    if (STATS && d2 >= B.lo2) ++L.st_band;
-    double ex, ey, ez;
-    query_exact(P, L.qin, ex, ey, ez);
-    const double e2 = exact_d2_at(ex, ey, ez, P.S.pts, P.S.pts64, scene_inexact, i);
-    if (d2 >= B.lo2 && e2 > B.r2) return;
-    if (B.any_inexact) d2 = __double2float_rn(e2);
-  }
-  if (L.count < (uint32_t)kSlab) L.out[L.count] = slab_entry(d2, i);
-  ++L.count;
-}
-
-template <bool STATS>
-__device__ __forceinline__ void collect_finish(const CollectParams& P, const CollectLane& L, uint32_t kmax) {
-  if (STATS) {
-    atomicAdd(&P.stats[kStatNodes], L.st_nodes);
-    atomicAdd(&P.stats[kStatLeafPoints], L.st_points);
-    atomicAdd(&P.stats[kStatInRadius], (unsigned long long)L.count);
-    atomicAdd(&P.stats[kStatBand], L.st_band);
-    atomicAdd(&P.stats[kStatLeafPairs], L.st_pairs);
-    atomicMax(&P.stats[kStatMaxLeafPoints], (unsigned long long)L.count);
-  }
-  const uint32_t count = L.count;
-  P.counts[L.qin] = count < kmax ? count : kmax;
-  uint8_t fl = count > kmax ? 1 : 0;
-  if (count > (uint32_t)kSlab) {
-    fl |= 2;
-    const unsigned int h = atomicAdd(&P.small[0], 1u);
-    P.heavy_list[h] = L.qin;
-    P.heavy_m[h] = count;
-    if (P.heavy_t) P.heavy_t[h] = L.t;
-  } else if (count > 128u) {
-    fl |= 4;
-    P.big_list[atomicAdd(&P.small[3], 1u)] = L.t;
-  } else if (count > 64u) {
-    fl |= 4;
-    P.mid_list[atomicAdd(&P.small[2], 1u)] = L.t;
-  }
-  QueryInfo qi;
-  query_exact(P, L.qin, qi.ex, qi.ey, qi.ez);
-  qi.qid = __float_as_uint(L.q.w);
-  qi.meta = (count < (uint32_t)kSlab ? count : (uint32_t)kSlab) | ((fl & 1) ? kQueryOverflow : 0u) |
-            ((fl & 2) ? kQueryGeneric : 0u) | ((fl & 4) ? kQueryBig : 0u) | (kmax << kQueryKmaxShift);
-  P.qinfo[L.t] = qi;
-  P.flags[L.qin] = fl;
-  if (P.overflow_out) P.overflow_out[L.qin] = fl & 1;
-}
-
-__device__ __forceinline__ void collect_init(const CollectParams& P, uint32_t t, CollectLane& L) {
-  L.t = t;
-  L.qin = P.qorder[t];
-  L.q = P.qpts[L.qin];
-  L.count = 0;
-  L.out = P.slab + slab_base(t);
-  L.st_nodes = L.st_points = L.st_band = L.st_pairs = 0;
-}
-
-// Tests the points of leaf bucket [first, first + cnt) against the lane's
-// query.  `test` false: the lane only takes part in the (warp-uniform) loads.
-// Four point loads are issued before their tests (more loads in flight per
-// warp; measured 6% faster at the 32-register budget than one at a time).
-template <bool STATS>
-__device__ __forceinline__ void collect_leaf(const CollectParams& P, const DevBands& B, int scene_inexact,
-                                             CollectLane& L, int first, int cnt, bool test) {
-  constexpr int kGroup = 4;
-  int i = first;
-  const int end = first + cnt;
-  for (; i + kGroup <= end; i += kGroup) {
-    float4 p[kGroup];
-#pragma unroll
-    for (int u = 0; u < kGroup; ++u) p[u] = __ldg(&P.S.pts[i + u]);
-    if (test) {
-#pragma unroll
-      for (int u = 0; u < kGroup; ++u) collect_point<STATS>(P, B, scene_inexact, L, (uint32_t)(i + u), p[u]);
-    }
-  }
-  for (; i < end; ++i) {
-    const float4 p = __ldg(&P.S.pts[i]);
-    if (test) collect_point<STATS>(P, B, scene_inexact, L, (uint32_t)i, p);
-  }
-}
-
-// Point-major form of collect_leaf for a packet: lane j holds point
-// first + j of the bucket (cnt <= 32), and the warp takes the queries whose
-// sphere reaches the bucket (`active`, one bit per lane) one at a time: the
-// query's coordinates are broadcast, every lane tests its point, and the hits
-// go to consecutive entries of that query's slab row (one coalesced store).
-// The loop runs once per reaching query instead of once per point, and lanes
-// whose query misses the bucket cost nothing.  The decisions are
-// collect_point's (FP32 outside the band, FP64 inside); only the order of a
-// query's slab entries differs, which the emit's sort does not see.
-template <bool STATS>
-__device__ __forceinline__ void collect_leaf_pm(const CollectParams& P, const DevBands& B, int scene_inexact,
-                                                CollectLane& L, uint32_t t0, int lane, int first, int cnt,
-                                                unsigned int active) {
-  const bool has = lane < cnt;
-  const uint32_t i = (uint32_t)(first + (has ? lane : 0));
-  const float4 p = __ldg(&P.S.pts[i]);
-  const unsigned int lt_mask = (1u << lane) - 1u;
-  if (STATS) {
-    L.st_points += cnt;
-    if ((active >> lane) & 1u) L.st_pairs += cnt;
-  }
-  while (active) {
-    const int q = __ffs(active) - 1;
-    active &= active - 1u;
-    const float qx = __shfl_sync(0xffffffffu, L.q.x, q);
-    const float qy = __shfl_sync(0xffffffffu, L.q.y, q);
-    const float qz = __shfl_sync(0xffffffffu, L.q.z, q);
-    const float dx = p.x - qx, dy = p.y - qy, dz = p.z - qz;
-    float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-    bool hit = has && d2 <= B.hi2;
-    const bool check = hit && (d2 >= B.lo2 || B.any_inexact);
-    if (__any_sync(0xffffffffu, check)) {
-      const uint32_t qin = __shfl_sync(0xffffffffu, L.qin, q);
-      if (check) {
-        double ex, ey, ez;
-        query_exact(P, qin, ex, ey, ez);
-        if (STATS && d2 >= B.lo2) ++L.st_band;
-        const double e2 = exact_d2_at(ex, ey, ez, P.S.pts, P.S.pts64, scene_inexact, i);
-        if (d2 >= B.lo2 && e2 > B.r2)
-          hit = false;
-        else if (B.any_inexact)
-          d2 = __double2float_rn(e2);
-      }
-    }
-    const unsigned int hits = __ballot_sync(0xffffffffu, hit);
-    if (hits) {
-      const uint32_t c0 = __shfl_sync(0xffffffffu, L.count, q);
-      if (hit) {
-        const uint32_t pos = c0 + (uint32_t)__popc(hits & lt_mask);
-        if (pos < (uint32_t)kSlab) P.slab[slab_base(t0 + (uint32_t)q) + pos] = slab_entry(d2, i);
-      }
-      if (lane == q) L.count = c0 + (uint32_t)__popc(hits);
-    }
-  }
-}
-
-// One thread per query, queries in Morton order.  Stackless walk over the
-// rope-linked nodes, while-while style: a lane advances through internal
-// nodes until it stands on an overlapping leaf bucket, then the lanes test
-// their buckets together.
-template <bool STATS>
-__global__ void __launch_bounds__(256) k_collect(CollectParams P) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= P.nq) return;
-  const DevBands B = *P.bands;
-  const SceneView& S = P.S;
-  const int scene_inexact = *S.inexact;
-  CollectLane L;
-  collect_init(P, t, L);
-  int cur = S.n > 0 ? 0 : kRopeEnd;
-  while (cur != kRopeEnd) {
-    int first = 0, cnt = 0;
-    while (cur != kRopeEnd) {
-      const float4 a = __ldg(&S.nodes[2 * cur]), b = __ldg(&S.nodes[2 * cur + 1]);
-      if (STATS) ++L.st_nodes;
-      const int hit = __float_as_int(a.w);
-      const bool over = box_d2(L.q.x, L.q.y, L.q.z, a, b) <= B.box_hi2;
-      if (over && hit >= 0) {
-        ++cur;  // internal node: its left child is the next record
-        continue;
-      }
-      cur = __float_as_int(b.w);
-      if (over) {
-        first = leaf_first(hit);
-        cnt = leaf_count(hit);
-        break;
-      }
-    }
-    if (STATS) {
-      L.st_points += cnt;
-      L.st_pairs += cnt;
-    }
-    collect_leaf<STATS>(P, B, scene_inexact, L, first, cnt, true);
-  }
-  collect_finish<STATS>(P, L, P.kmax);
-}
-
-// One warp per 32 Morton-consecutive queries (packet traversal): the warp
-// walks the rope-linked nodes once, entering a node when any lane's query
-// sphere overlaps it.  Node and point loads are warp-uniform (one request
-// each) and the control flow never diverges; each lane tests leaf points
-// against its own query.  CUBE: internal nodes are tested against the
-// query's bounding cube (six compares against bounds rounded outward; it
-// never rejects a node the sphere test accepts), leaf buckets against the
-// sphere.  BATCH: several problems (a problem batch, or several requests on
-// one scene): each warp walks its problem's subtree with its problem's bands
-// and kmax; kept out of the single-problem instantiation, whose registers it
-// would cost.
-// LEAF: how a reached leaf bucket is tested -- 0 lane-major (collect_leaf:
-// every lane loops over the bucket's points), 1 point-major (collect_leaf_pm:
-// the warp loops over the reaching queries), 2 either, chosen per bucket
-// (warp-uniform): point-major when at most kHybridRatio reaching queries per
-// point, i.e. when few of the packet's spheres reach the bucket.
-constexpr int kLeafLaneMajor = 0, kLeafPointMajor = 1, kLeafHybrid = 2;
-// The packet walk for processing ranks t & ~31 .. (t & ~31) + 31 (lane t & 31).
-template <bool STATS, bool CUBE, bool BATCH, int LEAF>
-__device__ __forceinline__ void collect_packet_body(const CollectParams& P, uint32_t t) {
-  // a problem batch pads every problem to whole warps, so a warp has one problem
-  const uint32_t prob = BATCH ? P.warp_prob[t >> 5] : 0u;
-  const bool valid = t < P.nq && (!BATCH || P.qorder[t] != kNone);
-  if (BATCH && !valid && t < P.nq) P.qinfo[t] = QueryInfo{0.0, 0.0, 0.0, 0u, 0u};  // padding: nothing to emit
-  const DevBands B = P.bands[prob];
-  const SceneView& S = P.S;
-  const int scene_inexact = *S.inexact;
-  CollectLane L;
-  if (valid) {
-    collect_init(P, t, L);
-  } else {
-    L.q = make_float4(INFINITY, INFINITY, INFINITY, 0.f);  // never overlaps
-    L.count = 0;
-    L.out = nullptr;
-    L.st_nodes = L.st_points = L.st_band = L.st_pairs = 0;
-  }
-  float3 clo, chi;  // query cube, CUBE only
-  if (CUBE) {
-    const float h = sqrtf(B.box_hi2) * (1.0f + 4.0f * kU);  // >= the sphere radius
-    clo = make_float3(__fsub_rd(L.q.x, h), __fsub_rd(L.q.y, h), __fsub_rd(L.q.z, h));
-    chi = make_float3(__fadd_ru(L.q.x, h), __fadd_ru(L.q.y, h), __fadd_ru(L.q.z, h));
-  }
-  // the walk covers the problem's subtree: from its root to the root's rope
-  int cur = S.n > 0 ? 0 : kRopeEnd, end = kRopeEnd;
-  if (BATCH) {
-    cur = S.prob_root[prob];
-    if (cur != kRopeEnd) end = __float_as_int(__ldg(&S.nodes[2 * cur + 1]).w);
-  }
-  while (cur != end) {
-    const float4 a = __ldg(&S.nodes[2 * cur]), b = __ldg(&S.nodes[2 * cur + 1]);
-    if (STATS) ++L.st_nodes;
-    const int hit = __float_as_int(a.w);
-    bool over;
-    if (CUBE && hit >= 0)
-      over = valid && a.x <= chi.x && b.x >= clo.x && a.y <= chi.y && b.y >= clo.y && a.z <= chi.z && b.z >= clo.z;
-    else
-      over = valid && box_d2(L.q.x, L.q.y, L.q.z, a, b) <= B.box_hi2;
-    const unsigned int reach = __ballot_sync(0xffffffffu, over);
-    if (reach) {
-      if (hit >= 0) {
-        ++cur;  // internal node: its left child is the next record
-        continue;
-      }
-      const int first = leaf_first(hit), cnt = leaf_count(hit);
-      const bool pm = LEAF == kLeafPointMajor || (LEAF == kLeafHybrid && 2 * __popc(reach) <= cnt);
-      if (pm) {
-        collect_leaf_pm<STATS>(P, B, scene_inexact, L, t & ~31u, (int)(threadIdx.x & 31), first, cnt, reach);
-      } else {
-        if (STATS) {
-          L.st_points += cnt;
-          if (over) L.st_pairs += cnt;
-        }
-        collect_leaf<STATS>(P, B, scene_inexact, L, first, cnt, over);
-      }
-    }
-    cur = __float_as_int(b.w);
-  }
-  if (valid) collect_finish<STATS>(P, L, BATCH ? P.prob_kmax[prob] : P.kmax);
-}
-
-template <bool STATS, bool CUBE, bool BATCH, int MIN_BLOCKS, int LEAF = kLeafLaneMajor>
-__global__ void __launch_bounds__(256, MIN_BLOCKS) k_collect_packet(CollectParams P) {
-  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
-  if (!__any_sync(0xffffffffu, t < P.nq)) return;  // whole warp past the end
-  collect_packet_body<STATS, CUBE, BATCH, LEAF>(P, t);
-}
-
-// ---- heavy queries: radius refinement -------------------------------------------
-// A query with more than kSlab points in radius needs only its kmax (<= 64)
-// nearest.  If at least kmax points lie within a smaller radius r', those kmax
-// nearest are all among them, so the query is collected again at r' and then
-// sorted and emitted like any other query (its rows and counts still refer to
-// the original radius: the kmax nearest within r).  r' is chosen from the
-// in-radius count (cube-root scaling towards ~2 kmax points) inside a bracket
-// [lo, hi] that every pass narrows; queries still unresolved after a few
-// passes (for instance many points at one distance) take the generic path.
 
 // The bands of DevBands recomputed for another radius (same formulas; the
 // FP32 e_abs is rounded up, which only widens them).
@@ -950,324 +253,397 @@ __device__ __forceinline__ DevBands bands_at_radius(const DevBands& base, double
   b.lo2 = r_lo > 0.0 ? __double2float_rd(r_lo * r_lo) : 0.0f;
   b.box_hi2 = __double2float_ru((double)hi2 * (1.0 + 1.0e-6));
   b.r2 = radius * radius;
+  set_band_top(b);
   return b;
 }
 
-struct RefineParams {
-  CollectParams C;         // scene, queries, processing order, bands, slab
-  const uint32_t* qprob;   // problem of each query (input order); nullptr: one problem
-  const uint32_t* work;    // processing ranks to collect again
-  const double* rad;       // their radii
-  uint32_t nwork;
-  uint32_t* cnt;           // out: in-radius count at rad (all of them, not only the kSlab stored)
-  // device-driven form (captured graphs): the count is read from *nwork_dev, the
-  // packet kernel runs when it is >= packet_min and the warp kernel otherwise,
-  // and both stride over the work with whatever grid they were given
-  const unsigned int* nwork_dev;
-  uint32_t packet_min;
-};
-
-__device__ __forceinline__ uint32_t refine_count(const RefineParams& R, bool packet_kernel) {
-  if (!R.nwork_dev) return R.nwork;
-  const uint32_t n = *R.nwork_dev;
-  return (n >= R.packet_min) == packet_kernel ? n : 0u;
+// Which points of four buckets are within the query's radius, each decided in
+// FP64 (a lane calls it when one of them lies inside the band).
+__device__ __noinline__ uint32_t exact_buckets_mask(const float4* pts, const double* pts64, int inexact,
+                                                    const double* rq, int qstride, double r2, uint4 four,
+                                                    uint32_t empty) {
+  const double ex = rq[1], ey = rq[2], ez = qstride == 4 ? rq[3] : 0.0;
+  uint32_t mask = 0;
+  for (int i = 0; i < 4 * kBucketPoints; ++i) {
+    const uint32_t b = i < 8 ? four.x : i < 16 ? four.y : i < 24 ? four.z : four.w;
+    if (b != empty && exact_d2_at(ex, ey, ez, pts, pts64, inexact, b * kBucketPoints + (i & 7)) <= r2) mask |= 1u << i;
+  }
+  return mask;
 }
 
-// One warp per work item: the warp walks the query's subtree once (node
-// tests warp-uniform) and its lanes test a leaf bucket's points together,
-// appending accepted points with a ballot prefix.  The accept rule is
-// collect_point's (FP32 outside the band, FP64 inside).  Heavy queries are few
-// and scattered, so a packet of 32 of them would walk the union of 32 regions.
-__device__ __forceinline__ void collect_refine_warp(const RefineParams& R, uint32_t j, int lane, int scene_inexact) {
-  const CollectParams& P = R.C;
+// One warp walks a tree for one query and its lanes test the reached buckets'
+// points together, four buckets at a time: visit(i, p, has) runs on every lane
+// with its point (has false: no point) and returns true, on all of them, to
+// end the walk.
+template <typename Point>
+__device__ __forceinline__ void walk_single(const SceneView& S, const TreeShape* T, const float4& q,
+                                            const float& reach2, WalkStack& stack, int lane, Point&& point) {
+  const PacketBox box{q.x, q.y, q.z, q.x, q.y, q.z};
+  const uint32_t bucket0 = __ldg(&T->base[0]);
+  walk_wide(S, T, box, nullptr, reach2, stack, lane, [&](uint32_t first, uint32_t mask) {
+    while (mask) {
+      // lane group g (eight lanes) takes the g-th set bucket
+      uint32_t m = mask;
+      for (int g = 0; g < (lane >> 3); ++g) m &= m - 1u;
+      const bool has = m != 0u;
+      const uint32_t i = (bucket0 + first + (has ? (uint32_t)(__ffs((int)m) - 1) : 0u)) * kBucketPoints + (lane & 7);
+      const float4 p = __ldg(&S.pts[i]);
+      if (point(i, p, has)) return true;
+#pragma unroll
+      for (int g = 0; g < 4; ++g) mask &= mask - 1u;
+    }
+    return false;
+  });
+}
+
+// A warp's queue of buckets that hold in-radius points, one column per lane:
+// (bucket << 8) | the points' bits, the bucket counted within the tree.  A
+// store per bucket, kept or overwritten, instead of an append per point keeps
+// the walk free of divergent steps (on the clustered sets a query gets 32
+// points from 10 buckets); the lanes expand their words together when the queue
+// is flushed, four indices to a 16-byte store.
+constexpr int kQueueWords = 25;  // the last row only takes stores of lanes without a hit
+struct CollectWarp {
+  uint32_t queue[kQueueWords][32];
+  __align__(16) uint32_t list[kBucketList];
+  WalkStack stack;
+};
+
+// A packet's walk: every lane with `active` collects its points within band B
+// (their number in *count); the others keep what they have.
+template <int DIM>
+__device__ __forceinline__ void collect_walk(const CollectParams& P, const TreeShape* T, const DevBands& B,
+                                             int scene_inexact, const float4& q, uint32_t qin, uint32_t t,
+                                             bool active, CollectWarp& W, int lane, const PacketBox& box,
+                                             const PacketBox* limit, float reach2, uint32_t* count) {
   const SceneView& S = P.S;
-  const uint32_t t = R.work[j], qin = P.qorder[t];
-  const uint32_t prob = R.qprob ? R.qprob[qin] : 0u;
-  const DevBands LB = bands_at_radius(P.bands[prob], R.rad[j]);
+  const uint32_t bucket0 = __ldg(&T->base[0]);
+  BucketQuery bq;
+  bq.set(q.x, q.y, q.z, B.top);
+  // near < band: in the band; never for a lane that collects nothing
+  const int band = active ? (int)(0x80000001u + __float_as_uint(B.width)) : (int)0x80000000;
+  const uint32_t keep = active ? 0xffffffffu : 0u;
+  uint32_t found = 0;      // points
+  int words = 0;           // words in the queue
+  uint32_t pending = 0;    // points in the queue
+  uint32_t stored = 0;     // indices stored, a multiple of four until the last flush
+  // Stores the queued points in fours; a rest of at most three stays queued
+  // unless `last` (whose last store may hold up to three stray indices).
+  auto flush = [&](bool last) {
+    __syncwarp();
+    uint32_t fours = last ? (pending + 3) / 4 : pending / 4;
+    const uint32_t room = ((uint32_t)kSlab - stored) / 4;  // beyond kSlab they are only counted
+    const bool full = fours > room;
+    if (full) fours = room;
+    const uint32_t most = __reduce_max_sync(0xffffffffu, fours);
+    uint32_t bits = 0, word = 0, first = 0;
+    int w = 0;
+    uint32_t* out = P.slab + slab_base(t) + stored;
+    for (uint32_t k = 0; k < most; ++k) {
+      if (k < fours) {
+        uint32_t i[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          if (bits == 0 && w < words) {
+            word = W.queue[w++][lane];
+            bits = word & 255u;
+            first = (bucket0 + (word >> 8)) * kBucketPoints;
+          }
+          i[u] = first + (bits ? (uint32_t)(__ffs((int)bits) - 1) : 0u);
+          bits &= bits - 1u;
+        }
+        *reinterpret_cast<uint4*>(out + 4 * k) = make_uint4(i[0], i[1], i[2], i[3]);
+      }
+    }
+    stored += 4 * fours;
+    int rest = 0;
+    if (!full && !last) {
+      if (bits) W.queue[rest++][lane] = (word & ~255u) | bits;
+      while (w < words) W.queue[rest++][lane] = W.queue[w++][lane];
+      pending -= 4 * fours;
+    } else {
+      pending = 0;
+    }
+    words = rest;
+    __syncwarp();
+  };
+  walk_fours(S, T, box, limit, reach2, W.stack, W.list, lane, 32u, [&](const uint4& four) {
+    int near;
+    uint32_t hits = buckets_mask<DIM, true>(S.bucket_pts, four, bq, &near);
+    if (near < band)
+      hits = exact_buckets_mask(S.pts, S.pts64, scene_inexact, P.qraw + (size_t)qin * P.qstride, P.qstride, B.r2,
+                                four, S.slots / kBucketPoints);
+    hits &= keep;
+    found += __popc(hits);
+    pending += __popc(hits);
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const uint32_t bucket = u == 0 ? four.x : u == 1 ? four.y : u == 2 ? four.z : four.w;
+      const uint32_t byte = (hits >> (8 * u)) & 255u;
+      W.queue[words][lane] = ((bucket - bucket0) << 8) | byte;  // kept when it has a hit
+      words += byte != 0u;
+    }
+    if (__any_sync(0xffffffffu, words > kQueueWords - 5)) flush(false);
+    return false;
+  });
+  flush(true);
+  if (active) *count = found;
+}
+
+// What a packet walk that keeps no candidates needs of shared memory.
+struct PacketWarp {
+  __align__(16) uint32_t list[kBucketList];
+  WalkStack stack;
+};
+
+// The same for one query by the whole warp (all arguments warp-uniform).
+__device__ __noinline__ uint32_t collect_alone(const CollectParams& P, const TreeShape* T, const DevBands& B,
+                                               int scene_inexact, uint32_t qin, uint32_t t, WalkStack& stack) {
+  const SceneView& S = P.S;
+  const int lane = threadIdx.x & 31;
   const float4 q = P.qpts[qin];
   const double* rq = P.qraw + (size_t)qin * P.qstride;
-  const double ex = rq[1], ey = rq[2], ez = P.qstride == 4 ? rq[3] : 0.0;
-  unsigned long long* out = P.slab + slab_base(t);
-  int cur = S.n > 0 ? 0 : kRopeEnd, end = kRopeEnd;
-  if (S.prob_root) {
-    cur = S.prob_root[prob];
-    if (cur != kRopeEnd) end = __float_as_int(__ldg(&S.nodes[2 * cur + 1]).w);
-  }
-  const unsigned int lt = (1u << lane) - 1u;
+  uint32_t* out = P.slab + slab_base(t);
   uint32_t count = 0;
-  while (cur != end) {
-    const float4 a = __ldg(&S.nodes[2 * cur]), b = __ldg(&S.nodes[2 * cur + 1]);
-    const int hit = __float_as_int(a.w);
-    if (box_d2(q.x, q.y, q.z, a, b) <= LB.box_hi2) {
-      if (hit >= 0) {
-        ++cur;
-        continue;
-      }
-      const int first = leaf_first(hit), cnt = leaf_count(hit);
-      bool acc = false;
-      float key = 0.f;
-      const uint32_t i = (uint32_t)(first + lane);
-      if (lane < cnt) {
-        const float4 p = __ldg(&S.pts[i]);
-        const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-        key = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-        acc = key <= LB.hi2;
-        if (acc && (key >= LB.lo2 || LB.any_inexact)) {
-          const double e2 = exact_d2_at(ex, ey, ez, S.pts, S.pts64, scene_inexact, i);
-          if (key >= LB.lo2 && e2 > LB.r2) acc = false;
-          if (LB.any_inexact) key = __double2float_rn(e2);
-        }
-      }
-      const unsigned int m = __ballot_sync(0xffffffffu, acc);
-      if (acc) {
-        const uint32_t pos = count + __popc(m & lt);
-        if (pos < (uint32_t)kSlab) out[pos] = slab_entry(key, i);
-      }
-      count += __popc(m);
-    }
-    cur = __float_as_int(b.w);
-  }
-  if (lane == 0) R.cnt[j] = count;
+  walk_single(S, T, q, B.box_hi2, stack, lane, [&](uint32_t i, const float4& p, bool has) {
+    const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    bool hit = has && d2 <= B.hi2;
+    if (hit && d2 >= B.lo2)
+      hit = exact_d2_at(rq[1], rq[2], P.qstride == 4 ? rq[3] : 0.0, S.pts, S.pts64, scene_inexact, i) <= B.r2;
+    const uint32_t hits = __ballot_sync(0xffffffffu, hit);
+    const uint32_t at = count + __popc(hits & ((1u << lane) - 1u));
+    if (hit && at < (uint32_t)kSlab) out[at] = i;
+    count += __popc(hits);
+    return false;
+  });
+  return count;
 }
 
-__global__ void __launch_bounds__(256) k_collect_refine(RefineParams R) {
-  const uint32_t n = refine_count(R, false);
-  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  uint32_t j = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5);
-  if (j >= n) return;  // whole warp
-  const int scene_inexact = *R.C.S.inexact;
-  for (; j < n; j += warps) collect_refine_warp(R, j, threadIdx.x & 31, scene_inexact);
-}
+// A query whose radius holds more than kSlab points needs only its kmax (<= 64)
+// nearest.  If at least kmax points lie within a smaller radius r', those kmax
+// nearest are all among them, so the query is collected again at r' (its rows
+// and counts still refer to the original radius).  r' is chosen from the
+// in-radius count (cube-root scaling towards ~2 kmax points) inside a bracket
+// [lo, hi] that every pass narrows; a query still unresolved after the passes
+// (many points at one distance) takes the generic path, which gathers within
+// the smallest tested radius that holds its rows.  The passes run inside the
+// collect, by the packet that holds the query: the lanes are neighbours, the
+// nodes are in the caches, and nothing is listed or read back.
+constexpr int kRefinePasses = 6;
 
-// One thread per work item, warp-packet walks (the form for many heavy
-// queries, which then cluster in space): the lanes of a warp that share a
-// subtree root walk it together (a problem batch can mix roots in a warp).
-__device__ __forceinline__ void collect_refine_packet(const RefineParams& R, uint32_t j, bool valid,
-                                                      int scene_inexact) {
-  const CollectParams& P = R.C;
-  const SceneView& S = P.S;
-  CollectLane L;
-  uint32_t prob = 0;
-  DevBands LB = P.bands[0];
-  int root = kRopeEnd, end = kRopeEnd;
-  if (valid) {
-    collect_init(P, R.work[j], L);
-    prob = R.qprob ? R.qprob[L.qin] : 0u;
-    LB = bands_at_radius(P.bands[prob], R.rad[j]);
-    root = S.prob_root ? S.prob_root[prob] : (S.n > 0 ? 0 : kRopeEnd);
-    if (root != kRopeEnd) end = __float_as_int(__ldg(&S.nodes[2 * root + 1]).w);
-  } else {
-    L.q = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
-    L.count = 0;
-    L.out = nullptr;
-  }
-  bool todo = valid && root != kRopeEnd;
-  while (true) {
-    const unsigned int pending = __ballot_sync(0xffffffffu, todo);
-    if (!pending) break;
-    const int leader = __ffs(pending) - 1;
-    const int r0 = __shfl_sync(0xffffffffu, root, leader), e0 = __shfl_sync(0xffffffffu, end, leader);
-    const bool mine = todo && root == r0;
-    int cur = r0;
-    while (cur != e0) {
-      const float4 a = __ldg(&S.nodes[2 * cur]), b = __ldg(&S.nodes[2 * cur + 1]);
-      const int hit = __float_as_int(a.w);
-      const bool over = mine && box_d2(L.q.x, L.q.y, L.q.z, a, b) <= LB.box_hi2;
-      if (__any_sync(0xffffffffu, over)) {
-        if (hit >= 0) {
-          ++cur;
-          continue;
-        }
-        collect_leaf<false>(P, LB, scene_inexact, L, leaf_first(hit), leaf_count(hit), over);
-      }
-      cur = __float_as_int(b.w);
-    }
-    todo = todo && !mine;
-  }
-  if (valid) R.cnt[j] = L.count;
-}
-
-// The same walk for one scene without problem subtrees (many heavy queries of a
-// plain or prepared scene): no per-lane roots, and close to the collect's occupancy.
-__global__ void __launch_bounds__(256, 6) k_collect_refine_packet_scene(RefineParams R) {
-  const uint32_t n = refine_count(R, true);
-  const uint32_t stride = gridDim.x * blockDim.x;
-  uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;  // warp-uniform
-  if (base >= n) return;  // whole warp
-  const CollectParams& P = R.C;
-  const SceneView& S = P.S;
-  const int scene_inexact = *S.inexact;
-  for (; base < n; base += stride) {
-    const uint32_t j = base + (threadIdx.x & 31);
-    const bool valid = j < n;
-    CollectLane L;
-    DevBands LB = P.bands[0];
-    if (valid) {
-      collect_init(P, R.work[j], L);
-      LB = bands_at_radius(P.bands[0], R.rad[j]);
-    } else {
-      L.q = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
-      L.count = 0;
-      L.out = nullptr;
-    }
-    int cur = S.n > 0 ? 0 : kRopeEnd;
-    while (cur != kRopeEnd) {
-      const float4 a = __ldg(&S.nodes[2 * cur]), b = __ldg(&S.nodes[2 * cur + 1]);
-      const int hit = __float_as_int(a.w);
-      const bool over = valid && box_d2(L.q.x, L.q.y, L.q.z, a, b) <= LB.box_hi2;
-      if (__any_sync(0xffffffffu, over)) {
-        if (hit >= 0) {
-          ++cur;
-          continue;
-        }
-        collect_leaf<false>(P, LB, scene_inexact, L, leaf_first(hit), leaf_count(hit), over);
-      }
-      cur = __float_as_int(b.w);
-    }
-    if (valid) R.cnt[j] = L.count;
-  }
-}
-
-__global__ void __launch_bounds__(256) k_collect_refine_packet(RefineParams R) {
-  const uint32_t n = refine_count(R, true);
-  const uint32_t stride = gridDim.x * blockDim.x;
-  uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u;  // warp-uniform
-  if (base >= n) return;  // whole warp
-  const int scene_inexact = *R.C.S.inexact;
-  for (; base < n; base += stride) {
-    const uint32_t j = base + (threadIdx.x & 31);
-    collect_refine_packet(R, j, j < n, scene_inexact);
-  }
-}
-
-struct RefineUpdate {
-  const uint32_t* qorder;
-  const uint32_t* qprob;      // nullptr: one problem
-  const uint32_t* prob_kmax;  // nullptr: kmax below
-  uint32_t kmax;
-  QueryInfo* qinfo;
-  uint8_t* flags;
-  uint32_t* mid_list;
-  uint32_t* big_list;
-  unsigned int* small;        // [2] mid_list length, [3] big_list length
-  // this pass
-  const uint32_t* work;
-  const double* rad;
-  const double* lo;
-  const double* hi;
-  const uint32_t* full;       // in-radius count at radius frad (at least kmax points)
-  const double* frad;         // the original radius, or a smaller tested one that held more than kSlab
-  const uint32_t* cnt;
-  uint32_t nwork;
-  // next pass (or, on the last pass, the generic path's list)
-  uint32_t* next_work;
-  double* next_rad;
-  double* next_lo;
-  double* next_hi;
-  uint32_t* next_full;
-  double* next_frad;
-  unsigned int* next_count;
-  uint32_t* generic_qin;      // last pass: unresolved queries (input index), their counts at
-  uint32_t* generic_m;        // generic_rad: the generic path gathers within that radius
-  double* generic_rad;
-  int last;
-  const unsigned int* nwork_dev;  // non-null: the count is read here (captured graphs)
+struct RefineState {
+  float rad, lo, hi, frad;  // frad < 0: the original radius
+  uint32_t total, full;     // in-radius counts at the original radius and at frad
+  bool active, generic;
 };
 
-// One work item: resolves it (emit lists), lists it for the generic path (last
-// pass), or returns true with its next-pass radius, bracket and bound.
-__device__ __forceinline__ bool refine_update_one(const RefineUpdate& U, uint32_t j, uint32_t& t, double& est,
-                                                  double& l, double& h, uint32_t& f, double& fr) {
-  t = U.work[j];
-  const uint32_t qin = U.qorder[t], c = U.cnt[j];
-  const uint32_t kmax = U.prob_kmax ? U.prob_kmax[U.qprob ? U.qprob[qin] : 0u] : U.kmax;
-  if (c >= kmax && c <= (uint32_t)kSlab) {  // resolved: the slab holds every point within rad
-    // A resolved query goes to a list kernel whatever its count (k_emit_list<4>
-    // sorts up to 128): k_emit may run while the refinement does, and it skips
-    // the query under both the collect's record (generic) and this one (big).
-    uint8_t fl = (uint8_t)((U.flags[qin] & ~6u) | (c > 64u ? 4u : 0u));
-    U.flags[qin] = fl;
-    U.qinfo[t].meta = c | ((fl & 1) ? kQueryOverflow : 0u) | kQueryBig | (kmax << kQueryKmaxShift);
-    if (c > 128u)
-      U.big_list[atomicAdd(&U.small[3], 1u)] = t;
-    else
-      U.mid_list[atomicAdd(&U.small[2], 1u)] = t;
-    return false;
+// After pass `pass` found c points: done, or the next radius in st.rad.
+__device__ __forceinline__ void refine_step(RefineState& st, int pass, uint32_t c, uint32_t kmax, double radius) {
+  if (pass == 0) {
+    st.total = st.full = c;
+    st.frad = -1.f;
+    st.lo = 0.f;
+    st.hi = __double2float_ru(radius);
+    st.rad = st.hi;
   }
-  // a tested radius with more than kSlab (>= kmax) points in it also holds the
-  // kmax nearest; the smallest such radius bounds the generic path's gather
-  f = U.full[j];
-  fr = U.frad[j];
-  if (c > (uint32_t)kSlab && c < f) {
-    f = c;
-    fr = U.rad[j];
+  if (c <= (uint32_t)kSlab && (pass == 0 || c >= kmax)) {
+    st.active = false;
+    return;
   }
-  if (U.last) {
-    const unsigned int k = atomicAdd(U.next_count, 1u);
-    U.generic_qin[k] = qin;
-    U.generic_m[k] = f;
-    U.generic_rad[k] = fr;
-    return false;
+  if (pass > 0) {
+    if (c > (uint32_t)kSlab && c < st.full) {
+      st.full = c;
+      st.frad = st.rad;
+    }
+    if (c < kmax) st.lo = st.rad;
+    else st.hi = st.rad;
   }
-  const double r = U.rad[j];
-  l = U.lo[j];
-  h = U.hi[j];
-  if (c < kmax) l = r; else h = r;
-  est = r * cbrt(2.0 * kmax / (double)(c > 0u ? c : 1u));
-  if (!(est > l && est < h)) est = 0.5 * (l + h);
-  return true;
+  if (kmax > (uint32_t)kMaxList || pass == kRefinePasses) {
+    st.active = false;
+    st.generic = true;
+    return;
+  }
+  float est = st.rad * cbrtf(2.0f * (float)kmax / (float)(c > 0u ? c : 1u));
+  if (!(est > st.lo && est < st.hi)) est = 0.5f * (st.lo + st.hi);
+  st.rad = est;
 }
 
-// The next pass's work keeps each warp's items in their order (one atomic per
-// warp): items come in processing (Morton) order, so a packet of the next pass
-// still walks one region.
-__global__ void k_refine_update(RefineUpdate U) {
-  const uint32_t n = U.nwork_dev ? *U.nwork_dev : U.nwork;
-  const int lane = threadIdx.x & 31;
-  const uint32_t stride = gridDim.x * blockDim.x;
-  for (uint32_t base = (blockIdx.x * blockDim.x + threadIdx.x) & ~31u; base < n; base += stride) {  // warp-uniform
-    const uint32_t j = base + lane;
-    uint32_t t = 0, f = 0;
-    double est = 0.0, l = 0.0, h = 0.0, fr = 0.0;
-    const bool next = j < n && refine_update_one(U, j, t, est, l, h, f, fr);
-    const unsigned int m = __ballot_sync(0xffffffffu, next);
-    if (!m) continue;
-    unsigned int first = 0;
-    if (lane == 0) first = atomicAdd(U.next_count, (unsigned int)__popc(m));
-    first = __shfl_sync(0xffffffffu, first, 0);
-    if (next) {
-      const unsigned int k = first + __popc(m & ((1u << lane) - 1u));
-      U.next_work[k] = t;
-      U.next_rad[k] = est;
-      U.next_lo[k] = l;
-      U.next_hi[k] = h;
-      U.next_full[k] = f;
-      U.next_frad[k] = fr;
+__device__ __forceinline__ void collect_finish(const CollectParams& P, uint32_t t, uint32_t qin,
+                                               const RefineState& st, uint32_t points, uint32_t kmax,
+                                               double radius) {
+  if (P.stats) {
+    atomicAdd(&P.stats[kStatInRadius], (unsigned long long)st.total);
+    atomicMax(&P.stats[kStatMaxLeafPoints], (unsigned long long)st.total);
+    if (st.total > (uint32_t)kSlab && !st.generic) atomicAdd(&P.stats[kStatRefined], 1ull);
+    if (points > 64u && !st.generic) atomicAdd(&P.stats[kStatLargeQueries], 1ull);
+  }
+  P.counts[qin] = st.total < kmax ? st.total : kmax;
+  const bool over = st.total > kmax;
+  uint32_t meta = ((kmax < (uint32_t)kSlab ? kmax : (uint32_t)kSlab) << kQueryKmaxShift);
+  if (st.generic) {
+    meta |= kQueryGeneric;
+    const unsigned int h = atomicAdd(&P.small[0], 1u);
+    P.heavy_list[h] = qin;
+    P.heavy_m[h] = st.full;
+    P.heavy_rad[h] = st.frad < 0.f ? radius : (double)st.frad;
+    P.heavy_t[h] = t;
+  } else {
+    meta |= points;
+    if (points > 128u) {
+      meta |= kQueryBig;
+      P.big_list[atomicAdd(&P.small[3], 1u)] = t;
+    } else if (points > 64u) {
+      meta |= kQueryBig;
+      P.mid_list[atomicAdd(&P.small[2], 1u)] = t;
     }
   }
+  const double* r = P.qraw + (size_t)qin * P.qstride;
+  QueryInfo qi;
+  qi.ex = r[1];
+  qi.ey = r[2];
+  qi.ez = P.qstride == 4 ? r[3] : 0.0;
+  qi.qid = __float_as_uint(P.qpts[qin].w);
+  qi.meta = meta;
+  P.qinfo[t] = qi;
+  P.flags[qin] = (over ? 1 : 0) | (st.generic ? 2 : 0);
+  if (P.overflow_out) P.overflow_out[qin] = over ? 1 : 0;
 }
 
-// The first refinement pass's work: the collect pass's heavy queries (listed
-// by input index with their full counts), radius scaled from the full count.
-__global__ void k_refine_init(const uint32_t* heavy_qin, const uint32_t* heavy_m, const uint32_t* heavy_t,
-                              uint32_t H, const uint32_t* qprob, const double* prob_radius, double radius,
-                              const uint32_t* prob_kmax, uint32_t kmax, uint32_t* work, double* rad, double* lo,
-                              double* hi, uint32_t* full, double* frad, const unsigned int* H_dev) {
-  if (H_dev) H = *H_dev;  // captured graphs: the collect pass's heavy count
-  for (uint32_t h = blockIdx.x * blockDim.x + threadIdx.x; h < H; h += gridDim.x * blockDim.x) {
-    const uint32_t qin = heavy_qin[h], p = qprob ? qprob[qin] : 0u;
-    const uint32_t m = heavy_m[h];
-    work[h] = heavy_t[h];
-    const double r = prob_radius ? prob_radius[p] : radius;
-    const uint32_t k = prob_kmax ? prob_kmax[p] : kmax;
-    rad[h] = r * cbrt(2.0 * k / (double)m);
-    hi[h] = r;
-    frad[h] = r;
-    lo[h] = 0.0;
-    full[h] = m;
+// The record of a KNN query (no points: k_knn_single writes its rows).
+__device__ __forceinline__ void collect_finish_knn(const CollectParams& P, uint32_t t, uint32_t qin,
+                                                   uint32_t points, uint32_t kmax) {
+  uint32_t meta = points ? kmax << kQueryKmaxShift | points : 0u;
+  if (points > 128u) {
+    meta |= kQueryBig;
+    P.big_list[atomicAdd(&P.small[3], 1u)] = t;
+  } else if (points > 64u) {
+    meta |= kQueryBig;
+    P.mid_list[atomicAdd(&P.small[2], 1u)] = t;
+  }
+  const double* r = P.qraw + (size_t)qin * P.qstride;
+  P.qinfo[t] = QueryInfo{r[1], r[2], P.qstride == 4 ? r[3] : 0.0, __float_as_uint(P.qpts[qin].w), meta};
+}
+
+// One warp per 32 curve-consecutive queries (a packet): the warp walks the
+// wide tree once for the box around them (or around each run of them that is
+// worth it, see cut_packet), then tests every reached bucket's eight points
+// with each lane's query.  Node, bucket and control flow are warp-uniform.
+// BATCH: several problems (a problem batch, or several requests on one scene):
+// each warp has one problem, its tree, its bands and its kmax.  OWN: every
+// query has a radius of its own (KNN).
+// A packet of the clustered 1M x 1M sets takes 18 node steps and 87 buckets;
+// what bounds it is instruction issue (about 45 instructions per bucket).
+template <int DIM, bool BATCH, bool OWN>
+__device__ __forceinline__ void collect_packet_body(const CollectParams& P, uint32_t t, CollectWarp& W) {
+  const int lane = threadIdx.x & 31;
+  // a problem batch pads every problem to whole warps, so a warp has one problem
+  // (lanes past the packet's width hold no rank: the problem is lane 0's)
+  const uint32_t prob = BATCH ? P.warp_prob[(t - (uint32_t)lane) >> 5] : 0u;
+  const bool rank = (uint32_t)lane < P.width && t < P.nq;
+  const uint32_t qin = rank ? P.qorder[t] : kNone;
+  const bool valid = qin != kNone;
+  if (BATCH && !valid && rank) P.qinfo[t] = QueryInfo{0.0, 0.0, 0.0, 0u, 0u};  // padding: nothing to emit
+  const uint32_t kmax = BATCH ? P.prob_kmax[prob] : P.kmax;
+  const double radius = OWN ? (valid ? P.rank_radius[t] : 0.0) : BATCH ? P.prob_radius[prob] : P.radius;
+  const TreeShape* T = P.S.trees + (BATCH ? prob * P.S.tree_stride : 0u);
+  const int scene_inexact = *P.S.inexact;
+  const float4 q = valid ? P.qpts[qin] : make_float4(0.f, 0.f, 0.f, 0.f);
+  DevBands B = P.bands[prob];
+  if (OWN) B = bands_at_radius(B, radius);
+  RefineState st{};
+  st.active = valid;
+  bool left = false;  // to k_collect_single
+  uint32_t count = 0;
+  for (int pass = 0;; ++pass) {
+    cut_packet(
+        P.S, T, q, B.box_hi2, OWN || pass > 0, st.active, W.stack, lane,
+        [&](bool mine, const PacketBox& box, const PacketBox* limit, float reach2) {
+          collect_walk<DIM>(P, T, B, scene_inexact, q, qin, t, mine, W, lane, box, limit, reach2, &count);
+        },
+        [&](uint32_t run) {
+          if (OWN || pass == 0) {  // a warp of its own for each of them
+            uint32_t at = 0;
+            if (lane == 0) at = atomicAdd(&P.small[6], (unsigned int)__popc(run));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if ((run >> lane) & 1u) {
+              P.single_list[at + __popc(run & ((1u << lane) - 1u))] = t;
+              left = true;
+            }
+          } else {
+            for (; run; run &= run - 1u) {
+              const int from = __ffs((int)run) - 1;
+              const DevBands one = bands_at_radius(P.bands[prob], (double)__shfl_sync(0xffffffffu, st.rad, from));
+              const uint32_t c = collect_alone(P, T, one, scene_inexact, __shfl_sync(0xffffffffu, qin, from),
+                                               __shfl_sync(0xffffffffu, t, from), W.stack);
+              if (lane == from) count = c;
+            }
+          }
+        });
+    if (left) st.active = false;
+    if (OWN) break;
+    if (st.active) refine_step(st, pass, count, kmax, radius);
+    if (!__any_sync(0xffffffffu, st.active)) break;
+    B = bands_at_radius(P.bands[prob], (double)st.rad);
+  }
+  if (OWN) {
+    // a radius that holds too many points (it only bounds the k-th distance):
+    // k_knn_single finds the k nearest with a shrinking one
+    const bool heavy = valid && !left && count > (uint32_t)kSlab;
+    const uint32_t m = __ballot_sync(0xffffffffu, heavy);
+    if (m) {
+      uint32_t at = 0;
+      if (lane == 0) at = atomicAdd(&P.small[6], (unsigned int)__popc(m));
+      at = __shfl_sync(0xffffffffu, at, 0);
+      if (heavy) P.single_list[at + __popc(m & ((1u << lane) - 1u))] = t;
+    }
+    if (valid) collect_finish_knn(P, t, qin, left || heavy ? 0u : count, kmax);
+    return;
+  }
+  if (valid && !left) collect_finish(P, t, qin, st, count, kmax, radius);
+}
+
+constexpr int kCollectThreads = 128;
+
+template <int DIM, bool BATCH, bool OWN>
+__global__ void __launch_bounds__(kCollectThreads, 6) k_collect_packet(const __grid_constant__ CollectParams P) {
+  __shared__ CollectWarp warps[kCollectThreads / 32];
+  const uint32_t t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * P.width + (threadIdx.x & 31);
+  if (!__any_sync(0xffffffffu, t < P.nq)) return;  // whole warp past the end
+  collect_packet_body<DIM, BATCH, OWN>(P, t, warps[threadIdx.x >> 5]);
+}
+
+// One warp per query: every query of a call too small to fill the GPU with
+// packets (`listed` false), where the walk's latency is what counts, or those
+// the packets left.
+__global__ void __launch_bounds__(128) k_collect_single(const __grid_constant__ CollectParams P, bool listed) {
+  __shared__ WalkStack stacks[128 / 32];
+  const int lane = threadIdx.x & 31;
+  const uint32_t n = listed ? P.small[6] : P.nq;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; j < n; j += warps) {
+    const uint32_t t = listed ? P.single_list[j] : j;
+    const uint32_t qin = P.qorder[t];
+    if (qin == kNone) {
+      if (lane == 0) P.qinfo[t] = QueryInfo{0.0, 0.0, 0.0, 0u, 0u};
+      continue;
+    }
+    const uint32_t prob = P.warp_prob ? P.warp_prob[t >> 5] : 0u;
+    const uint32_t kmax = P.warp_prob ? P.prob_kmax[prob] : P.kmax;
+    const double radius = P.warp_prob ? P.prob_radius[prob] : P.radius;
+    DevBands B = P.bands[prob];
+    RefineState st{};
+    st.active = true;
+    uint32_t count;
+    for (int pass = 0;; ++pass) {
+      count = collect_alone(P, P.S.trees + prob * P.S.tree_stride, B, *P.S.inexact, qin, t, stacks[threadIdx.x >> 5]);
+      refine_step(st, pass, count, kmax, radius);
+      if (!st.active) break;
+      B = bands_at_radius(P.bands[prob], (double)st.rad);
+    }
+    if (lane == 0) collect_finish(P, t, qin, st, count, kmax, radius);
   }
 }
-
 
 // ---- emit: warp per query -----------------------------------------------------
 // Emitted row writer.
@@ -1293,7 +669,7 @@ struct RowSink {
 struct EmitParams {
   SceneView S;
   uint32_t nq;
-  unsigned long long* slab;
+  const uint32_t* slab;
   const QueryInfo* qinfo;     // by processing rank
   const unsigned long long* poff;  // first row of each query, by processing rank
   RowSink sink;
@@ -1312,19 +688,11 @@ struct EmitParams {
   int range = 0;
 };
 
-// A deferred query's sorted packed keys live in slab entries its candidates do
-// not use: from entry 64 for at most 64 candidates, from entry 128 for at most
-// 128 (room for 256 keys).
-__device__ __forceinline__ uint32_t* deferred_keys(unsigned long long* slab, uint32_t t, int n) {
-  return reinterpret_cast<uint32_t*>(slab + slab_base(t) + (n <= 64 ? 64 : 128));
-}
-
-// Packed sort element: the FP32 d2 key with its low SHIFT mantissa bits
-// replaced by the slab slot.  Valid keys are below 0x80000000, so the padding
-// value 0xFFFFFFFF sorts last.  Two elements whose truncated keys differ by two
-// units or more are in exact order (the FP32 keys are within a few ulps of
-// the exact FP64 d2, far less than 2^SHIFT ulps); closer pairs are re-decided
-// exactly.
+// Packed sort element: the exact FP64 d2 rounded to FP32 with its low SHIFT
+// mantissa bits replaced by the candidate's slot.  Valid keys are below
+// 0x80000000, so the padding value 0xFFFFFFFF sorts last.  Two elements whose
+// truncated keys differ by two units or more are in exact order; closer pairs
+// are re-decided exactly.
 template <int SHIFT>
 __device__ __forceinline__ uint32_t pack_key(uint32_t key_bits, uint32_t slot) {
   return (key_bits & ~((1u << SHIFT) - 1u)) | slot;
@@ -1364,27 +732,29 @@ __device__ __forceinline__ void warp_bitonic_striped(uint32_t (&v)[E], int lane)
   }
 }
 
-// Odd-even transposition over a warp's sorted buffer, one thread, restricted
-// to neighbours whose truncated keys differ by at most one unit, until no swap
-// happens (bounded by n passes).  Runs only when such a pair exists.
-__device__ __noinline__ void exact_fixup_sorted(uint32_t* buf, int n, int shift, const unsigned long long* ent,
-                                                SceneView S, int inexact, double ex, double ey, double ez) {
+// Odd-even transposition over a warp's sorted buffer (the pairs of one parity
+// are disjoint, so the lanes take them in parallel), restricted to neighbours
+// whose truncated keys differ by at most one unit, until no swap happens
+// (bounded by n passes).  Runs only when such a pair exists.
+__device__ __noinline__ void exact_fixup_sorted(uint32_t* buf, int n, int shift, const uint32_t* cand,
+                                                const float4* pts, const double* pts64, const uint32_t* perm,
+                                                int inexact, double ex, double ey, double ez, int lane) {
   const uint32_t mask = (1u << shift) - 1u;
   for (int pass = 0; pass < n; ++pass) {
     bool changed = false;
     for (int parity = 0; parity < 2; ++parity) {
-      for (int i = parity; i + 1 < n; i += 2) {
+      for (int i = parity + 2 * lane; i + 1 < n; i += 64) {
         const uint32_t a = buf[i], b = buf[i + 1];
         if ((b >> shift) - (a >> shift) > 1u) continue;
-        if (exact_before(ex, ey, ez, S.pts, S.pts64, S.perm, inexact, (uint32_t)ent[b & mask],
-                         (uint32_t)ent[a & mask])) {
+        if (exact_before(ex, ey, ez, pts, pts64, perm, inexact, cand[b & mask], cand[a & mask])) {
           buf[i] = b;
           buf[i + 1] = a;
           changed = true;
         }
       }
+      __syncwarp();
     }
-    if (!changed) break;
+    if (!__any_sync(0xffffffffu, changed)) break;
   }
 }
 
@@ -1410,54 +780,66 @@ __device__ __forceinline__ int exact_window(const uint32_t (&v)[E], int n, int k
   return m;
 }
 
-// The window of exact_window for keys sorted in a shared-memory buffer (k_emit_fixup).
-__device__ __forceinline__ int exact_window_sorted(const uint32_t* keys, int n, int kk, int shift) {
-  if (kk >= n) return n;
-  const uint32_t limit = (keys[kk - 1] >> shift) + 1u;
-  int m = kk;
-  while (m < n && (keys[m] >> shift) <= limit) ++m;
-  return m;
-}
-
-// What a warp needs of one query before it sorts: three independent loads
-// (the query's record, its first row and slab entry `lane`), so a query costs
-// one memory round trip before the sort and one (the point gather) after it.
+// What a warp needs of one query before it sorts: three independent loads (the
+// query's record, its first row and candidate `lane`), so a query costs one
+// memory round trip before the point gather.
 struct EmitQuery {
   QueryInfo qi;
   unsigned long long base;  // first row of the query
-  unsigned long long e0;    // slab entry `lane` (read before the count is known; unused beyond it)
+  uint32_t i0;              // candidate `lane` (read before the count is known; unused beyond it)
 };
 
 __device__ __forceinline__ void emit_load(const EmitParams& P, uint32_t t, int lane, EmitQuery& q) {
   q.qi = P.qinfo[t];
   q.base = P.poff[t];
-  q.e0 = P.slab[slab_base(t) + lane];  // inside the query's kSlab entries whatever its count
+  q.i0 = P.slab[slab_base(t) + lane];  // inside the query's kSlab entries whatever its count
 }
+
+// Per-warp shared memory of an emit: distance and id of each candidate, for the
+// lane that writes its row.
+template <int E>
+struct EmitWarp {
+  double dist[32 * E];
+  uint32_t nid[32 * E];
+};
 
 // Sorts the query's n <= 32 * E candidates by the reference's key and writes
 // its first min(n, kmax) rows; lane l writes rows l, l + 32, ... so each store
-// instruction covers 32 consecutive rows.  When two neighbours need the exact
-// comparison, DEFER == false re-decides them here through `wbuf` (shared
-// memory); DEFER == true leaves the sorted list in the query's spare slab
-// entries and queues the query for k_emit_fixup, which keeps this kernel free
-// of the exact comparison's call (and of the registers that call needs).
+// instruction covers 32 consecutive rows.  The points are gathered once: the
+// exact distance gives the sort key, and waits in shared memory for the lane
+// that writes the row.  When two neighbours need the exact comparison, DEFER
+// == false re-decides them here through `wbuf` and `cand` (shared memory, 32 * E
+// words each); DEFER == true queues the query for k_emit_fixup, which keeps this
+// kernel free of the exact comparison's call (and of the registers that call
+// needs).
 template <int E, bool DEFER>
 __device__ __forceinline__ void emit_query(const EmitParams& P, uint32_t t, const EmitQuery& q, int n, int lane,
-                                           uint32_t* wbuf) {
+                                           EmitWarp<E>& W, uint32_t* cand, uint32_t* wbuf) {
   constexpr int SHIFT = E == 1 ? 5 : E == 2 ? 6 : E == 4 ? 7 : 8;
   constexpr uint32_t kMask = (1u << SHIFT) - 1u;
-  const unsigned long long* ent = P.slab + slab_base(t);
-  uint32_t v[E], ids[E];
+  const double ex = q.qi.ex, ey = q.qi.ey, ez = q.qi.ez;
+  const int inexact = *P.S.inexact;
+  uint32_t v[E];
 #pragma unroll
   for (int r = 0; r < E; ++r) {
     const int s = (r << 5) | lane;
+    v[r] = 0xFFFFFFFFu;
     if (s < n) {
-      const unsigned long long e = r == 0 ? q.e0 : ent[s];
-      v[r] = pack_key<SHIFT>((uint32_t)(e >> 32), (uint32_t)s);
-      ids[r] = (uint32_t)e;
-    } else {
-      v[r] = 0xFFFFFFFFu;
-      ids[r] = 0u;
+      const uint32_t i = r == 0 ? q.i0 : P.slab[slab_base(t) + s];
+      const float4 p = __ldg(&P.S.pts[i]);
+      double sx = p.x, sy = p.y, sz = p.z;
+      if (inexact) {
+        const double* pp = P.S.pts64 + 3ull * i;
+        sx = pp[0];
+        sy = pp[1];
+        sz = pp[2];
+      }
+      const double dx = __dsub_rn(sx, ex), dy = __dsub_rn(sy, ey), dz = __dsub_rn(sz, ez);
+      const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+      v[r] = pack_key<SHIFT>(__float_as_uint(__double2float_rn(d2)), (uint32_t)s);
+      W.dist[s] = __dsqrt_rn(d2);
+      W.nid[s] = __float_as_uint(p.w);
+      if (!DEFER) cand[s] = i;
     }
   }
   warp_bitonic_striped<E>(v, lane);
@@ -1473,62 +855,33 @@ __device__ __forceinline__ void emit_query(const EmitParams& P, uint32_t t, cons
     if (lane == 31) nx = r + 1 < E ? wrap : 0xFFFFFFFFu;
     amb |= ((r << 5) | lane) + 1 < m && (nx >> SHIFT) - (v[r] >> SHIFT) <= 1u;
   }
-  const double ex = q.qi.ex, ey = q.qi.ey, ez = q.qi.ez;
-  const int inexact = *P.S.inexact;
   if (__any_sync(0xffffffffu, amb)) {
     if constexpr (DEFER) {
-      static_assert(E <= 4, "a deferred query needs spare slab entries");
-      uint32_t* spare = deferred_keys(P.slab, t, n);
-#pragma unroll
-      for (int r = 0; r < E; ++r) spare[(r << 5) | lane] = v[r];
       if (lane == 0) P.fix_list[atomicAdd(P.fix_count, 1u)] = t;
+      __syncwarp();
       return;
     } else {
 #pragma unroll
       for (int r = 0; r < E; ++r) wbuf[(r << 5) | lane] = v[r];
       __syncwarp();
-      if (lane == 0) exact_fixup_sorted(wbuf, m, SHIFT, ent, P.S, inexact, ex, ey, ez);
-      __syncwarp();
+      exact_fixup_sorted(wbuf, m, SHIFT, cand, P.S.pts, P.S.pts64, P.S.perm, inexact, ex, ey, ez, lane);
 #pragma unroll
       for (int r = 0; r < E; ++r) v[r] = wbuf[(r << 5) | lane];
-      __syncwarp();
     }
   }
+  __syncwarp();
 #pragma unroll
   for (int r = 0; r < E; ++r) {
     const int i = (r << 5) | lane;
-    const uint32_t slot = v[r] & kMask;
-    uint32_t idx;
-    if (E <= 2) {  // the entry of slot s sits in lane s % 32, register s / 32
-      idx = __shfl_sync(0xffffffffu, ids[0], slot & 31);
-      if (E == 2) {
-        const uint32_t hi = __shfl_sync(0xffffffffu, ids[E - 1], slot & 31);
-        if (slot >= 32) idx = hi;
-      }
-    } else {
-      idx = i < kk ? (uint32_t)ent[slot] : 0u;
-    }
     if (i < kk) {
-      const float4 p = __ldg(&P.S.pts[idx]);
-      double sx, sy, sz;
-      if (inexact) {
-        const double* pp = P.S.pts64 + 3ull * idx;
-        sx = pp[0];
-        sy = pp[1];
-        sz = pp[2];
-      } else {
-        sx = p.x;
-        sy = p.y;
-        sz = p.z;
-      }
-      const double dx = __dsub_rn(sx, ex), dy = __dsub_rn(sy, ey), dz = __dsub_rn(sz, ez);
-      const double dist = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz)));
-      P.sink.put(q.base + i, q.qi.qid, __float_as_uint(p.w), dist, (uint32_t)i + 1);
+      const uint32_t slot = v[r] & kMask;
+      P.sink.put(q.base + i, q.qi.qid, W.nid[slot], W.dist[slot], (uint32_t)i + 1);
     }
   }
+  __syncwarp();  // the shared memory is free again
 }
 
-// Warp per query in processing (Morton) order for the queries with at most
+// Warp per query in processing (curve) order for the queries with at most
 // 64 candidates; queries with 65..kSlab candidates are k_emit_list's, those on
 // the generic path get their rows from k_expand.
 constexpr int kEmitThreads = 256;
@@ -1538,8 +891,10 @@ constexpr int kEmitThreads = 256;
 // instead of short blocks of eight queries retiring and launching.
 constexpr int kEmitBlocksPerSm = 8;
 
-__global__ void __launch_bounds__(kEmitThreads, kEmitBlocksPerSm) k_emit(EmitParams P) {
+__global__ void __launch_bounds__(kEmitThreads, kEmitBlocksPerSm) k_emit(const __grid_constant__ EmitParams P) {
+  __shared__ EmitWarp<2> shared[kEmitThreads / 32];
   const int lane = threadIdx.x & 31;
+  EmitWarp<2>& W = shared[threadIdx.x >> 5];
   const uint32_t warps = gridDim.x * (kEmitThreads / 32);
   const uint32_t total = P.order ? P.out_hi - P.out_lo : P.nq;  // P.order: one range of output ranks
   for (uint32_t w = blockIdx.x * (kEmitThreads / 32) + (threadIdx.x >> 5); w < total; w += warps) {
@@ -1550,9 +905,9 @@ __global__ void __launch_bounds__(kEmitThreads, kEmitBlocksPerSm) k_emit(EmitPar
     const int n = (int)(meta & kQueryCountMask);
     if ((meta & (kQueryGeneric | kQueryBig)) || n == 0) continue;
     if (n <= 32)
-      emit_query<1, true>(P, t, q, n, lane, nullptr);
+      emit_query<1, true>(P, t, q, n, lane, reinterpret_cast<EmitWarp<1>&>(W), nullptr, nullptr);
     else
-      emit_query<2, true>(P, t, q, n, lane, nullptr);
+      emit_query<2, true>(P, t, q, n, lane, W, nullptr, nullptr);
   }
 }
 
@@ -1563,61 +918,358 @@ inline unsigned int emit_grid(uint64_t queries) {
   return (unsigned int)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
 
-// The queries the emit kernels queued, one warp per query: the sorted keys go
-// to shared memory, the warp runs odd-even transposition over them (the
-// pairs of one parity are disjoint, so the lanes take them in parallel)
-// re-deciding neighbours within one truncated unit exactly, until a pass
-// swaps nothing; then it writes the rows.  The queue length is read on the
-// device, so no host round trip is needed.
+// The queries the emit kernels queued (at most 128 candidates), one warp per
+// query, near ties decided in place.  The queue length is read on the device,
+// so no host round trip is needed.
 constexpr int kFixupThreads = 128;
 
-__global__ void __launch_bounds__(kFixupThreads) k_emit_fixup(EmitParams P) {
-  __shared__ uint32_t sk[kFixupThreads / 32][128];
+__global__ void __launch_bounds__(kFixupThreads) k_emit_fixup(const __grid_constant__ EmitParams P) {
+  __shared__ EmitWarp<4> shared[kFixupThreads / 32];
+  __shared__ uint32_t cands[kFixupThreads / 32][128], keys[kFixupThreads / 32][128];
   const unsigned int m = *P.fix_count;
   const unsigned int first = P.fix_begin ? *P.fix_begin : 0u;
-  const int lane = threadIdx.x & 31;
-  uint32_t* keys = sk[threadIdx.x >> 5];
-  const int inexact = *P.S.inexact;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint64_t warps = ((uint64_t)gridDim.x * blockDim.x) >> 5;
   for (uint64_t j = first + (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); j < m; j += warps) {
     const uint32_t t = P.fix_list[j];
-    const QueryInfo qi = P.qinfo[t];
-    const int n = (int)(qi.meta & kQueryCountMask);  // <= 128 for a deferred query
-    const int shift = n <= 32 ? 5 : n <= 64 ? 6 : 7;
-    const uint32_t mask = (1u << shift) - 1u;
-    const unsigned long long* ent = P.slab + slab_base(t);
-    const uint32_t* src = deferred_keys(P.slab, t, n);
-    for (int i = lane; i < n; i += 32) keys[i] = src[i];
-    __syncwarp();
-    const int kmax = query_kmax(qi.meta);
-    const int kk = n < kmax ? n : kmax;
-    const int w = exact_window_sorted(keys, n, kk, shift);  // the elements the first kk rows can come from
-    for (int pass = 0; pass < w; ++pass) {
-      bool changed = false;
-      for (int parity = 0; parity < 2; ++parity) {
-        for (int i = parity + 2 * lane; i + 1 < w; i += 64) {
-          const uint32_t a = keys[i], b = keys[i + 1];
-          if ((b >> shift) - (a >> shift) > 1u) continue;
-          if (exact_before(qi.ex, qi.ey, qi.ez, P.S.pts, P.S.pts64, P.S.perm, inexact, (uint32_t)ent[b & mask],
-                           (uint32_t)ent[a & mask])) {
-            keys[i] = b;
-            keys[i + 1] = a;
-            changed = true;
-          }
+    EmitQuery q;
+    emit_load(P, t, lane, q);
+    emit_query<4, false>(P, t, q, (int)(q.qi.meta & kQueryCountMask), lane, shared[warp], cands[warp], keys[warp]);
+  }
+}
+
+// ---- k nearest ---------------------------------------------------------------
+// k <= 64 goes through the fixed-radius machinery: a radius that holds every
+// query's k nearest is read off the points around its place on the curve,
+// the collect gathers what lies within it, and the emit sorts and keeps k.
+
+// First sorted point whose curve code is not below `code`.
+__device__ __forceinline__ uint32_t curve_position(const uint32_t* __restrict__ codes, uint32_t n, uint32_t code) {
+  uint32_t lo = 0, hi = n;
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (__ldg(&codes[mid]) < code) lo = mid + 1;
+    else hi = mid;
+  }
+  return lo;
+}
+
+// Ascending bitonic steps over a thread's registers: a full sort, or (MERGE)
+// only the last merge of a bitonic sequence.
+template <int N, bool MERGE>
+__device__ __forceinline__ void thread_bitonic(float (&v)[N]) {
+#pragma unroll
+  for (int k = MERGE ? N : 2; k <= N; k <<= 1) {
+#pragma unroll
+    for (int j = k >> 1; j > 0; j >>= 1) {
+#pragma unroll
+      for (int i = 0; i < N; ++i) {
+        const int o = i ^ j;
+        if (o > i) {
+          const bool up = (i & k) == 0 || k == N;
+          const float a = v[i], b = v[o];
+          v[i] = up ? fminf(a, b) : fmaxf(a, b);
+          v[o] = up ? fmaxf(a, b) : fminf(a, b);
         }
-        __syncwarp();
       }
-      if (!__any_sync(0xffffffffu, changed)) break;
+    }
+  }
+}
+
+// A radius that holds each query's k nearest (k <= KP): the k-th smallest FP32
+// distance among the 4 KP points around the query's place on the curve, widened
+// by the FP32 error.  One thread per query keeps the KP smallest in registers:
+// each further KP distances are sorted by a bitonic network and merged, about
+// 20 instructions per point and lane and no shared memory.  On the clustered
+// 1M x 1M sets 4 KP points bound k = 16 by 46 points on average (2 KP: 71,
+// 8 KP: 37, at twice this kernel's cost).
+template <int DIM, int KP>
+__global__ void __launch_bounds__(128) k_knn_radius(SceneView S, const uint32_t* __restrict__ scodes,
+                                                   const float4* __restrict__ qpts,
+                                                   const uint32_t* __restrict__ qorder,
+                                                   const uint32_t* __restrict__ qcodes, uint32_t nq, uint32_t k,
+                                                   const DevBands* bands, double* __restrict__ radius) {
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= nq) return;
+  const float4 q = qpts[qorder[t]];
+  const uint32_t buckets = (S.n + kBucketPoints - 1) / kBucketPoints;
+  constexpr uint32_t kWindow = KP / 2;  // buckets
+  const uint32_t at = curve_position(scodes, S.n, qcodes[t]) / kBucketPoints;
+  uint32_t b0 = at > kWindow / 2 ? at - kWindow / 2 : 0u;
+  if (b0 + kWindow > buckets) b0 = buckets > kWindow ? buckets - kWindow : 0u;
+  BucketQuery bq;
+  bq.set(q.x, q.y, q.z, 0.f);
+  float best[KP];
+#pragma unroll
+  for (int i = 0; i < KP; ++i) best[i] = INFINITY;
+  for (uint32_t w = 0; w < kWindow; w += KP / 8) {
+    float v[KP];
+#pragma unroll
+    for (int g = 0; g < KP / 8; ++g) {
+      const uint32_t b = b0 + w + g;
+      float d2[8];
+      bucket_d2<DIM>(S.bucket_pts, b < buckets ? b : buckets - 1, bq, d2);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[8 * g + j] = b < buckets ? d2[j] : INFINITY;
+    }
+    thread_bitonic<KP, false>(v);
+#pragma unroll
+    for (int i = 0; i < KP; ++i) best[i] = fminf(best[i], v[KP - 1 - i]);
+    thread_bitonic<KP, true>(best);
+  }
+  const uint32_t kk = k < S.n ? k : S.n;
+  float r2 = best[KP - 1];
+#pragma unroll
+  for (int i = 0; i < KP - 1; ++i)
+    if ((uint32_t)i + 1 == kk) r2 = best[i];
+  // 1e-22 covers squares that underflow
+  radius[t] = sqrt((double)r2) * (1.0 + (double)bands->rho) + (double)bands->e_abs + 1.0e-22;
+}
+
+// k nearest of single queries, a warp per query: the sorted list of the k best
+// lies in registers (entry l and l + 32 in lane l) under the exact order
+// (FP64 distance, id, search input index), and the walk's reach shrinks with its
+// last entry.  For the few queries whose radius holds more points than a slab
+// row (duplicates, mixed densities), and for callers without scratch.
+struct SingleParams {
+  SceneView S;
+  const float4* qpts;
+  const double* qraw;
+  int qstride;
+  const DevBands* bands;
+  uint32_t k;
+  const uint32_t* work;           // processing ranks (nullptr: every rank)
+  const unsigned int* nwork_dev;  // their number (nullptr: nwork)
+  uint32_t nwork;
+  const uint32_t* qorder;         // processing rank -> query input index
+  const double* rank_radius;      // a radius that holds the k nearest, by processing rank
+  const uint32_t* qcodes;         // without rank_radius: curve codes by processing rank
+  const uint32_t* scodes;
+  const unsigned long long* poff; // rows: first row by processing rank
+  RowSink sink;
+  uint32_t* nearest;              // instead of rows: the nearest point by query input index
+};
+
+struct SingleEntry {
+  double d;
+  uint32_t i;
+};
+__device__ __forceinline__ bool entry_before(const SceneView& S, const SingleEntry& a, const SingleEntry& b) {
+  if (a.d != b.d) return a.d < b.d;
+  if (a.i == kNone || b.i == kNone) return b.i == kNone && a.i != kNone;
+  const uint32_t na = __float_as_uint(__ldg(&S.pts[a.i].w)), nb = __float_as_uint(__ldg(&S.pts[b.i].w));
+  if (na != nb) return na < nb;
+  return __ldg(&S.perm[a.i]) < __ldg(&S.perm[b.i]);
+}
+
+__global__ void __launch_bounds__(256) k_knn_single(SingleParams P) {
+  __shared__ WalkStack stacks[256 / 32];
+  const int lane = threadIdx.x & 31;
+  const SceneView& S = P.S;
+  const uint32_t n = P.nwork_dev ? *P.nwork_dev : P.nwork;
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  const DevBands B = *P.bands;
+  const int scene_inexact = *S.inexact;
+  for (uint32_t j = (uint32_t)(((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5); j < n; j += warps) {
+    const uint32_t t = P.work ? P.work[j] : j;
+    const uint32_t qin = P.qorder ? P.qorder[t] : t;
+    const float4 q = P.qpts[qin];
+    const double* rq = P.qraw + (size_t)qin * P.qstride;
+    const double ex = rq[1], ey = rq[2], ez = P.qstride == 4 ? rq[3] : 0.0;
+    double r;
+    if (P.rank_radius) {
+      r = P.rank_radius[t];
+    } else {  // k = 1: the nearest of the 32 points around the query's place on the curve
+      const uint32_t at = curve_position(P.scodes, S.n, P.qcodes[t]);
+      uint32_t a = at > 16u ? at - 16u : 0u;
+      if (a + 32u > S.n) a = S.n > 32u ? S.n - 32u : 0u;
+      const float4 p = __ldg(&S.pts[a + (uint32_t)lane < S.n ? a + lane : a]);
+      const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+      const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+      r = sqrt((double)__uint_as_float(__reduce_min_sync(0xffffffffu, __float_as_uint(d2)))) *
+              (1.0 + (double)B.rho) + (double)B.e_abs + 1.0e-22;
+    }
+    float hi2, reach2;
+    auto set_reach = [&](double radius) {
+      const double w = radius * (1.0 + (double)B.rho) + (double)B.e_abs + 1.0e-18;
+      hi2 = fmaxf(__double2float_ru(w * w), B.floor2);
+      reach2 = __fmul_ru(hi2, 1.000001f);
+    };
+    set_reach(r);
+    SingleEntry e0{INFINITY, kNone}, e1{INFINITY, kNone};
+    const int last = (int)(P.k < S.n ? P.k : S.n) - 1;
+    walk_single(S, S.trees, q, reach2, stacks[threadIdx.x >> 5], lane, [&](uint32_t i, const float4& p, bool has) {
+      const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+      const bool pass = has && fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= hi2;
+      unsigned int m = __ballot_sync(0xffffffffu, pass);
+      if (!m) return false;
+      SingleEntry mine{INFINITY, kNone};
+      if (pass) mine = SingleEntry{__dsqrt_rn(exact_d2_at(ex, ey, ez, S.pts, S.pts64, scene_inexact, i)), i};
+      bool changed = false;
+      while (m) {
+        const int from = __ffs((int)m) - 1;
+        m &= m - 1u;
+        const SingleEntry c{__shfl_sync(0xffffffffu, mine.d, from), __shfl_sync(0xffffffffu, mine.i, from)};
+        const int pos = __popc(__ballot_sync(0xffffffffu, entry_before(S, e0, c))) +
+                        __popc(__ballot_sync(0xffffffffu, entry_before(S, e1, c)));
+        if (pos > last) continue;
+        changed = true;
+        SingleEntry u0{__shfl_up_sync(0xffffffffu, e0.d, 1), __shfl_up_sync(0xffffffffu, e0.i, 1)};
+        SingleEntry u1{__shfl_up_sync(0xffffffffu, e1.d, 1), __shfl_up_sync(0xffffffffu, e1.i, 1)};
+        const SingleEntry top{__shfl_sync(0xffffffffu, e0.d, 31), __shfl_sync(0xffffffffu, e0.i, 31)};
+        if (lane == 0) u1 = top;
+        if (lane >= pos) e0 = lane == pos ? c : u0;
+        if (lane + 32 >= pos) e1 = lane + 32 == pos ? c : u1;
+      }
+      if (changed) {
+        const double k0 = __shfl_sync(0xffffffffu, e0.d, last & 31), k1 = __shfl_sync(0xffffffffu, e1.d, last & 31);
+        const double kth = last < 32 ? k0 : k1;
+        if (kth < r) {
+          r = kth;
+          set_reach(r);
+        }
+      }
+      return false;
+    });
+    if (P.nearest) {
+      if (lane == 0) P.nearest[qin] = e0.i == kNone ? 0u : e0.i;
+      continue;
     }
     const unsigned long long base = P.poff[t];
-    for (int i = lane; i < kk; i += 32) {
-      const uint32_t idx = (uint32_t)ent[keys[i] & mask];
-      const float4 p = __ldg(&P.S.pts[idx]);
-      const double dist = __dsqrt_rn(exact_d2_at(qi.ex, qi.ey, qi.ez, P.S.pts, P.S.pts64, inexact, idx));
-      P.sink.put(base + i, qi.qid, __float_as_uint(p.w), dist, (uint32_t)i + 1);
-    }
-    __syncwarp();
+    const uint32_t qid = __float_as_uint(q.w);
+    if (lane <= last && e0.i != kNone)
+      P.sink.put(base + lane, qid, __float_as_uint(__ldg(&S.pts[e0.i].w)), e0.d, (uint32_t)lane + 1);
+    if (lane + 32 <= last && e1.i != kNone)
+      P.sink.put(base + 32 + lane, qid, __float_as_uint(__ldg(&S.pts[e1.i].w)), e1.d, (uint32_t)lane + 33);
   }
+}
+
+// The nearest point of every query (directed Hausdorff), a packet of 32
+// queries per warp.  The smallest distance among 32 points around a query's
+// place on the curve bounds its search; the warp walks what that bound reaches
+// and shrinks its reach as the lanes' bounds fall.  Points whose FP32 distances
+// are closer than the error band are ordered exactly (FP64 distance, id,
+// search input index).
+struct NearestParams {
+  SceneView S;
+  const float4* qpts;
+  const double* qraw;
+  int qstride;
+  const uint32_t* qorder;
+  const uint32_t* qcodes;
+  const uint32_t* scodes;
+  uint32_t nq;
+  const DevBands* bands;
+  uint32_t* nearest;  // by query input index
+};
+
+// Whether point i at FP32 squared distance d2 orders before the best so far.
+__device__ __forceinline__ bool nearer(const NearestParams& P, const Ctx& c, uint32_t qin, float d2, uint32_t i,
+                                       float best, uint32_t besti) {
+  if (besti == kNone) return true;
+  const float tol = key_tol(c, fmaxf(d2, best));
+  if (best - d2 > tol) return true;
+  if (d2 - best > tol) return false;
+  const double* rq = P.qraw + (size_t)qin * P.qstride;
+  return exact_before(rq[1], rq[2], P.qstride == 4 ? rq[3] : 0.0, P.S.pts, P.S.pts64, P.S.perm, c.scene_inexact, i,
+                      besti);
+}
+
+// The nearest point of one query by the whole warp (packets whose queries lie
+// far apart); everything below `bound` may order first.
+__device__ __noinline__ uint32_t nearest_alone(const NearestParams& P, const Ctx& c, uint32_t qin, float bound,
+                                               WalkStack& stack) {
+  const float4 q = P.qpts[qin];
+  float best = INFINITY, reach2 = __fmul_ru(bound, 1.000001f);
+  uint32_t besti = kNone;
+  walk_single(P.S, P.S.trees, q, reach2, stack, (int)(threadIdx.x & 31),
+              [&](uint32_t i, const float4& p, bool has) {
+                const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+                const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                for (uint32_t m = __ballot_sync(0xffffffffu, has && d2 < bound); m; m &= m - 1u) {
+                  const int from = __ffs((int)m) - 1;
+                  const float cd = __shfl_sync(0xffffffffu, d2, from);
+                  const uint32_t ci = __shfl_sync(0xffffffffu, i, from);
+                  if (!nearer(P, c, qin, cd, ci, best, besti)) continue;
+                  best = cd;
+                  besti = ci;
+                  bound = fminf(bound, best + key_tol(c, best));
+                  reach2 = __fmul_ru(bound, 1.000001f);
+                }
+                return false;
+              });
+  return besti;
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(128) k_nearest(const __grid_constant__ NearestParams P) {
+  __shared__ PacketWarp warps[128 / 32];
+  const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
+  if (!__any_sync(0xffffffffu, t < P.nq)) return;  // whole warp past the end
+  const bool valid = t < P.nq;
+  const int lane = threadIdx.x & 31;
+  const SceneView& S = P.S;
+  const uint32_t tq = valid ? t : P.nq - 1;
+  const uint32_t qin = P.qorder[tq];
+  const float4 q = P.qpts[qin];
+  const DevBands B = *P.bands;
+  Ctx c;
+  c.scene_inexact = *S.inexact;
+  c.rho = B.rho;
+  c.e_abs = B.e_abs;
+  c.floor2 = B.floor2;
+  BucketQuery bq;
+  bq.set(q.x, q.y, q.z, 0.f);
+  const uint32_t buckets = (S.n + kBucketPoints - 1) / kBucketPoints;
+  const uint32_t at = curve_position(P.scodes, S.n, P.qcodes[tq]) / kBucketPoints;
+  uint32_t b0 = at > 2u ? at - 2u : 0u;
+  if (b0 + 4u > buckets) b0 = buckets > 4u ? buckets - 4u : 0u;
+  float best = INFINITY;
+  for (uint32_t w = b0; w < b0 + 4u && w < buckets; ++w) {
+    float d2[8];
+    bucket_d2<DIM>(S.bucket_pts, w, bq, d2);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) best = fminf(best, d2[j]);
+  }
+  uint32_t besti = kNone;
+  float bound = best + key_tol(c, best);  // what may still order first lies below it
+  bq.nd = pack2(-bound);
+  WalkStack& stack = warps[threadIdx.x >> 5].stack;
+  cut_packet(
+      S, S.trees, q, __fmul_ru(bound, 1.000001f), true, valid, stack, lane,
+      [&](bool mine, const PacketBox& box, const PacketBox* limit, float reach2) {
+        bq.nd = pack2(mine ? -bound : INFINITY);  // no candidates for the other lanes
+        walk_fours(S, S.trees, box, limit, reach2, stack, warps[threadIdx.x >> 5].list, lane, 4u,
+                   [&](const uint4& four) {
+                     uint32_t hits = buckets_mask<DIM, false>(S.bucket_pts, four, bq, nullptr);
+                     for (; hits; hits &= hits - 1u) {
+                       const int j = __ffs((int)hits) - 1;
+                       const uint32_t b = j < 8 ? four.x : j < 16 ? four.y : j < 24 ? four.z : four.w;
+                       const uint32_t i = b * kBucketPoints + (j & 7);
+                       const float4 p = __ldg(&S.pts[i]);
+                       const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+                       const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                       if (nearer(P, c, qin, d2, i, best, besti)) {
+                         best = d2;
+                         besti = i;
+                         bound = fminf(bound, best + key_tol(c, best));
+                         bq.nd = pack2(-bound);
+                       }
+                     }
+                     reach2 = __uint_as_float(__reduce_max_sync(
+                         0xffffffffu, __float_as_uint(mine ? __fmul_ru(bound, 1.000001f) : 0.f)));
+                     return false;
+                   });
+      },
+      [&](uint32_t run) {
+        for (; run; run &= run - 1u) {
+          const int from = __ffs((int)run) - 1;
+          const uint32_t i = nearest_alone(P, c, __shfl_sync(0xffffffffu, qin, from),
+                                           __shfl_sync(0xffffffffu, bound, from), stack);
+          if (lane == from) besti = i;
+        }
+      });
+  if (valid) P.nearest[qin] = besti == kNone ? 0u : besti;
 }
 
 // ---- ranked summaries ----------------------------------------------------------
@@ -1689,7 +1341,29 @@ __device__ __forceinline__ bool group_box_ok(const CountParams& P, const SceneVi
   return __dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)) <= r2;
 }
 
-__global__ void __launch_bounds__(256) k_count_packet(CountParams P) {
+// The count of one query by the whole warp (packets whose queries lie far apart).
+__device__ __noinline__ uint32_t count_alone(const CountParams& P, const DevBands& B, int scene_inexact, uint32_t qin,
+                                             WalkStack& stack) {
+  const SceneView& S = P.S;
+  const float4 q = P.qpts[qin];
+  const double* rq = P.qraw + (size_t)qin * P.qstride;
+  uint32_t count = 0;
+  walk_single(S, S.trees, q, B.box_hi2, stack, (int)(threadIdx.x & 31), [&](uint32_t i, const float4& p, bool has) {
+    const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
+    const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+    bool hit = has && d2 <= B.hi2;
+    if (hit && d2 >= B.lo2)
+      hit = exact_d2_at(rq[1], rq[2], P.qstride == 4 ? rq[3] : 0.0, S.pts, S.pts64, scene_inexact, i) <= B.r2;
+    if (hit && P.group_of) hit = group_box_ok(P, S, qin, i, B.r2);
+    count += __popc(__ballot_sync(0xffffffffu, hit));
+    return P.threshold != 0u && count >= P.threshold;
+  });
+  return P.threshold != 0u && count > P.threshold ? P.threshold : count;
+}
+
+template <int DIM>
+__global__ void __launch_bounds__(128) k_count_packet(const __grid_constant__ CountParams P) {
+  __shared__ PacketWarp warps[128 / 32];
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (!__any_sync(0xffffffffu, t < P.nq)) return;  // whole warp past the end
   const bool valid = t < P.nq;
@@ -1697,7 +1371,7 @@ __global__ void __launch_bounds__(256) k_count_packet(CountParams P) {
   const SceneView& S = P.S;
   const int scene_inexact = *S.inexact;
   uint32_t qin = 0;
-  float4 q = make_float4(INFINITY, INFINITY, INFINITY, 0.f);  // never overlaps
+  float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
   if (valid) {
     qin = P.qorder[t];
     q = P.qpts[qin];
@@ -1705,41 +1379,47 @@ __global__ void __launch_bounds__(256) k_count_packet(CountParams P) {
   const uint32_t thr = P.threshold;
   uint32_t count = 0;
   bool active = valid;
-  int cur = S.n > 0 ? 0 : kRopeEnd;
-  while (cur != kRopeEnd) {
-    const float4 a = __ldg(&S.nodes[2 * cur]), b = __ldg(&S.nodes[2 * cur + 1]);
-    const int hit = __float_as_int(a.w);
-    const bool over = active && box_d2(q.x, q.y, q.z, a, b) <= B.box_hi2;
-    if (__any_sync(0xffffffffu, over)) {
-      if (hit >= 0) {
-        ++cur;  // internal node: its left child is the next record
-        continue;
-      }
-      const int first = leaf_first(hit), cnt = leaf_count(hit);
-      bool test = over;
-      for (int i = first; i < first + cnt; ++i) {
-        const float4 p = __ldg(&S.pts[i]);
-        if (!test) continue;
-        const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-        const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-        if (d2 > B.hi2) continue;
-        if (d2 >= B.lo2) {
-          const double* rq = P.qraw + (size_t)qin * P.qstride;
-          const double e2 = exact_d2_at(rq[1], rq[2], P.qstride == 4 ? rq[3] : 0.0, S.pts, S.pts64, scene_inexact,
-                                        (uint32_t)i);
-          if (e2 > B.r2) continue;
+  const int lane = threadIdx.x & 31;
+  const TreeShape* T = S.trees;
+  const uint32_t bucket0 = __ldg(&T->base[0]);
+  BucketQuery bq;
+  bq.set(q.x, q.y, q.z, B.top);
+  const int band = valid ? (int)(0x80000001u + __float_as_uint(B.width)) : (int)0x80000000;
+  const float reach2 = B.box_hi2;
+  WalkStack& stack = warps[threadIdx.x >> 5].stack;
+  cut_packet(
+      S, T, q, reach2, false, valid, stack, lane,
+      [&](bool mine, const PacketBox& box, const PacketBox*, float reach) {
+        walk_fours(S, T, box, nullptr, reach, stack, warps[threadIdx.x >> 5].list, lane, 32u, [&](const uint4& four) {
+          int near;
+          uint32_t hits = buckets_mask<DIM, true>(S.bucket_pts, four, bq, &near);
+          if (near < band)
+            hits = exact_buckets_mask(S.pts, S.pts64, scene_inexact, P.qraw + (size_t)qin * P.qstride, P.qstride,
+                                      B.r2, four, S.slots / kBucketPoints);
+          if (!mine || !active) hits = 0;
+          if (P.group_of) {
+            for (uint32_t h = hits; h; h &= h - 1u) {
+              const int i = __ffs((int)h) - 1;
+              const uint32_t b = i < 8 ? four.x : i < 16 ? four.y : i < 24 ? four.z : four.w;
+              if (!group_box_ok(P, S, qin, b * kBucketPoints + (i & 7), B.r2)) hits &= ~(1u << i);
+            }
+          }
+          count += __popc(hits);
+          if (thr == 0u) return false;
+          if (count >= thr) {  // the count stops at the threshold
+            count = thr;
+            active = false;
+          }
+          return !__any_sync(0xffffffffu, mine && active);  // every query of the run reached its threshold
+        });
+      },
+      [&](uint32_t run) {
+        for (; run; run &= run - 1u) {
+          const int from = __ffs((int)run) - 1;
+          const uint32_t c = count_alone(P, B, scene_inexact, __shfl_sync(0xffffffffu, qin, from), stack);
+          if (lane == from) count = c;
         }
-        if (P.group_of && !group_box_ok(P, S, qin, (uint32_t)i, B.r2)) continue;
-        ++count;
-        if (thr != 0u && count >= thr) {
-          active = false;
-          test = false;
-        }
-      }
-      if (!__any_sync(0xffffffffu, active)) break;  // every query of the warp reached its threshold
-    }
-    cur = __float_as_int(b.w);
-  }
+      });
   const bool reached = valid && thr != 0u && count >= thr;
   if (valid) {
     const uint32_t id = __float_as_uint(q.w);
@@ -1757,7 +1437,8 @@ __global__ void __launch_bounds__(256) k_count_packet(CountParams P) {
 // Point groups: the nearest point within radius whose group box is also within
 // radius, by exact FP64 distance then smaller id (rtdl_optix_core.cpp:6215-6306);
 // one row per query at its input index, 0xFFFFFFFF / FLT_MAX when none.
-__global__ void __launch_bounds__(256) k_group_nearest_packet(CountParams P, RtdlFixedRadiusNeighborRow* rows) {
+__global__ void __launch_bounds__(128) k_group_nearest_packet(const __grid_constant__ CountParams P, RtdlFixedRadiusNeighborRow* rows) {
+  __shared__ PacketWarp warps[128 / 32];
   const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;
   if (!__any_sync(0xffffffffu, t < P.nq)) return;  // whole warp past the end
   const bool valid = t < P.nq;
@@ -1765,7 +1446,7 @@ __global__ void __launch_bounds__(256) k_group_nearest_packet(CountParams P, Rtd
   const SceneView& S = P.S;
   const int scene_inexact = *S.inexact;
   uint32_t qin = 0;
-  float4 q = make_float4(INFINITY, INFINITY, INFINITY, 0.f);
+  float4 q = make_float4(0.f, 0.f, 0.f, 0.f);
   if (valid) {
     qin = P.qorder[t];
     q = P.qpts[qin];
@@ -1773,37 +1454,74 @@ __global__ void __launch_bounds__(256) k_group_nearest_packet(CountParams P, Rtd
   double best = 0.0;
   uint32_t best_id = 0xFFFFFFFFu;
   bool found = false;
-  int cur = S.n > 0 ? 0 : kRopeEnd;
-  while (cur != kRopeEnd) {
-    const float4 a = __ldg(&S.nodes[2 * cur]), b = __ldg(&S.nodes[2 * cur + 1]);
-    const int hit = __float_as_int(a.w);
-    const bool over = valid && box_d2(q.x, q.y, q.z, a, b) <= B.box_hi2;
-    if (__any_sync(0xffffffffu, over)) {
-      if (hit >= 0) {
-        ++cur;
-        continue;
-      }
-      const int first = leaf_first(hit), cnt = leaf_count(hit);
-      for (int i = first; i < first + cnt; ++i) {
-        const float4 p = __ldg(&S.pts[i]);
-        if (!over) continue;
-        const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
-        if (fmaf(dz, dz, fmaf(dy, dy, dx * dx)) > B.hi2) continue;
-        const double* rq = P.qraw + (size_t)qin * P.qstride;
-        const double e2 = exact_d2_at(rq[1], rq[2], P.qstride == 4 ? rq[3] : 0.0, S.pts, S.pts64, scene_inexact,
-                                      (uint32_t)i);
-        if (e2 > B.r2) continue;
-        if (P.group_of && !group_box_ok(P, S, qin, (uint32_t)i, B.r2)) continue;
-        const uint32_t id = __float_as_uint(p.w);
-        if (!found || e2 < best || (e2 == best && id < best_id)) {
-          best = e2;
-          best_id = id;
-          found = true;
+  const int lane = threadIdx.x & 31;
+  const TreeShape* T = S.trees;
+  const uint32_t bucket0 = __ldg(&T->base[0]);
+  BucketQuery bq;
+  bq.set(q.x, q.y, q.z, B.top);  // every point that may be within radius, decided below
+  const float reach2 = B.box_hi2;
+  WalkStack& stack = warps[threadIdx.x >> 5].stack;
+  cut_packet(
+      S, T, q, reach2, false, valid, stack, lane,
+      [&](bool mine, const PacketBox& box, const PacketBox*, float reach) {
+        walk_fours(S, T, box, nullptr, reach, stack, warps[threadIdx.x >> 5].list, lane, 32u, [&](const uint4& four) {
+          uint32_t hits = buckets_mask<2, false>(S.bucket_pts, four, bq, nullptr);
+          if (!mine) hits = 0;
+          for (; hits; hits &= hits - 1u) {
+            const int j = __ffs((int)hits) - 1;
+            const uint32_t b = j < 8 ? four.x : j < 16 ? four.y : j < 24 ? four.z : four.w;
+            const uint32_t i = b * kBucketPoints + (j & 7);
+            const double* rq = P.qraw + (size_t)qin * P.qstride;
+            const double e2 = exact_d2_at(rq[1], rq[2], 0.0, S.pts, S.pts64, scene_inexact, i);
+            if (e2 > B.r2) continue;
+            if (P.group_of && !group_box_ok(P, S, qin, i, B.r2)) continue;
+            const uint32_t id = __float_as_uint(__ldg(&S.pts[i].w));
+            if (!found || e2 < best || (e2 == best && id < best_id)) {
+              best = e2;
+              best_id = id;
+              found = true;
+            }
+          }
+          return false;
+        });
+      },
+      [&](uint32_t run) {  // one query at a time, the lanes over its points
+        for (; run; run &= run - 1u) {
+          const int from = __ffs((int)run) - 1;
+          const uint32_t one = __shfl_sync(0xffffffffu, qin, from);
+          const float4 q1 = P.qpts[one];
+          const double* rq = P.qraw + (size_t)one * P.qstride;
+          double d = INFINITY;
+          uint32_t id = 0xFFFFFFFFu;
+          walk_single(S, T, q1, reach2, stack, lane, [&](uint32_t i, const float4& p, bool has) {
+            const float dx = p.x - q1.x, dy = p.y - q1.y;
+            if (has && fmaf(dy, dy, dx * dx) <= B.hi2) {
+              const double e2 = exact_d2_at(rq[1], rq[2], 0.0, S.pts, S.pts64, scene_inexact, i);
+              const uint32_t pid = __float_as_uint(p.w);
+              if (e2 <= B.r2 && (!P.group_of || group_box_ok(P, S, one, i, B.r2)) &&
+                  (e2 < d || (e2 == d && pid < id))) {
+                d = e2;
+                id = pid;
+              }
+            }
+            return false;
+          });
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            const double od = __shfl_xor_sync(0xffffffffu, d, o);
+            const uint32_t oid = __shfl_xor_sync(0xffffffffu, id, o);
+            if (od < d || (od == d && oid < id)) {
+              d = od;
+              id = oid;
+            }
+          }
+          if (lane == from && d < INFINITY) {
+            best = d;
+            best_id = id;
+            found = true;
+          }
         }
-      }
-    }
-    cur = __float_as_int(b.w);
-  }
+      });
   if (valid)
     rows[qin] = RtdlFixedRadiusNeighborRow{__float_as_uint(q.w), found ? best_id : 0xFFFFFFFFu,
                                            found ? __dsqrt_rn(best) : 3.4028234663852886e38};
@@ -1950,7 +1668,9 @@ template <int E, bool DEFER>
 // nwork_dev non-null (captured graphs): the list length is read there and the
 // warps stride over the list.
 __global__ void __launch_bounds__(kEmitListThreads)
-    k_emit_list(EmitParams P, const uint32_t* work, uint32_t nwork, const unsigned int* nwork_dev) {
+    k_emit_list(const __grid_constant__ EmitParams P, const uint32_t* work, uint32_t nwork, const unsigned int* nwork_dev) {
+  __shared__ EmitWarp<E> shared[kEmitListThreads / 32];
+  __shared__ uint32_t cands[DEFER ? 1 : kEmitListThreads / 32][DEFER ? 1 : 32 * E];
   __shared__ uint32_t wbuf[DEFER ? 1 : kEmitListThreads / 32][DEFER ? 1 : 32 * E];
   const int lane = threadIdx.x & 31;
   if (nwork_dev) nwork = *nwork_dev;
@@ -1965,7 +1685,8 @@ __global__ void __launch_bounds__(kEmitListThreads)
     EmitQuery q;
     emit_load(P, t, lane, q);
     const int n = (int)(q.qi.meta & kQueryCountMask);
-    emit_query<E, DEFER>(P, t, q, n, lane, DEFER ? nullptr : wbuf[threadIdx.x >> 5]);
+    emit_query<E, DEFER>(P, t, q, n, lane, shared[threadIdx.x >> 5], DEFER ? nullptr : cands[threadIdx.x >> 5],
+                         DEFER ? nullptr : wbuf[threadIdx.x >> 5]);
   }
 }
 
@@ -2025,25 +1746,30 @@ __global__ void k_chunk_rows(const unsigned long long* offsets, uint32_t nq, int
 // The next range's fix-ups start after this range's.
 __global__ void k_fix_advance(unsigned int* fix_begin, const unsigned int* fix_count) { *fix_begin = *fix_count; }
 
-__global__ void k_fill_i32(int* out, uint32_t n, int v) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) out[i] = v;
-}
-
 // Problem batch: *flag stays nonzero while every problem's query ids ascend.
 __global__ void k_batch_ids_sorted(const float4* qpts, const uint32_t* qprob, uint32_t n, unsigned int* flag) {
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x + 1; i < n; i += (uint64_t)gridDim.x * blockDim.x)
     if (qprob[i] == qprob[i - 1] && __float_as_uint(qpts[i].w) < __float_as_uint(qpts[i - 1].w)) *flag = 0u;
 }
 
-// Problem batch: one block per problem copies its sorted queries to the padded
-// processing order (kNone fills the last warp) and records each warp's problem.
-__global__ void k_batch_pad(const unsigned long long* qoff, const unsigned long long* pstart, const uint32_t* sorted,
-                            uint32_t* qorder, uint32_t* warp_prob) {
-  const uint32_t p = blockIdx.x;
-  const unsigned long long a = qoff[p], nqp = qoff[p + 1] - a, base = pstart[p], padded = pstart[p + 1] - base;
-  for (unsigned long long j = threadIdx.x; j < padded; j += blockDim.x) {
-    qorder[base + j] = j < nqp ? sorted[a + j] : kNone;
-    if ((j & 31) == 0) warp_prob[(base + j) >> 5] = p;
+// Problem batch: the sorted queries into the padded processing order (kNone
+// fills a problem's last warp) and each warp's problem.  A thread per rank
+// finds its problem by bisection (the same one for a whole warp); a block per
+// problem left one block copying the largest problem alone (0.51 ms for the 128
+// problems of 6M queries).
+__global__ void k_batch_pad(const unsigned long long* qoff, const unsigned long long* pstart, uint32_t problems,
+                            uint32_t np, const uint32_t* sorted, uint32_t* qorder, uint32_t* warp_prob) {
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < np; t += gridDim.x * blockDim.x) {
+    uint32_t lo = 0, hi = problems;  // first problem that starts after t
+    while (lo < hi) {
+      const uint32_t mid = (lo + hi) >> 1;
+      if (__ldg(&pstart[mid]) <= t) lo = mid + 1;
+      else hi = mid;
+    }
+    const uint32_t p = lo - 1;
+    const unsigned long long j = qoff[p] + (t - pstart[p]);
+    qorder[t] = j < qoff[p + 1] ? sorted[j] : kNone;
+    if ((t & 31u) == 0) warp_prob[t >> 5] = p;
   }
 }
 
@@ -2156,13 +1882,14 @@ __global__ void __launch_bounds__(kHeavyThreads)
 }
 
 // Generic-path gather for a radius query with more than kSlab candidates: one
-// warp per query walks the BVH with a warp-uniform stack; the lanes test a leaf
+// warp per query walks the tree; the lanes test the reached
 // bucket's points together and append in-radius candidates with a ballot
 // prefix (no atomics).
 __global__ void __launch_bounds__(32)
     k_heavy_gather_bvh(SceneView S, const float4* qpts, const double* qraw, int qstride, const uint32_t* heavy_list,
                        const unsigned long long* seg_off, const uint32_t* seg_size, const DevBands* bands,
                        const uint32_t* qprob, const double* item_rad, HeavyEntry* scratch, unsigned int* error) {
+  __shared__ WalkStack stack;
   const int lane = threadIdx.x;
   const uint32_t h = blockIdx.x;
   const uint32_t qin = heavy_list[h];
@@ -2174,45 +1901,28 @@ __global__ void __launch_bounds__(32)
   const uint32_t P2 = seg_size[h];
   const unsigned int lt_mask = (1u << lane) - 1u;
   uint32_t cnt = 0;
-  int cur = S.n > 0 ? 0 : kRopeEnd, end = kRopeEnd;
-  if (S.prob_root) {  // problem batch: the query's problem subtree only
-    cur = S.prob_root[prob];
-    if (cur != kRopeEnd) end = __float_as_int(__ldg(&S.nodes[2 * cur + 1]).w);
-  }
-  while (cur != end) {  // warp-uniform: every lane follows the same nodes
-    const float4 a = __ldg(&S.nodes[2 * cur]), b = __ldg(&S.nodes[2 * cur + 1]);
-    const int hit = __float_as_int(a.w);
-    if (box_d2(c.qx, c.qy, c.qz, a, b) <= B.box_hi2) {
-      if (hit >= 0) {
-        ++cur;  // internal node: its left child is the next record
-        continue;
-      }
-      const int first = leaf_first(hit), leaf = leaf_count(hit);
-      bool acc = false;
-      const uint32_t i = (uint32_t)(first + lane);
-      if (lane < leaf) {
-        const float4 p = __ldg(&S.pts[i]);
-        const float dx = p.x - c.qx, dy = p.y - c.qy, dz = p.z - c.qz;
-        const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-        acc = d2 <= B.hi2 && (d2 < B.lo2 || exact_d2(c, i) <= B.r2);
-      }
-      const unsigned int m = __ballot_sync(0xffffffffu, acc);
-      if (acc) {
-        const uint32_t pos = cnt + __popc(m & lt_mask);
-        if (pos < P2) {
-          HeavyEntry en;
-          en.key = (unsigned long long)__double_as_longlong(__dsqrt_rn(exact_d2(c, i)));
-          en.nid = __float_as_uint(__ldg(&S.pts[i].w));
-          en.sidx = i;
-          seg[pos] = en;
-        } else {
-          atomicOr(error, 2u);
-        }
-      }
-      cnt += __popc(m);
-    }
-    cur = __float_as_int(b.w);
-  }
+  const float4 q = make_float4(c.qx, c.qy, c.qz, 0.f);
+  walk_single(S, S.trees + prob * S.tree_stride, q, B.box_hi2, stack, lane,
+              [&](uint32_t i, const float4& p, bool has) {
+                const float dx = p.x - c.qx, dy = p.y - c.qy, dz = p.z - c.qz;
+                const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
+                const bool acc = has && d2 <= B.hi2 && (d2 < B.lo2 || exact_d2(c, i) <= B.r2);
+                const unsigned int m = __ballot_sync(0xffffffffu, acc);
+                if (acc) {
+                  const uint32_t pos = cnt + __popc(m & lt_mask);
+                  if (pos < P2) {
+                    HeavyEntry en;
+                    en.key = (unsigned long long)__double_as_longlong(__dsqrt_rn(exact_d2(c, i)));
+                    en.nid = __float_as_uint(p.w);
+                    en.sidx = i;
+                    seg[pos] = en;
+                  } else {
+                    atomicOr(error, 2u);
+                  }
+                }
+                cnt += __popc(m);
+                return false;
+              });
   for (uint32_t i = cnt + lane; i < P2; i += 32) {
     HeavyEntry en;
     en.key = ~0ull;
@@ -2301,13 +2011,10 @@ struct ExpandParams {
   const uint32_t* qrank;      // with work_list: input index -> output rank
 };
 
-// G consecutive threads per query (G = 32: a warp) write its rows with the
-// exact FP64 distance: all queries in output order, or the queries of
-// `work_list`.  G is at least the longest row list when it is known to be
-// short (nearest lists of k <= 16 rows), so a warp serves 32 / G queries and
-// their rows, consecutive in output order, with one set of stores.
-template <int G>
+// A warp per query writes its rows with the exact FP64 distance: all queries
+// in output order, or the queries of `work_list` (generic path).
 __global__ void __launch_bounds__(kExpandThreads) k_expand(ExpandParams P) {
+  constexpr int G = 32;
   const int lane = threadIdx.x & (G - 1);
   const uint64_t groups = ((uint64_t)gridDim.x * blockDim.x) / G;
   const bool ids_sorted = P.bands->ids_sorted != 0;
@@ -2327,7 +2034,7 @@ __global__ void __launch_bounds__(kExpandThreads) k_expand(ExpandParams P) {
                                      : P.temp + (size_t)qin * P.L;
     for (uint32_t s = lane; s < cnt; s += G) {
       const uint32_t sidx = src[s];
-      if (sidx >= P.S.n) {  // never expected: a generic-path slot without a candidate
+      if (sidx >= P.S.slots) {  // never expected: a generic-path slot without a candidate
         atomicOr(P.error, 4u);
         continue;
       }
@@ -2461,7 +2168,6 @@ struct Readback {
   unsigned int scene_bad;
   unsigned int query_bad;
   unsigned int fixups;
-  unsigned int refine_left;  // heavy queries still unresolved after a refinement pass
   unsigned long long chunk_rows[kDownloadChunks + 1];  // first row of each download range
 };
 
@@ -2541,7 +2247,7 @@ struct QueryPrep {
   float4* qpts = nullptr;
   DevBands* bands = nullptr;   // one, or one per problem of a batch
   uint32_t* qorder = nullptr;  // processing rank -> input index (a batch pads problems to whole warps: kNone)
-  uint32_t* qcodes = nullptr;  // Morton codes in processing order (qcodes[t] belongs to qorder[t]); single only
+  uint32_t* qcodes = nullptr;  // curve codes in processing order (qcodes[t] belongs to qorder[t]); single only
   uint32_t* oorder = nullptr;
   uint32_t nproc = 0;          // processing ranks
   const unsigned int* order_identity = nullptr;  // device flag: output order == input order
@@ -2552,7 +2258,6 @@ struct QueryPrep {
   unsigned int* sorted_flag = nullptr;
   unsigned long long* qoff = nullptr;  // device copy of the query offsets
   double* prob_radius = nullptr;       // radius of each problem
-  int* shared_roots = nullptr;         // requests against one plain scene: every problem's root is the scene's
   SceneView view{};                    // the scene as the traversal kernels see it
   const PreparedQueries* borrowed = nullptr;  // set: the query-side buffers belong to a prepared query set
 };
@@ -2592,7 +2297,7 @@ QueryPrep prepare_queries(Scene* sc, const void* queries_dev, uint32_t nq, bool 
   qp.order_identity = &qp.bands->ids_sorted;
   qp.view = sc->view();
   qp.qcodes = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq, s));
-  morton_codes(qp.qpts, nq, sc->dim, sc->stats, qp.qcodes, s);
+  curve_codes(qp.qpts, nq, sc->dim, sc->stats, qp.qcodes, s);
   iota_u32(qp.qorder, nq, s);
   radix_sort_pairs(qp.qcodes, qp.qorder, nq, 0, sc->dim == 3 ? 30 : 32, nullptr, &qp.qst->bad, s);
   if (want_output_order) {
@@ -2608,7 +2313,7 @@ QueryPrep prepare_queries(Scene* sc, const void* queries_dev, uint32_t nq, bool 
 }
 
 // A problem batch's query preparation: per-query problem ids, per-problem
-// bands and kmax, composite (problem, Morton) sort, processing order padded
+// bands and kmax, composite (problem, curve) sort, processing order padded
 // so each warp holds queries of one problem, and the output order (problem,
 // then query id, stable).
 QueryPrep prepare_queries_batch(Scene* sc, const void* queries_dev, uint32_t nq, const BatchSpec& bs,
@@ -2617,12 +2322,6 @@ QueryPrep prepare_queries_batch(Scene* sc, const void* queries_dev, uint32_t nq,
   QueryPrep qp;
   const bool shared = sc->problems == 0;  // several requests against one plain scene
   qp.view = sc->view();
-  if (shared) {
-    qp.shared_roots = static_cast<int*>(dev_alloc(sizeof(int) * P, s));
-    k_fill_i32<<<div_up(P, 256), 256, 0, s>>>(qp.shared_roots, P, sc->n > 0 ? 0 : kRopeEnd);
-    RTDL_LAUNCHED(1);
-    qp.view.prob_root = qp.shared_roots;
-  }
   std::vector<unsigned long long> pstart(P + 1, 0);
   for (uint32_t p = 0; p < P; ++p) pstart[p + 1] = pstart[p] + (bs.qoff[p + 1] - bs.qoff[p] + 31) / 32 * 32;
   if (pstart[P] > 0xFFFFFFFFull - 32) throw std::runtime_error("problem batch has too many queries");
@@ -2655,7 +2354,7 @@ QueryPrep prepare_queries_batch(Scene* sc, const void* queries_dev, uint32_t nq,
   }
   k_bands_batch<<<div_up(P, 128), 128, 0, s>>>(sc->stats, qp.qst, d_radius, P, qp.sorted_flag, qp.bands);
   RTDL_LAUNCHED(1);
-  // processing order: composite (problem, Morton in the problem's box) sort, padded per problem
+  // processing order: composite (problem, curve in the problem's box) sort, padded per problem
   uint32_t* codes = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * (nq ? nq : 1), s));
   uint32_t* sorted = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * (nq ? nq : 1), s));
   if (shared)
@@ -2664,7 +2363,7 @@ QueryPrep prepare_queries_batch(Scene* sc, const void* queries_dev, uint32_t nq,
     batch_codes(qp.qpts, qp.qprob, nq, sc->dim, sc->prob_stats, 1, sc->code_bits, codes, s);
   iota_u32(sorted, nq, s);
   radix_sort_pairs(codes, sorted, nq, 0, 32, nullptr, &qp.qst->bad, s);
-  k_batch_pad<<<P, 256, 0, s>>>(qp.qoff, d_pstart, sorted, qp.qorder, qp.warp_prob);
+  k_batch_pad<<<grid_for(qp.nproc, 256), 256, 0, s>>>(qp.qoff, d_pstart, P, qp.nproc, sorted, qp.qorder, qp.warp_prob);
   RTDL_LAUNCHED(1);
   // output order: by query id, then (stable) by problem; skipped when every
   // problem's ids are already ascending
@@ -2698,7 +2397,6 @@ void free_prep(QueryPrep& qp, cudaStream_t s) {
   dev_free(qp.prob_kmax, s);
   dev_free(qp.sorted_flag, s);
   dev_free(qp.qoff, s);
-  dev_free(qp.shared_roots, s);
   dev_free(qp.prob_radius, s);
 }
 
@@ -2775,236 +2473,60 @@ GenericOut run_generic_path(Scene* sc, const QueryPrep& qp, const void* queries_
   return g;
 }
 
-// Host side of the radius refinement (see k_collect_refine): up to kRefinePasses
-// passes over the unresolved heavy queries, each followed by an update that
-// resolves queries or narrows their radius; after the last pass the
-// unresolved ones are listed for the generic path.
-constexpr int kRefinePasses = 6;
+// Calls of at most this many queries collect a warp per query (32 warps on
+// every SM); above it packets fill the GPU.
+constexpr uint32_t kSingleQueries = kSmCount * 32;
 
-struct RefineOut {
-  uint32_t generic = 0, mid = 0, big = 0;
-  const uint32_t* generic_qin = nullptr;
-  const uint32_t* generic_m = nullptr;
-  const double* generic_rad = nullptr;  // the radius each generic query gathers within
-  std::vector<void*> buffers;  // released by the caller once the rows are out
-};
-
-RefineOut refine_heavy(const CollectParams& C, const QueryPrep& qp, double radius, uint32_t kmax, uint32_t H,
-                       const uint32_t* heavy_list, const uint32_t* heavy_m, const uint32_t* heavy_t,
-                       QueryInfo* qinfo, uint8_t* flags, uint32_t* mid_list, uint32_t* big_list, unsigned int* small,
-                       cudaStream_t s, const std::function<void()>& after_first_pass = {}) {
-  RefineOut out;
-  auto alloc = [&](size_t bytes) {
-    void* p = dev_alloc(bytes ? bytes : 1, s);
-    out.buffers.push_back(p);
-    return p;
-  };
-  uint32_t* work[2];
-  double *rad[2], *lo[2], *hi[2], *frad[2];
-  uint32_t* full[2];
-  for (int b = 0; b < 2; ++b) {
-    work[b] = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * H));
-    rad[b] = static_cast<double*>(alloc(sizeof(double) * H));
-    lo[b] = static_cast<double*>(alloc(sizeof(double) * H));
-    hi[b] = static_cast<double*>(alloc(sizeof(double) * H));
-    full[b] = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * H));
-    frad[b] = static_cast<double*>(alloc(sizeof(double) * H));
-  }
-  double* gen_rad = static_cast<double*>(alloc(sizeof(double) * H));
-  uint32_t* cnt = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * H));
-  uint32_t* gen_qin = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * H));
-  uint32_t* gen_m = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * H));
-  unsigned int* next_count = static_cast<unsigned int*>(alloc(sizeof(unsigned int)));
-  k_refine_init<<<div_up(H, 256), 256, 0, s>>>(heavy_list, heavy_m, heavy_t, H, qp.qprob, qp.prob_radius, radius,
-                                               qp.prob_kmax, kmax, work[0], rad[0], lo[0], hi[0], full[0],
-                                               frad[0], nullptr);
-  RTDL_LAUNCHED(1);
-  Readback* rb = pinned_readback();
-  uint32_t n = H;
-  int cur = 0;
-  for (int pass = 0; pass < kRefinePasses && n > 0; ++pass) {
-    const bool last = pass == kRefinePasses - 1;
-
-    RefineParams R;
-    R.C = C;
-    R.qprob = qp.qprob;
-    R.work = work[cur];
-    R.rad = rad[cur];
-    R.nwork = n;
-    R.cnt = cnt;
-    R.nwork_dev = nullptr;
-    R.packet_min = 0;
-    const bool scene_packet = n >= qp.nproc / 8 && !qp.qprob && !qp.view.prob_root;
-    if (n >= qp.nproc / 8) {  // many heavy queries: they cluster, a packet of them walks one region
-      if (scene_packet)
-        k_collect_refine_packet_scene<<<div_up(n, 256), 256, 0, s>>>(R);
-      else
-        k_collect_refine_packet<<<div_up(n, 256), 256, 0, s>>>(R);
-    } else
-      k_collect_refine<<<div_up((uint64_t)n * 32, 256), 256, 0, s>>>(R);
-    RTDL_CUDA_CHECK(cudaMemsetAsync(next_count, 0, sizeof(unsigned int), s));
-    RefineUpdate U;
-    U.qorder = qp.qorder;
-    U.qprob = qp.qprob;
-    U.prob_kmax = qp.prob_kmax;
-    U.kmax = kmax;
-    U.qinfo = qinfo;
-    U.flags = flags;
-    U.mid_list = mid_list;
-    U.big_list = big_list;
-    U.small = small;
-    U.work = work[cur];
-    U.rad = rad[cur];
-    U.lo = lo[cur];
-    U.hi = hi[cur];
-    U.full = full[cur];
-    U.frad = frad[cur];
-    U.cnt = cnt;
-    U.nwork = n;
-    U.nwork_dev = nullptr;
-    U.next_work = work[cur ^ 1];
-    U.next_rad = rad[cur ^ 1];
-    U.next_lo = lo[cur ^ 1];
-    U.next_hi = hi[cur ^ 1];
-    U.next_full = full[cur ^ 1];
-    U.next_frad = frad[cur ^ 1];
-    U.next_count = next_count;
-    U.generic_qin = gen_qin;
-    U.generic_m = gen_m;
-    U.generic_rad = gen_rad;
-    U.last = last ? 1 : 0;
-    k_refine_update<<<div_up(n, 256), 256, 0, s>>>(U);
-    RTDL_LAUNCHED(2);
-    if (pass == 0 && after_first_pass) after_first_pass();  // work the caller queues before the first wait
-
-    SmallReads reads(rb);
-    reads.add(&rb->refine_left, next_count, sizeof(unsigned int));
-    reads.launch(s);
-    RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
-    n = rb->refine_left;
-    if (last) out.generic = n;
-    cur ^= 1;
-  }
-  out.generic_qin = gen_qin;
-  out.generic_m = gen_m;
-  out.generic_rad = gen_rad;
-  SmallReads reads(rb);
-  reads.add(&rb->mid, small + 2, sizeof(unsigned int) * 2);
-  reads.launch(s);
-  RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
-  out.mid = rb->mid;
-  out.big = rb->big;
-  return out;
-}
-
-// The collect pass, by the tuning's traversal (a problem batch walks in packets).
-void launch_collect(const CollectParams& C, uint32_t np, uint32_t nq, bool batch, bool stats, cudaStream_t s) {
-  const int threads = tuning().block_threads;
-  const bool packet = tuning().traversal != 1 || batch;
-  if (packet) {
-    const unsigned int grid = div_up(np, threads);
-    const bool cube = tuning().traversal == 2;
-    // occupancy bounds chosen so neither variant spills (32 and 40 registers)
-    if (batch)  // several problems (traversal counters are not gathered here)
-      tuning().traversal == 4 ? k_collect_packet<false, false, true, 5, kLeafHybrid><<<grid, threads, 0, s>>>(C)
-                              : k_collect_packet<false, false, true, 5><<<grid, threads, 0, s>>>(C);
-    else if (tuning().traversal == 3)
-      stats ? k_collect_packet<true, false, false, 1, kLeafPointMajor><<<grid, threads, 0, s>>>(C)
-            : k_collect_packet<false, false, false, 6, kLeafPointMajor><<<grid, threads, 0, s>>>(C);
-    else if (tuning().traversal == 4)
-      stats ? k_collect_packet<true, false, false, 1, kLeafHybrid><<<grid, threads, 0, s>>>(C)
-            : k_collect_packet<false, false, false, 6, kLeafHybrid><<<grid, threads, 0, s>>>(C);
-    else if (stats)
-      cube ? k_collect_packet<true, true, false, 1><<<grid, threads, 0, s>>>(C)
-           : k_collect_packet<true, false, false, 1><<<grid, threads, 0, s>>>(C);
-    else
-      cube ? k_collect_packet<false, true, false, 6><<<grid, threads, 0, s>>>(C)
-           : k_collect_packet<false, false, false, 7><<<grid, threads, 0, s>>>(C);
-  } else {
-    if (stats)
-      k_collect<true><<<div_up(nq, threads), threads, 0, s>>>(C);
-    else
-      k_collect<false><<<div_up(nq, threads), threads, 0, s>>>(C);
-  }
+// The queries the packets left (their number is on the device).
+void launch_collect_left(const CollectParams& C, uint32_t np, cudaStream_t s) {
+  const unsigned int blocks = div_up(np, 128 / 32), cap = kSmCount * 8;
+  k_collect_single<<<blocks < cap ? blocks : cap, 128, 0, s>>>(C, true);
   RTDL_LAUNCHED(1);
 }
 
-// Buffers of the device-driven refinement (worst case: every processing rank).
-struct RefineDevice {
-  uint32_t* work[2];
-  double *rad[2], *lo[2], *hi[2], *frad[2];
-  uint32_t* full[2];
-  uint32_t *cnt, *gen_qin, *gen_m;
-  double* gen_rad;
-  unsigned int* pass_count;  // kRefinePasses: work left after each pass (after the last: the generic count)
-};
-
-// The radius refinement without host reads (captured graphs): every pass is
-// launched, each kernel reads its work count on the device and strides over it,
-// and both walk
-// forms are launched (the one the host-driven loop would not pick exits).
-// small[0] holds the collect pass's heavy count; D.pass_count[kRefinePasses-1]
-// ends with the number of queries left for the generic path.
-void enqueue_refine_device(const CollectParams& C, const uint32_t* qprob, const double* prob_radius, double radius,
-                           const uint32_t* prob_kmax, uint32_t kmax, uint32_t nproc, bool one_scene,
-                           QueryInfo* qinfo, uint8_t* flags, unsigned int* small, const RefineDevice& D,
-                           cudaStream_t s) {
-  RTDL_CUDA_CHECK(cudaMemsetAsync(D.pass_count, 0, sizeof(unsigned int) * kRefinePasses, s));
-  k_refine_init<<<kSmCount * 4, 256, 0, s>>>(C.heavy_list, C.heavy_m, C.heavy_t, 0, qprob, prob_radius, radius,
-                                             prob_kmax, kmax, D.work[0], D.rad[0], D.lo[0], D.hi[0], D.full[0],
-                                             D.frad[0], small);
-  RTDL_LAUNCHED(1);
-  int cur = 0;
-  for (int pass = 0; pass < kRefinePasses; ++pass) {
-    const unsigned int* n_dev = pass == 0 ? small : D.pass_count + pass - 1;
-    RefineParams R;
-    R.C = C;
-    R.qprob = qprob;
-    R.work = D.work[cur];
-    R.rad = D.rad[cur];
-    R.nwork = 0;
-    R.cnt = D.cnt;
-    R.nwork_dev = n_dev;
-    R.packet_min = nproc / 8;  // the host-driven loop's choice between the two forms
-    if (one_scene)
-      k_collect_refine_packet_scene<<<kStrideBlocks, 256, 0, s>>>(R);
-    else
-      k_collect_refine_packet<<<kStrideBlocks, 256, 0, s>>>(R);
-    k_collect_refine<<<kStrideBlocks, 256, 0, s>>>(R);
-    RefineUpdate U;
-    U.qorder = C.qorder;
-    U.qprob = qprob;
-    U.prob_kmax = prob_kmax;
-    U.kmax = kmax;
-    U.qinfo = qinfo;
-    U.flags = flags;
-    U.mid_list = C.mid_list;
-    U.big_list = C.big_list;
-    U.small = small;
-    U.work = D.work[cur];
-    U.rad = D.rad[cur];
-    U.lo = D.lo[cur];
-    U.hi = D.hi[cur];
-    U.full = D.full[cur];
-    U.frad = D.frad[cur];
-    U.cnt = D.cnt;
-    U.nwork = 0;
-    U.next_work = D.work[cur ^ 1];
-    U.next_rad = D.rad[cur ^ 1];
-    U.next_lo = D.lo[cur ^ 1];
-    U.next_hi = D.hi[cur ^ 1];
-    U.next_full = D.full[cur ^ 1];
-    U.next_frad = D.frad[cur ^ 1];
-    U.next_count = D.pass_count + pass;
-    U.generic_qin = D.gen_qin;
-    U.generic_m = D.gen_m;
-    U.generic_rad = D.gen_rad;
-    U.last = pass == kRefinePasses - 1 ? 1 : 0;
-    U.nwork_dev = n_dev;
-    k_refine_update<<<kSmCount * 4, 256, 0, s>>>(U);
-    RTDL_LAUNCHED(3);
-    cur ^= 1;
+// The collect pass over np processing ranks.
+void launch_collect(CollectParams& C, uint32_t np, bool batch, cudaStream_t s) {
+  if (np <= kSingleQueries && !C.rank_radius) {
+    k_collect_single<<<div_up(np, 128 / 32), 128, 0, s>>>(C, false);
+    RTDL_LAUNCHED(1);
+    return;
   }
+  // Full packets once they give every SM 24 warps (what the registers allow);
+  // fewer queries per packet below that, where the longest packet sets the time:
+  // a packet of eight meets half the buckets of one of 32.
+  C.width = np >= 32u * 24u * kSmCount ? 32u : np >= 16u * 24u * kSmCount ? 16u : 8u;
+  const unsigned int grid = div_up((uint64_t)div_up(np, C.width) * 32, kCollectThreads);
+  const bool flat = C.qstride == 3;
+  if (batch)
+    flat ? k_collect_packet<2, true, false><<<grid, kCollectThreads, 0, s>>>(C)
+         : k_collect_packet<3, true, false><<<grid, kCollectThreads, 0, s>>>(C);
+  else if (C.rank_radius)
+    flat ? k_collect_packet<2, false, true><<<grid, kCollectThreads, 0, s>>>(C)
+         : k_collect_packet<3, false, true><<<grid, kCollectThreads, 0, s>>>(C);
+  else
+    flat ? k_collect_packet<2, false, false><<<grid, kCollectThreads, 0, s>>>(C)
+         : k_collect_packet<3, false, false><<<grid, kCollectThreads, 0, s>>>(C);
+  RTDL_LAUNCHED(1);
+  if (!C.rank_radius) launch_collect_left(C, np, s);
+}
+
+void launch_emit(const EmitParams& E, uint32_t queries, cudaStream_t s) {
+  k_emit<<<emit_grid(queries), kEmitThreads, 0, s>>>(E);
+  RTDL_LAUNCHED(1);
+}
+
+// Blocks of the kernels that stride over a device list of at most np queries.
+inline unsigned int list_grid(uint32_t np) {
+  const unsigned int blocks = div_up(np, kEmitListThreads / 32);
+  return blocks < kStrideBlocks ? blocks : kStrideBlocks;
+}
+static_assert(kEmitListThreads == kFixupThreads, "list_grid serves both");
+
+// The list kernels over the collect's lists (lengths in small[2], small[3]).
+void launch_emit_lists(const EmitParams& E, const CollectParams& C, uint32_t np, cudaStream_t s) {
+  k_emit_list<4, true><<<list_grid(np), kEmitListThreads, 0, s>>>(E, C.mid_list, 0, C.small + 2);
+  k_emit_list<8, false><<<list_grid(np), kEmitListThreads, 0, s>>>(E, C.big_list, 0, C.small + 3);
+  RTDL_LAUNCHED(2);
 }
 
 void check_readback(const Readback& r) {
@@ -3040,43 +2562,24 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
     RTDL_LAUNCHED(1);
   }
   if (timer) timer->mark("query_prep");
-  unsigned long long* slab =
-      static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long) * slab_base((uint32_t)np1), s));
-  uint32_t* counts = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq1, s));
-  QueryInfo* qinfo = static_cast<QueryInfo*>(dev_alloc(sizeof(QueryInfo) * np1, s));
-  uint8_t* flags = static_cast<uint8_t*>(dev_alloc(nq1, s));
-  uint32_t* heavy_list = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq1, s));
-  uint32_t* heavy_m = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq1, s));
-  uint32_t* heavy_t = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq1, s));
-  uint32_t* mid_list = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * np1, s));
-  uint32_t* big_list = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * np1, s));
-  uint32_t* fix_list = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * np1, s));
-  unsigned int* small = static_cast<unsigned int*>(dev_alloc(sizeof(unsigned int) * 8, s));
-  unsigned long long* offsets = static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long) * (nq + 1), s));
-  unsigned long long* poff = static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long) * np1, s));
+  std::vector<void*> bufs;
+  auto alloc = [&](size_t bytes) {
+    void* p = dev_alloc(bytes ? bytes : 1, s);
+    bufs.push_back(p);
+    return p;
+  };
+  uint32_t* counts = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * nq1));
+  unsigned int* small = static_cast<unsigned int*>(alloc(sizeof(unsigned int) * 8));
+  unsigned long long* offsets = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * ((size_t)nq + 1)));
+  unsigned long long* poff = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * np1));
   unsigned long long* prob_rows =
-      bs ? static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long) * (bs->problems + 1), s)) : nullptr;
+      bs ? static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * (bs->problems + 1))) : nullptr;
   RTDL_CUDA_CHECK(cudaMemsetAsync(small, 0, sizeof(unsigned int) * 8, s));
   GenericOut g;
-  std::vector<void*> refine_bufs;
   auto cleanup = [&]() {
     g.release(s);
-    for (void* p : refine_bufs) dev_free(p, s);
-    dev_free(prob_rows, s);
-    dev_free(poff, s);
     if (!pq) dev_free(qrank, s);
-    dev_free(slab, s);
-    dev_free(counts, s);
-    dev_free(qinfo, s);
-    dev_free(flags, s);
-    dev_free(heavy_list, s);
-    dev_free(heavy_m, s);
-    dev_free(heavy_t, s);
-    dev_free(mid_list, s);
-    dev_free(big_list, s);
-    dev_free(fix_list, s);
-    dev_free(small, s);
-    dev_free(offsets, s);
+    for (void* p : bufs) dev_free(p, s);
     free_prep(qp, s);
   };
   try {
@@ -3088,33 +2591,36 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
     C.qorder = qp.qorder;
     C.nq = np;
     C.kmax = kmax;
+    C.radius = radius;
     C.bands = qp.bands;
     C.warp_prob = qp.warp_prob;
     C.prob_kmax = qp.prob_kmax;
-    C.slab = slab;
+    C.prob_radius = qp.prob_radius;
+    C.rank_radius = nullptr;
+    C.slab = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * slab_base((uint32_t)np1)));
     C.counts = counts;
-    C.qinfo = qinfo;
-    C.flags = flags;
-    C.heavy_list = heavy_list;
-    C.heavy_m = heavy_m;
-    C.heavy_t = heavy_t;
-    C.mid_list = mid_list;
-    C.big_list = big_list;
+    C.qinfo = static_cast<QueryInfo*>(alloc(sizeof(QueryInfo) * np1));
+    C.flags = static_cast<uint8_t*>(alloc(nq1));
+    C.heavy_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * nq1));
+    C.heavy_m = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * nq1));
+    C.heavy_rad = static_cast<double*>(alloc(sizeof(double) * nq1));
+    C.heavy_t = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * nq1));
+    C.mid_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * np1));
+    C.big_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * np1));
+    C.single_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * np1));
     C.small = small;
     C.overflow_out = overflow_dev;
     C.stats = nullptr;
     const bool stats = stats_enabled();
     if (stats) {
-      C.stats = static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long) * kStatCount, s));
+      C.stats = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * kStatCount));
       RTDL_CUDA_CHECK(cudaMemsetAsync(C.stats, 0, sizeof(unsigned long long) * kStatCount, s));
     }
     if (timer) timer->mark("setup");
-    launch_collect(C, np, nq, bs != nullptr, stats, s);
-    if (stats) {
+    launch_collect(C, np, bs != nullptr, s);
+    if (stats)
       RTDL_CUDA_CHECK(cudaMemcpyAsync(last_stats().data(), C.stats, sizeof(unsigned long long) * kStatCount,
                                       cudaMemcpyDeviceToHost, s));
-      dev_free(C.stats, s);
-    }
     if (timer) timer->mark("traverse");
     if (witness) {
       k_witness_offsets<<<grid_for(nq + 1, 256), 256, 0, s>>>(qp.oorder, qp.order_identity, nq, offsets);
@@ -3129,7 +2635,27 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
                                       cudaMemcpyDeviceToHost, s));
     }
     if (timer) timer->mark("scan");
-    auto launch_expand = [&](uint32_t n_generic, const uint32_t* list) {
+    Readback* rb = pinned_readback();
+    SmallReads reads(rb);
+    // the row count, the list lengths and the input checks; waits
+    auto read_counts = [&]() {
+      reads.add(&rb->rows, offsets + nq, sizeof(unsigned long long));
+      reads.add(&rb->heavy, small, sizeof(unsigned int) * 4);
+      reads.add(&rb->fixups, small + 4, sizeof(unsigned int));
+      reads.add(&rb->scene_bad, &sc->stats->bad, sizeof(unsigned int));
+      reads.add(&rb->query_bad, &qp.qst->bad, sizeof(unsigned int));
+      reads.launch(s);
+      RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
+      check_readback(*rb);
+      res.rows = rb->rows;
+      res.heavy = rb->heavy;
+      return *rb;
+    };
+    // queries whose candidates were not kept: gathered within the smallest
+    // tested radius that holds their rows, sorted and written
+    auto generic_path = [&](uint32_t n) {
+      g = run_generic_path(sc, qp, queries_dev, qstride, n, C.heavy_list, C.heavy_m, kmax, false, small + 1, s,
+                           C.heavy_rad);
       ExpandParams X;
       X.S = sc->view();
       X.qpts = qp.qpts;
@@ -3137,10 +2663,10 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
       X.qstride = qstride;
       X.oorder = qp.oorder;
       X.bands = qp.bands;
-      X.nq = n_generic;
+      X.nq = n;
       X.L = kSlab;
       X.counts = counts;
-      X.flags = flags;
+      X.flags = C.flags;
       X.temp = nullptr;  // unused with a work list
       X.heavy_out = g.heavy_out;
       X.heavy_out_off = g.heavy_out_off;
@@ -3150,269 +2676,133 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
       X.ranked = predicate == kFrn ? 0 : 1;
       X.overflow_out = nullptr;
       X.error = small + 1;
-      X.work_list = list;
+      X.work_list = C.heavy_list;
       X.qrank = qrank;
-      k_expand<32><<<grid_for((uint64_t)n_generic * 32, kExpandThreads), kExpandThreads, 0, s>>>(X);
+      k_expand<<<grid_for((uint64_t)n * 32, kExpandThreads), kExpandThreads, 0, s>>>(X);
       RTDL_LAUNCHED(1);
+      if (stats) last_stats()[kStatGenericQueries] = n;
     };
-    // Rows only counted: the total is known after the scan (no refinement, no emit).
+    // Rows only counted: the total is known after the scan (no emit).
     const bool count_only = rows_alloc == nullptr && rows_dev == nullptr && !bs && !ss && !witness;
-    Readback* rb = pinned_readback();
     if (count_only) {
-      SmallReads reads(rb);
-      reads.add(&rb->rows, offsets + nq, sizeof(unsigned long long));
-      reads.add(&rb->heavy, small, sizeof(unsigned int) * 4);
-      reads.add(&rb->scene_bad, &sc->stats->bad, sizeof(unsigned int));
-      reads.add(&rb->query_bad, &qp.qst->bad, sizeof(unsigned int));
-      reads.launch(s);
-      RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
-      check_readback(*rb);
-      res.rows = rb->rows;
+      read_counts();
     } else {
       // rows copied to the host range by range as they are emitted
       bool chunked = dl != nullptr && (dl->alloc != nullptr || dl->host_fixed != nullptr) && rows_alloc != nullptr &&
                      !bs && !ss && !witness &&
                      nq >= (uint32_t)kDownloadChunks * 1024u;
-      SmallReads reads(rb);
-      if (chunked) {
-        unsigned long long* chunk_dev =
-            static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long) * (kDownloadChunks + 1), s));
-        refine_bufs.push_back(chunk_dev);
-        k_chunk_rows<<<1, 32, 0, s>>>(offsets, nq, kDownloadChunks, chunk_dev);
-        RTDL_LAUNCHED(1);
-        reads.add(rb->chunk_rows, chunk_dev, sizeof(unsigned long long) * (kDownloadChunks + 1));
+      const size_t row_size = predicate == kFrn ? 16 : 24;
+      Readback r{};
+      if (rows_alloc != nullptr) {  // the row buffer is sized from the count
+        if (chunked) {
+          unsigned long long* chunk_dev =
+              static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * (kDownloadChunks + 1)));
+          k_chunk_rows<<<1, 32, 0, s>>>(offsets, nq, kDownloadChunks, chunk_dev);
+          RTDL_LAUNCHED(1);
+          reads.add(rb->chunk_rows, chunk_dev, sizeof(unsigned long long) * (kDownloadChunks + 1));
+        }
+        r = read_counts();
+        if (res.rows == 0) chunked = false;
+        rows_dev = res.rows ? dev_alloc(row_size * res.rows, s) : nullptr;
+        rows_capacity = res.rows;
+        *rows_alloc = rows_dev;
       }
-      reads.add(&rb->rows, offsets + nq, sizeof(unsigned long long));
-      reads.add(&rb->heavy, small, sizeof(unsigned int) * 4);
-      reads.add(&rb->scene_bad, &sc->stats->bad, sizeof(unsigned int));
-      reads.add(&rb->query_bad, &qp.qst->bad, sizeof(unsigned int));
-      reads.launch(s);
-      RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
-      const Readback r = *rb;
-      check_readback(r);
-      res.rows = r.rows;
-      if (res.rows == 0) chunked = false;
-      uint32_t mid = r.mid, big = r.big, generic = r.heavy;
-      const uint32_t* generic_list = heavy_list;
-      const uint32_t* generic_m = heavy_m;
-      const double* generic_rad = nullptr;
-      auto emit_params = [&]() {
-        EmitParams E;
-        E.S = sc->view();
-        E.nq = np;
-        E.slab = slab;
-        E.qinfo = qinfo;
-        E.poff = poff;
-        E.sink.rows = rows_dev;
-        E.sink.capacity = rows_dev ? rows_capacity : 0;
-        E.sink.ranked = predicate == kFrn ? 0 : 1;
-        E.fix_list = fix_list;
-        E.fix_count = small + 4;
-        return E;
-      };
-      if (r.heavy > 0 && rows_alloc == nullptr && !witness) {
-        // Rows into a given device buffer: the emit does not wait for the heavy
-        // queries.  Three streams: the list kernels of the collect's 65..kSlab
-        // candidate queries (their counts are final) are queued first on the
-        // second stream, the first refinement pass on the third, then k_emit
-        // on this one; the refinement's later passes (each reads its count
-        // back to the host), the generic path and the list kernels of the
-        // queries it resolved follow on the third stream.  k_emit skips a
-        // heavy query whichever of its records it reads: the collect marked
-        // it generic, the pass that resolves it marks it for a list kernel
-        // and appends it to a list after the collect's entries.
-        cudaStream_t ls = aux_stream(0), rs = aux_stream(1);
-        static thread_local cudaEvent_t ev_offsets = nullptr, ev_lists = nullptr, ev_refined = nullptr;
-        if (!ev_offsets) {
-          RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_offsets, cudaEventDisableTiming));
-          RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_lists, cudaEventDisableTiming));
-          RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_refined, cudaEventDisableTiming));
-        }
-        k_proc_offsets<<<grid_for(np, 256), 256, 0, s>>>(qp.qorder, qrank, offsets, np, poff);
+      if (witness && rows_dev) {
+        k_witness_fill<<<grid_for(nq, 256), 256, 0, s>>>(qp.qpts, nq, static_cast<RtdlFixedRadiusNeighborRow*>(rows_dev),
+                                                         rows_capacity);
         RTDL_LAUNCHED(1);
-        RTDL_CUDA_CHECK(cudaEventRecord(ev_offsets, s));
-        RTDL_CUDA_CHECK(cudaStreamWaitEvent(ls, ev_offsets, 0));
-        RTDL_CUDA_CHECK(cudaStreamWaitEvent(rs, ev_offsets, 0));
-        const EmitParams E = emit_params();
-        auto launch_lists = [&](uint32_t first_mid, uint32_t n_mid, uint32_t first_big, uint32_t n_big,
-                                cudaStream_t st) {
-          if (n_mid > 0) {
-            k_emit_list<4, true><<<div_up((uint64_t)n_mid * 32, kEmitListThreads), kEmitListThreads, 0, st>>>(
-                E, mid_list + first_mid, n_mid, nullptr);
-            RTDL_LAUNCHED(1);
-          }
-          if (n_big > 0) {
-            k_emit_list<8, false><<<div_up((uint64_t)n_big * 32, kEmitListThreads), kEmitListThreads, 0, st>>>(
-                E, big_list + first_big, n_big, nullptr);
-            RTDL_LAUNCHED(1);
-          }
-        };
-        launch_lists(0, r.mid, 0, r.big, ls);
-        RTDL_CUDA_CHECK(cudaEventRecord(ev_lists, ls));
-        RefineOut ro = refine_heavy(C, qp, radius, kmax, r.heavy, heavy_list, heavy_m, heavy_t, qinfo, flags, mid_list,
-                                    big_list, small, rs, [&]() {
-                                      k_emit<<<emit_grid(np), kEmitThreads, 0, s>>>(E);
-                                      RTDL_LAUNCHED(1);
-                                    });
-        refine_bufs = ro.buffers;
-        generic = ro.generic;
-        res.heavy = generic;
-        if (stats) {
-          last_stats()[kStatGenericQueries] = generic;
-          last_stats()[kStatLargeQueries] = ro.mid + ro.big;
-          last_stats()[kStatRefined] = r.heavy - generic;
+      }
+      k_proc_offsets<<<grid_for(np, 256), 256, 0, s>>>(qp.qorder, qrank, offsets, np, poff);
+      RTDL_LAUNCHED(1);
+      EmitParams E;
+      E.S = sc->view();
+      E.nq = np;
+      E.slab = C.slab;
+      E.qinfo = C.qinfo;
+      E.poff = poff;
+      E.sink.rows = rows_dev;
+      E.sink.capacity = rows_dev ? rows_capacity : 0;
+      E.sink.ranked = predicate == kFrn ? 0 : 1;
+      E.fix_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * np1));
+      E.fix_count = small + 4;
+      if (chunked) {
+        if (dl->host_fixed) {
+          dl->host = dl->host_fixed;
+          dl->pinned = true;
+        } else {
+          dl->host = dl->alloc(row_size * res.rows, &dl->pinned);
         }
-        // the gather is bounded by each query's smallest tested radius that holds its rows
-        if (generic > 0)
-          g = run_generic_path(sc, qp, queries_dev, qstride, generic, ro.generic_qin, ro.generic_m, kmax, false,
-                               small + 1, rs, ro.generic_rad);
-        launch_lists(r.mid, ro.mid - r.mid, r.big, ro.big - r.big, rs);
-        RTDL_CUDA_CHECK(cudaEventRecord(ev_refined, rs));
-        RTDL_CUDA_CHECK(cudaStreamWaitEvent(s, ev_lists, 0));
-        RTDL_CUDA_CHECK(cudaStreamWaitEvent(s, ev_refined, 0));
-        k_emit_fixup<<<kSmCount * 4, kFixupThreads, 0, s>>>(E);
+        // Range by range in output order: each range's queries are emitted
+        // (the list kernels and k_emit skip queries outside it), its deferred
+        // queries fixed up, and the copy of its rows queued on the copy
+        // stream, which overlaps the emission of the ranges after it.  The
+        // generic queries' rows are written first.
+        const uint32_t mid = r.mid, big = r.big;
+        if (r.heavy > 0) generic_path(r.heavy);
+        uint32_t* eorder = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * nq1));
+        k_emit_order<<<grid_for(np, 256), 256, 0, s>>>(qp.qorder, qrank, np, eorder);
         RTDL_LAUNCHED(1);
-        if (generic > 0) launch_expand(generic, ro.generic_qin);
-        if (timer) timer->mark("emit");
-        SmallReads end_reads(rb);
-        end_reads.add(&rb->error, small + 1, sizeof(unsigned int));
-        end_reads.add(&rb->fixups, small + 4, sizeof(unsigned int));
-        end_reads.launch(s);
-        RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
-        if (stats) last_stats()[kStatEmitFixups] = rb->fixups;
-        if (rb->error & 6u) throw std::runtime_error("generic neighbor path produced an inconsistent candidate count");
+        // the two list kernels' work, partitioned by range (list lengths in small[2], small[3])
+        constexpr uint32_t C8 = kDownloadChunks, kPart = 3 * C8 + 1;
+        unsigned int* part = static_cast<unsigned int*>(alloc(sizeof(unsigned int) * 2 * kPart));
+        RTDL_CUDA_CHECK(cudaMemsetAsync(part, 0, sizeof(unsigned int) * 2 * kPart, s));
+        uint32_t* lists_by_range[2] = {nullptr, nullptr};
+        const uint32_t list_len[2] = {mid, big};
+        uint32_t* lists[2] = {C.mid_list, C.big_list};
+        for (int l = 0; l < 2; ++l) {
+          if (list_len[l] == 0) continue;
+          lists_by_range[l] = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * list_len[l]));
+          const unsigned int grid = grid_for(list_len[l], 256);
+          k_range_count<<<grid, 256, 0, s>>>(lists[l], small + 2 + l, qp.qorder, qrank, nq, C8, part + l * kPart);
+          k_range_starts<<<1, 1, 0, s>>>(C8, part + l * kPart);
+          k_range_scatter<<<grid, 256, 0, s>>>(lists[l], small + 2 + l, qp.qorder, qrank, nq, C8, part + l * kPart,
+                                               lists_by_range[l]);
+          RTDL_LAUNCHED(3);
+        }
+        E.order = eorder;
+        E.fix_begin = small + 5;
+        static thread_local cudaEvent_t ev_range[kDownloadChunks] = {};
+        unsigned long long first[kDownloadChunks + 1];
+        for (int c = 0; c <= kDownloadChunks; ++c) first[c] = r.chunk_rows[c];
+        if (first[kDownloadChunks] != res.rows) throw std::runtime_error("row ranges disagree with the row count");
+        for (int c = 0; c < (int)C8; ++c) {
+          if (first[c + 1] == first[c]) continue;  // no rows in this range
+          E.out_lo = (uint32_t)((uint64_t)nq * (uint32_t)c / C8);
+          E.out_hi = (uint32_t)((uint64_t)nq * (uint32_t)(c + 1) / C8);
+          E.range = c;
+          // the list kernels stride over the range's part: grids sized for an even split
+          if (mid > 0) {
+            E.list_start = part + C8;
+            k_emit_list<4, true><<<div_up((uint64_t)div_up(mid, C8) * 32, kEmitListThreads), kEmitListThreads, 0, s>>>(
+                E, lists_by_range[0], 0, nullptr);
+          }
+          if (big > 0) {
+            E.list_start = part + kPart + C8;
+            k_emit_list<8, false><<<div_up((uint64_t)div_up(big, C8) * 32, kEmitListThreads), kEmitListThreads, 0,
+                                    s>>>(E, lists_by_range[1], 0, nullptr);
+          }
+          E.list_start = nullptr;
+          launch_emit(E, E.out_hi - E.out_lo, s);
+          k_emit_fixup<<<kSmCount * 4, kFixupThreads, 0, s>>>(E);
+          k_fix_advance<<<1, 1, 0, s>>>(small + 5, small + 4);
+          RTDL_LAUNCHED(4);
+          if (!ev_range[c]) RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_range[c], cudaEventDisableTiming));
+          RTDL_CUDA_CHECK(cudaEventRecord(ev_range[c], s));
+          RTDL_CUDA_CHECK(cudaStreamWaitEvent(dl->copy, ev_range[c], 0));
+          RTDL_CUDA_CHECK(cudaMemcpyAsync(static_cast<char*>(dl->host) + first[c] * row_size,
+                                          static_cast<const char*>(rows_dev) + first[c] * row_size,
+                                          (first[c + 1] - first[c]) * row_size, cudaMemcpyDeviceToHost, dl->copy));
+          ++dl->copies;
+        }
       } else {
-        if (r.heavy > 0) {
-          // queries with more than kSlab points in radius: collect again at smaller radii
-          RefineOut ro = refine_heavy(C, qp, radius, kmax, r.heavy, heavy_list, heavy_m, heavy_t, qinfo, flags, mid_list,
-                                      big_list, small, s);
-          refine_bufs = ro.buffers;
-          generic = ro.generic;
-          generic_list = ro.generic_qin;
-          generic_m = ro.generic_m;
-          generic_rad = ro.generic_rad;
-          mid = ro.mid;
-          big = ro.big;
-          if (timer) timer->mark("refine");
-        }
-        res.heavy = generic;
-        if (stats) {
-          last_stats()[kStatGenericQueries] = generic;
-          last_stats()[kStatLargeQueries] = mid + big;
-          last_stats()[kStatRefined] = r.heavy - generic;
-        }
-        if (generic > 0) {
-          // the gather is bounded by each query's smallest tested radius that holds its rows
-          g = run_generic_path(sc, qp, queries_dev, qstride, generic, generic_list, generic_m, kmax, false, small + 1, s,
-                               generic_rad);
-          if (timer) timer->mark("generic_path");
-        }
-        if (rows_alloc != nullptr) {
-          const size_t row_size = predicate == kFrn ? 16 : 24;
-          rows_dev = res.rows ? dev_alloc(row_size * res.rows, s) : nullptr;
-          rows_capacity = res.rows;
-          *rows_alloc = rows_dev;
-        }
-        if (witness && rows_dev) {
-          k_witness_fill<<<grid_for(nq, 256), 256, 0, s>>>(qp.qpts, nq, static_cast<RtdlFixedRadiusNeighborRow*>(rows_dev),
-                                                           rows_capacity);
-          RTDL_LAUNCHED(1);
-        }
-        k_proc_offsets<<<grid_for(np, 256), 256, 0, s>>>(qp.qorder, qrank, offsets, np, poff);
-        RTDL_LAUNCHED(1);
-        if (chunked) {
-          const size_t row_size = predicate == kFrn ? 16 : 24;
-          if (dl->host_fixed) {
-            dl->host = dl->host_fixed;
-            dl->pinned = true;
-          } else {
-            dl->host = dl->alloc(row_size * res.rows, &dl->pinned);
-          }
-        }
-        EmitParams E = emit_params();
-        if (chunked) {
-          // Range by range in output order: each range's queries are emitted
-          // (the list kernels and k_emit skip queries outside it), its deferred
-          // queries fixed up, and the copy of its rows queued on the copy
-          // stream, which overlaps the emission of the ranges after it.  The
-          // generic queries' rows are written first.
-          if (generic > 0) launch_expand(generic, generic_list);
-          uint32_t* eorder = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq1, s));
-          refine_bufs.push_back(eorder);
-          k_emit_order<<<grid_for(np, 256), 256, 0, s>>>(qp.qorder, qrank, np, eorder);
-          RTDL_LAUNCHED(1);
-          // the two list kernels' work, partitioned by range (list lengths in small[2], small[3])
-          constexpr uint32_t C = kDownloadChunks, kPart = 3 * C + 1;
-          unsigned int* part = static_cast<unsigned int*>(dev_alloc(sizeof(unsigned int) * 2 * kPart, s));
-          refine_bufs.push_back(part);
-          RTDL_CUDA_CHECK(cudaMemsetAsync(part, 0, sizeof(unsigned int) * 2 * kPart, s));
-          uint32_t* lists_by_range[2] = {nullptr, nullptr};
-          const uint32_t list_len[2] = {mid, big};
-          uint32_t* lists[2] = {mid_list, big_list};
-          for (int l = 0; l < 2; ++l) {
-            if (list_len[l] == 0) continue;
-            lists_by_range[l] = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * list_len[l], s));
-            refine_bufs.push_back(lists_by_range[l]);
-            const unsigned int grid = grid_for(list_len[l], 256);
-            k_range_count<<<grid, 256, 0, s>>>(lists[l], small + 2 + l, qp.qorder, qrank, nq, C, part + l * kPart);
-            k_range_starts<<<1, 1, 0, s>>>(C, part + l * kPart);
-            k_range_scatter<<<grid, 256, 0, s>>>(lists[l], small + 2 + l, qp.qorder, qrank, nq, C, part + l * kPart,
-                                                 lists_by_range[l]);
-            RTDL_LAUNCHED(3);
-          }
-          E.order = eorder;
-          E.fix_begin = small + 5;
-          static thread_local cudaEvent_t ev_range[kDownloadChunks] = {};
-          unsigned long long first[kDownloadChunks + 1];
-          for (int c = 0; c <= kDownloadChunks; ++c) first[c] = r.chunk_rows[c];
-          if (first[kDownloadChunks] != res.rows) throw std::runtime_error("row ranges disagree with the row count");
-          const size_t row_size = predicate == kFrn ? 16 : 24;
-          for (int c = 0; c < (int)C; ++c) {
-            if (first[c + 1] == first[c]) continue;  // no rows in this range
-            E.out_lo = (uint32_t)((uint64_t)nq * (uint32_t)c / C);
-            E.out_hi = (uint32_t)((uint64_t)nq * (uint32_t)(c + 1) / C);
-            E.range = c;
-            // the list kernels stride over the range's part: grids sized for an even split
-            if (mid > 0) {
-              E.list_start = part + C;
-              k_emit_list<4, true><<<div_up((uint64_t)div_up(mid, C) * 32, kEmitListThreads), kEmitListThreads, 0, s>>>(
-                  E, lists_by_range[0], 0, nullptr);
-            }
-            if (big > 0) {
-              E.list_start = part + kPart + C;
-              k_emit_list<8, false><<<div_up((uint64_t)div_up(big, C) * 32, kEmitListThreads), kEmitListThreads, 0,
-                                      s>>>(E, lists_by_range[1], 0, nullptr);
-            }
-            E.list_start = nullptr;
-            k_emit<<<emit_grid(E.out_hi - E.out_lo), kEmitThreads, 0, s>>>(E);
-            k_emit_fixup<<<kSmCount * 4, kFixupThreads, 0, s>>>(E);
-            k_fix_advance<<<1, 1, 0, s>>>(small + 5, small + 4);
-            RTDL_LAUNCHED(5);
-            if (!ev_range[c]) RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_range[c], cudaEventDisableTiming));
-            RTDL_CUDA_CHECK(cudaEventRecord(ev_range[c], s));
-            RTDL_CUDA_CHECK(cudaStreamWaitEvent(dl->copy, ev_range[c], 0));
-            RTDL_CUDA_CHECK(cudaMemcpyAsync(static_cast<char*>(dl->host) + first[c] * row_size,
-                                            static_cast<const char*>(rows_dev) + first[c] * row_size,
-                                            (first[c + 1] - first[c]) * row_size, cudaMemcpyDeviceToHost, dl->copy));
-            ++dl->copies;
-          }
-          if (timer) timer->mark("emit");
-          SmallReads end_reads(rb);
-          end_reads.add(&rb->error, small + 1, sizeof(unsigned int));
-          end_reads.add(&rb->fixups, small + 4, sizeof(unsigned int));
-          end_reads.launch(s);
-          RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
-          if (stats) last_stats()[kStatEmitFixups] = rb->fixups;
-          if (rb->error & 6u) throw std::runtime_error("generic neighbor path produced an inconsistent candidate count");
-          cleanup();
-          return res;
-        }
         // The list kernels (queries with 65..kSlab candidates: few warps, long
-        // sorts) run on the second stream beside k_emit, so each fills the
+        // sorts) read their lengths on the device, so nothing waits for the
+        // host between the collect and the rows.  In calls that fill the GPU
+        // they run on the second stream beside k_emit, so each fills the
         // other's partial waves; they write disjoint rows, and the fix-up waits
         // for both.
         static thread_local cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-        const bool side = mid > 0 || big > 0;
+        const bool side = np > kSingleQueries;
         cudaStream_t ls = s;
         if (side) {
           if (!ev_fork) {
@@ -3423,35 +2813,29 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
           RTDL_CUDA_CHECK(cudaEventRecord(ev_fork, s));
           RTDL_CUDA_CHECK(cudaStreamWaitEvent(ls, ev_fork, 0));
         }
-        if (mid > 0) {
-          k_emit_list<4, true><<<div_up((uint64_t)mid * 32, kEmitListThreads), kEmitListThreads, 0, ls>>>(E, mid_list,
-                                                                                                       mid, nullptr);
-          RTDL_LAUNCHED(1);
-        }
-        if (big > 0) {
-          k_emit_list<8, false><<<div_up((uint64_t)big * 32, kEmitListThreads), kEmitListThreads, 0, ls>>>(E, big_list,
-                                                                                                        big, nullptr);
-          RTDL_LAUNCHED(1);
-        }
-        k_emit<<<emit_grid(np), kEmitThreads, 0, s>>>(E);
-        RTDL_LAUNCHED(1);
+        launch_emit_lists(E, C, np, ls);
+        launch_emit(E, np, s);
         if (side) {
           RTDL_CUDA_CHECK(cudaEventRecord(ev_join, ls));
           RTDL_CUDA_CHECK(cudaStreamWaitEvent(s, ev_join, 0));
         }
-        k_emit_fixup<<<kSmCount * 4, kFixupThreads, 0, s>>>(E);
+        k_emit_fixup<<<list_grid(np), kFixupThreads, 0, s>>>(E);
         RTDL_LAUNCHED(1);
-        if (generic > 0) {
-          launch_expand(generic, generic_list);
-        }
-        if (timer) timer->mark("emit");
-        SmallReads end_reads(rb);
-        end_reads.add(&rb->error, small + 1, sizeof(unsigned int));
-        end_reads.add(&rb->fixups, small + 4, sizeof(unsigned int));
-        end_reads.launch(s);
+        r = read_counts();
+        if (r.heavy > 0) generic_path(r.heavy);
+      }
+      if (timer) timer->mark("emit");
+      if (chunked || r.heavy > 0) {
+        reads.add(&rb->error, small + 1, sizeof(unsigned int));
+        reads.add(&rb->fixups, small + 4, sizeof(unsigned int));
+        reads.launch(s);
         RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
-        if (stats) last_stats()[kStatEmitFixups] = rb->fixups;
         if (rb->error & 6u) throw std::runtime_error("generic neighbor path produced an inconsistent candidate count");
+      }
+      if (stats) last_stats()[kStatEmitFixups] = rb->fixups;
+      if (chunked) {
+        cleanup();
+        return res;
       }
     }
     if (ss) {
@@ -3472,8 +2856,7 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
     }
   } catch (...) {
     sync_quietly(s);
-    sync_quietly(aux_stream(0));  // the refinement and the list kernels may run there
-    sync_quietly(aux_stream(1));
+    sync_quietly(aux_stream(0));  // the list kernels may run there
     dev_free(summary_rows, s);
     cleanup();
     throw;
@@ -3571,9 +2954,11 @@ void count_walk(Scene* sc, const void* queries_dev, uint32_t nq, double radius, 
     P.group_of = group_of;
     P.group_boxes = group_boxes;
     if (nearest_rows)
-      k_group_nearest_packet<<<div_up(nq, 256), 256, 0, s>>>(P, nearest_rows);
+      k_group_nearest_packet<<<div_up(nq, 128), 128, 0, s>>>(P, nearest_rows);
+    else if (sc->dim == 3)
+      k_count_packet<3><<<div_up(nq, 128), 128, 0, s>>>(P);
     else
-      k_count_packet<<<div_up(nq, 256), 256, 0, s>>>(P);
+      k_count_packet<2><<<div_up(nq, 128), 128, 0, s>>>(P);
     RTDL_LAUNCHED(1);
     Readback* rb = pinned_readback();
     RTDL_CUDA_CHECK(cudaMemcpyAsync(&rb->scene_bad, &sc->stats->bad, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
@@ -3600,7 +2985,7 @@ void run_count_threshold(Scene* sc, const void* queries_dev, uint32_t nq, double
 }
 
 PointGroupScene* point_group_create(const RtdlPoint* points, size_t count, const RtdlPointGroupBounds2D* groups,
-                                    size_t group_count, double max_radius, int leaf_size, cudaStream_t s) {
+                                    size_t group_count, double max_radius, cudaStream_t s) {
   size_t total = 0;
   for (size_t g = 0; g < group_count; ++g) {
     const RtdlPointGroupBounds2D& G = groups[g];
@@ -3643,7 +3028,7 @@ PointGroupScene* point_group_create(const RtdlPoint* points, size_t count, const
     }
     if (!boxes.empty())
       RTDL_CUDA_CHECK(cudaMemcpyAsync(pg->boxes, boxes.data(), sizeof(double) * boxes.size(), cudaMemcpyHostToDevice, s));
-    pg->sc = build_scene(d_pts, (uint32_t)total, 2, s, leaf_size);
+    pg->sc = build_scene(d_pts, (uint32_t)total, 2, s);
     unsigned int bad = 0;
     RTDL_CUDA_CHECK(cudaMemcpyAsync(&bad, &pg->sc->stats->bad, sizeof(bad), cudaMemcpyDeviceToHost, s));
     RTDL_CUDA_CHECK(cudaStreamSynchronize(s));  // the host vectors stay alive until the copies are done
@@ -3725,14 +3110,14 @@ QueryResult run_build_and_query(const BuildQueryInputs& in, int predicate, doubl
       RTDL_CUDA_CHECK(cudaMemcpyAsync(*query_owned, in.query_host, qbytes, cudaMemcpyHostToDevice, s));
       q = *query_owned;
     }
-    Scene* sc = build_scene(in.search_dev, in.ns, in.dim, s, scene_leaf_size());
+    Scene* sc = build_scene(in.search_dev, in.ns, in.dim, s);
     *scene_out = sc;
     if (timer) timer->mark("build");
     return run_query(sc, q, in.nq, predicate, radius, limit, rows_dev, rows_capacity, rows_alloc, overflow_dev, s,
                      timer);
   }
   // the query side does not need the scene until its bands: it is prepared on
-  // `aux` (own-box Morton order) while the scene builds on `s`
+  // `aux` (own-box curve order) while the scene builds on `s`
   static thread_local cudaEvent_t ev_start = nullptr, ev_ready = nullptr;
   if (!ev_start) {
     RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_start, cudaEventDisableTiming));
@@ -3740,7 +3125,7 @@ QueryResult run_build_and_query(const BuildQueryInputs& in, int predicate, doubl
   }
   RTDL_CUDA_CHECK(cudaEventRecord(ev_start, s));
   RTDL_CUDA_CHECK(cudaStreamWaitEvent(aux, ev_start, 0));  // whatever the caller queued on s comes first
-  Scene* sc = build_scene(in.search_dev, in.ns, in.dim, s, scene_leaf_size());
+  Scene* sc = build_scene(in.search_dev, in.ns, in.dim, s);
   *scene_out = sc;
   const void* q = in.query_dev;
   if (in.query_host) {  // a pageable copy holds the host; the build is already queued
@@ -3787,7 +3172,7 @@ QueryResult run_build_and_query_chunked(const BuildQueryInputs& in, int predicat
   *scene_out = nullptr;
   const size_t rec = in.dim == 3 ? sizeof(RtdlPoint3D) : sizeof(RtdlPoint);
   const size_t row_size = predicate == kFrn ? sizeof(RtdlFixedRadiusNeighborRow) : sizeof(RtdlKnnNeighborRow);
-  // Each range's query set is uploaded and prepared (Morton order, its own
+  // Each range's query set is uploaded and prepared (curve order, its own
   // statistics) on a third stream one range ahead: the first range's beside
   // the scene build, every later one beside the query of the range before it.
   cudaStream_t ps = aux_stream(1);
@@ -3842,7 +3227,7 @@ QueryResult run_build_and_query_chunked(const BuildQueryInputs& in, int predicat
     RTDL_CUDA_CHECK(cudaEventRecord(ev_start, s));
     RTDL_CUDA_CHECK(cudaStreamWaitEvent(ps, ev_start, 0));
     prepare_range(0);
-    Scene* sc = build_scene(in.search_dev, in.ns, in.dim, s, scene_leaf_size());
+    Scene* sc = build_scene(in.search_dev, in.ns, in.dim, s);
     *scene_out = sc;
     if (timer) timer->mark("build");
     for (int c = 0; c < chunks; ++c) {
@@ -3897,11 +3282,10 @@ constexpr unsigned int kGraphStatusOverflow = 1u;  // traversal stack overflow (
 constexpr unsigned int kGraphStatusGeneric = 2u;   // heavy queries left for the generic path
 constexpr unsigned int kBatchGraphStatusRows = 4u;  // a batch graph's rows exceed the caller's row buffer
 
-__global__ void k_graph_status(const unsigned int* small, const unsigned int* pass_count, uint32_t requests,
-                               unsigned int* status) {
+__global__ void k_graph_status(const unsigned int* small, uint32_t requests, unsigned int* status) {
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < requests; r += gridDim.x * blockDim.x)
     status[r] = ((small[8 * (size_t)r + 1] & 1u) ? kGraphStatusOverflow : 0u) |
-                (pass_count[(size_t)r * kRefinePasses + kRefinePasses - 1] ? kGraphStatusGeneric : 0u);
+                (small[8 * (size_t)r] ? kGraphStatusGeneric : 0u);
 }
 
 
@@ -3916,23 +3300,18 @@ struct SummaryGraph {
   std::vector<uint32_t> kmax;
   std::vector<void*> buffers;  // device, released at destroy
   DevBands* bands = nullptr;   // one per request
-  unsigned long long* slab = nullptr;
+  uint32_t* slab = nullptr;
   uint32_t* counts = nullptr;
   QueryInfo* qinfo = nullptr;
   uint8_t* flags = nullptr;
   uint32_t *heavy_list = nullptr, *heavy_m = nullptr, *heavy_t = nullptr;
+  double* heavy_rad = nullptr;
+  uint32_t* single_list = nullptr;
   uint32_t *mid_list = nullptr, *big_list = nullptr, *fix_list = nullptr;
   unsigned int* small = nullptr;       // 8 counters per request (CollectParams::small)
-  unsigned int* pass_count = nullptr;  // kRefinePasses per request: work left after each pass
   unsigned long long *offsets = nullptr, *poff = nullptr;
   void* scan_ws = nullptr;
   void* rows = nullptr;  // nq * kcap rows
-  uint32_t* work[2] = {nullptr, nullptr};
-  double *rad[2] = {nullptr, nullptr}, *lo[2] = {nullptr, nullptr}, *hi[2] = {nullptr, nullptr};
-  uint32_t* full[2] = {nullptr, nullptr};
-  double* frad[2] = {nullptr, nullptr};
-  double* gen_rad = nullptr;
-  uint32_t *cnt = nullptr, *gen_qin = nullptr, *gen_m = nullptr;
   SummaryPartial* partial = nullptr;
   uint32_t summary_blocks = 0;
   RtdlFixedRadiusRankedNeighborAggregate* agg = nullptr;  // one per request
@@ -3968,7 +3347,6 @@ void graph_enqueue_request(SummaryGraph* g, uint32_t r, cudaStream_t s) {
   const double radius = g->radius[r];
   const uint32_t kmax = g->kmax[r];
   unsigned int* small = g->small + 8 * (size_t)r;
-  unsigned int* pc = g->pass_count + (size_t)r * kRefinePasses;
   k_bands<<<1, 32, 0, s>>>(sc->stats, pq->qst, radius, 1, g->bands + r);
   RTDL_LAUNCHED(1);
   CollectParams C;
@@ -3979,39 +3357,28 @@ void graph_enqueue_request(SummaryGraph* g, uint32_t r, cudaStream_t s) {
   C.qorder = pq->qorder;
   C.nq = np;
   C.kmax = kmax;
+  C.radius = radius;
   C.bands = g->bands + r;
   C.warp_prob = nullptr;
   C.prob_kmax = nullptr;
+  C.prob_radius = nullptr;
   C.slab = g->slab;
   C.counts = g->counts;
   C.qinfo = g->qinfo;
   C.flags = g->flags;
   C.heavy_list = g->heavy_list;
   C.heavy_m = g->heavy_m;
+  C.heavy_rad = g->heavy_rad;
   C.heavy_t = g->heavy_t;
   C.mid_list = g->mid_list;
   C.big_list = g->big_list;
+  C.single_list = g->single_list;
   C.small = small;
   C.overflow_out = nullptr;
+  C.rank_radius = nullptr;
   C.stats = nullptr;
-  launch_collect(C, np, nq, false, false, s);
+  launch_collect(C, np, false, s);
   scan_counts_u64_ws(g->counts, pq->oorder, pq->identity, nq, g->offsets, g->scan_ws, s);
-  // heavy queries: every refinement pass is launched; each reads its work count
-  RefineDevice D;
-  for (int b2 = 0; b2 < 2; ++b2) {
-    D.work[b2] = g->work[b2];
-    D.rad[b2] = g->rad[b2];
-    D.lo[b2] = g->lo[b2];
-    D.hi[b2] = g->hi[b2];
-    D.frad[b2] = g->frad[b2];
-    D.full[b2] = g->full[b2];
-  }
-  D.cnt = g->cnt;
-  D.gen_qin = g->gen_qin;
-  D.gen_m = g->gen_m;
-  D.gen_rad = g->gen_rad;
-  D.pass_count = pc;
-  enqueue_refine_device(C, nullptr, nullptr, radius, nullptr, kmax, np, true, g->qinfo, g->flags, small, D, s);
   k_proc_offsets<<<grid_for(np, 256), 256, 0, s>>>(pq->qorder, pq->qrank, g->offsets, np, g->poff);
   RTDL_LAUNCHED(1);
   EmitParams E;
@@ -4025,15 +3392,14 @@ void graph_enqueue_request(SummaryGraph* g, uint32_t r, cudaStream_t s) {
   E.sink.ranked = 0;
   E.fix_list = g->fix_list;
   E.fix_count = small + 4;
-  k_emit<<<emit_grid(np), kEmitThreads, 0, s>>>(E);
-  k_emit_list<4, true><<<kStrideBlocks, kEmitListThreads, 0, s>>>(E, g->mid_list, 0, small + 2);
-  k_emit_list<8, false><<<kStrideBlocks, kEmitListThreads, 0, s>>>(E, g->big_list, 0, small + 3);
-  k_emit_fixup<<<kSmCount * 4, kFixupThreads, 0, s>>>(E);
+  launch_emit(E, np, s);
+  launch_emit_lists(E, C, np, s);
+  k_emit_fixup<<<list_grid(np), kFixupThreads, 0, s>>>(E);
   k_summarize<<<g->summary_blocks, kSummaryThreads, 0, s>>>(static_cast<const RtdlFixedRadiusNeighborRow*>(g->rows),
                                                             g->offsets, pq->oorder, pq->identity, pq->qpts, nq,
                                                             nullptr, g->partial);
   k_summary_final<<<1, 1024, 0, s>>>(g->partial, g->summary_blocks, nq, g->agg + r);
-  RTDL_LAUNCHED(6);
+  RTDL_LAUNCHED(3);
 }
 
 void graph_release(SummaryGraph* g) {
@@ -4050,9 +3416,8 @@ void graph_capture(SummaryGraph* g) {
   RTDL_CUDA_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   try {
     RTDL_CUDA_CHECK(cudaMemsetAsync(g->small, 0, sizeof(unsigned int) * 8 * (size_t)g->R, s));
-    RTDL_CUDA_CHECK(cudaMemsetAsync(g->pass_count, 0, sizeof(unsigned int) * kRefinePasses * (size_t)g->R, s));
     for (uint32_t r = 0; r < g->R; ++r) graph_enqueue_request(g, r, s);
-    k_graph_status<<<div_up(g->R, 256), 256, 0, s>>>(g->small, g->pass_count, g->R, g->status);
+    k_graph_status<<<div_up(g->R, 256), 256, 0, s>>>(g->small, g->R, g->status);
     RTDL_LAUNCHED(1);
   } catch (...) {
     cudaGraph_t partial = nullptr;
@@ -4129,7 +3494,7 @@ SummaryGraph* summary_graph_create(Scene* sc, const PreparedQueries* pq, const d
     };
     const size_t n = g->nq, R = g->R;
     g->bands = static_cast<DevBands*>(alloc(sizeof(DevBands) * R));
-    g->slab = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * slab_base(g->nq)));
+    g->slab = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * slab_base(g->nq)));
     g->counts = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
     g->qinfo = static_cast<QueryInfo*>(alloc(sizeof(QueryInfo) * n));
     g->flags = static_cast<uint8_t*>(alloc(n));
@@ -4140,23 +3505,12 @@ SummaryGraph* summary_graph_create(Scene* sc, const PreparedQueries* pq, const d
     g->big_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
     g->fix_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
     g->small = static_cast<unsigned int*>(alloc(sizeof(unsigned int) * 8 * R));
-    g->pass_count = static_cast<unsigned int*>(alloc(sizeof(unsigned int) * kRefinePasses * R));
     g->offsets = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * (n + 1)));
     g->poff = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * n));
     g->scan_ws = alloc(scan_workspace_bytes(g->nq));
     graph_size_rows(g);
-    for (int b = 0; b < 2; ++b) {
-      g->work[b] = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
-      g->rad[b] = static_cast<double*>(alloc(sizeof(double) * n));
-      g->lo[b] = static_cast<double*>(alloc(sizeof(double) * n));
-      g->hi[b] = static_cast<double*>(alloc(sizeof(double) * n));
-      g->full[b] = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
-      g->frad[b] = static_cast<double*>(alloc(sizeof(double) * n));
-    }
-    g->cnt = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
-    g->gen_qin = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
-    g->gen_m = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
-    g->gen_rad = static_cast<double*>(alloc(sizeof(double) * n));
+    g->heavy_rad = static_cast<double*>(alloc(sizeof(double) * n));
+    g->single_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
     g->summary_blocks = div_up((uint64_t)n * 32, kSummaryThreads);
     g->partial = static_cast<SummaryPartial*>(alloc(sizeof(SummaryPartial) * g->summary_blocks));
     g->agg = static_cast<RtdlFixedRadiusRankedNeighborAggregate*>(
@@ -4258,7 +3612,7 @@ PreparedQueries* prepare_query_set(const void* records_dev, uint32_t n, int dim,
     k_identity_flag<<<1, 32, 0, s>>>(pq->qst, pq->identity);
     RTDL_LAUNCHED(1);
     uint32_t* codes = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * n1, s));
-    morton_codes(pq->qpts, n, dim, pq->qst, codes, s);  // the set's own box: the order only groups neighbours
+    curve_codes(pq->qpts, n, dim, pq->qst, codes, s);  // the set's own box: the order only groups neighbours
     iota_u32(pq->qorder, n, s);
     radix_sort_pairs(codes, pq->qorder, n, 0, dim == 3 ? 30 : 32, nullptr, &pq->qst->bad, s);
     k_extract_ids<<<grid_for(n, 256), 256, 0, s>>>(pq->qpts, n, codes);
@@ -4311,30 +3665,179 @@ QueryResult run_query_batch(Scene* sc, const void* queries_dev, const BatchSpec&
                           overflow_dev, s, timer, &bs);
 }
 
-// The list kernels take their per-lane lists in dynamic shared memory
-// (block_threads x list length x 8 B, at most kMaxList x 256 x 8 = 128 KiB).
-// The limit a launch may ask for is a per-function attribute of each device:
-// it is raised once per device to that largest size, never per launch, so
-// concurrent calls with different k cannot lower it under one another.
-void ensure_pass1_shared_memory() {
-  static std::mutex m;
-  static std::vector<bool> done;
-  int dev = 0;
-  RTDL_CUDA_CHECK(cudaGetDevice(&dev));
-  std::lock_guard<std::mutex> g(m);
-  if ((int)done.size() <= dev) done.resize(dev + 1, false);
-  if (done[dev]) return;
-  const int most = kMaxList * 256 * 8;
-  RTDL_CUDA_CHECK(cudaFuncSetAttribute(k_pass1<true, true, kWalkRope>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-  RTDL_CUDA_CHECK(cudaFuncSetAttribute(k_pass1<true, false, kWalkRope>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-  RTDL_CUDA_CHECK(cudaFuncSetAttribute(k_pass1<true, true, kWalkNear>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-  RTDL_CUDA_CHECK(cudaFuncSetAttribute(k_pass1<true, false, kWalkNear>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-  RTDL_CUDA_CHECK(cudaFuncSetAttribute(k_pass1<true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-  RTDL_CUDA_CHECK(cudaFuncSetAttribute(k_pass1<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-  RTDL_CUDA_CHECK(cudaFuncSetAttribute(k_pass1<false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-  RTDL_CUDA_CHECK(cudaFuncSetAttribute(k_pass1<false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-  done[dev] = true;
+namespace {
+
+// Row offsets by processing rank when every query has `rows` rows.
+__global__ void k_uniform_offsets(const uint32_t* qorder, const uint32_t* qrank, uint32_t nq, uint32_t rows,
+                                  unsigned long long* poff) {
+  for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < nq; t += (uint64_t)gridDim.x * blockDim.x)
+    poff[t] = (unsigned long long)qrank[qorder[t]] * rows;
 }
+
+template <int KP>
+void launch_knn_radius(const Scene* sc, const QueryPrep& qp, uint32_t nq, uint32_t k, double* radius, cudaStream_t s) {
+  if (sc->dim == 3)
+    k_knn_radius<3, KP><<<div_up(nq, 128), 128, 0, s>>>(sc->view(), sc->codes, qp.qpts, qp.qorder, qp.qcodes, nq, k,
+                                                       qp.bands, radius);
+  else
+    k_knn_radius<2, KP><<<div_up(nq, 128), 128, 0, s>>>(sc->view(), sc->codes, qp.qpts, qp.qorder, qp.qcodes, nq, k,
+                                                       qp.bands, radius);
+  RTDL_LAUNCHED(1);
+}
+
+// Processing ranks answered at a time by run_knn: bounds the slab (4 GiB).
+constexpr uint32_t kKnnRanks = 1u << 22;
+
+// knn_rows with k <= 64: every query has min(k, n) rows, so nothing is scanned
+// and the host reads nothing back before the rows are written.
+QueryResult run_knn(Scene* sc, const void* queries_dev, uint32_t nq, uint32_t k, void* rows_dev, size_t rows_capacity,
+                    void** rows_alloc, uint8_t* overflow_dev, cudaStream_t s, PhaseTimer* timer) {
+  QueryResult res;
+  const int qstride = sc->dim == 3 ? 4 : 3;
+  const uint32_t kk = k < sc->n ? k : sc->n;
+  std::vector<void*> bufs;
+  QueryPrep qp = prepare_queries(sc, queries_dev, nq, false, 0.0, true, s);
+  auto alloc = [&](size_t bytes) {
+    void* p = dev_alloc(bytes ? bytes : 1, s);
+    bufs.push_back(p);
+    return p;
+  };
+  auto cleanup = [&]() {
+    for (void* p : bufs) dev_free(p, s);
+    free_prep(qp, s);
+  };
+  try {
+    uint32_t* qrank = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * nq));
+    k_invert<<<grid_for(nq, 256), 256, 0, s>>>(qp.oorder, nq, qp.order_identity, qrank);
+    RTDL_LAUNCHED(1);
+    if (timer) timer->mark("query_prep");
+    res.rows = (unsigned long long)nq * kk;
+    if (rows_alloc != nullptr) {
+      rows_dev = dev_alloc(sizeof(RtdlKnnNeighborRow) * res.rows, s);
+      rows_capacity = res.rows;
+      *rows_alloc = rows_dev;
+    }
+    if (overflow_dev) RTDL_CUDA_CHECK(cudaMemsetAsync(overflow_dev, 0, nq, s));
+    const bool stats = stats_enabled();
+    if (rows_dev) {
+      const uint32_t most = nq < kKnnRanks ? nq : kKnnRanks;
+      double* radius = static_cast<double*>(alloc(sizeof(double) * nq));
+      unsigned long long* poff = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * nq));
+      k_uniform_offsets<<<grid_for(nq, 256), 256, 0, s>>>(qp.qorder, qrank, nq, kk, poff);
+      RTDL_LAUNCHED(1);
+      if (kk <= 8) launch_knn_radius<8>(sc, qp, nq, k, radius, s);
+      else if (kk <= 16) launch_knn_radius<16>(sc, qp, nq, k, radius, s);
+      else if (kk <= 32) launch_knn_radius<32>(sc, qp, nq, k, radius, s);
+      else launch_knn_radius<64>(sc, qp, nq, k, radius, s);
+      unsigned int* small = static_cast<unsigned int*>(alloc(sizeof(unsigned int) * 8));
+      CollectParams C;
+      C.S = qp.view;
+      C.qpts = qp.qpts;
+      C.qraw = static_cast<const double*>(queries_dev);
+      C.qstride = qstride;
+      C.kmax = kk;
+      C.radius = 0.0;
+      C.bands = qp.bands;
+      C.warp_prob = nullptr;
+      C.prob_kmax = nullptr;
+      C.prob_radius = nullptr;
+      C.slab = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * slab_base(most)));
+      C.counts = nullptr;
+      C.qinfo = static_cast<QueryInfo*>(alloc(sizeof(QueryInfo) * most));
+      C.flags = nullptr;
+      C.heavy_list = C.heavy_m = C.heavy_t = nullptr;
+      C.heavy_rad = nullptr;
+      C.mid_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * most));
+      C.big_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * most));
+      C.single_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * most));
+      C.small = small;
+      C.overflow_out = nullptr;
+      C.stats = nullptr;
+      if (stats) {
+        C.stats = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * kStatCount));
+        RTDL_CUDA_CHECK(cudaMemsetAsync(C.stats, 0, sizeof(unsigned long long) * kStatCount, s));
+      }
+      EmitParams E;
+      E.S = sc->view();
+      E.slab = C.slab;
+      E.qinfo = C.qinfo;
+      E.sink.rows = rows_dev;
+      E.sink.capacity = rows_capacity;
+      E.sink.ranked = 1;
+      E.fix_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * most));
+      E.fix_count = small + 4;
+      for (uint32_t t0 = 0; t0 < nq; t0 += most) {  // kernels see one range of ranks at a time
+        const uint32_t np = nq - t0 < most ? nq - t0 : most;
+        RTDL_CUDA_CHECK(cudaMemsetAsync(small, 0, sizeof(unsigned int) * 8, s));
+        C.qorder = qp.qorder + t0;
+        C.nq = np;
+        C.rank_radius = radius + t0;
+        E.nq = np;
+        E.poff = poff + t0;
+        SingleParams H{};
+        H.S = sc->view();
+        H.qpts = qp.qpts;
+        H.qraw = C.qraw;
+        H.qstride = qstride;
+        H.bands = qp.bands;
+        H.k = kk;
+        H.qorder = C.qorder;
+        H.rank_radius = C.rank_radius;
+        H.poff = E.poff;
+        H.sink = E.sink;
+        if (np <= kSingleQueries) {  // too few for packets: a warp per query throughout
+          H.nwork = np;
+          k_knn_single<<<div_up(np, 256 / 32), 256, 0, s>>>(H);
+          RTDL_LAUNCHED(1);
+          continue;
+        }
+        launch_collect(C, np, false, s);
+        // the queries the packets left, beside the emit kernels (disjoint rows)
+        static thread_local cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+        if (!ev_fork) {
+          RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
+          RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
+        }
+        cudaStream_t ls = aux_stream();
+        RTDL_CUDA_CHECK(cudaEventRecord(ev_fork, s));
+        RTDL_CUDA_CHECK(cudaStreamWaitEvent(ls, ev_fork, 0));
+        H.work = C.single_list;
+        H.nwork_dev = small + 6;
+        k_knn_single<<<kSmCount * 4, 256, 0, ls>>>(H);
+        launch_emit_lists(E, C, np, ls);
+        RTDL_CUDA_CHECK(cudaEventRecord(ev_join, ls));
+        launch_emit(E, np, s);
+        RTDL_CUDA_CHECK(cudaStreamWaitEvent(s, ev_join, 0));
+        k_emit_fixup<<<list_grid(np), kFixupThreads, 0, s>>>(E);
+        RTDL_LAUNCHED(2);
+      }
+      if (stats)
+        RTDL_CUDA_CHECK(cudaMemcpyAsync(last_stats().data(), C.stats, sizeof(unsigned long long) * kStatCount,
+                                        cudaMemcpyDeviceToHost, s));
+    }
+    if (timer) timer->mark("traverse");
+    Readback* rb = pinned_readback();
+    SmallReads reads(rb);
+    reads.add(&rb->scene_bad, &sc->stats->bad, sizeof(unsigned int));
+    reads.add(&rb->query_bad, &qp.qst->bad, sizeof(unsigned int));
+    reads.launch(s);
+    RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
+    throw_if_bad(rb->scene_bad | rb->query_bad);
+  } catch (...) {
+    sync_quietly(s);
+    sync_quietly(aux_stream());  // the list kernels may run there
+    if (rows_alloc && *rows_alloc) {
+      dev_free(*rows_alloc, s);
+      *rows_alloc = nullptr;
+    }
+    cleanup();
+    throw;
+  }
+  cleanup();
+  return res;
+}
+
+}  // namespace
 
 QueryResult run_query(Scene* sc, const void* queries_dev, uint32_t nq, int predicate, double radius, uint32_t limit,
                       void* rows_dev, size_t rows_capacity, void** rows_alloc, uint8_t* overflow_dev, cudaStream_t s,
@@ -4342,7 +3845,6 @@ QueryResult run_query(Scene* sc, const void* queries_dev, uint32_t nq, int predi
   QueryResult res;
   if (rows_alloc) *rows_alloc = nullptr;
   if (sc->problems) throw std::runtime_error("a problem batch is queried with the batch entry points");
-  const bool knn = predicate == kKnn;
   const int qstride = sc->dim == 3 ? 4 : 3;
   if (nq == 0) return res;
   if (sc->n == 0) {
@@ -4350,17 +3852,17 @@ QueryResult run_query(Scene* sc, const void* queries_dev, uint32_t nq, int predi
     return res;
   }
   if (timer) timer->mark("start");
-  if (!knn && limit <= (uint32_t)kMaxList)
+  if (predicate != kKnn)
     return run_radius_query(sc, queries_dev, nq, predicate, radius, limit, rows_dev, rows_capacity, rows_alloc,
                             overflow_dev, s, timer);
-  QueryPrep qp = prepare_queries(sc, queries_dev, nq, !knn, radius, true, s);
-  const bool all_heavy = knn && limit > (uint32_t)kMaxList;
-  const int L = all_heavy ? 1 : (int)(limit < (uint32_t)kMaxList ? limit : (uint32_t)kMaxList);
+  if (limit <= (uint32_t)kMaxList)
+    return run_knn(sc, queries_dev, nq, limit, rows_dev, rows_capacity, rows_alloc, overflow_dev, s, timer);
+  // k > 64: every query takes the generic path over the whole scene
+  QueryPrep qp = prepare_queries(sc, queries_dev, nq, false, radius, true, s);
   if (timer) timer->mark("query_prep");
-
   uint32_t* counts = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq, s));
   uint8_t* flags = static_cast<uint8_t*>(dev_alloc(nq, s));
-  uint32_t* temp = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * (size_t)nq * L, s));
+  uint32_t* temp = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * (size_t)nq, s));
   uint32_t* heavy_list = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq, s));
   uint32_t* heavy_m = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq, s));
   unsigned int* small = static_cast<unsigned int*>(dev_alloc(sizeof(unsigned int) * 4, s));  // heavy count, error
@@ -4379,59 +3881,9 @@ QueryResult run_query(Scene* sc, const void* queries_dev, uint32_t nq, int predi
     free_prep(qp, s);
   };
   try {
-    if (all_heavy) {
-      k_mark_all_heavy<<<grid_for(nq, 256), 256, 0, s>>>(qp.qorder, nq, sc->n, limit, counts, flags, temp,
-                                                         heavy_list, heavy_m);
-      RTDL_LAUNCHED(1);
-      RTDL_CUDA_CHECK(cudaMemcpyAsync(small, &nq, sizeof(uint32_t), cudaMemcpyHostToDevice, s));
-      RTDL_CUDA_CHECK(cudaStreamSynchronize(s));  // nq lives on this host stack frame
-    } else {
-      Pass1Params P;
-      P.S = sc->view();
-      P.qpts = qp.qpts;
-      P.qraw = static_cast<const double*>(queries_dev);
-      P.qstride = qstride;
-      P.qorder = qp.qorder;
-      P.nq = nq;
-      P.kmax = limit;
-      P.L = L;
-      P.bands = qp.bands;
-      P.temp = temp;
-      P.counts = counts;
-      P.flags = flags;
-      P.heavy_list = heavy_list;
-      P.heavy_m = heavy_m;
-      P.heavy_count = small;
-      P.error = small + 1;
-      const int threads = tuning().block_threads;
-      const size_t shm = (size_t)threads * L * 8;
-      const unsigned int blocks = div_up(nq, threads);
-      const bool stats = stats_enabled();
-      P.stats = nullptr;
-      P.qcodes = qp.qcodes;
-      P.scodes = sc->codes;
-      if (stats) {
-        P.stats = static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long) * kStatCount, s));
-        RTDL_CUDA_CHECK(cudaMemsetAsync(P.stats, 0, sizeof(unsigned long long) * kStatCount, s));
-      }
-      ensure_pass1_shared_memory();
-      auto launch = [&](auto kernel) { kernel<<<blocks, threads, shm, s>>>(P); };
-      const int walk = tuning().traversal == 1 ? kWalkLane : L >= kNearFirstMinList ? kWalkNear : kWalkRope;
-      if (knn) {
-        if (walk == kWalkNear) stats ? launch(k_pass1<true, true, kWalkNear>) : launch(k_pass1<true, false, kWalkNear>);
-        else if (walk == kWalkRope) stats ? launch(k_pass1<true, true, kWalkRope>) : launch(k_pass1<true, false, kWalkRope>);
-        else stats ? launch(k_pass1<true, true>) : launch(k_pass1<true, false>);
-      } else {
-        if (stats) launch(k_pass1<false, true>);
-        else launch(k_pass1<false, false>);
-      }
-      RTDL_LAUNCHED(1);
-      if (stats) {
-        RTDL_CUDA_CHECK(cudaMemcpyAsync(last_stats().data(), P.stats, sizeof(unsigned long long) * kStatCount,
-                                        cudaMemcpyDeviceToHost, s));
-        dev_free(P.stats, s);
-      }
-    }
+    k_mark_all_heavy<<<grid_for(nq, 256), 256, 0, s>>>(qp.qorder, nq, sc->n, limit, counts, flags, temp, heavy_list,
+                                                       heavy_m);
+    RTDL_LAUNCHED(1);
     if (timer) timer->mark("traverse");
     scan_counts_u64(counts, qp.oorder, &qp.bands->ids_sorted, nq, offsets, s);
     if (timer) timer->mark("scan");
@@ -4439,22 +3891,17 @@ QueryResult run_query(Scene* sc, const void* queries_dev, uint32_t nq, int predi
     Readback* rb = pinned_readback();
     SmallReads reads(rb);
     reads.add(&rb->rows, offsets + nq, sizeof(unsigned long long));
-    reads.add(&rb->heavy, small, sizeof(unsigned int) * 2);
     reads.add(&rb->scene_bad, &sc->stats->bad, sizeof(unsigned int));
     reads.add(&rb->query_bad, &qp.qst->bad, sizeof(unsigned int));
     reads.launch(s);
     RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
-    const Readback r = *rb;
-    check_readback(r);
-    res.rows = r.rows;
-    res.heavy = r.heavy;
-    if (r.heavy > 0) {
-      g = run_generic_path(sc, qp, queries_dev, qstride, r.heavy, heavy_list, heavy_m, limit, knn, small + 1, s);
-      if (timer) timer->mark("generic_path");
-    }
+    throw_if_bad(rb->scene_bad | rb->query_bad);
+    res.rows = rb->rows;
+    res.heavy = nq;
+    g = run_generic_path(sc, qp, queries_dev, qstride, nq, heavy_list, heavy_m, limit, true, small + 1, s);
+    if (timer) timer->mark("generic_path");
     if (rows_alloc != nullptr) {
-      const size_t row_size = predicate == kFrn ? 16 : 24;
-      rows_dev = res.rows ? dev_alloc(row_size * res.rows, s) : nullptr;
+      rows_dev = res.rows ? dev_alloc(sizeof(RtdlKnnNeighborRow) * res.rows, s) : nullptr;
       rows_capacity = res.rows;
       *rows_alloc = rows_dev;
     }
@@ -4467,7 +3914,7 @@ QueryResult run_query(Scene* sc, const void* queries_dev, uint32_t nq, int predi
       E.oorder = qp.oorder;
       E.bands = qp.bands;
       E.nq = nq;
-      E.L = L;
+      E.L = 1;
       E.counts = counts;
       E.flags = flags;
       E.temp = temp;
@@ -4476,28 +3923,17 @@ QueryResult run_query(Scene* sc, const void* queries_dev, uint32_t nq, int predi
       E.offsets = offsets;
       E.rows = rows_dev;
       E.capacity = rows_dev ? rows_capacity : 0;
-      E.ranked = predicate == kFrn ? 0 : 1;
+      E.ranked = 1;
       E.overflow_out = overflow_dev;
       E.error = small + 1;
       E.work_list = nullptr;
       E.qrank = nullptr;
-      // lists of at most L rows unless some query took the generic path
-      const int group = (r.heavy > 0 || L > 16) ? 32 : L > 8 ? 16 : L > 4 ? 8 : L > 2 ? 4 : L > 1 ? 2 : 1;
-      const unsigned int blocks = grid_for((uint64_t)nq * group, kExpandThreads);
-      switch (group) {
-        case 1: k_expand<1><<<blocks, kExpandThreads, 0, s>>>(E); break;
-        case 2: k_expand<2><<<blocks, kExpandThreads, 0, s>>>(E); break;
-        case 4: k_expand<4><<<blocks, kExpandThreads, 0, s>>>(E); break;
-        case 8: k_expand<8><<<blocks, kExpandThreads, 0, s>>>(E); break;
-        case 16: k_expand<16><<<blocks, kExpandThreads, 0, s>>>(E); break;
-        default: k_expand<32><<<blocks, kExpandThreads, 0, s>>>(E); break;
-      }
+      k_expand<<<grid_for((uint64_t)nq * 32, kExpandThreads), kExpandThreads, 0, s>>>(E);
       RTDL_LAUNCHED(1);
     }
     if (timer) timer->mark("emit");
     RTDL_CUDA_CHECK(cudaMemcpyAsync(&rb->error, small + 1, sizeof(unsigned int), cudaMemcpyDeviceToHost, s));
     RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
-    if (rb->error & 8u) throw std::runtime_error("LBVH traversal stack overflow");
     if (rb->error & 6u) throw std::runtime_error("generic neighbor path produced an inconsistent candidate count");
   } catch (...) {
     sync_quietly(s);
@@ -4516,36 +3952,22 @@ HausdorffResult run_directed_hausdorff(Scene* sc, const void* queries_dev, uint3
   if (timer) timer->mark("start");
   QueryPrep qp = prepare_queries(sc, queries_dev, nq, false, 0.0, false, s);
   if (timer) timer->mark("query_prep");
-  uint32_t* counts = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq, s));
-  uint8_t* flags = static_cast<uint8_t*>(dev_alloc(nq, s));
   uint32_t* temp = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq, s));
-  unsigned int* small = static_cast<unsigned int*>(dev_alloc(sizeof(unsigned int) * 4, s));
-  RTDL_CUDA_CHECK(cudaMemsetAsync(small, 0, sizeof(unsigned int) * 4, s));
-  Pass1Params P;
+  NearestParams P;
   P.S = sc->view();
   P.qpts = qp.qpts;
   P.qraw = static_cast<const double*>(queries_dev);
   P.qstride = qstride;
   P.qorder = qp.qorder;
-  P.nq = nq;
-  P.kmax = 1;
-  P.L = 1;
-  P.bands = qp.bands;
-  P.temp = temp;
-  P.counts = counts;
-  P.flags = flags;
-  P.heavy_list = nullptr;
-  P.heavy_m = nullptr;
-  P.heavy_count = small;
-  P.error = small + 1;
-  const int threads = tuning().block_threads;
-  P.stats = nullptr;
   P.qcodes = qp.qcodes;
   P.scodes = sc->codes;
-  if (tuning().traversal != 1)
-    k_pass1<true, false, kWalkRope><<<div_up(nq, threads), threads, (size_t)threads * 8, s>>>(P);
+  P.nq = nq;
+  P.bands = qp.bands;
+  P.nearest = temp;
+  if (sc->dim == 3)
+    k_nearest<3><<<div_up(nq, 128), 128, 0, s>>>(P);
   else
-    k_pass1<true, false><<<div_up(nq, threads), threads, (size_t)threads * 8, s>>>(P);
+    k_nearest<2><<<div_up(nq, 128), 128, 0, s>>>(P);
   RTDL_LAUNCHED(1);
   if (timer) timer->mark("traverse");
   const unsigned int blocks = grid_for(nq, 256) < 2 * kSmCount ? grid_for(nq, 256) : 2 * kSmCount;
@@ -4562,22 +3984,17 @@ HausdorffResult run_directed_hausdorff(Scene* sc, const void* queries_dev, uint3
   reads.add(rb->chunk_rows, best, sizeof(Witness));
   reads.add(&rb->scene_bad, &sc->stats->bad, sizeof(unsigned int));
   reads.add(&rb->query_bad, &qp.qst->bad, sizeof(unsigned int));
-  reads.add(&rb->error, small + 1, sizeof(unsigned int));
   reads.launch(s);
   RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
   Witness w;
   memcpy(&w, rb->chunk_rows, sizeof(Witness));
-  const unsigned int bad[3] = {rb->scene_bad, rb->query_bad, rb->error};
+  const unsigned int bad = rb->scene_bad | rb->query_bad;
   if (timer) timer->mark("reduce");
-  dev_free(counts, s);
-  dev_free(flags, s);
   dev_free(temp, s);
-  dev_free(small, s);
   dev_free(partial, s);
   dev_free(best, s);
   free_prep(qp, s);
-  throw_if_bad(bad[0] | bad[1]);
-  if (bad[2] & 8u) throw std::runtime_error("LBVH traversal stack overflow");
+  throw_if_bad(bad);
   HausdorffResult out;
   unsigned long long db = w.dist;
   memcpy(&out.distance, &db, sizeof(double));
@@ -4606,15 +4023,11 @@ constexpr size_t align256(size_t v) { return (v + 255) & ~(size_t)255; }
 struct NoAllocLayout {  // byte offsets into the scratch array, 256-B aligned
   static constexpr size_t kStats = 0;
   static constexpr size_t kBands = align256(kStats + sizeof(PointStats));
-  static constexpr size_t kSmall = align256(kBands + sizeof(DevBands));
-  static constexpr size_t kBest = align256(kSmall + 4 * sizeof(unsigned int));
+  static constexpr size_t kBest = align256(kBands + sizeof(DevBands));
   static constexpr size_t kPartial = align256(kBest + sizeof(Witness));
   static constexpr size_t kQpts = align256(kPartial + kNoAllocReduceBlocks * sizeof(Witness));
-  static constexpr size_t kOrder = align256(kQpts + (size_t)kNoAllocMaxQueries * sizeof(float4));
-  static constexpr size_t kTemp = align256(kOrder + (size_t)kNoAllocMaxQueries * sizeof(uint32_t));
-  static constexpr size_t kCounts = align256(kTemp + (size_t)kNoAllocMaxQueries * sizeof(uint32_t));
-  static constexpr size_t kFlags = align256(kCounts + (size_t)kNoAllocMaxQueries * sizeof(uint32_t));
-  static constexpr size_t kCodes = align256(kFlags + (size_t)kNoAllocMaxQueries);
+  static constexpr size_t kTemp = align256(kQpts + (size_t)kNoAllocMaxQueries * sizeof(float4));
+  static constexpr size_t kCodes = align256(kTemp + (size_t)kNoAllocMaxQueries * sizeof(uint32_t));
   static constexpr size_t kTotal = align256(kCodes + (size_t)kNoAllocMaxQueries * sizeof(uint32_t));
 };
 
@@ -4669,45 +4082,29 @@ void run_directed_hausdorff_noalloc(Scene* sc, const void* queries_dev, uint32_t
   unsigned char* base = noalloc_scratch_for_current_device();
   PointStats* qst = reinterpret_cast<PointStats*>(base + NoAllocLayout::kStats);
   DevBands* bands = reinterpret_cast<DevBands*>(base + NoAllocLayout::kBands);
-  unsigned int* small = reinterpret_cast<unsigned int*>(base + NoAllocLayout::kSmall);
   Witness* best = reinterpret_cast<Witness*>(base + NoAllocLayout::kBest);
   Witness* partial = reinterpret_cast<Witness*>(base + NoAllocLayout::kPartial);
   float4* qpts = reinterpret_cast<float4*>(base + NoAllocLayout::kQpts);
-  uint32_t* qorder = reinterpret_cast<uint32_t*>(base + NoAllocLayout::kOrder);
   uint32_t* temp = reinterpret_cast<uint32_t*>(base + NoAllocLayout::kTemp);
-  uint32_t* counts = reinterpret_cast<uint32_t*>(base + NoAllocLayout::kCounts);
-  uint8_t* flags = reinterpret_cast<uint8_t*>(base + NoAllocLayout::kFlags);
   uint32_t* codes = reinterpret_cast<uint32_t*>(base + NoAllocLayout::kCodes);
   // The array keeps the previous call's contents: reset what must start at zero.
   reset_stats(qst, s);
-  RTDL_CUDA_CHECK(cudaMemsetAsync(small, 0, 4 * sizeof(unsigned int), s));
   prep_points(queries_dev, nq, sc->dim, qpts, qst, s);
   k_bands<<<1, 32, 0, s>>>(sc->stats, qst, 0.0, 0, bands);
   RTDL_LAUNCHED(1);
-  iota_u32(qorder, nq, s);  // input order: no sort, hence no sort scratch
-  morton_codes(qpts, nq, sc->dim, sc->stats, codes, s);  // seeds the nearest search (input order)
-  Pass1Params P;
+  curve_codes(qpts, nq, sc->dim, sc->stats, codes, s);  // input order (no sort, hence no sort scratch)
+  SingleParams P{};
   P.S = sc->view();
   P.qpts = qpts;
   P.qraw = static_cast<const double*>(queries_dev);
   P.qstride = sc->dim == 3 ? 4 : 3;
-  P.qorder = qorder;
-  P.nq = nq;
-  P.kmax = 1;
-  P.L = 1;
   P.bands = bands;
-  P.temp = temp;
-  P.counts = counts;
-  P.flags = flags;
-  P.heavy_list = nullptr;
-  P.heavy_m = nullptr;
-  P.heavy_count = small;
-  P.error = small + 1;
-  P.stats = nullptr;
+  P.k = 1;
+  P.nwork = nq;
   P.qcodes = codes;
   P.scodes = sc->codes;
-  const int threads = tuning().block_threads;
-  k_pass1<true, false><<<div_up(nq, threads), threads, (size_t)threads * 8, s>>>(P);
+  P.nearest = temp;
+  k_knn_single<<<grid_for((uint64_t)nq * 32, 256), 256, 0, s>>>(P);
   RTDL_LAUNCHED(1);
   const unsigned int blocks = grid_for(nq, 256) < kNoAllocReduceBlocks ? grid_for(nq, 256) : kNoAllocReduceBlocks;
   k_nearest_reduce<<<blocks, 256, 0, s>>>(sc->view(), qpts, static_cast<const double*>(queries_dev), P.qstride, nq,
@@ -4720,7 +4117,7 @@ void run_directed_hausdorff_noalloc(Scene* sc, const void* queries_dev, uint32_t
 
 // ---- captured graphs over prepared problem batches --------------------------
 // Many uneven fixed-radius problems, already built into problem batches
-// (build_scene_batch: one LBVH per batch, each problem one subtree), answered
+// (build_scene_batch: each problem a tree of its own), answered
 // by one CUDA graph replay with no host read-back inside.  Per batch the graph
 // holds ONE persistent collect launch -- a grid that fills the GPU once, whose
 // warps take 32-query packets (one problem each) from a device work queue
@@ -4751,8 +4148,9 @@ __global__ void k_empty_batch_rows(const unsigned long long* base, uint32_t prob
 }
 
 // Persistent collect over one batch: 32-query packets from a work queue.
-template <int MIN_BLOCKS, int LEAF>
-__global__ void __launch_bounds__(256, MIN_BLOCKS) k_collect_persistent(CollectParams P, unsigned int* queue) {
+template <int DIM>
+__global__ void __launch_bounds__(kCollectThreads, 6) k_collect_persistent(const __grid_constant__ CollectParams P, unsigned int* queue) {
+  __shared__ CollectWarp warps[kCollectThreads / 32];
   const uint32_t packets = (P.nq + 31u) / 32u;
   const uint32_t lane = threadIdx.x & 31u;
   for (;;) {
@@ -4760,18 +4158,15 @@ __global__ void __launch_bounds__(256, MIN_BLOCKS) k_collect_persistent(CollectP
     if (lane == 0) item = atomicAdd(queue, 1u);
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= packets) return;
-    collect_packet_body<false, false, true, LEAF>(P, item * 32u + lane);
+    collect_packet_body<DIM, true, false>(P, item * 32u + lane, warps[threadIdx.x >> 5]);
   }
 }
 
-constexpr int kPersistentMinBlocks = 5;
-
-__global__ void k_batch_graph_status(const unsigned int* small, const unsigned int* pass_count, uint32_t batches,
-                                     const unsigned long long* total, unsigned long long capacity,
+__global__ void k_batch_graph_status(const unsigned int* small, uint32_t batches, const unsigned long long* total, unsigned long long capacity,
                                      unsigned int* status) {
   for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < batches; b += gridDim.x * blockDim.x)
     status[b] = ((small[8 * (size_t)b + 1] & 1u) ? kGraphStatusOverflow : 0u) |
-                (pass_count[(size_t)b * kRefinePasses + kRefinePasses - 1] ? kGraphStatusGeneric : 0u) |
+                (small[8 * (size_t)b] ? kGraphStatusGeneric : 0u) |
                 (*total > capacity ? kBatchGraphStatusRows : 0u);
 }
 
@@ -4799,18 +4194,18 @@ struct BatchGraph {
   unsigned long long capacity = 0;
   std::vector<void*> buffers;
   // scratch shared by the batches (sized for the largest)
-  unsigned long long* slab = nullptr;
+  uint32_t* slab = nullptr;
   uint32_t* counts = nullptr;
   QueryInfo* qinfo = nullptr;
   uint8_t* flags = nullptr;
   uint32_t *heavy_list = nullptr, *heavy_m = nullptr, *heavy_t = nullptr;
+  double* heavy_rad = nullptr;
+  uint32_t* single_list = nullptr;
   uint32_t *mid_list = nullptr, *big_list = nullptr, *fix_list = nullptr;
   unsigned long long* poff = nullptr;
   void* scan_ws = nullptr;
-  RefineDevice D{};
   // per batch
   unsigned int* small = nullptr;        // 8 counters per batch
-  unsigned int* pass_count = nullptr;   // kRefinePasses per batch
   unsigned int* queue = nullptr;        // work-queue counter per batch
   unsigned long long* base = nullptr;   // batches + 1: first row of each batch, then the total
   unsigned long long* prob_rows = nullptr;  // problems + 1: first row of each problem, then the total
@@ -4818,7 +4213,6 @@ struct BatchGraph {
   unsigned int* status_host = nullptr;      // pinned
   unsigned long long* rows_host = nullptr;  // pinned, problems + 1
   unsigned int persistent_grid = 0;
-  bool hybrid = true;  // leaf buckets tested lane- or point-major per bucket (the tuning at creation)
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
   int kernels = 0;
@@ -4846,35 +4240,38 @@ void batch_graph_enqueue(BatchGraph* g, uint32_t i, cudaStream_t s) {
   C.qorder = b.qp.qorder;
   C.nq = b.qp.nproc;
   C.kmax = kmax;
+  C.width = 32;
+  C.radius = 0.0;
   C.bands = b.qp.bands;
   C.warp_prob = b.qp.warp_prob;
   C.prob_kmax = b.qp.prob_kmax;
+  C.prob_radius = b.qp.prob_radius;
   C.slab = g->slab;
   C.counts = g->counts;
   C.qinfo = g->qinfo;
   C.flags = g->flags;
   C.heavy_list = g->heavy_list;
   C.heavy_m = g->heavy_m;
+  C.heavy_rad = g->heavy_rad;
   C.heavy_t = g->heavy_t;
   C.mid_list = g->mid_list;
   C.big_list = g->big_list;
+  C.single_list = g->single_list;
   C.small = small;
   C.overflow_out = nullptr;
+  C.rank_radius = nullptr;
   C.stats = nullptr;
   const uint32_t np = b.qp.nproc;
-  if (g->hybrid)
-    k_collect_persistent<kPersistentMinBlocks, kLeafHybrid><<<g->persistent_grid, 256, 0, s>>>(C, g->queue + i);
+  if (b.sc->dim == 3)
+    k_collect_persistent<3><<<g->persistent_grid, kCollectThreads, 0, s>>>(C, g->queue + i);
   else
-    k_collect_persistent<kPersistentMinBlocks, kLeafLaneMajor><<<g->persistent_grid, 256, 0, s>>>(C, g->queue + i);
+    k_collect_persistent<2><<<g->persistent_grid, kCollectThreads, 0, s>>>(C, g->queue + i);
+  launch_collect_left(C, b.qp.nproc, s);
   RTDL_LAUNCHED(1);
   scan_counts_u64_ws(g->counts, b.qp.oorder, b.qp.order_identity, b.nq, b.offsets, g->scan_ws, s);
   k_add_row_base<<<grid_for(b.nq + 1, 256), 256, 0, s>>>(b.offsets, b.nq, g->base + i, g->base + i + 1);
   k_problem_rows<<<div_up(b.problems + 1, 256), 256, 0, s>>>(b.offsets, b.qp.qoff, b.problems, g->prob_rows + b.p0);
   RTDL_LAUNCHED(2);
-  RefineDevice D = g->D;
-  D.pass_count = g->pass_count + (size_t)i * kRefinePasses;
-  enqueue_refine_device(C, b.qp.qprob, b.qp.prob_radius, 0.0, b.qp.prob_kmax, kmax, np, false, g->qinfo, g->flags,
-                        small, D, s);
   k_proc_offsets<<<grid_for(np, 256), 256, 0, s>>>(b.qp.qorder, b.qrank, b.offsets, np, g->poff);
   RTDL_LAUNCHED(1);
   EmitParams E;
@@ -4888,11 +4285,10 @@ void batch_graph_enqueue(BatchGraph* g, uint32_t i, cudaStream_t s) {
   E.sink.ranked = 0;
   E.fix_list = g->fix_list;
   E.fix_count = small + 4;
-  k_emit<<<emit_grid(np), kEmitThreads, 0, s>>>(E);
-  k_emit_list<4, true><<<kStrideBlocks, kEmitListThreads, 0, s>>>(E, g->mid_list, 0, small + 2);
-  k_emit_list<8, false><<<kStrideBlocks, kEmitListThreads, 0, s>>>(E, g->big_list, 0, small + 3);
-  k_emit_fixup<<<kSmCount * 4, kFixupThreads, 0, s>>>(E);
-  RTDL_LAUNCHED(4);
+  launch_emit(E, np, s);
+  launch_emit_lists(E, C, np, s);
+  k_emit_fixup<<<list_grid(np), kFixupThreads, 0, s>>>(E);
+  RTDL_LAUNCHED(1);
 }
 
 void batch_graph_release(BatchGraph* g) {
@@ -4910,11 +4306,10 @@ void batch_graph_capture(BatchGraph* g) {
   RTDL_CUDA_CHECK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
   try {
     RTDL_CUDA_CHECK(cudaMemsetAsync(g->small, 0, sizeof(unsigned int) * 8 * (size_t)B, s));
-    RTDL_CUDA_CHECK(cudaMemsetAsync(g->pass_count, 0, sizeof(unsigned int) * kRefinePasses * (size_t)B, s));
     RTDL_CUDA_CHECK(cudaMemsetAsync(g->queue, 0, sizeof(unsigned int) * B, s));
     RTDL_CUDA_CHECK(cudaMemsetAsync(g->base, 0, sizeof(unsigned long long), s));
     for (uint32_t i = 0; i < B; ++i) batch_graph_enqueue(g, i, s);
-    k_batch_graph_status<<<div_up(B, 256), 256, 0, s>>>(g->small, g->pass_count, B, g->base + B, g->capacity,
+    k_batch_graph_status<<<div_up(B, 256), 256, 0, s>>>(g->small, B, g->base + B, g->capacity,
                                                         g->status);
     RTDL_LAUNCHED(1);
   } catch (...) {
@@ -5009,7 +4404,7 @@ BatchGraph* batch_graph_create(Scene* const* batches, uint32_t batch_count, cons
       g->buffers.push_back(p);
       return p;
     };
-    g->slab = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * slab_base((uint32_t)n)));
+    g->slab = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * slab_base((uint32_t)n)));
     g->counts = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * nqm));
     g->qinfo = static_cast<QueryInfo*>(alloc(sizeof(QueryInfo) * n));
     g->flags = static_cast<uint8_t*>(alloc(nqm));
@@ -5021,20 +4416,9 @@ BatchGraph* batch_graph_create(Scene* const* batches, uint32_t batch_count, cons
     g->fix_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
     g->poff = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * n));
     g->scan_ws = alloc(scan_workspace_bytes((uint32_t)nqm));
-    for (int k = 0; k < 2; ++k) {
-      g->D.work[k] = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
-      g->D.rad[k] = static_cast<double*>(alloc(sizeof(double) * n));
-      g->D.lo[k] = static_cast<double*>(alloc(sizeof(double) * n));
-      g->D.hi[k] = static_cast<double*>(alloc(sizeof(double) * n));
-      g->D.full[k] = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
-      g->D.frad[k] = static_cast<double*>(alloc(sizeof(double) * n));
-    }
-    g->D.cnt = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * nqm));
-    g->D.gen_qin = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * nqm));
-    g->D.gen_m = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * nqm));
-    g->D.gen_rad = static_cast<double*>(alloc(sizeof(double) * nqm));
+    g->heavy_rad = static_cast<double*>(alloc(sizeof(double) * nqm));
+    g->single_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
     g->small = static_cast<unsigned int*>(alloc(sizeof(unsigned int) * 8 * B));
-    g->pass_count = static_cast<unsigned int*>(alloc(sizeof(unsigned int) * kRefinePasses * B));
     g->queue = static_cast<unsigned int*>(alloc(sizeof(unsigned int) * B));
     g->base = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * (B + 1)));
     g->prob_rows = static_cast<unsigned long long*>(alloc(sizeof(unsigned long long) * ((size_t)g->problems + 1)));
@@ -5042,14 +4426,13 @@ BatchGraph* batch_graph_create(Scene* const* batches, uint32_t batch_count, cons
     RTDL_CUDA_CHECK(cudaMemsetAsync(g->prob_rows, 0, sizeof(unsigned long long) * ((size_t)g->problems + 1), s));
     RTDL_CUDA_CHECK(cudaMallocHost(&g->status_host, sizeof(unsigned int) * B));
     RTDL_CUDA_CHECK(cudaMallocHost(&g->rows_host, sizeof(unsigned long long) * ((size_t)g->problems + 1)));
-    g->hybrid = tuning().traversal == 4;
     int per_sm = 0;
-    if (g->hybrid)
-      RTDL_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per_sm, k_collect_persistent<kPersistentMinBlocks, kLeafHybrid>, 256, 0));
+    if (batches[0]->dim == 3)
+      RTDL_CUDA_CHECK(
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_collect_persistent<3>, kCollectThreads, 0));
     else
-      RTDL_CUDA_CHECK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-          &per_sm, k_collect_persistent<kPersistentMinBlocks, kLeafLaneMajor>, 256, 0));
+      RTDL_CUDA_CHECK(
+          cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_collect_persistent<2>, kCollectThreads, 0));
     int sms = kSmCount;
     RTDL_CUDA_CHECK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, g->device));
     g->persistent_grid = (unsigned int)(sms * (per_sm > 0 ? per_sm : 1));

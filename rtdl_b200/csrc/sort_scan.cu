@@ -1,6 +1,6 @@
 // sort_scan.cu -- device prefix scans and a stable LSD radix sort, written for
-// this library (no CUB): the LBVH build sorts Morton codes with it, the query
-// path sorts queries into Morton order and into query-id order, and row
+// this library (no CUB): the LBVH build sorts curve codes with it, the query
+// path sorts queries into curve order and into query-id order, and row
 // offsets come from the scan.
 //
 // Scan: reduce-then-scan over 2,048-element tiles (256 threads x 8 items), a
