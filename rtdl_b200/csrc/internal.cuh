@@ -209,13 +209,23 @@ size_t scan_workspace_bytes(uint32_t n);
 void scan_counts_u64_ws(const uint32_t* counts, const uint32_t* order, const unsigned int* identity_flag, uint32_t n,
                         unsigned long long* out, void* workspace, cudaStream_t s);
 // Stable LSD radix sort of (key, value) pairs over bits [begin_bit, end_bit),
-// 8 bits per pass.  The result is left in keys/vals.  When *skip_flag != 0
-// (device memory) every pass returns immediately and the input stays in place.
+// 8 bits per pass.  The result is left in keys/vals.  iota: the values of the
+// input are 0, 1, ... (vals is only written).  When *skip_flag != 0 (device
+// memory) every pass returns immediately and keys/vals stay as they are.
 // A look-back wait that runs out sets kBadSortWait in *wait_error (the sorted
 // set's PointStats::bad), which the caller's input check turns into an error.
-void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, int begin_bit, int end_bit,
+void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, int begin_bit, int end_bit, bool iota,
                       const unsigned int* skip_flag, unsigned int* wait_error, cudaStream_t s);
-void iota_u32(uint32_t* out, uint32_t n, cudaStream_t s);
+// The same in two steps, for a kernel that makes the keys and counts their
+// digits on the way (count_digits): the first returns the counters, zeroed (256
+// per pass; nullptr: the set is small enough to need none), the second sorts.
+struct SortWork {
+  uint32_t* words = nullptr;
+  int begin_bit = 0, passes = 0;
+};
+uint32_t* radix_sort_counts(uint32_t n, int begin_bit, int end_bit, SortWork& w, cudaStream_t s);
+void radix_sort_counted(uint32_t* keys, uint32_t* vals, uint32_t n, bool iota, SortWork& w,
+                        const unsigned int* skip_flag, unsigned int* wait_error, cudaStream_t s);
 
 // ---- scene build (lbvh.cu) -------------------------------------------------
 // `points` is a device AoS of RtdlPoint (dim 2) or RtdlPoint3D (dim 3).
@@ -234,14 +244,16 @@ void batch_problem_ids(const unsigned long long* offsets_dev, uint32_t problems,
 void batch_boxes(const float4* pts, const uint32_t* pid, uint32_t n, PointStats* prob_stats, uint32_t problems,
                  cudaStream_t s);
 void batch_codes(const float4* pts, const uint32_t* pid, uint32_t n, int dim, const PointStats* prob_stats,
-                 int stats_stride, int code_bits, uint32_t* codes, cudaStream_t s);
+                 int stats_stride, int code_bits, uint32_t* codes, uint32_t* digit_counts, cudaStream_t s);
 void destroy_scene(Scene* sc);
 // Converts AoS points to float4 (w = id bits) and accumulates statistics.
 void prep_points(const void* points_dev, uint32_t n, int dim, float4* out, PointStats* stats, cudaStream_t s);
 void reset_stats(PointStats* stats, cudaStream_t s);
 // Hilbert codes relative to the box held in `box_stats` (clamped).
+// digit_counts (optional): radix_sort_counts' counters over all the code's bits.
 void curve_codes(const float4* pts, uint32_t n, int dim, const PointStats* box_stats, uint32_t* codes,
-                  cudaStream_t s);
+                 uint32_t* digit_counts, cudaStream_t s);
+inline int curve_bits(int dim) { return dim == 3 ? 30 : 32; }
 
 // ---- queries (query.cu) -----------------------------------------------------
 enum Predicate { kFrn = 0, kBounded = 1, kKnn = 2 };

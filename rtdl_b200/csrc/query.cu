@@ -1806,7 +1806,8 @@ __global__ void k_mark_all_heavy(const uint32_t* qorder, uint32_t nq, uint32_t n
   }
 }
 
-__global__ void k_extract_ids(const float4* qpts, uint32_t n, uint32_t* ids) {
+__global__ void k_extract_ids(const float4* qpts, uint32_t n, const unsigned int* skip, uint32_t* ids) {
+  if (*skip) return;  // the ids ascend: nothing is sorted
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
     ids[i] = __float_as_uint(qpts[i].w);
 }
@@ -2297,16 +2298,16 @@ QueryPrep prepare_queries(Scene* sc, const void* queries_dev, uint32_t nq, bool 
   qp.order_identity = &qp.bands->ids_sorted;
   qp.view = sc->view();
   qp.qcodes = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq, s));
-  curve_codes(qp.qpts, nq, sc->dim, sc->stats, qp.qcodes, s);
-  iota_u32(qp.qorder, nq, s);
-  radix_sort_pairs(qp.qcodes, qp.qorder, nq, 0, sc->dim == 3 ? 30 : 32, nullptr, &qp.qst->bad, s);
+  SortWork sort;
+  uint32_t* digits = radix_sort_counts(nq, 0, curve_bits(sc->dim), sort, s);
+  curve_codes(qp.qpts, nq, sc->dim, sc->stats, qp.qcodes, digits, s);
+  radix_sort_counted(qp.qcodes, qp.qorder, nq, true, sort, nullptr, &qp.qst->bad, s);
   if (want_output_order) {
     qp.oorder = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq, s));
     uint32_t* ids = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq, s));
-    k_extract_ids<<<grid_for(nq, 256), 256, 0, s>>>(qp.qpts, nq, ids);
+    k_extract_ids<<<grid_for(nq, 256), 256, 0, s>>>(qp.qpts, nq, &qp.bands->ids_sorted, ids);
     RTDL_LAUNCHED(1);
-    iota_u32(qp.oorder, nq, s);
-    radix_sort_pairs(ids, qp.oorder, nq, 0, 32, &qp.bands->ids_sorted, &qp.qst->bad, s);
+    radix_sort_pairs(ids, qp.oorder, nq, 0, 32, true, &qp.bands->ids_sorted, &qp.qst->bad, s);
     dev_free(ids, s);
   }
   return qp;
@@ -2357,24 +2358,24 @@ QueryPrep prepare_queries_batch(Scene* sc, const void* queries_dev, uint32_t nq,
   // processing order: composite (problem, curve in the problem's box) sort, padded per problem
   uint32_t* codes = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * (nq ? nq : 1), s));
   uint32_t* sorted = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * (nq ? nq : 1), s));
+  SortWork sort;
+  uint32_t* digits = radix_sort_counts(nq, 0, 32, sort, s);
   if (shared)
-    batch_codes(qp.qpts, qp.qprob, nq, sc->dim, sc->stats, 0, batch_code_bits(P, sc->dim), codes, s);
+    batch_codes(qp.qpts, qp.qprob, nq, sc->dim, sc->stats, 0, batch_code_bits(P, sc->dim), codes, digits, s);
   else
-    batch_codes(qp.qpts, qp.qprob, nq, sc->dim, sc->prob_stats, 1, sc->code_bits, codes, s);
-  iota_u32(sorted, nq, s);
-  radix_sort_pairs(codes, sorted, nq, 0, 32, nullptr, &qp.qst->bad, s);
+    batch_codes(qp.qpts, qp.qprob, nq, sc->dim, sc->prob_stats, 1, sc->code_bits, codes, digits, s);
+  radix_sort_counted(codes, sorted, nq, true, sort, nullptr, &qp.qst->bad, s);
   k_batch_pad<<<grid_for(qp.nproc, 256), 256, 0, s>>>(qp.qoff, d_pstart, P, qp.nproc, sorted, qp.qorder, qp.warp_prob);
   RTDL_LAUNCHED(1);
   // output order: by query id, then (stable) by problem; skipped when every
   // problem's ids are already ascending
   qp.oorder = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * (nq ? nq : 1), s));
-  iota_u32(qp.oorder, nq, s);
-  k_extract_ids<<<grid_for(nq, 256), 256, 0, s>>>(qp.qpts, nq, codes);
+  k_extract_ids<<<grid_for(nq, 256), 256, 0, s>>>(qp.qpts, nq, qp.sorted_flag, codes);
   RTDL_LAUNCHED(1);
-  radix_sort_pairs(codes, qp.oorder, nq, 0, 32, qp.sorted_flag, &qp.qst->bad, s);
+  radix_sort_pairs(codes, qp.oorder, nq, 0, 32, true, qp.sorted_flag, &qp.qst->bad, s);
   k_gather_u32<<<grid_for(nq, 256), 256, 0, s>>>(qp.qprob, qp.oorder, nq, qp.sorted_flag, codes);
   RTDL_LAUNCHED(1);
-  radix_sort_pairs(codes, qp.oorder, nq, 0, batch_problem_bits(P), qp.sorted_flag, &qp.qst->bad, s);
+  radix_sort_pairs(codes, qp.oorder, nq, 0, batch_problem_bits(P), false, qp.sorted_flag, &qp.qst->bad, s);
   dev_free(codes, s);
   dev_free(sorted, s);
   dev_free(d_pstart, s);
@@ -3612,13 +3613,13 @@ PreparedQueries* prepare_query_set(const void* records_dev, uint32_t n, int dim,
     k_identity_flag<<<1, 32, 0, s>>>(pq->qst, pq->identity);
     RTDL_LAUNCHED(1);
     uint32_t* codes = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * n1, s));
-    curve_codes(pq->qpts, n, dim, pq->qst, codes, s);  // the set's own box: the order only groups neighbours
-    iota_u32(pq->qorder, n, s);
-    radix_sort_pairs(codes, pq->qorder, n, 0, dim == 3 ? 30 : 32, nullptr, &pq->qst->bad, s);
-    k_extract_ids<<<grid_for(n, 256), 256, 0, s>>>(pq->qpts, n, codes);
+    SortWork sort;
+    uint32_t* digits = radix_sort_counts(n, 0, curve_bits(dim), sort, s);
+    curve_codes(pq->qpts, n, dim, pq->qst, codes, digits, s);  // the set's own box: the order only groups neighbours
+    radix_sort_counted(codes, pq->qorder, n, true, sort, nullptr, &pq->qst->bad, s);
+    k_extract_ids<<<grid_for(n, 256), 256, 0, s>>>(pq->qpts, n, pq->identity, codes);
     RTDL_LAUNCHED(1);
-    iota_u32(pq->oorder, n, s);
-    radix_sort_pairs(codes, pq->oorder, n, 0, 32, pq->identity, &pq->qst->bad, s);
+    radix_sort_pairs(codes, pq->oorder, n, 0, 32, true, pq->identity, &pq->qst->bad, s);
     k_invert<<<grid_for(n, 256), 256, 0, s>>>(pq->oorder, n, pq->identity, pq->qrank);
     RTDL_LAUNCHED(1);
     dev_free(codes, s);
@@ -4092,7 +4093,7 @@ void run_directed_hausdorff_noalloc(Scene* sc, const void* queries_dev, uint32_t
   prep_points(queries_dev, nq, sc->dim, qpts, qst, s);
   k_bands<<<1, 32, 0, s>>>(sc->stats, qst, 0.0, 0, bands);
   RTDL_LAUNCHED(1);
-  curve_codes(qpts, nq, sc->dim, sc->stats, codes, s);  // input order (no sort, hence no sort scratch)
+  curve_codes(qpts, nq, sc->dim, sc->stats, codes, nullptr, s);  // input order (no sort, hence no sort scratch)
   SingleParams P{};
   P.S = sc->view();
   P.qpts = qpts;

@@ -6,22 +6,23 @@
 // Scan: reduce-then-scan over 2,048-element tiles (256 threads x 8 items), a
 // single-block pass over the tile sums, then a downsweep.  Deterministic and
 // free of inter-block waits.
-// Radix sort: 8-bit digits.  One kernel counts the digits of every pass in a
-// single read of the keys; then one scatter kernel per pass.  A scatter block
-// takes the next tile index from a counter, counts its tile's digits, and
-// finds each digit's offset among the earlier tiles by decoupled look-back
-// (Merrill and Garland, "Single-pass Parallel Prefix Scan with Decoupled
-// Look-back", 2016): per (tile, digit) a status word holds either the tile's
-// own count or the inclusive count over tiles 0..tile, and a block walks back
-// over the earlier tiles' words until it meets an inclusive one.  Tile indices
-// are handed out in the order blocks start, so every tile a block waits on
-// belongs to a block that is already running; each wait is still bounded and
-// reports through an error word when it runs out.  Inside a tile each warp
-// owns a contiguous run: the warp counts its digits (a key's peers from eight
-// ballots on the digit's bits, one shared-memory add per digit group; 1% faster
-// at 4M keys than __match_any_sync), a block-wide scan over (digit, warp)
-// turns the counts into bases, and the warp then places its keys in order, so
-// the sort stays stable.
+// Radix sort: 8-bit digits.  The digits of every pass are counted in one read
+// of the keys (by the kernel that makes the codes, or by a kernel of its own);
+// then one scatter kernel per pass.  A scatter block takes the next tile index
+// from a counter, ranks its tile's keys, and finds each digit's offset among
+// the earlier tiles by decoupled look-back (Merrill and Garland, "Single-pass
+// Parallel Prefix Scan with Decoupled Look-back", 2016): per (tile, digit) a
+// status word holds either the tile's own count or the inclusive count over
+// tiles 0..tile, and a block walks back over the earlier tiles' words, four at
+// a time, until it meets an inclusive one.  Tile indices are handed out in the
+// order blocks start, so every tile a block waits on belongs to a block that is
+// already running; each wait is still bounded and reports through an error word
+// when it runs out.  Inside a tile each warp owns a contiguous run of 16 keys
+// per lane: a key's peers come from eight ballots on its digit's bits, and one
+// shared-memory add per digit group gives the group its place after the warp's
+// earlier keys, so the sort stays stable and every key is ranked once.  Keys
+// and values are all loaded before the ranking starts.
+// A set of at most one tile is sorted by one block, all passes in one launch.
 #include <cuda/atomic>
 
 #include "internal.cuh"
@@ -35,7 +36,7 @@ constexpr int kScanItems = 8;
 constexpr int kScanTile = kScanThreads * kScanItems;
 
 constexpr int kSortThreads = 256;
-constexpr int kSortItems = 8;
+constexpr int kSortItems = 16;
 constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int kSortWarps = kSortThreads / 32;
 
@@ -210,19 +211,48 @@ __global__ void __launch_bounds__(kSortThreads) k_radix_hist_all(const uint32_t*
   }
 }
 
+// A warp's ranking of its run: rank[i] is the place of the lane's i-th key among
+// the warp's keys of the same digit; wcnt (the warp's 256 digit counts, zeroed)
+// ends with the totals.
+__device__ __forceinline__ void rank_run(const uint32_t (&key)[kSortItems], uint32_t valid_items, int shift,
+                                         unsigned int* wcnt, int lane, uint16_t (&rank)[kSortItems]) {
+  const unsigned int lt_mask = (1u << lane) - 1u;
+#pragma unroll
+  for (int i = 0; i < kSortItems; ++i) {
+    const bool valid = (valid_items >> i) & 1u;
+    const uint32_t d = (key[i] >> shift) & 255u;
+    const unsigned int peers = digit_peers(d, valid);
+    unsigned int before = 0;
+    if (valid) before = wcnt[d];
+    __syncwarp();
+    if (valid && (peers & lt_mask) == 0) wcnt[d] = before + __popc(peers);
+    __syncwarp();
+    rank[i] = (uint16_t)(before + __popc(peers & lt_mask));
+  }
+}
+
+__global__ void k_copy_pairs(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+                             uint32_t* __restrict__ keys, uint32_t* __restrict__ vals, uint32_t n,
+                             const unsigned int* skip) {
+  if (skip != nullptr && *skip) return;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
+    keys[i] = keys_in[i];
+    vals[i] = vals_in[i];
+  }
+}
+
+// iota: the values of the input are the indices 0, 1, ... (vals_in is not read).
 __global__ void __launch_bounds__(kSortThreads)
     k_radix_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-                     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n, int shift,
+                     uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, uint32_t n, int shift, bool iota,
                      const uint32_t* __restrict__ digit_counts, uint32_t* status, unsigned int* tile_counter,
                      unsigned int* wait_error, const unsigned int* skip) {
   if (skip != nullptr && *skip) return;
   __shared__ unsigned int wcnt[kSortWarps][256];  // a warp's digit counts, then its tile-local digit bases
-  __shared__ unsigned int dbase[256];             // tile-local start of each digit
-  __shared__ unsigned int gbase[256];             // global start of each digit for this tile
+  __shared__ unsigned int gbase[256];             // global start of each digit for this tile, less its tile-local start
   __shared__ unsigned int total, tile_s;
   __shared__ uint32_t skeys[kSortTile], svals[kSortTile];
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  const unsigned int lt_mask = (1u << lane) - 1u;
   if (t == 0) tile_s = atomicAdd(tile_counter, 1u);
 #pragma unroll
   for (int w = 0; w < kSortWarps; ++w) wcnt[w][t] = 0;
@@ -230,18 +260,22 @@ __global__ void __launch_bounds__(kSortThreads)
   const uint32_t tile = tile_s;
   // the warp's run of the tile: kSortItems rounds of 32 consecutive keys
   const uint64_t tile0 = (uint64_t)tile * kSortTile;
-  const uint64_t base = tile0 + (uint64_t)warp * (kSortItems * 32);
-  uint32_t key[kSortItems];
+  const uint64_t base = tile0 + (uint64_t)warp * (kSortItems * 32) + lane;
+  uint32_t key[kSortItems], val[kSortItems], valid = 0;
 #pragma unroll
   for (int i = 0; i < kSortItems; ++i) {
-    const uint64_t idx = base + (uint64_t)i * 32 + lane;
-    const bool valid = idx < n;
-    key[i] = valid ? keys_in[idx] : 0u;
-    const uint32_t d = (key[i] >> shift) & 255u;
-    const unsigned int peers = digit_peers(d, valid);
-    if (valid && (peers & lt_mask) == 0) wcnt[warp][d] += __popc(peers);
-    __syncwarp();
+    const uint64_t idx = base + (uint64_t)i * 32;
+    const bool in = idx < n;
+    valid |= in ? 1u << i : 0u;
+    key[i] = in ? keys_in[idx] : 0u;
   }
+#pragma unroll
+  for (int i = 0; i < kSortItems; ++i) {
+    const uint64_t idx = base + (uint64_t)i * 32;
+    val[i] = iota ? (uint32_t)idx : (valid >> i) & 1u ? vals_in[idx] : 0u;
+  }
+  uint16_t rank[kSortItems];
+  rank_run(key, valid, shift, wcnt[warp], lane, rank);
   __syncthreads();
   // thread t owns digit t: offsets of the warps within the digit and the
   // tile's count of the digit
@@ -256,54 +290,56 @@ __global__ void __launch_bounds__(kSortThreads)
   // offset among them
   cuda::atomic_ref<uint32_t, cuda::thread_scope_device> mine(status[(uint64_t)tile * 256 + t]);
   uint32_t before = 0;
-  if (tile == 0) {
-    mine.store(kLookInclusive | r, cuda::memory_order_relaxed);
-  } else {
-    mine.store(kLookLocal | r, cuda::memory_order_relaxed);
+  mine.store((tile == 0 ? kLookInclusive : kLookLocal) | r, cuda::memory_order_relaxed);
+  // the tile's own layout while the earlier tiles publish theirs
+  const unsigned int db = block_exclusive_scan<unsigned int>(r, &total);
+  const unsigned int dstart = block_exclusive_scan<unsigned int>(digit_counts[t], &total);
+#pragma unroll
+  for (int w = 0; w < kSortWarps; ++w) wcnt[w][t] += db;
+  if (tile != 0) {
+    constexpr int kBack = 4;  // status words read at a time
     int64_t j = (int64_t)tile - 1;
     int spins = 0;
-    while (j >= 0) {
-      cuda::atomic_ref<uint32_t, cuda::thread_scope_device> w(status[(uint64_t)j * 256 + t]);
-      const uint32_t v = w.load(cuda::memory_order_relaxed);
-      if (v & kLookInclusive) {
-        before += v & kLookValue;
-        break;
+    bool found = false;
+    while (!found && j >= 0) {
+      uint32_t v[kBack];
+#pragma unroll
+      for (int b = 0; b < kBack; ++b) {
+        v[b] = kLookInclusive;  // before tile 0: nothing
+        if (j - b >= 0) {
+          cuda::atomic_ref<uint32_t, cuda::thread_scope_device> w(status[(uint64_t)(j - b) * 256 + t]);
+          v[b] = w.load(cuda::memory_order_relaxed);
+        }
       }
-      if (v & kLookLocal) {
-        before += v & kLookValue;
-        --j;
-        continue;
+      int used = 0;
+#pragma unroll
+      for (int b = 0; b < kBack; ++b) {
+        if (found || used != b || !(v[b] & (kLookInclusive | kLookLocal))) continue;
+        before += v[b] & kLookValue;
+        found = (v[b] & kLookInclusive) != 0;
+        ++used;
       }
-      if (++spins > kLookSpinLimit) {
-        atomicOr(wait_error, kBadSortWait);
-        break;
+      j -= used;
+      if (used == 0) {
+        if (++spins > kLookSpinLimit) {
+          atomicOr(wait_error, kBadSortWait);
+          break;
+        }
+        __nanosleep(32);
       }
-      __nanosleep(64);
     }
     mine.store(kLookInclusive | ((before + r) & kLookValue), cuda::memory_order_relaxed);
   }
-  const unsigned int db = block_exclusive_scan<unsigned int>(r, &total);
-  const unsigned int dstart = block_exclusive_scan<unsigned int>(digit_counts[t], &total);
-  dbase[t] = db;
-  gbase[t] = dstart + before;
-#pragma unroll
-  for (int w = 0; w < kSortWarps; ++w) wcnt[w][t] += db;
+  gbase[t] = dstart + before - db;
   __syncthreads();
-  // place the keys in the tile's digit order in shared memory (stable)
+  // the keys into the tile's digit order in shared memory (stable)
 #pragma unroll
   for (int i = 0; i < kSortItems; ++i) {
-    const uint64_t idx = base + (uint64_t)i * 32 + lane;
-    const bool valid = idx < n;
-    const uint32_t d = (key[i] >> shift) & 255u;
-    const unsigned int peers = digit_peers(d, valid);
-    if (valid) {
-      const unsigned int pos = wcnt[warp][d] + __popc(peers & lt_mask);
+    if ((valid >> i) & 1u) {
+      const unsigned int pos = wcnt[warp][(key[i] >> shift) & 255u] + rank[i];
       skeys[pos] = key[i];
-      svals[pos] = vals_in[idx];
+      svals[pos] = val[i];
     }
-    __syncwarp();
-    if (valid && (peers & lt_mask) == 0) wcnt[warp][d] += __popc(peers);
-    __syncwarp();
   }
   __syncthreads();
   // write out: consecutive threads take consecutive keys of a digit's run,
@@ -312,8 +348,7 @@ __global__ void __launch_bounds__(kSortThreads)
   const unsigned int tile_n = (unsigned int)(n - tile0 < (uint64_t)kSortTile ? n - tile0 : (uint64_t)kSortTile);
   for (unsigned int j = t; j < tile_n; j += kSortThreads) {
     const uint32_t k = skeys[j];
-    const uint32_t d = (k >> shift) & 255u;
-    const unsigned int pos = gbase[d] + (j - dbase[d]);
+    const unsigned int pos = gbase[(k >> shift) & 255u] + j;
     if (pos < n) {
       keys_out[pos] = k;
       vals_out[pos] = svals[j];
@@ -321,9 +356,58 @@ __global__ void __launch_bounds__(kSortThreads)
   }
 }
 
-__global__ void k_iota(uint32_t* out, uint32_t n) {
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-    out[i] = (uint32_t)i;
+// At most kSortTile keys: every pass in one block, in place.
+__global__ void __launch_bounds__(kSortThreads) k_radix_small(uint32_t* keys, uint32_t* vals, uint32_t n,
+                                                             int begin_bit, int passes, bool iota,
+                                                             const unsigned int* skip) {
+  if (skip != nullptr && *skip) return;
+  __shared__ unsigned int wcnt[kSortWarps][256];
+  __shared__ unsigned int total;
+  __shared__ uint32_t skeys[kSortTile], svals[kSortTile];
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  const uint32_t base = (uint32_t)warp * (kSortItems * 32) + lane;
+  for (int p = 0; p < passes; ++p) {
+    const int shift = begin_bit + 8 * p;
+    uint32_t key[kSortItems], val[kSortItems], valid = 0;
+#pragma unroll
+    for (int i = 0; i < kSortItems; ++i) {
+      const uint32_t idx = base + (uint32_t)i * 32;
+      const bool in = idx < n;
+      valid |= in ? 1u << i : 0u;
+      key[i] = !in ? 0u : p == 0 ? keys[idx] : skeys[idx];
+      val[i] = !in ? 0u : p > 0 ? svals[idx] : iota ? idx : vals[idx];
+    }
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) wcnt[w][t] = 0;
+    __syncthreads();
+    uint16_t rank[kSortItems];
+    rank_run(key, valid, shift, wcnt[warp], lane, rank);
+    __syncthreads();
+    unsigned int r = 0;
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) {
+      const unsigned int c = wcnt[w][t];
+      wcnt[w][t] = r;
+      r += c;
+    }
+    const unsigned int db = block_exclusive_scan<unsigned int>(r, &total);
+#pragma unroll
+    for (int w = 0; w < kSortWarps; ++w) wcnt[w][t] += db;
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < kSortItems; ++i) {
+      if ((valid >> i) & 1u) {
+        const unsigned int pos = wcnt[warp][(key[i] >> shift) & 255u] + rank[i];
+        skeys[pos] = key[i];
+        svals[pos] = val[i];
+      }
+    }
+    __syncthreads();
+  }
+  for (uint32_t j = t; j < n; j += kSortThreads) {
+    keys[j] = skeys[j];
+    vals[j] = svals[j];
+  }
 }
 
 }  // namespace
@@ -343,58 +427,67 @@ void scan_counts_u64_ws(const uint32_t* counts, const uint32_t* order, const uns
   scan_impl<unsigned long long>(counts, order, identity_flag, n, out, static_cast<unsigned long long*>(workspace), s);
 }
 
-void iota_u32(uint32_t* out, uint32_t n, cudaStream_t s) {
-  if (n == 0) return;
-  unsigned int blocks = div_up(n, 256);
-  if (blocks > 8 * kSmCount * 4) blocks = 8 * kSmCount * 4;
-  k_iota<<<blocks, 256, 0, s>>>(out, n);
-  RTDL_LAUNCHED(1);
-}
-
-void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, int begin_bit, int end_bit,
-                      const unsigned int* skip_flag, unsigned int* wait_error, cudaStream_t s) {
-  if (n <= 1 || end_bit <= begin_bit) return;
+uint32_t* radix_sort_counts(uint32_t n, int begin_bit, int end_bit, SortWork& w, cudaStream_t s) {
   if (n > kLookValue) throw std::runtime_error("radix sort input too large");
   if (begin_bit < 0 || end_bit > 32) throw std::runtime_error("radix sort bit range must lie in [0, 32)");
-  int passes = (end_bit - begin_bit + 7) / 8;
-  if (passes & 1) ++passes;  // even pass count leaves the result in the caller's buffers
-  int real = 0;              // passes that sort (the rest only copy)
-  while (real < passes && begin_bit + 8 * real < 32) ++real;
+  w = SortWork{};
+  w.begin_bit = begin_bit;
+  if (end_bit <= begin_bit) throw std::runtime_error("radix sort of no bits");
+  w.passes = (end_bit - begin_bit + 7) / 8;
+  if (n <= (uint32_t)kSortTile) return nullptr;  // one block counts for itself
   const uint32_t tiles = div_up(n, kSortTile);
+  // per pass: 256 digit counts, a tile counter and tiles x 256 status words
+  const size_t words = (256 + 1 + (size_t)tiles * 256) * (size_t)w.passes;
+  w.words = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * words, s));
+  RTDL_CUDA_CHECK(cudaMemsetAsync(w.words, 0, sizeof(uint32_t) * words, s));
+  return w.words;
+}
+
+void radix_sort_counted(uint32_t* keys, uint32_t* vals, uint32_t n, bool iota, SortWork& w,
+                        const unsigned int* skip_flag, unsigned int* wait_error, cudaStream_t s) {
+  if (n == 0) return;
+  if (n <= (uint32_t)kSortTile) {
+    k_radix_small<<<1, kSortThreads, 0, s>>>(keys, vals, n, w.begin_bit, w.passes, iota, skip_flag);
+    RTDL_LAUNCHED(1);
+    return;
+  }
+  const uint32_t tiles = div_up(n, kSortTile);
+  uint32_t* counts = w.words;                                         // passes x 256
+  unsigned int* tile_counters = w.words + 256 * (size_t)w.passes;     // passes
+  uint32_t* status = w.words + 257 * (size_t)w.passes;                // passes x tiles x 256
   uint32_t* keys_alt = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * n, s));
   uint32_t* vals_alt = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * n, s));
-  // per sorting pass: 256 digit counts, a tile counter and tiles x 256 status words
-  const size_t per_pass = 256 + 1 + (size_t)tiles * 256;
-  const size_t work_words = per_pass * (size_t)real;
-  uint32_t* work = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * work_words, s));
-  RTDL_CUDA_CHECK(cudaMemsetAsync(work, 0, sizeof(uint32_t) * work_words, s));
-  uint32_t* counts = work;                                    // real x 256
-  unsigned int* tile_counters = work + 256 * (size_t)real;    // real
-  uint32_t* status = work + 257 * (size_t)real;               // real x tiles x 256
-  unsigned int hist_blocks = div_up(n, kSortThreads * 8);
-  if (hist_blocks > (unsigned int)kSmCount * 2) hist_blocks = kSmCount * 2;
-  k_radix_hist_all<<<hist_blocks, kSortThreads, 0, s>>>(keys, n, begin_bit, real, counts, skip_flag);
-  RTDL_LAUNCHED(1);
   uint32_t *ki = keys, *vi = vals, *ko = keys_alt, *vo = vals_alt;
-  for (int p = 0; p < passes; ++p) {
-    const int shift = begin_bit + 8 * p;
-    if (p < real) {
-      k_radix_onesweep<<<tiles, kSortThreads, 0, s>>>(ki, vi, ko, vo, n, shift, counts + 256 * p, status +
-                                                      (size_t)p * tiles * 256, tile_counters + p, wait_error,
-                                                      skip_flag);
-      RTDL_LAUNCHED(1);
-    } else {
-      // A padding pass beyond the key width: a plain copy keeps the ping-pong even.
-      RTDL_CUDA_CHECK(cudaMemcpyAsync(ko, ki, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
-      RTDL_CUDA_CHECK(cudaMemcpyAsync(vo, vi, sizeof(uint32_t) * n, cudaMemcpyDeviceToDevice, s));
-    }
-    RTDL_CUDA_CHECK(cudaGetLastError());
+  for (int p = 0; p < w.passes; ++p) {
+    k_radix_onesweep<<<tiles, kSortThreads, 0, s>>>(ki, vi, ko, vo, n, w.begin_bit + 8 * p, iota && p == 0,
+                                                    counts + 256 * p, status + (size_t)p * tiles * 256,
+                                                    tile_counters + p, wait_error, skip_flag);
+    RTDL_LAUNCHED(1);
     uint32_t* tk = ki; ki = ko; ko = tk;
     uint32_t* tv = vi; vi = vo; vo = tv;
   }
+  if (w.passes & 1) {  // an odd number of passes ends in the other buffers
+    k_copy_pairs<<<tiles, kSortThreads, 0, s>>>(ki, vi, keys, vals, n, skip_flag);
+    RTDL_LAUNCHED(1);
+  }
   dev_free(keys_alt, s);
   dev_free(vals_alt, s);
-  dev_free(work, s);
+  dev_free(w.words, s);
+  w.words = nullptr;
+}
+
+void radix_sort_pairs(uint32_t* keys, uint32_t* vals, uint32_t n, int begin_bit, int end_bit, bool iota,
+                      const unsigned int* skip_flag, unsigned int* wait_error, cudaStream_t s) {
+  if (n == 0 || end_bit <= begin_bit) return;
+  SortWork w;
+  uint32_t* counts = radix_sort_counts(n, begin_bit, end_bit, w, s);
+  if (counts) {
+    unsigned int hist_blocks = div_up(n, kSortThreads * 8);
+    if (hist_blocks > (unsigned int)kSmCount * 2) hist_blocks = kSmCount * 2;
+    k_radix_hist_all<<<hist_blocks, kSortThreads, 0, s>>>(keys, n, begin_bit, w.passes, counts, skip_flag);
+    RTDL_LAUNCHED(1);
+  }
+  radix_sort_counted(keys, vals, n, iota, w, skip_flag, wait_error, s);
 }
 
 }  // namespace rtdl_b200
