@@ -204,7 +204,7 @@ struct __align__(16) QueryInfo {
 };
 constexpr uint32_t kQueryCountMask = 511u;
 constexpr uint32_t kQueryGeneric = 1u << 18;  // candidates not kept: generic path
-constexpr uint32_t kQueryBig = 1u << 19;      // 65..kSlab candidates: k_emit_list
+constexpr uint32_t kQueryBig = 1u << 19;      // 65..kSlab candidates: k_emit_mid, k_emit_big
 constexpr int kQueryKmaxShift = 20;           // kmax, at most kSlab
 __device__ __forceinline__ int query_kmax(uint32_t meta) { return (int)((meta >> kQueryKmaxShift) & 511u); }
 
@@ -677,7 +677,7 @@ struct EmitParams {
   unsigned int* fix_count;
   // Emission of one range [out_lo, out_hi) of output ranks (rows copied to the
   // host range by range): k_emit takes the range's queries through `order`
-  // (output rank -> processing rank), k_emit_list the range's part
+  // (output rank -> processing rank), k_emit_mid and k_emit_big the range's part
   // [list_start[range], list_start[range + 1]) of its list partitioned by
   // range, and the fix-up the queue from `*fix_begin`.  All null: every
   // query at once.
@@ -807,15 +807,12 @@ struct EmitWarp {
 // its first min(n, kmax) rows; lane l writes rows l, l + 32, ... so each store
 // instruction covers 32 consecutive rows.  The points are gathered once: the
 // exact distance gives the sort key, and waits in shared memory for the lane
-// that writes the row.  When two neighbours need the exact comparison, DEFER
-// == false re-decides them here through `wbuf` and `cand` (shared memory, 32 * E
-// words each); DEFER == true queues the query for k_emit_fixup, which keeps this
-// kernel free of the exact comparison's call (and of the registers that call
-// needs).
-template <int E, bool DEFER>
+// that writes the row.  Neighbours that need the exact comparison are re-decided
+// through `wbuf` and `cand` (shared memory, 32 * E words each).
+template <int E>
 __device__ __forceinline__ void emit_query(const EmitParams& P, uint32_t t, const EmitQuery& q, int n, int lane,
                                            EmitWarp<E>& W, uint32_t* cand, uint32_t* wbuf) {
-  constexpr int SHIFT = E == 1 ? 5 : E == 2 ? 6 : E == 4 ? 7 : 8;
+  constexpr int SHIFT = E == 4 ? 7 : 8;
   constexpr uint32_t kMask = (1u << SHIFT) - 1u;
   const double ex = q.qi.ex, ey = q.qi.ey, ez = q.qi.ez;
   const int inexact = *P.S.inexact;
@@ -839,7 +836,7 @@ __device__ __forceinline__ void emit_query(const EmitParams& P, uint32_t t, cons
       v[r] = pack_key<SHIFT>(__float_as_uint(__double2float_rn(d2)), (uint32_t)s);
       W.dist[s] = __dsqrt_rn(d2);
       W.nid[s] = __float_as_uint(p.w);
-      if (!DEFER) cand[s] = i;
+      cand[s] = i;
     }
   }
   warp_bitonic_striped<E>(v, lane);
@@ -856,18 +853,12 @@ __device__ __forceinline__ void emit_query(const EmitParams& P, uint32_t t, cons
     amb |= ((r << 5) | lane) + 1 < m && (nx >> SHIFT) - (v[r] >> SHIFT) <= 1u;
   }
   if (__any_sync(0xffffffffu, amb)) {
-    if constexpr (DEFER) {
-      if (lane == 0) P.fix_list[atomicAdd(P.fix_count, 1u)] = t;
-      __syncwarp();
-      return;
-    } else {
 #pragma unroll
-      for (int r = 0; r < E; ++r) wbuf[(r << 5) | lane] = v[r];
-      __syncwarp();
-      exact_fixup_sorted(wbuf, m, SHIFT, cand, P.S.pts, P.S.pts64, P.S.perm, inexact, ex, ey, ez, lane);
+    for (int r = 0; r < E; ++r) wbuf[(r << 5) | lane] = v[r];
+    __syncwarp();
+    exact_fixup_sorted(wbuf, m, SHIFT, cand, P.S.pts, P.S.pts64, P.S.perm, inexact, ex, ey, ez, lane);
 #pragma unroll
-      for (int r = 0; r < E; ++r) v[r] = wbuf[(r << 5) | lane];
-    }
+    for (int r = 0; r < E; ++r) v[r] = wbuf[(r << 5) | lane];
   }
   __syncwarp();
 #pragma unroll
@@ -881,39 +872,212 @@ __device__ __forceinline__ void emit_query(const EmitParams& P, uint32_t t, cons
   __syncwarp();  // the shared memory is free again
 }
 
-// Warp per query in processing (curve) order for the queries with at most
-// 64 candidates; queries with 65..kSlab candidates are k_emit_list's, those on
-// the generic path get their rows from k_expand.
-constexpr int kEmitThreads = 256;
-
-// The grid fills the GPU once (emit_grid) and each warp strides over the
-// queries: a warp takes its next query as soon as it is done with one,
-// instead of short blocks of eight queries retiring and launching.
-constexpr int kEmitBlocksPerSm = 8;
-
-__global__ void __launch_bounds__(kEmitThreads, kEmitBlocksPerSm) k_emit(const __grid_constant__ EmitParams P) {
-  __shared__ EmitWarp<2> shared[kEmitThreads / 32];
-  const int lane = threadIdx.x & 31;
-  EmitWarp<2>& W = shared[threadIdx.x >> 5];
-  const uint32_t warps = gridDim.x * (kEmitThreads / 32);
-  const uint32_t total = P.order ? P.out_hi - P.out_lo : P.nq;  // P.order: one range of output ranks
-  for (uint32_t w = blockIdx.x * (kEmitThreads / 32) + (threadIdx.x >> 5); w < total; w += warps) {
-    const uint32_t t = P.order ? P.order[P.out_lo + w] : w;
-    EmitQuery q;
-    emit_load(P, t, lane, q);
-    const uint32_t meta = q.qi.meta;
-    const int n = (int)(meta & kQueryCountMask);
-    if ((meta & (kQueryGeneric | kQueryBig)) || n == 0) continue;
-    if (n <= 32)
-      emit_query<1, true>(P, t, q, n, lane, reinterpret_cast<EmitWarp<1>&>(W), nullptr, nullptr);
-    else
-      emit_query<2, true>(P, t, q, n, lane, W, nullptr, nullptr);
+// ---- emit: a group of lanes per query ---------------------------------------
+// Sorted keys of a group of GL lanes, R per lane: element lane * R + r.  Each
+// merge starts by comparing element e of a block with its mirror image, so all
+// later steps ascend: the steps inside a lane are plain min/max pairs, and only
+// a stride of R elements or more takes a shuffle.  64 keys cost 6 shuffles a
+// register over 8 lanes (12 per query), where a warp with two keys a lane
+// needs 40 per query.
+template <int GL, int R>
+__device__ __forceinline__ void group_sort(uint32_t (&v)[R], int gl) {
+#pragma unroll
+  for (int k = 2; k <= GL * R; k <<= 1) {
+    if (k <= R) {
+#pragma unroll
+      for (int r = 0; r < R; ++r) {
+        const int o = r ^ (k - 1);
+        if (o > r) {
+          const uint32_t a = v[r], b = v[o];
+          v[r] = min(a, b);
+          v[o] = max(a, b);
+        }
+      }
+    } else {
+      const bool lower = (gl & (k / R / 2)) == 0;
+      uint32_t w[R];
+#pragma unroll
+      for (int r = 0; r < R; ++r) w[r] = __shfl_xor_sync(0xffffffffu, v[R - 1 - r], k / R - 1);
+#pragma unroll
+      for (int r = 0; r < R; ++r) v[r] = lower ? min(v[r], w[r]) : max(v[r], w[r]);
+    }
+#pragma unroll
+    for (int j = k >> 2; j > 0; j >>= 1) {
+      if (j >= R) {
+        const bool lower = (gl & (j / R)) == 0;
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const uint32_t w = __shfl_xor_sync(0xffffffffu, v[r], j / R);
+          v[r] = lower ? min(v[r], w) : max(v[r], w);
+        }
+      } else {
+#pragma unroll
+        for (int r = 0; r < R; ++r) {
+          const int o = r ^ j;
+          if (o > r) {
+            const uint32_t a = v[r], b = v[o];
+            v[r] = min(a, b);
+            v[o] = max(a, b);
+          }
+        }
+      }
+    }
   }
 }
 
-// Blocks of k_emit for `queries` warps of work: one resident wave at most.
+// Shared memory of a warp whose groups of GL lanes hold up to 8 * GL candidates
+// each: exact squared distance and id by slot, and the slots in sorted order.
+// The rows are padded so that the groups of a warp use different banks.
+template <int GL>
+struct EmitGroups {
+  static constexpr int kGroups = 32 / GL, kCap = 8 * GL;
+  double d2[kGroups][kCap + 8];
+  uint32_t nid[kGroups][kCap + 8];
+  uint8_t slot[kGroups][kCap + 8];
+};
+
+// Sorts a group's n <= GL * R candidates by the reference's key and writes its
+// first min(n, kmax) rows (n == 0: the group has nothing to do).  The points are
+// gathered once, four loads of a lane in flight; the square root is taken only
+// for the rows that are written.  A query whose near ties need the exact
+// comparison is queued for k_emit_fixup.  All lanes of the warp call this.
+template <int GL, int R>
+__device__ __forceinline__ void emit_group(const EmitParams& P, uint32_t t, const QueryInfo& qi,
+                                           unsigned long long base, const uint32_t (&first)[4], int n, int nmax,
+                                           int lane, EmitGroups<GL>& W) {
+  constexpr int SHIFT = GL * R == 16 ? 4 : GL * R == 32 ? 5 : GL * R == 64 ? 6 : 7;
+  static_assert(GL * R == 1 << SHIFT, "a slot fills the key's low bits");
+  constexpr uint32_t kMask = (1u << SHIFT) - 1u;
+  constexpr int H = R < 4 ? R : 4;
+  const int gl = lane & (GL - 1), g = lane / GL;
+  const int inexact = *P.S.inexact;
+  uint32_t v[R];
+#pragma unroll
+  for (int h = 0; h < R; h += H) {
+#pragma unroll
+    for (int r = h; r < h + H; ++r) v[r] = 0xFFFFFFFFu;
+    if (h * GL >= nmax) continue;  // nothing here in any group
+    uint32_t id[H];
+    float4 p[H];
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      const int s = (h + r) * GL + gl;
+      id[r] = 0;
+      if (s < n) id[r] = h == 0 ? first[r] : P.slab[slab_base(t) + s];
+    }
+#pragma unroll
+    for (int r = 0; r < H; ++r) p[r] = __ldg(&P.S.pts[id[r]]);
+#pragma unroll
+    for (int r = 0; r < H; ++r) {
+      const int s = (h + r) * GL + gl;
+      if (s < n) {
+        double sx = p[r].x, sy = p[r].y, sz = p[r].z;
+        if (inexact) {
+          const double* pp = P.S.pts64 + 3ull * id[r];
+          sx = pp[0];
+          sy = pp[1];
+          sz = pp[2];
+        }
+        const double dx = __dsub_rn(sx, qi.ex), dy = __dsub_rn(sy, qi.ey), dz = __dsub_rn(sz, qi.ez);
+        const double d2 = __dadd_rn(__dadd_rn(__dmul_rn(dx, dx), __dmul_rn(dy, dy)), __dmul_rn(dz, dz));
+        v[h + r] = pack_key<SHIFT>(__float_as_uint(__double2float_rn(d2)), (uint32_t)s);
+        W.d2[g][s] = d2;
+        W.nid[g][s] = __float_as_uint(p[r].w);
+      }
+    }
+  }
+  group_sort<GL, R>(v, gl);
+  const int kmax = query_kmax(qi.meta);
+  const int kk = n < kmax ? n : kmax;
+  // Near ties matter among the elements that can become rows: up to one unit
+  // above element kk - 1 (all of them when every candidate is a row).
+  uint32_t limit = 0x7FFFFFFFu >> SHIFT;
+  {
+    const int c = kk > 0 ? kk - 1 : 0;
+    uint32_t vc = v[0];
+#pragma unroll
+    for (int r = 1; r < R; ++r)
+      if ((c & (R - 1)) == r) vc = v[r];
+    vc = __shfl_sync(0xffffffffu, vc, c / R, GL);
+    if (kk < n) limit = (vc >> SHIFT) + 1u;
+  }
+  uint32_t next = __shfl_down_sync(0xffffffffu, v[0], 1, GL);
+  if (gl == GL - 1) next = 0xFFFFFFFFu;
+  bool amb = false;
+#pragma unroll
+  for (int r = 0; r < R; ++r) {
+    const uint32_t nx = (r + 1 < R ? v[r + 1 < R ? r + 1 : r] : next) >> SHIFT;
+    amb |= nx <= limit && nx - (v[r] >> SHIFT) <= 1u;
+  }
+  const unsigned int any = __ballot_sync(0xffffffffu, amb) >> (lane & ~(GL - 1));
+  const bool defer = (any & (GL == 32 ? 0xFFFFFFFFu : (1u << (GL & 31)) - 1u)) != 0;
+  if (defer && gl == 0) P.fix_list[atomicAdd(P.fix_count, 1u)] = t;
+  if (R == 2) {
+    *reinterpret_cast<uint16_t*>(&W.slot[g][gl * R]) = (uint16_t)((v[0] & kMask) | (v[1] & kMask) << 8);
+  } else {
+#pragma unroll
+    for (int r = 0; r < R; r += 4)
+      *reinterpret_cast<uint32_t*>(&W.slot[g][gl * R + r]) =
+          (v[r] & kMask) | (v[r + 1 < R ? r + 1 : r] & kMask) << 8 | (v[r + 2 < R ? r + 2 : r] & kMask) << 16 |
+          (v[r + 3 < R ? r + 3 : r] & kMask) << 24;
+  }
+  __syncwarp();
+  const int rows = defer ? 0 : kk;
+  for (int i = gl; i < rows; i += GL) {
+    const uint32_t slot = W.slot[g][i];
+    P.sink.put(base + i, qi.qid, W.nid[g][slot], __dsqrt_rn(W.d2[g][slot]), (uint32_t)i + 1);
+  }
+  __syncwarp();  // the shared memory is free again
+}
+
+// A warp's 32 / GL queries (t of this lane's group; live: the group has one that
+// is this kernel's): the records, first rows and first candidates in one round
+// trip, then the network for the largest count in the warp.
+template <int GL>
+__device__ __forceinline__ void emit_groups(const EmitParams& P, uint32_t t, bool live, uint32_t skip, int lane,
+                                            EmitGroups<GL>& W) {
+  const QueryInfo qi = P.qinfo[t];
+  const unsigned long long base = P.poff[t];
+  uint32_t first[4];  // read before the count is known; inside the query's kSlab entries whatever it is
+#pragma unroll
+  for (int r = 0; r < 4; ++r) first[r] = P.slab[slab_base(t) + r * GL + (lane & (GL - 1))];
+  const int n = live && !(qi.meta & skip) ? (int)(qi.meta & kQueryCountMask) : 0;
+  const int nmax = (int)__reduce_max_sync(0xffffffffu, (unsigned int)n);
+  if (nmax == 0) return;
+  if (nmax <= 2 * GL) emit_group<GL, 2>(P, t, qi, base, first, n, nmax, lane, W);
+  else if (nmax <= 4 * GL) emit_group<GL, 4>(P, t, qi, base, first, n, nmax, lane, W);
+  else emit_group<GL, 8>(P, t, qi, base, first, n, nmax, lane, W);
+}
+
+// Queries with at most 64 candidates in processing (curve) order, eight lanes
+// each; queries with 65..kSlab candidates are k_emit_mid's and k_emit_big's, those on the
+// generic path get their rows from k_expand.
+constexpr int kEmitThreads = 256;
+constexpr int kEmitLanes = 8;
+
+// The grid fills the GPU once (emit_grid) and each warp strides over the
+// queries: a warp takes its next four as soon as it is done with some, instead
+// of short blocks retiring and launching.
+constexpr int kEmitBlocksPerSm = 4;
+
+__global__ void __launch_bounds__(kEmitThreads, kEmitBlocksPerSm) k_emit(const __grid_constant__ EmitParams P) {
+  __shared__ EmitGroups<kEmitLanes> shared[kEmitThreads / 32];
+  constexpr uint32_t kQueries = 32 / kEmitLanes;
+  const int lane = threadIdx.x & 31;
+  const uint32_t warps = gridDim.x * (kEmitThreads / 32);
+  const uint32_t total = P.order ? P.out_hi - P.out_lo : P.nq;  // P.order: one range of output ranks
+  for (uint32_t w = blockIdx.x * (kEmitThreads / 32) + (threadIdx.x >> 5); (uint64_t)w * kQueries < total; w += warps) {
+    const uint32_t j = w * kQueries + lane / kEmitLanes;
+    const bool live = j < total;
+    const uint32_t o = live ? j : total - 1;
+    emit_groups<kEmitLanes>(P, P.order ? P.order[P.out_lo + o] : o, live, kQueryGeneric | kQueryBig, lane,
+                            shared[threadIdx.x >> 5]);
+  }
+}
+
+// Blocks of k_emit for `queries` queries: one resident wave at most.
 inline unsigned int emit_grid(uint64_t queries) {
-  const uint64_t blocks = div_up(queries * 32, (uint64_t)kEmitThreads);
+  const uint64_t blocks = div_up(queries * kEmitLanes, (uint64_t)kEmitThreads);
   const uint64_t cap = (uint64_t)kSmCount * kEmitBlocksPerSm;
   return (unsigned int)(blocks < cap ? (blocks > 0 ? blocks : 1) : cap);
 }
@@ -934,7 +1098,7 @@ __global__ void __launch_bounds__(kFixupThreads) k_emit_fixup(const __grid_const
     const uint32_t t = P.fix_list[j];
     EmitQuery q;
     emit_load(P, t, lane, q);
-    emit_query<4, false>(P, t, q, (int)(q.qi.meta & kQueryCountMask), lane, shared[warp], cands[warp], keys[warp]);
+    emit_query<4>(P, t, q, (int)(q.qi.meta & kQueryCountMask), lane, shared[warp], cands[warp], keys[warp]);
   }
 }
 
@@ -1659,34 +1823,48 @@ __global__ void k_proc_offsets(const uint32_t* qorder, const uint32_t* qrank, co
   }
 }
 
-// One warp per query of a work list (processing ranks): E = 4 for 65..128
-// candidates (exact fixups deferred to k_emit_fixup), E = 8 for 129..kSlab
-// (fixups in place through shared memory).
 constexpr int kEmitListThreads = 128;
 
-template <int E, bool DEFER>
-// nwork_dev non-null (captured graphs): the list length is read there and the
-// warps stride over the list.
-__global__ void __launch_bounds__(kEmitListThreads)
-    k_emit_list(const __grid_constant__ EmitParams P, const uint32_t* work, uint32_t nwork, const unsigned int* nwork_dev) {
-  __shared__ EmitWarp<E> shared[kEmitListThreads / 32];
-  __shared__ uint32_t cands[DEFER ? 1 : kEmitListThreads / 32][DEFER ? 1 : 32 * E];
-  __shared__ uint32_t wbuf[DEFER ? 1 : kEmitListThreads / 32][DEFER ? 1 : 32 * E];
-  const int lane = threadIdx.x & 31;
-  if (nwork_dev) nwork = *nwork_dev;
-  uint32_t begin = 0;
-  if (P.list_start) {  // one range of output ranks
+// The part of a work list (processing ranks) a list kernel takes: the list's
+// length is read on the device, or one range of output ranks.
+__device__ __forceinline__ void list_part(const EmitParams& P, const unsigned int* nwork_dev, uint32_t& begin,
+                                          uint32_t& end) {
+  begin = 0;
+  if (nwork_dev) end = *nwork_dev;
+  if (P.list_start) {
     begin = P.list_start[P.range];
-    nwork = P.list_start[P.range + 1];
+    end = P.list_start[P.range + 1];
   }
+}
+
+// 65..128 candidates: 16 lanes per query (exact fixups deferred to k_emit_fixup).
+__global__ void __launch_bounds__(kEmitListThreads)
+    k_emit_mid(const __grid_constant__ EmitParams P, const uint32_t* work, uint32_t nwork, const unsigned int* nwork_dev) {
+  __shared__ EmitGroups<16> shared[kEmitListThreads / 32];
+  const int lane = threadIdx.x & 31;
+  uint32_t begin, end = nwork;
+  list_part(P, nwork_dev, begin, end);
   const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t j = begin + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); j < nwork; j += warps) {  // whole warps
+  for (uint32_t w = begin + 2 * ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); w < end; w += 2 * warps) {
+    const uint32_t j = w + lane / 16;
+    emit_groups<16>(P, work[j < end ? j : w], j < end, 0u, lane, shared[threadIdx.x >> 5]);
+  }
+}
+
+// 129..kSlab candidates: a warp per query, fixups in place through shared memory.
+__global__ void __launch_bounds__(kEmitListThreads)
+    k_emit_big(const __grid_constant__ EmitParams P, const uint32_t* work, uint32_t nwork, const unsigned int* nwork_dev) {
+  __shared__ EmitWarp<8> shared[kEmitListThreads / 32];
+  __shared__ uint32_t cands[kEmitListThreads / 32][256], wbuf[kEmitListThreads / 32][256];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t begin, end = nwork;
+  list_part(P, nwork_dev, begin, end);
+  const uint32_t warps = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t j = begin + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); j < end; j += warps) {  // whole warps
     const uint32_t t = work[j];
     EmitQuery q;
     emit_load(P, t, lane, q);
-    const int n = (int)(q.qi.meta & kQueryCountMask);
-    emit_query<E, DEFER>(P, t, q, n, lane, shared[threadIdx.x >> 5], DEFER ? nullptr : cands[threadIdx.x >> 5],
-                         DEFER ? nullptr : wbuf[threadIdx.x >> 5]);
+    emit_query<8>(P, t, q, (int)(q.qi.meta & kQueryCountMask), lane, shared[warp], cands[warp], wbuf[warp]);
   }
 }
 
@@ -2525,8 +2703,8 @@ static_assert(kEmitListThreads == kFixupThreads, "list_grid serves both");
 
 // The list kernels over the collect's lists (lengths in small[2], small[3]).
 void launch_emit_lists(const EmitParams& E, const CollectParams& C, uint32_t np, cudaStream_t s) {
-  k_emit_list<4, true><<<list_grid(np), kEmitListThreads, 0, s>>>(E, C.mid_list, 0, C.small + 2);
-  k_emit_list<8, false><<<list_grid(np), kEmitListThreads, 0, s>>>(E, C.big_list, 0, C.small + 3);
+  k_emit_mid<<<list_grid(np), kEmitListThreads, 0, s>>>(E, C.mid_list, 0, C.small + 2);
+  k_emit_big<<<list_grid(np), kEmitListThreads, 0, s>>>(E, C.big_list, 0, C.small + 3);
   RTDL_LAUNCHED(2);
 }
 
@@ -2774,12 +2952,12 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
           // the list kernels stride over the range's part: grids sized for an even split
           if (mid > 0) {
             E.list_start = part + C8;
-            k_emit_list<4, true><<<div_up((uint64_t)div_up(mid, C8) * 32, kEmitListThreads), kEmitListThreads, 0, s>>>(
+            k_emit_mid<<<div_up((uint64_t)div_up(mid, C8) * 32, kEmitListThreads), kEmitListThreads, 0, s>>>(
                 E, lists_by_range[0], 0, nullptr);
           }
           if (big > 0) {
             E.list_start = part + kPart + C8;
-            k_emit_list<8, false><<<div_up((uint64_t)div_up(big, C8) * 32, kEmitListThreads), kEmitListThreads, 0,
+            k_emit_big<<<div_up((uint64_t)div_up(big, C8) * 32, kEmitListThreads), kEmitListThreads, 0,
                                     s>>>(E, lists_by_range[1], 0, nullptr);
           }
           E.list_start = nullptr;
