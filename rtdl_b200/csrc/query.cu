@@ -606,7 +606,7 @@ __device__ __forceinline__ void collect_packet_body(const CollectParams& P, uint
 constexpr int kCollectThreads = 128;
 
 template <int DIM, bool BATCH, bool OWN>
-__global__ void __launch_bounds__(kCollectThreads, 6) k_collect_packet(const __grid_constant__ CollectParams P) {
+__global__ void __launch_bounds__(kCollectThreads, OWN ? 6 : 7) k_collect_packet(const __grid_constant__ CollectParams P) {
   __shared__ CollectWarp warps[kCollectThreads / 32];
   const uint32_t t = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * P.width + (threadIdx.x & 31);
   if (!__any_sync(0xffffffffu, t < P.nq)) return;  // whole warp past the end
@@ -1308,6 +1308,31 @@ __global__ void __launch_bounds__(256) k_knn_single(SingleParams P) {
   }
 }
 
+// ---- nearest point and the Hausdorff witness ------------------------------------
+struct Witness {
+  unsigned long long dist;  // FP64 bits
+  uint32_t qid, nid;
+};
+// max by (distance, -query_id, -neighbor_id)
+__device__ __forceinline__ bool witness_better(const Witness& a, const Witness& b) {
+  if (a.dist != b.dist) return a.dist > b.dist;
+  if (a.qid != b.qid) return a.qid < b.qid;
+  return a.nid < b.nid;
+}
+
+// The best witness of a warp, in every lane.
+__device__ __forceinline__ Witness warp_witness(Witness best) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    Witness other;
+    other.dist = __shfl_xor_sync(0xffffffffu, best.dist, o);
+    other.qid = __shfl_xor_sync(0xffffffffu, best.qid, o);
+    other.nid = __shfl_xor_sync(0xffffffffu, best.nid, o);
+    if (witness_better(other, best)) best = other;
+  }
+  return best;
+}
+
 // The nearest point of every query (directed Hausdorff), a packet of 32
 // queries per warp.  The smallest distance among 32 points around a query's
 // place on the curve bounds its search; the warp walks what that bound reaches
@@ -1437,12 +1462,12 @@ __global__ void __launch_bounds__(128) k_nearest(const __grid_constant__ Nearest
 }
 
 // ---- ranked summaries ----------------------------------------------------------
-// One warp per query in output order reads the query's rows (contiguous) and
-// reduces them to the reference's ranked summary: count, first and last row,
-// and the distances added one by one in row order (so the sum is the one a
-// sequential loop over the rows gives).  Each block also writes its queries'
-// partial aggregate (in warp order), which k_summary_final reduces in block
-// order: the aggregate is the same on every run.
+// A query's rows (contiguous, in output order) are reduced to the reference's
+// ranked summary: count, first and last row, and the distances added one by one
+// in row order (so the sum is the one a sequential loop over the rows gives).
+// Every eight consecutive queries also give a partial aggregate, added in query
+// order, which k_summary_final reduces in a fixed order: the aggregate is the
+// same on every run.
 struct SummaryPartial {
   unsigned long long count, nearest, kth;
   double sum;
@@ -1736,49 +1761,58 @@ struct SummarySpec {
 };
 
 
-constexpr int kSummaryThreads = 256;
+constexpr int kSummaryThreads = 128;
+constexpr int kSummaryGroup = 8;  // queries per partial aggregate
 
+// A thread per query.  The sum of a query's distances is a chain of FP64 adds;
+// with a warp per query every add cost the warp two shuffles for one query, here
+// 32 chains share them, and a thread keeps eight distance loads in flight.
 __global__ void __launch_bounds__(kSummaryThreads)
-    k_summarize(const RtdlFixedRadiusNeighborRow* rows, const unsigned long long* offsets, const uint32_t* oorder,
-                const unsigned int* identity, const float4* qpts, uint32_t nq,
-                RtdlFixedRadiusRankedNeighborSummary* summaries, SummaryPartial* partial) {
-  __shared__ SummaryPartial wsum[kSummaryThreads / 32];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const uint64_t j = ((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    k_summarize(const RtdlFixedRadiusNeighborRow* __restrict__ rows, const unsigned long long* __restrict__ offsets,
+                const uint32_t* __restrict__ oorder, const unsigned int* __restrict__ identity,
+                const float4* __restrict__ qpts, uint32_t nq, RtdlFixedRadiusRankedNeighborSummary* summaries,
+                SummaryPartial* partial) {
+  __shared__ SummaryPartial per_query[kSummaryThreads];
+  const uint64_t j = (uint64_t)blockIdx.x * kSummaryThreads + threadIdx.x;
   SummaryPartial mine{0ull, 0ull, 0ull, 0.0};
-  if (j < nq) {  // warp-uniform
+  if (j < nq) {
     const uint32_t qin = *identity ? (uint32_t)j : oorder[j];
     const unsigned long long a = offsets[j], b = offsets[j + 1];
-    const int cnt = (int)(b - a);  // at most 64
-    double d0 = 0.0, d1 = 0.0;
-    if (lane < cnt) d0 = rows[a + lane].distance;
-    if (lane + 32 < cnt) d1 = rows[a + 32 + lane].distance;
+    const uint32_t cnt = (uint32_t)(b - a);
     double sum = 0.0;
-    for (int i = 0; i < cnt; ++i) sum += __shfl_sync(0xffffffffu, i < 32 ? d0 : d1, i & 31);
+    for (uint32_t i = 0; i < cnt; i += 8) {
+      double d[8];
+#pragma unroll
+      for (uint32_t u = 0; u < 8; ++u) d[u] = i + u < cnt ? rows[a + i + u].distance : 0.0;
+#pragma unroll
+      for (uint32_t u = 0; u < 8; ++u)
+        if (i + u < cnt) sum += d[u];
+    }
     RtdlFixedRadiusRankedNeighborSummary sm;
     sm.query_id = __float_as_uint(qpts[qin].w);
-    sm.neighbor_count = (uint32_t)cnt;
+    sm.neighbor_count = cnt;
     sm.nearest_neighbor_id = cnt ? rows[a].neighbor_id : 0xFFFFFFFFu;
     sm.kth_neighbor_id = cnt ? rows[b - 1].neighbor_id : 0xFFFFFFFFu;
     sm.nearest_distance = cnt ? rows[a].distance : 0.0;
     sm.kth_distance = cnt ? rows[b - 1].distance : 0.0;
     sm.sum_distance = sum;
-    if (lane == 0) {
-      if (summaries) summaries[qin] = sm;
-      mine = SummaryPartial{(unsigned long long)cnt, sm.nearest_neighbor_id, sm.kth_neighbor_id, sum};
-    }
+    if (summaries) summaries[qin] = sm;
+    mine = SummaryPartial{(unsigned long long)cnt, sm.nearest_neighbor_id, sm.kth_neighbor_id, sum};
   }
-  if (lane == 0) wsum[warp] = mine;
+  per_query[threadIdx.x] = mine;
   __syncthreads();
-  if (threadIdx.x == 0) {
+  const uint32_t g = threadIdx.x;
+  const uint64_t out = (uint64_t)blockIdx.x * (kSummaryThreads / kSummaryGroup) + g;
+  if (g < kSummaryThreads / kSummaryGroup && out * kSummaryGroup < nq) {
     SummaryPartial acc{0ull, 0ull, 0ull, 0.0};
-    for (int w = 0; w < kSummaryThreads / 32; ++w) {
-      acc.count += wsum[w].count;
-      acc.nearest += wsum[w].nearest;
-      acc.kth += wsum[w].kth;
-      acc.sum += wsum[w].sum;
+    for (int w = 0; w < kSummaryGroup; ++w) {
+      const SummaryPartial& q = per_query[g * kSummaryGroup + w];
+      acc.count += q.count;
+      acc.nearest += q.nearest;
+      acc.kth += q.kth;
+      acc.sum += q.sum;
     }
-    partial[blockIdx.x] = acc;
+    partial[out] = acc;
   }
 }
 
@@ -2249,17 +2283,6 @@ __global__ void __launch_bounds__(kExpandThreads) k_expand(ExpandParams P) {
 }
 
 // ---- directed Hausdorff: FP64 max over per-query nearest distances ---------
-struct Witness {
-  unsigned long long dist;  // FP64 bits
-  uint32_t qid, nid;
-};
-// max by (distance, -query_id, -neighbor_id)
-__device__ __forceinline__ bool witness_better(const Witness& a, const Witness& b) {
-  if (a.dist != b.dist) return a.dist > b.dist;
-  if (a.qid != b.qid) return a.qid < b.qid;
-  return a.nid < b.nid;
-}
-
 __global__ void __launch_bounds__(256)
     k_nearest_reduce(SceneView S, const float4* qpts, const double* qraw, int qstride, uint32_t nq,
                      const uint32_t* temp, double* nearest_dist, uint32_t* nearest_id, Witness* partial) {
@@ -2293,14 +2316,7 @@ __global__ void __launch_bounds__(256)
     }
   }
   if (!have) best = Witness{0ull, kNone, kNone};
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    Witness other;
-    other.dist = __shfl_xor_sync(0xffffffffu, best.dist, o);
-    other.qid = __shfl_xor_sync(0xffffffffu, best.qid, o);
-    other.nid = __shfl_xor_sync(0xffffffffu, best.nid, o);
-    if (witness_better(other, best)) best = other;
-  }
+  best = warp_witness(best);
   if ((threadIdx.x & 31) == 0) warp_best[threadIdx.x >> 5] = best;
   __syncthreads();
   if (threadIdx.x == 0) {
@@ -2311,12 +2327,21 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-__global__ void k_witness_final(const Witness* partial, int n, Witness* out) {
-  if (threadIdx.x != 0) return;
-  Witness b = partial[0];
-  for (int i = 1; i < n; ++i)
-    if (witness_better(partial[i], b)) b = partial[i];
-  *out = b;
+// The best of n witnesses; one block.
+__global__ void __launch_bounds__(256) k_witness_best(const Witness* __restrict__ in, uint32_t n, Witness* out) {
+  __shared__ Witness warp_best[8];
+  Witness best{0ull, kNone, kNone};
+  for (uint32_t i = threadIdx.x; i < n; i += 256) {
+    const Witness w = in[i];
+    if (witness_better(w, best)) best = w;
+  }
+  best = warp_witness(best);
+  if ((threadIdx.x & 31) == 0) warp_best[threadIdx.x >> 5] = best;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    best = warp_witness(threadIdx.x < 8 ? warp_best[threadIdx.x] : Witness{0ull, kNone, kNone});
+    if (threadIdx.x == 0) *out = best;
+  }
 }
 
 bool stats_enabled() {
@@ -3018,14 +3043,14 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
       }
     }
     if (ss) {
-      const uint32_t blocks = div_up((uint64_t)nq * 32, kSummaryThreads);
-      SummaryPartial* partial = static_cast<SummaryPartial*>(dev_alloc(sizeof(SummaryPartial) * blocks, s));
+      const uint32_t parts = div_up(nq, kSummaryGroup);
+      SummaryPartial* partial = static_cast<SummaryPartial*>(dev_alloc(sizeof(SummaryPartial) * parts, s));
       RtdlFixedRadiusRankedNeighborAggregate* agg = static_cast<RtdlFixedRadiusRankedNeighborAggregate*>(
           dev_alloc(sizeof(RtdlFixedRadiusRankedNeighborAggregate), s));
-      k_summarize<<<blocks, kSummaryThreads, 0, s>>>(static_cast<const RtdlFixedRadiusNeighborRow*>(summary_rows),
+      k_summarize<<<div_up(nq, kSummaryThreads), kSummaryThreads, 0, s>>>(static_cast<const RtdlFixedRadiusNeighborRow*>(summary_rows),
                                                     offsets, qp.oorder, qp.order_identity, qp.qpts, nq,
                                                     ss->summaries_dev, partial);
-      k_summary_final<<<1, 1024, 0, s>>>(partial, blocks, nq, agg);
+      k_summary_final<<<1, 1024, 0, s>>>(partial, parts, nq, agg);
       RTDL_LAUNCHED(2);
       RTDL_CUDA_CHECK(cudaMemcpyAsync(ss->aggregate_host, agg, sizeof(*agg), cudaMemcpyDeviceToHost, s));
       RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
@@ -3492,7 +3517,7 @@ struct SummaryGraph {
   void* scan_ws = nullptr;
   void* rows = nullptr;  // nq * kcap rows
   SummaryPartial* partial = nullptr;
-  uint32_t summary_blocks = 0;
+  uint32_t summary_parts = 0;
   RtdlFixedRadiusRankedNeighborAggregate* agg = nullptr;  // one per request
   unsigned int* status = nullptr;                         // one per request
   RtdlFixedRadiusRankedNeighborAggregate* agg_host = nullptr;  // pinned
@@ -3574,10 +3599,10 @@ void graph_enqueue_request(SummaryGraph* g, uint32_t r, cudaStream_t s) {
   launch_emit(E, np, s);
   launch_emit_lists(E, C, np, s);
   k_emit_fixup<<<list_grid(np), kFixupThreads, 0, s>>>(E);
-  k_summarize<<<g->summary_blocks, kSummaryThreads, 0, s>>>(static_cast<const RtdlFixedRadiusNeighborRow*>(g->rows),
+  k_summarize<<<div_up(nq, kSummaryThreads), kSummaryThreads, 0, s>>>(static_cast<const RtdlFixedRadiusNeighborRow*>(g->rows),
                                                             g->offsets, pq->oorder, pq->identity, pq->qpts, nq,
                                                             nullptr, g->partial);
-  k_summary_final<<<1, 1024, 0, s>>>(g->partial, g->summary_blocks, nq, g->agg + r);
+  k_summary_final<<<1, 1024, 0, s>>>(g->partial, g->summary_parts, nq, g->agg + r);
   RTDL_LAUNCHED(3);
 }
 
@@ -3690,8 +3715,8 @@ SummaryGraph* summary_graph_create(Scene* sc, const PreparedQueries* pq, const d
     graph_size_rows(g);
     g->heavy_rad = static_cast<double*>(alloc(sizeof(double) * n));
     g->single_list = static_cast<uint32_t*>(alloc(sizeof(uint32_t) * n));
-    g->summary_blocks = div_up((uint64_t)n * 32, kSummaryThreads);
-    g->partial = static_cast<SummaryPartial*>(alloc(sizeof(SummaryPartial) * g->summary_blocks));
+    g->summary_parts = div_up(n, kSummaryGroup);
+    g->partial = static_cast<SummaryPartial*>(alloc(sizeof(SummaryPartial) * g->summary_parts));
     g->agg = static_cast<RtdlFixedRadiusRankedNeighborAggregate*>(
         alloc(sizeof(RtdlFixedRadiusRankedNeighborAggregate) * R));
     g->status = static_cast<unsigned int*>(alloc(sizeof(unsigned int) * R));
@@ -4132,6 +4157,9 @@ HausdorffResult run_directed_hausdorff(Scene* sc, const void* queries_dev, uint3
   QueryPrep qp = prepare_queries(sc, queries_dev, nq, false, 0.0, false, s);
   if (timer) timer->mark("query_prep");
   uint32_t* temp = static_cast<uint32_t*>(dev_alloc(sizeof(uint32_t) * nq, s));
+  const unsigned int blocks = grid_for(nq, 256) < 8 * kSmCount ? grid_for(nq, 256) : 8 * kSmCount;
+  Witness* partial = static_cast<Witness*>(dev_alloc(sizeof(Witness) * blocks, s));
+  Witness* best = static_cast<Witness*>(dev_alloc(sizeof(Witness), s));
   NearestParams P;
   P.S = sc->view();
   P.qpts = qp.qpts;
@@ -4149,12 +4177,9 @@ HausdorffResult run_directed_hausdorff(Scene* sc, const void* queries_dev, uint3
     k_nearest<2><<<div_up(nq, 128), 128, 0, s>>>(P);
   RTDL_LAUNCHED(1);
   if (timer) timer->mark("traverse");
-  const unsigned int blocks = grid_for(nq, 256) < 2 * kSmCount ? grid_for(nq, 256) : 2 * kSmCount;
-  Witness* partial = static_cast<Witness*>(dev_alloc(sizeof(Witness) * blocks, s));
-  Witness* best = static_cast<Witness*>(dev_alloc(sizeof(Witness), s));
   k_nearest_reduce<<<blocks, 256, 0, s>>>(sc->view(), qp.qpts, static_cast<const double*>(queries_dev), qstride, nq,
                                           temp, nearest_dist_dev, nearest_id_dev, partial);
-  k_witness_final<<<1, 32, 0, s>>>(partial, (int)blocks, best);
+  k_witness_best<<<1, 256, 0, s>>>(partial, blocks, best);
   RTDL_LAUNCHED(2);
   // one read of the witness (into the record's row-range words) and the error words
   Readback* rb = pinned_readback();
@@ -4288,7 +4313,7 @@ void run_directed_hausdorff_noalloc(Scene* sc, const void* queries_dev, uint32_t
   const unsigned int blocks = grid_for(nq, 256) < kNoAllocReduceBlocks ? grid_for(nq, 256) : kNoAllocReduceBlocks;
   k_nearest_reduce<<<blocks, 256, 0, s>>>(sc->view(), qpts, static_cast<const double*>(queries_dev), P.qstride, nq,
                                           temp, nearest_dist_dev, nearest_id_dev, partial);
-  k_witness_final<<<1, 32, 0, s>>>(partial, (int)blocks, best);
+  k_witness_best<<<1, 256, 0, s>>>(partial, blocks, best);
   k_noalloc_finish<<<1, 32, 0, s>>>(best, sc->stats, qst, witness_dev);
   RTDL_LAUNCHED(3);
 }
