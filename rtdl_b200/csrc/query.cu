@@ -2688,6 +2688,19 @@ void launch_collect_left(const CollectParams& C, uint32_t np, cudaStream_t s) {
   RTDL_LAUNCHED(1);
 }
 
+// Queries per packet: full packets once they give every SM `warps` of them, fewer
+// below that, where the longest packet sets the time (a packet of eight meets
+// half the buckets of one of 32).  A plain call's packets are alike: 24 warps are
+// what an SM holds, and asking for 96 took a 262k-query summary from 1550 to
+// 1835 us.  The problems of a batch are not, and short packets fill its last
+// wave: with 96 instead of 24 (32 always, in a batch graph) six served requests
+// went from 1190 to 1060 us, batches of 6 and 31 small problems from 725 and 770
+// to 660 and 675, a graph of 8 problems from 785 to 650; 192 gave the same.
+uint32_t packet_width(uint32_t np, bool batch) {
+  const uint64_t warps = batch ? 96 : 24;
+  return np >= 32u * warps * kSmCount ? 32u : np >= 16u * warps * kSmCount ? 16u : 8u;
+}
+
 // The collect pass over np processing ranks.
 void launch_collect(CollectParams& C, uint32_t np, bool batch, cudaStream_t s) {
   if (np <= kSingleQueries && !C.rank_radius) {
@@ -2695,10 +2708,7 @@ void launch_collect(CollectParams& C, uint32_t np, bool batch, cudaStream_t s) {
     RTDL_LAUNCHED(1);
     return;
   }
-  // Full packets once they give every SM 24 warps (what the registers allow);
-  // fewer queries per packet below that, where the longest packet sets the time:
-  // a packet of eight meets half the buckets of one of 32.
-  C.width = np >= 32u * 24u * kSmCount ? 32u : np >= 16u * 24u * kSmCount ? 16u : 8u;
+  C.width = packet_width(np, batch);
   const unsigned int grid = div_up((uint64_t)div_up(np, C.width) * 32, kCollectThreads);
   const bool flat = C.qstride == 3;
   if (batch)
@@ -4355,14 +4365,14 @@ __global__ void k_empty_batch_rows(const unsigned long long* base, uint32_t prob
 template <int DIM>
 __global__ void __launch_bounds__(kCollectThreads, 6) k_collect_persistent(const __grid_constant__ CollectParams P, unsigned int* queue) {
   __shared__ CollectWarp warps[kCollectThreads / 32];
-  const uint32_t packets = (P.nq + 31u) / 32u;
+  const uint32_t packets = (P.nq + P.width - 1u) / P.width;
   const uint32_t lane = threadIdx.x & 31u;
   for (;;) {
     uint32_t item = 0;
     if (lane == 0) item = atomicAdd(queue, 1u);
     item = __shfl_sync(0xffffffffu, item, 0);
     if (item >= packets) return;
-    collect_packet_body<DIM, true, false>(P, item * 32u + lane, warps[threadIdx.x >> 5]);
+    collect_packet_body<DIM, true, false>(P, item * P.width + lane, warps[threadIdx.x >> 5]);
   }
 }
 
@@ -4444,7 +4454,7 @@ void batch_graph_enqueue(BatchGraph* g, uint32_t i, cudaStream_t s) {
   C.qorder = b.qp.qorder;
   C.nq = b.qp.nproc;
   C.kmax = kmax;
-  C.width = 32;
+  C.width = packet_width(b.qp.nproc, true);
   C.radius = 0.0;
   C.bands = b.qp.bands;
   C.warp_prob = b.qp.warp_prob;
