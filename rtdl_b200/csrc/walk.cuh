@@ -239,17 +239,18 @@ __device__ __forceinline__ void walk_fours(const SceneView& S, const TreeShape* 
   __syncwarp();
 }
 
-// Whether the box meets at most `most` nodes of level LEAF.
+// How many nodes of level LEAF the box meets; the count may stop once it is
+// above `most`.
 template <int LEAF>
-__device__ __forceinline__ bool few_nodes(const SceneView& S, const TreeShape* __restrict__ T, const PacketBox& box,
-                                          const PacketBox* limit, float reach2, WalkStack& stack, int lane,
-                                          uint32_t most) {
+__device__ __forceinline__ uint32_t nodes_met(const SceneView& S, const TreeShape* __restrict__ T, const PacketBox& box,
+                                              const PacketBox* limit, float reach2, WalkStack& stack, int lane,
+                                              uint32_t most) {
   uint32_t nodes = 0;
   walk_wide<LEAF>(S, T, box, limit, reach2, stack, lane, [&](uint32_t, uint32_t mask) {
     nodes += __popc(mask);
     return nodes > most;
   });
-  return nodes <= most;
+  return nodes;
 }
 
 // Cuts a packet into runs of neighbouring queries that are worth walking
@@ -259,10 +260,12 @@ __device__ __forceinline__ bool few_nodes(const SceneView& S, const TreeShape* _
 // its box meets and a query alone 350 and 12 per bucket, so a run of s queries
 // is walked together when its box meets at most 10 s buckets, else its halves
 // are tried, and runs of four that still do not fit go to single().  The
-// buckets are only counted (a step per level-1 node) when the level-1 nodes,
-// which hold 32 buckets and of which a box meets about 6 each, are many (a
-// count of about five steps over the upper levels), and neither is counted
-// when the box is at most 8 times one query's cube and all radii are equal (on
+// buckets are only counted (a step per level-1 node) when the number of level-1
+// nodes, which hold 32 buckets and of which a box meets about 6 each, does not
+// decide (a count of about five steps over the upper levels): up to s / 2 + 4
+// fit, more than 2 s do not (counting the buckets of every hopeless run kept the
+// last packets of a 65k-query shell 25 us longer; with s for 2 s too many went
+// alone, 1.03 -> 2.2 ms for six served requests).  Neither is counted when the box is at most 8 times one query's cube and all radii are equal (on
 // the clustered 1M x 1M sets it is 5.8 times, 14 nodes and 87 buckets).
 // Judged by the nodes alone a packet could still meet 1,000 buckets, and a few
 // such packets kept the kernel running 0.2 ms after the rest had ended.
@@ -291,9 +294,11 @@ __device__ __forceinline__ void cut_packet(const SceneView& S, const TreeShape* 
         fits = (box.hx - box.lx + w) * (box.hy - box.ly + w) * (box.hz - box.lz + w) <= 8.f * w * w * w;
       }
       const PacketBox* lim = own_radii ? &limit : nullptr;
-      if (!fits)
-        fits = few_nodes<1>(S, T, box, lim, reach2, stack, lane, (uint32_t)s / 2 + 4) ||
-               few_nodes<0>(S, T, box, lim, reach2, stack, lane, (uint32_t)s * 10);
+      if (!fits) {
+        const uint32_t w = (uint32_t)s, met = nodes_met<1>(S, T, box, lim, reach2, stack, lane, 2 * w);
+        fits = met <= w / 2 + 4 ||
+               (met <= 2 * w && nodes_met<0>(S, T, box, lim, reach2, stack, lane, 10 * w) <= 10 * w);
+      }
       if (!fits && s > 4) {
         s >>= 1;
         continue;
