@@ -259,16 +259,19 @@ __device__ __forceinline__ uint32_t nodes_met(const SceneView& S, const TreeShap
 // few queries over many points.  A walk costs about 50 instructions per bucket
 // its box meets and a query alone 350 and 12 per bucket, so a run of s queries
 // is walked together when its box meets at most 10 s buckets, else its halves
-// are tried, and runs of four that still do not fit go to single().  The
+// are tried, and runs of four that still do not fit go to single() (6 s and
+// 16 s: KNN k = 32 of 100k queries 1.26 and 1.12 ms against 1.08).  The
 // buckets are only counted (a step per level-1 node) when the number of level-1
 // nodes, which hold 32 buckets and of which a box meets about 6 each, does not
 // decide (a count of about five steps over the upper levels): up to s / 2 + 4
-// fit, more than 2 s do not (counting the buckets of every hopeless run kept the
-// last packets of a 65k-query shell 25 us longer; with s for 2 s too many went
-// alone, 1.03 -> 2.2 ms for six served requests).  Neither is counted when the box is at most 8 times one query's cube and all radii are equal (on
-// the clustered 1M x 1M sets it is 5.8 times, 14 nodes and 87 buckets).
-// Judged by the nodes alone a packet could still meet 1,000 buckets, and a few
-// such packets kept the kernel running 0.2 ms after the rest had ended.
+// fit, more than 2 s do not.  Counting the buckets of every hopeless run kept
+// the last packets of a 65k-query shell 25 us longer; with s in place of 2 s too
+// many queries went alone (six served requests 1.03 -> 2.2 ms).  Neither is
+// counted when the box is at most 8 times one query's cube and all radii are
+// equal (on the clustered 1M x 1M sets it is 5.8 times, 14 nodes and 87
+// buckets).  Judged by the nodes alone a packet could still meet 1,000 buckets,
+// and a few such packets kept the kernel running 0.2 ms after the rest had
+// ended.
 // walk(mine, box, limit, reach2) gets the lanes of a run, single(mask) the
 // lanes that go alone.
 template <typename Walk, typename Single>
@@ -278,7 +281,11 @@ __device__ __forceinline__ void cut_packet(const SceneView& S, const TreeShape* 
   const uint32_t act = __ballot_sync(0xffffffffu, active);
   const float half = own_radii ? reach_half_width(lane_reach2) : 0.f;
   int s = 32;
-  for (int at = 0; at < 32;) {
+  // A narrow packet starts at its own width, so the limits fit its queries (a
+  // 65k-query shell 360 -> 310 us, a 20k-query summary 336 -> 261).  With radii of
+  // their own the queries left over cost too much (KNN k = 32 1.06 -> 1.26 ms).
+  while (!own_radii && s > 4 && (act >> (s / 2)) == 0) s >>= 1;
+  for (int at = 0; at < 32 && (act >> at) != 0;) {
     const uint32_t run = act & ((0xffffffffu >> (32 - s)) << at);
     if (run) {
       const bool mine = (run >> lane) & 1u;
