@@ -388,7 +388,7 @@ def secondary_leg(workload: str, steps: int, warmup: int, k: int = 16) -> dict:
         dist_equal = _bits_equal(got["distance"], exp["distance"])
         max_err = float(np.max(np.abs(got["distance"] - exp["distance"])))
         alg_bytes = len(probe) * 16 + len(build) * 16 + units * 24
-        kernel = "k_pass1<KNN> (nearest-list LBVH walk)"
+        kernel = "k_collect_packet<OWN> (radius from the curve window, packet walk)"
         full = {}
         ref = digests.get("knn16_1m")
         if ref and k == 16 and len(probe) == len(build) == 1 << 20:
@@ -408,7 +408,7 @@ def secondary_leg(workload: str, steps: int, warmup: int, k: int = 16) -> dict:
         dist_equal = _bits_equal(got_d[sample], dist)
         max_err = float(np.max(np.abs(got_d[sample] - dist)))
         alg_bytes = len(probe) * 16 + len(build) * 16 + len(probe) * 12
-        kernel = "k_pass1<KNN> with k = 1 (nearest LBVH walk)"
+        kernel = "k_nearest (packet walk)"
         full = {}
         ref = digests.get("hausdorff_4m")
         if ref:
@@ -1237,7 +1237,7 @@ def main(argv=None) -> int:
         dom, dom_kernel, dom_ms, dom_bytes = ("k_collect_packet (packet LBVH walk, FP32 test + FP64 band)",
                                               "k_collect_packet", traverse_ms, traverse_bytes)
     else:
-        dom, dom_kernel, dom_ms, dom_bytes = ("k_emit + k_emit_list (exact FP64 sort and row emission)",
+        dom, dom_kernel, dom_ms, dom_bytes = ("k_emit + k_emit_mid + k_emit_big (exact FP64 sort and row emission)",
                                               "k_emit", emit_ms, emit_bytes)
     achieved = dom_bytes / (dom_ms / 1e3) / 1e9
     traffic = measured_traffic(dom_kernel, "clustered_3d_fixed_radius", N_PROBE, N_BUILD)

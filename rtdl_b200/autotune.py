@@ -1,13 +1,10 @@
 """Autotuner for the fixed-radius path: picks the kernel configuration per shape class.
 
-The knobs (``rtdl_b200_set_tuning``): the LBVH leaf-bucket size (points per
-leaf, the traversal's tile), the collect traversal (``packet``: one warp walks
-the tree for 32 neighbouring queries; ``packet_cube``: the same with the
-query's bounding cube tested at internal nodes; ``packet_points``: the same
-with leaf buckets tested a lane per point, the reaching queries in turn;
-``packet_hybrid``, the library default: the one of those two leaf tests that
-costs less for each bucket; ``lane``: one thread per query) and the collect
-block size.  A shape class is the dimension plus the
+The knobs (``rtdl_b200_set_tuning``) are the leaf-bucket size, the collect
+traversal and the collect block size.  The library's walks have one form now
+(8-point buckets; packets or a warp per query, chosen per call and per packet),
+so every setting runs the same kernels and the candidates differ by timing noise
+only; the class stays for callers that use it.  A shape class is the dimension plus the
 log2 buckets of the build size, the query count and the mean in-radius count
 (from a sampled query).  :meth:`Autotuner.tune` times every candidate on the
 caller's device-resident data with CUDA events (min of ``repeats``), keeps

@@ -1050,14 +1050,17 @@ __device__ __forceinline__ void emit_groups(const EmitParams& P, uint32_t t, boo
 }
 
 // Queries with at most 64 candidates in processing (curve) order, eight lanes
-// each; queries with 65..kSlab candidates are k_emit_mid's and k_emit_big's, those on the
+// each (1M clustered queries: 253 us; a warp each took 325, with the load/store
+// pipe 71% busy, half of it shuffles).  Bound by the latency of the point
+// gathers.  Queries with 65..kSlab candidates are k_emit_mid's and k_emit_big's, those on the
 // generic path get their rows from k_expand.
 constexpr int kEmitThreads = 256;
 constexpr int kEmitLanes = 8;
 
 // The grid fills the GPU once (emit_grid) and each warp strides over the
 // queries: a warp takes its next four as soon as it is done with some, instead
-// of short blocks retiring and launching.
+// of short blocks retiring and launching.  Four blocks: 64 registers without
+// spills (three blocks 2460, five 2361 and four 2264 us for a batch's emit phase).
 constexpr int kEmitBlocksPerSm = 4;
 
 __global__ void __launch_bounds__(kEmitThreads, kEmitBlocksPerSm) k_emit(const __grid_constant__ EmitParams P) {
@@ -1766,7 +1769,8 @@ constexpr int kSummaryGroup = 8;  // queries per partial aggregate
 
 // A thread per query.  The sum of a query's distances is a chain of FP64 adds;
 // with a warp per query every add cost the warp two shuffles for one query, here
-// 32 chains share them, and a thread keeps eight distance loads in flight.
+// 32 chains share a warp, and a thread keeps eight distance loads in flight.  262k
+// queries with 50 rows each: 58 us, a warp per query 190.
 __global__ void __launch_bounds__(kSummaryThreads)
     k_summarize(const RtdlFixedRadiusNeighborRow* __restrict__ rows, const unsigned long long* __restrict__ offsets,
                 const uint32_t* __restrict__ oorder, const unsigned int* __restrict__ identity,
@@ -1871,7 +1875,8 @@ __device__ __forceinline__ void list_part(const EmitParams& P, const unsigned in
   }
 }
 
-// 65..128 candidates: 16 lanes per query (exact fixups deferred to k_emit_fixup).
+// 65..128 candidates: 16 lanes per query (exact fixups deferred to k_emit_fixup);
+// 99 us for the 13% of 1M clustered queries, 141 with a warp per query.
 __global__ void __launch_bounds__(kEmitListThreads)
     k_emit_mid(const __grid_constant__ EmitParams P, const uint32_t* work, uint32_t nwork, const unsigned int* nwork_dev) {
   __shared__ EmitGroups<16> shared[kEmitListThreads / 32];
@@ -2283,6 +2288,10 @@ __global__ void __launch_bounds__(kExpandThreads) k_expand(ExpandParams P) {
 }
 
 // ---- directed Hausdorff: FP64 max over per-query nearest distances ---------
+// Exact distances of the nearest points in input order, and a witness per block.
+// A chain of two dependent loads per query, the second scattered: with two
+// blocks per SM and one thread over the partial results 172 us for 4M queries,
+// with eight and k_witness_best 104.
 __global__ void __launch_bounds__(256)
     k_nearest_reduce(SceneView S, const float4* qpts, const double* qraw, int qstride, uint32_t nq,
                      const uint32_t* temp, double* nearest_dist, uint32_t* nearest_id, Witness* partial) {

@@ -215,22 +215,23 @@ def _plan(kernel_name, predicate, precision, build_input, probe_input, query_inp
     )
     fields = tuple((f, _EMIT_FIELD_TYPES.get(f, "unknown")) for f in emit_fields)
     if predicate == "knn_rows":
-        steps = (f"Build an LBVH over `{search_input.name}` on the device (Morton codes, radix sort, Karras "
-                 "hierarchy, refit).",
-                 f"For each point of `{query_input.name}`, seed a nearest list from the Morton window, walk the "
-                 "tree in FP32, re-decide the k-th-distance band in FP64.",
+        steps = (f"Build an LBVH over `{search_input.name}` on the device (Hilbert codes, radix sort, 8-point "
+                 "buckets, 32-ary levels).",
+                 f"For each point of `{query_input.name}`, take a radius that holds its k nearest from its window on "
+                 "the curve, collect within it in FP32, re-decide the radius band in FP64.",
                  f"Emit the k={options['k']!r} nearest rows per query with 1-based neighbor_rank, ordered by "
                  "(distance, neighbor_id), grouped by query_id.")
-        programs = ("k_pass1<KNN>", "k_expand")
+        programs = ("k_knn_radius", "k_collect_packet", "k_knn_single", "k_emit", "k_emit_mid", "k_emit_big",
+                    "k_emit_fixup")
     else:
-        steps = (f"Build an LBVH over `{search_input.name}` on the device (Morton codes, radix sort, Karras "
-                 "hierarchy, refit).",
+        steps = (f"Build an LBVH over `{search_input.name}` on the device (Hilbert codes, radix sort, 8-point "
+                 "buckets, 32-ary levels).",
                  f"Collect the points of `{search_input.name}` within the inclusive radius={options['radius']!r} "
                  "of each query in FP32; re-decide the radius band in FP64.",
                  f"Sort each query's candidates by (distance, neighbor_id), keep the k_max={options['k_max']!r} "
                  "nearest, emit rows grouped by query_id with exact FP64 distances"
                  + (" and 1-based neighbor_rank." if predicate == "bounded_knn_rows" else "."))
-        programs = ("k_collect_packet", "k_emit", "k_emit_list", "k_emit_fixup", "k_heavy_gather_bvh")
+        programs = ("k_collect_packet", "k_emit", "k_emit_mid", "k_emit_big", "k_emit_fixup", "k_heavy_gather_bvh")
     return B200ExecutionPlan(
         kernel_name=kernel_name,
         workload_kind=predicate,
@@ -246,8 +247,8 @@ def _plan(kernel_name, predicate, precision, build_input, probe_input, query_inp
         host_steps=steps,
         device_programs=programs,
         output_record=(record, fields),
-        bvh_policy="LBVH built on the device per call (or once per prepared scene); collapsed leaf buckets, "
-                   "rope-linked pre-order records",
+        bvh_policy="LBVH built on the device per call (or once per prepared scene); 8-point buckets under "
+                   "implicit 32-ary levels",
         predicate_options=options,
         query_input=query_input.name,
         search_input=search_input.name,
