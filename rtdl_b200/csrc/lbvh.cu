@@ -679,6 +679,10 @@ Scene* build_scene_impl(const void* points_dev, uint32_t n, int dim, cudaStream_
     sc->prob_stats = static_cast<PointStats*>(dev_alloc(sizeof(PointStats) * problems, s));
   }
   if (n == 0) {
+    // trees of no buckets, where every walk ends at once
+    const size_t bytes = sizeof(TreeShape) * (batch ? problems : 1);
+    sc->trees = static_cast<TreeShape*>(dev_alloc(bytes, s));
+    RTDL_CUDA_CHECK(cudaMemsetAsync(sc->trees, 0, bytes, s));
     if (batch) batch_boxes(nullptr, nullptr, 0, sc->prob_stats, problems, s);
     return sc;
   }

@@ -1576,7 +1576,6 @@ __global__ void __launch_bounds__(128) k_count_packet(const __grid_constant__ Co
   bool active = valid;
   const int lane = threadIdx.x & 31;
   const TreeShape* T = S.trees;
-  const uint32_t bucket0 = __ldg(&T->base[0]);
   BucketQuery bq;
   bq.set(q.x, q.y, q.z, B.top);
   const int band = valid ? (int)(0x80000001u + __float_as_uint(B.width)) : (int)0x80000000;
@@ -1651,7 +1650,6 @@ __global__ void __launch_bounds__(128) k_group_nearest_packet(const __grid_const
   bool found = false;
   const int lane = threadIdx.x & 31;
   const TreeShape* T = S.trees;
-  const uint32_t bucket0 = __ldg(&T->base[0]);
   BucketQuery bq;
   bq.set(q.x, q.y, q.z, B.top);  // every point that may be within radius, decided below
   const float reach2 = B.box_hi2;
