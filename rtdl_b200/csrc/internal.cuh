@@ -92,7 +92,8 @@ constexpr uint32_t kMaxScenePoints = 1u << 26;
 
 // Wide tree over the points in curve order, what the fixed-radius walks read.
 // Eight consecutive points make a bucket (the last one of a problem is filled
-// up with points at infinity, which no radius reaches), 32 consecutive buckets
+// up with points at infinity, which every walk leaves out, at an infinite
+// radius too: see walk_single and set_band_top), 32 consecutive buckets
 // a level-1 node, 32 of those a level-2 node, and so on until a level has at
 // most 32 nodes: no links, no splits.  A warp tests a node's 32 children in
 // one step, one per lane, with coalesced loads; 1M points take four levels

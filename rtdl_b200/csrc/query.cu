@@ -272,9 +272,10 @@ __device__ __noinline__ uint32_t exact_buckets_mask(const float4* pts, const dou
 }
 
 // One warp walks a tree for one query and its lanes test the reached buckets'
-// points together, four buckets at a time: visit(i, p, has) runs on every lane
-// with its point (has false: no point) and returns true, on all of them, to
-// end the walk.
+// points together, four buckets at a time: point(i, p, has) runs on every lane
+// with its point and returns true, on all of them, to end the walk.  has is
+// false where there is no bucket and for the points at infinity that fill one
+// up, which a radius whose square overflows would hold.
 template <typename Point>
 __device__ __forceinline__ void walk_single(const SceneView& S, const TreeShape* T, const float4& q,
                                             const float& reach2, WalkStack& stack, int lane, Point&& point) {
@@ -285,10 +286,9 @@ __device__ __forceinline__ void walk_single(const SceneView& S, const TreeShape*
       // lane group g (eight lanes) takes the g-th set bucket
       uint32_t m = mask;
       for (int g = 0; g < (lane >> 3); ++g) m &= m - 1u;
-      const bool has = m != 0u;
-      const uint32_t i = (bucket0 + first + (has ? (uint32_t)(__ffs((int)m) - 1) : 0u)) * kBucketPoints + (lane & 7);
+      const uint32_t i = (bucket0 + first + (m ? (uint32_t)(__ffs((int)m) - 1) : 0u)) * kBucketPoints + (lane & 7);
       const float4 p = __ldg(&S.pts[i]);
-      if (point(i, p, has)) return true;
+      if (point(i, p, m != 0u && p.x < INFINITY)) return true;
 #pragma unroll
       for (int g = 0; g < 4; ++g) mask &= mask - 1u;
     }
