@@ -21,6 +21,7 @@
 #include <vector>
 
 #include "internal.cuh"
+#include "per_device.cuh"
 
 namespace rtdl_b200 {
 
@@ -384,8 +385,7 @@ void run_rows_call(const void* q, size_t nq, const void* sp, size_t ns, int dim,
     const size_t row_size = predicate == kFrn ? sizeof(RtdlFixedRadiusNeighborRow) : sizeof(RtdlKnnNeighborRow);
     void* host;
     if (dl.host) {  // the copies were queued while the rows were emitted
-      static thread_local cudaEvent_t ev_copied = nullptr;
-      if (!ev_copied) RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_copied, cudaEventDisableTiming));
+      const cudaEvent_t ev_copied = aux_event(kEventCopied);
       RTDL_CUDA_CHECK(cudaEventRecord(ev_copied, dl.copy));
       RTDL_CUDA_CHECK(cudaStreamWaitEvent(s, ev_copied, 0));
       RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
@@ -421,17 +421,26 @@ struct PreparedHandle {
 
 }  // namespace
 
-
 cudaStream_t aux_stream(int which) {
-  static thread_local std::map<std::pair<int, int>, cudaStream_t> streams;
+  static thread_local PerDevice<cudaStream_t> streams;
   int dev = 0;
   RTDL_CUDA_CHECK(cudaGetDevice(&dev));
-  auto it = streams.find({dev, which});
-  if (it != streams.end()) return it->second;
-  cudaStream_t s;
-  RTDL_CUDA_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-  streams[{dev, which}] = s;
-  return s;
+  return streams.get(dev, which, [] {
+    cudaStream_t s;
+    RTDL_CUDA_CHECK(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    return s;
+  });
+}
+
+cudaEvent_t aux_event(AuxEvent which) {
+  static thread_local PerDevice<cudaEvent_t> events;
+  int dev = 0;
+  RTDL_CUDA_CHECK(cudaGetDevice(&dev));
+  return events.get(dev, which, [] {
+    cudaEvent_t e;
+    RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    return e;
+  });
 }
 }  // namespace rtdl_b200
 

@@ -395,6 +395,11 @@ QueryResult run_build_and_query_chunked(const BuildQueryInputs& in, int predicat
 // run_build_and_query and the row copies, 1 the heavy queries' refinement
 // beside the emit kernels and the query ranges' preparation one range ahead.
 cudaStream_t aux_stream(int which = 0);
+// The events that order this thread's streams on the current device.  A wait
+// holds what its event stood for when it was queued, so an event is recorded
+// again as soon as that is done.
+enum AuxEvent { kEventStart, kEventReady, kEventFork, kEventJoin, kEventRange, kEventCopied };
+cudaEvent_t aux_event(AuxEvent which);
 // Ranked-summary aggregates of several (radius, k_max) requests over one
 // prepared query set and one plain scene, captured once as a CUDA graph over
 // buffers allocated at creation (worst-case sizes) and replayed on the graph's

@@ -2985,7 +2985,6 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
         }
         E.order = eorder;
         E.fix_begin = small + 5;
-        static thread_local cudaEvent_t ev_range[kDownloadChunks] = {};
         unsigned long long first[kDownloadChunks + 1];
         for (int c = 0; c <= kDownloadChunks; ++c) first[c] = r.chunk_rows[c];
         if (first[kDownloadChunks] != res.rows) throw std::runtime_error("row ranges disagree with the row count");
@@ -3010,9 +3009,9 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
           k_emit_fixup<<<kSmCount * 4, kFixupThreads, 0, s>>>(E);
           k_fix_advance<<<1, 1, 0, s>>>(small + 5, small + 4);
           RTDL_LAUNCHED(4);
-          if (!ev_range[c]) RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_range[c], cudaEventDisableTiming));
-          RTDL_CUDA_CHECK(cudaEventRecord(ev_range[c], s));
-          RTDL_CUDA_CHECK(cudaStreamWaitEvent(dl->copy, ev_range[c], 0));
+          const cudaEvent_t ev_range = aux_event(kEventRange);
+          RTDL_CUDA_CHECK(cudaEventRecord(ev_range, s));
+          RTDL_CUDA_CHECK(cudaStreamWaitEvent(dl->copy, ev_range, 0));
           RTDL_CUDA_CHECK(cudaMemcpyAsync(static_cast<char*>(dl->host) + first[c] * row_size,
                                           static_cast<const char*>(rows_dev) + first[c] * row_size,
                                           (first[c + 1] - first[c]) * row_size, cudaMemcpyDeviceToHost, dl->copy));
@@ -3025,14 +3024,10 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
         // they run on the second stream beside k_emit, so each fills the
         // other's partial waves; they write disjoint rows, and the fix-up waits
         // for both.
-        static thread_local cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
         const bool side = np > kSingleQueries;
         cudaStream_t ls = s;
         if (side) {
-          if (!ev_fork) {
-            RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-            RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
-          }
+          const cudaEvent_t ev_fork = aux_event(kEventFork);
           ls = aux_stream();
           RTDL_CUDA_CHECK(cudaEventRecord(ev_fork, s));
           RTDL_CUDA_CHECK(cudaStreamWaitEvent(ls, ev_fork, 0));
@@ -3040,6 +3035,7 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
         launch_emit_lists(E, C, np, ls);
         launch_emit(E, np, s);
         if (side) {
+          const cudaEvent_t ev_join = aux_event(kEventJoin);
           RTDL_CUDA_CHECK(cudaEventRecord(ev_join, ls));
           RTDL_CUDA_CHECK(cudaStreamWaitEvent(s, ev_join, 0));
         }
@@ -3342,11 +3338,7 @@ QueryResult run_build_and_query(const BuildQueryInputs& in, int predicate, doubl
   }
   // the query side does not need the scene until its bands: it is prepared on
   // `aux` (own-box curve order) while the scene builds on `s`
-  static thread_local cudaEvent_t ev_start = nullptr, ev_ready = nullptr;
-  if (!ev_start) {
-    RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_start, cudaEventDisableTiming));
-    RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_ready, cudaEventDisableTiming));
-  }
+  const cudaEvent_t ev_start = aux_event(kEventStart), ev_ready = aux_event(kEventReady);
   RTDL_CUDA_CHECK(cudaEventRecord(ev_start, s));
   RTDL_CUDA_CHECK(cudaStreamWaitEvent(aux, ev_start, 0));  // whatever the caller queued on s comes first
   Scene* sc = build_scene(in.search_dev, in.ns, in.dim, s);
@@ -3446,8 +3438,7 @@ QueryResult run_build_and_query_chunked(const BuildQueryInputs& in, int predicat
   QueryResult total;
   try {
     // the query side waits for what the caller queued on s (the search set's upload)
-    static thread_local cudaEvent_t ev_start = nullptr;
-    if (!ev_start) RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_start, cudaEventDisableTiming));
+    const cudaEvent_t ev_start = aux_event(kEventStart);
     RTDL_CUDA_CHECK(cudaEventRecord(ev_start, s));
     RTDL_CUDA_CHECK(cudaStreamWaitEvent(ps, ev_start, 0));
     prepare_range(0);
@@ -3485,8 +3476,7 @@ QueryResult run_build_and_query_chunked(const BuildQueryInputs& in, int predicat
     }
     if (timer) timer->mark("queries");
     // the rows are released on `s` once it has waited for the copies
-    static thread_local cudaEvent_t ev_copied = nullptr;
-    if (!ev_copied) RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_copied, cudaEventDisableTiming));
+    const cudaEvent_t ev_copied = aux_event(kEventCopied);
     RTDL_CUDA_CHECK(cudaEventRecord(ev_copied, copy));
     RTDL_CUDA_CHECK(cudaStreamWaitEvent(s, ev_copied, 0));
     release();
@@ -4017,11 +4007,7 @@ QueryResult run_knn(Scene* sc, const void* queries_dev, uint32_t nq, uint32_t k,
         }
         launch_collect(C, np, false, s);
         // the queries the packets left, beside the emit kernels (disjoint rows)
-        static thread_local cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
-        if (!ev_fork) {
-          RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_fork, cudaEventDisableTiming));
-          RTDL_CUDA_CHECK(cudaEventCreateWithFlags(&ev_join, cudaEventDisableTiming));
-        }
+        const cudaEvent_t ev_fork = aux_event(kEventFork), ev_join = aux_event(kEventJoin);
         cudaStream_t ls = aux_stream();
         RTDL_CUDA_CHECK(cudaEventRecord(ev_fork, s));
         RTDL_CUDA_CHECK(cudaStreamWaitEvent(ls, ev_fork, 0));
