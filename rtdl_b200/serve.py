@@ -41,9 +41,11 @@ import numpy as np
 from .runtime import FRN_ROW_DTYPE, KNN_ROW_DTYPE, POINT2D_DTYPE, POINT3D_DTYPE, B200Scene
 
 FRN, KNN = "fixed_radius_neighbors", "knn_rows"
-_SLAB_BYTES_PER_PROBE = 256 * 8  # candidate slab entries per probe
+_SLAB_BYTES_PER_PROBE = 256 * 4  # candidate slab of one probe, fixed radius and KNN of k <= 64 alike
+_SLAB_PROBES_KNN = 1 << 22       # probes a KNN call answers at a time, over one slab
+_PACKET_PROBES = 32              # a fixed-radius request of a group is padded to whole packets
 _SCRATCH_BYTES_PER_PROBE = 160   # per-probe records, lists and orders of one call
-_SCENE_BYTES_PER_POINT = 112     # points, exact coordinates, order, codes, nodes
+_SCENE_BYTES_PER_POINT = 112     # points, exact coordinates, buckets, nodes, order, codes, and the build's scratch
 
 
 @dataclass
@@ -72,11 +74,18 @@ class Request:
 
 
 def request_bytes(op: str, probes: int, limit: int, dimension: int) -> int:
-    """Device memory one request is charged at admission."""
+    """Device memory one request is charged at admission: its records and rows, and what its call allocates
+    (the slab is most of that).  KNN of k > 64 keeps no slab; its candidates' scratch grows with the scene and is
+    not charged."""
     rec = 32 if dimension == 3 else 24
     row = 16 if op == FRN else 24
-    slab = _SLAB_BYTES_PER_PROBE if op == FRN else 4 * max(limit, 1)
-    return probes * (rec + row * max(limit, 1) + slab + _SCRATCH_BYTES_PER_PROBE)
+    if op == FRN:
+        ranks = -(-probes // _PACKET_PROBES) * _PACKET_PROBES
+        slab, scratch = ranks * _SLAB_BYTES_PER_PROBE, ranks * _SCRATCH_BYTES_PER_PROBE
+    else:
+        slab = min(probes, _SLAB_PROBES_KNN) * _SLAB_BYTES_PER_PROBE if limit <= 64 else probes * 4 * limit
+        scratch = probes * _SCRATCH_BYTES_PER_PROBE
+    return probes * (rec + row * max(limit, 1)) + slab + scratch
 
 
 class _Budget:
