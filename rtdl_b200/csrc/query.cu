@@ -1197,7 +1197,11 @@ __global__ void __launch_bounds__(128) k_knn_radius(SceneView S, const uint32_t*
 // lies in registers (entry l and l + 32 in lane l) under the exact order
 // (FP64 distance, id, search input index), and the walk's reach shrinks with its
 // last entry.  For the few queries whose radius holds more points than a slab
-// row (duplicates, mixed densities), and for callers without scratch.
+// row (duplicates, mixed densities), and for callers without scratch.  Where
+// many points tie at the k-th distance the time is the points', so 32 of them are
+// compared with the last entry at once and only what orders before it is
+// inserted, a warp step each: k = 16 of 100k queries over 200 sites of 1,000
+// points 7.45 -> 1.86 ms (every point inserted or refused by itself before).
 struct SingleParams {
   SceneView S;
   const float4* qpts;
@@ -1263,15 +1267,16 @@ __global__ void __launch_bounds__(256) k_knn_single(SingleParams P) {
       reach2 = __fmul_ru(hi2, 1.000001f);
     };
     set_reach(r);
-    SingleEntry e0{INFINITY, kNone}, e1{INFINITY, kNone};
+    SingleEntry e0{INFINITY, kNone}, e1{INFINITY, kNone}, kth{INFINITY, kNone};
     const int last = (int)(P.k < S.n ? P.k : S.n) - 1;
     walk_single(S, S.trees, q, reach2, stacks[threadIdx.x >> 5], lane, [&](uint32_t i, const float4& p, bool has) {
       const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
       const bool pass = has && fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= hi2;
-      unsigned int m = __ballot_sync(0xffffffffu, pass);
-      if (!m) return false;
+      if (!__any_sync(0xffffffffu, pass)) return false;
       SingleEntry mine{INFINITY, kNone};
       if (pass) mine = SingleEntry{__dsqrt_rn(exact_d2_at(ex, ey, ez, S.pts, S.pts64, scene_inexact, i)), i};
+      // only what orders before the list's last entry is inserted, one at a time
+      unsigned int m = __ballot_sync(0xffffffffu, pass && entry_before(S, mine, kth));
       bool changed = false;
       while (m) {
         const int from = __ffs((int)m) - 1;
@@ -1289,10 +1294,10 @@ __global__ void __launch_bounds__(256) k_knn_single(SingleParams P) {
         if (lane + 32 >= pos) e1 = lane + 32 == pos ? c : u1;
       }
       if (changed) {
-        const double k0 = __shfl_sync(0xffffffffu, e0.d, last & 31), k1 = __shfl_sync(0xffffffffu, e1.d, last & 31);
-        const double kth = last < 32 ? k0 : k1;
-        if (kth < r) {
-          r = kth;
+        kth.d = __shfl_sync(0xffffffffu, last < 32 ? e0.d : e1.d, last & 31);
+        kth.i = __shfl_sync(0xffffffffu, last < 32 ? e0.i : e1.i, last & 31);
+        if (kth.d < r) {
+          r = kth.d;
           set_reach(r);
         }
       }
