@@ -257,18 +257,24 @@ __device__ __forceinline__ DevBands bands_at_radius(const DevBands& base, double
   return b;
 }
 
-// Which points of four buckets are within the query's radius, each decided in
-// FP64 (a lane calls it when one of them lies inside the band).
-__device__ __noinline__ uint32_t exact_buckets_mask(const float4* pts, const double* pts64, int inexact,
-                                                    const double* rq, int qstride, double r2, uint4 four,
-                                                    uint32_t empty) {
-  const double ex = rq[1], ey = rq[2], ez = qstride == 4 ? rq[3] : 0.0;
-  uint32_t mask = 0;
-  for (int i = 0; i < 4 * kBucketPoints; ++i) {
-    const uint32_t b = i < 8 ? four.x : i < 16 ? four.y : i < 24 ? four.z : four.w;
-    if (b != empty && exact_d2_at(ex, ey, ez, pts, pts64, inexact, b * kBucketPoints + (i & 7)) <= r2) mask |= 1u << i;
+// Which of the hits among four buckets' points are within the query's radius:
+// those whose FP32 distance is not below the band, in FP64 (a lane calls it
+// when a hit lies inside the band; `lo` is the band's lower edge in the bucket
+// test's form).  On a lattice whose spacing divides the radius most packets
+// come here: counts of 60k queries over 1M points 932 us with all 32 points
+// decided in FP64, 696 with the hits taken one by one, 556 so.
+template <int DIM>
+__device__ __noinline__ uint32_t exact_buckets_mask(const SceneView& S, int inexact, const double* rq, float4 q,
+                                                    float lo, double r2, uint4 four, uint32_t hits) {
+  BucketQuery bq;
+  bq.set(q.x, q.y, q.z, lo);
+  for (uint32_t m = hits & ~buckets_mask<DIM, false>(S.bucket_pts, four, bq, nullptr); m; m &= m - 1u) {
+    const int j = __ffs((int)m) - 1;
+    const uint32_t b = j < 8 ? four.x : j < 16 ? four.y : j < 24 ? four.z : four.w;
+    if (!(exact_d2_at(rq[1], rq[2], DIM == 3 ? rq[3] : 0.0, S.pts, S.pts64, inexact, b * kBucketPoints + (j & 7)) <= r2))
+      hits &= ~(1u << j);
   }
-  return mask;
+  return hits;
 }
 
 // One warp walks a tree for one query and its lanes test the reached buckets'
@@ -371,8 +377,8 @@ __device__ __forceinline__ void collect_walk(const CollectParams& P, const TreeS
     int near;
     uint32_t hits = buckets_mask<DIM, true>(S.bucket_pts, four, bq, &near);
     if (near < band)
-      hits = exact_buckets_mask(S.pts, S.pts64, scene_inexact, P.qraw + (size_t)qin * P.qstride, P.qstride, B.r2,
-                                four, S.slots / kBucketPoints);
+      hits = exact_buckets_mask<DIM>(S, scene_inexact, P.qraw + (size_t)qin * P.qstride, q,
+                                     __fsub_rd(B.top, B.width), B.r2, four, hits);
     hits &= keep;
     found += __popc(hits);
     pending += __popc(hits);
@@ -1593,8 +1599,8 @@ __global__ void __launch_bounds__(128) k_count_packet(const __grid_constant__ Co
           int near;
           uint32_t hits = buckets_mask<DIM, true>(S.bucket_pts, four, bq, &near);
           if (near < band)
-            hits = exact_buckets_mask(S.pts, S.pts64, scene_inexact, P.qraw + (size_t)qin * P.qstride, P.qstride,
-                                      B.r2, four, S.slots / kBucketPoints);
+            hits = exact_buckets_mask<DIM>(S, scene_inexact, P.qraw + (size_t)qin * P.qstride, q,
+                                           __fsub_rd(B.top, B.width), B.r2, four, hits);
           if (!mine || !active) hits = 0;
           if (P.group_of) {
             for (uint32_t h = hits; h; h &= h - 1u) {
