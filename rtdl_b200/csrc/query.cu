@@ -316,8 +316,11 @@ struct CollectWarp {
 };
 
 // A packet's walk: every lane with `active` collects its points within band B
-// (their number in *count); the others keep what they have.
-template <int DIM>
+// (their number in *count); the others keep what they have.  BAND: the radius
+// decides the rows, so points inside the band are decided in FP64.  A KNN radius
+// only has to hold the k nearest: what lies just outside it may come along (it
+// is widened from the distance of a point, which would always lie in the band).
+template <int DIM, bool BAND>
 __device__ __forceinline__ void collect_walk(const CollectParams& P, const TreeShape* T, const DevBands& B,
                                              int scene_inexact, const float4& q, uint32_t qin, uint32_t t,
                                              bool active, CollectWarp& W, int lane, const PacketBox& box,
@@ -375,8 +378,8 @@ __device__ __forceinline__ void collect_walk(const CollectParams& P, const TreeS
   };
   walk_fours(S, T, box, limit, reach2, W.stack, W.list, lane, 32u, [&](const uint4& four) {
     int near;
-    uint32_t hits = buckets_mask<DIM, true>(S.bucket_pts, four, bq, &near);
-    if (near < band)
+    uint32_t hits = buckets_mask<DIM, BAND>(S.bucket_pts, four, bq, &near);
+    if (BAND && near < band)
       hits = exact_buckets_mask<DIM>(S, scene_inexact, P.qraw + (size_t)qin * P.qstride, q,
                                      __fsub_rd(B.top, B.width), B.r2, four, hits);
     hits &= keep;
@@ -565,7 +568,7 @@ __device__ __forceinline__ void collect_packet_body(const CollectParams& P, uint
     cut_packet(
         P.S, T, q, B.box_hi2, OWN || pass > 0, st.active, W.stack, lane,
         [&](bool mine, const PacketBox& box, const PacketBox* limit, float reach2) {
-          collect_walk<DIM>(P, T, B, scene_inexact, q, qin, t, mine, W, lane, box, limit, reach2, &count);
+          collect_walk<DIM, !OWN>(P, T, B, scene_inexact, q, qin, t, mine, W, lane, box, limit, reach2, &count);
         },
         [&](uint32_t run) {
           if (OWN || pass == 0) {  // a warp of its own for each of them
