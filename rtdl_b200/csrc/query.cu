@@ -2705,6 +2705,20 @@ GenericOut run_generic_path(Scene* sc, const QueryPrep& qp, const void* queries_
 // every SM); above it packets fill the GPU.
 constexpr uint32_t kSingleQueries = kSmCount * 32;
 
+// Whether the queries of a call on one scene walk alone, a warp each, because
+// they are few or lie far apart among its points: the box around a packet then
+// holds little that its queries share.  Time of walking alone over the packets'
+// (fixed radius with 0.5, 32 and 130 in radius; KNN k = 1, 8, 32; uniform and
+// clustered points): 3D, 10k queries 0.70 to 0.95 at any number of points, 40k
+// over 1M points 0.61 to 0.87, 80k over 2M 0.57 to 0.82, 120k over 1M 0.77 to
+// 0.97, 160k 0.93 to 1.16; 2D, 20k over 1M points 0.63 to 0.96, 40k 0.72 to 1.19.
+// With 11,000 in radius 3D packets share more: 40k over 1M points 0.80, 80k 1.35.
+// Nearest points of 40k queries over 1M in 3D: 213 us and 373.
+inline bool queries_alone(uint64_t queries, uint64_t points, int dim) {
+  return dim == 3 ? queries <= 3 * kSingleQueries || 16 * queries <= points
+                  : queries <= kSingleQueries || 50 * queries <= points;
+}
+
 // The queries the packets left (their number is on the device).
 void launch_collect_left(const CollectParams& C, uint32_t np, cudaStream_t s) {
   const unsigned int blocks = div_up(np, 128 / 32), cap = kSmCount * 8;
@@ -2727,7 +2741,7 @@ uint32_t packet_width(uint32_t np, bool batch) {
 
 // The collect pass over np processing ranks.
 void launch_collect(CollectParams& C, uint32_t np, bool batch, cudaStream_t s) {
-  if (np <= kSingleQueries && !C.rank_radius) {
+  if (!C.rank_radius && (batch ? np <= kSingleQueries : queries_alone(np, C.S.n, C.qstride - 1))) {
     k_collect_single<<<div_up(np, 128 / 32), 128, 0, s>>>(C, false);
     RTDL_LAUNCHED(1);
     return;
@@ -4013,7 +4027,7 @@ QueryResult run_knn(Scene* sc, const void* queries_dev, uint32_t nq, uint32_t k,
         H.rank_radius = C.rank_radius;
         H.poff = E.poff;
         H.sink = E.sink;
-        if (np <= kSingleQueries) {  // too few for packets: a warp per query throughout
+        if (queries_alone(np, sc->n, sc->dim)) {
           H.nwork = np;
           k_knn_single<<<div_up(np, 256 / 32), 256, 0, s>>>(H);
           RTDL_LAUNCHED(1);
@@ -4191,7 +4205,21 @@ HausdorffResult run_directed_hausdorff(Scene* sc, const void* queries_dev, uint3
   P.nq = nq;
   P.bands = qp.bands;
   P.nearest = temp;
-  if (sc->dim == 3)
+  if (queries_alone(nq, sc->n, sc->dim)) {
+    SingleParams H{};
+    H.S = P.S;
+    H.qpts = P.qpts;
+    H.qraw = P.qraw;
+    H.qstride = qstride;
+    H.bands = P.bands;
+    H.k = 1;
+    H.nwork = nq;
+    H.qorder = P.qorder;
+    H.qcodes = P.qcodes;
+    H.scodes = P.scodes;
+    H.nearest = temp;
+    k_knn_single<<<div_up(nq, 256 / 32), 256, 0, s>>>(H);
+  } else if (sc->dim == 3)
     k_nearest<3><<<div_up(nq, 128), 128, 0, s>>>(P);
   else
     k_nearest<2><<<div_up(nq, 128), 128, 0, s>>>(P);
