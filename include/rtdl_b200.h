@@ -623,9 +623,10 @@ RTDL_B200_API int rtdl_b200_get_last_phase_timings(const char** names_out, doubl
 /* Traversal counters of this thread's last query, recorded only when the
  * environment variable RTDL_B200_STATS is set at load time: nodes visited,
  * leaf points tested, in-radius candidates, list inserts, list shifts, FP64
- * band re-decisions, largest in-radius count of one query.  The walks count
- * in-radius candidates and their largest number; nodes, leaf points, inserts,
- * shifts and band re-decisions read 0.  Returns the number of counters. */
+ * band re-decisions, largest in-radius count of one query.  The fixed-radius and
+ * KNN (k <= 64) walks count in-radius candidates and their largest number (KNN:
+ * within the radius that bounds the query's k nearest); nodes, leaf points,
+ * inserts, shifts and band re-decisions read 0.  Returns the number of counters. */
 RTDL_B200_API int rtdl_b200_get_last_query_stats(unsigned long long* values_out, int capacity);
 
 /* Number of kernels this library has launched in the process so far (all

@@ -522,6 +522,11 @@ __device__ __forceinline__ void collect_finish(const CollectParams& P, uint32_t 
 // The record of a KNN query (no points: k_knn_single writes its rows).
 __device__ __forceinline__ void collect_finish_knn(const CollectParams& P, uint32_t t, uint32_t qin,
                                                    uint32_t points, uint32_t kmax) {
+  if (P.stats && points) {  // (k_knn_single counts its own)
+    atomicAdd(&P.stats[kStatInRadius], (unsigned long long)points);
+    atomicMax(&P.stats[kStatMaxLeafPoints], (unsigned long long)points);
+    if (points > 64u) atomicAdd(&P.stats[kStatLargeQueries], 1ull);
+  }
   uint32_t meta = points ? kmax << kQueryKmaxShift | points : 0u;
   if (points > 128u) {
     meta |= kQueryBig;
@@ -1235,6 +1240,7 @@ struct SingleParams {
   const unsigned long long* poff; // rows: first row by processing rank
   RowSink sink;
   uint32_t* nearest;              // instead of rows: the nearest point by query input index
+  unsigned long long* stats;      // STATS
 };
 
 struct SingleEntry {
@@ -1249,6 +1255,9 @@ __device__ __forceinline__ bool entry_before(const SceneView& S, const SingleEnt
   return __ldg(&S.perm[a.i]) < __ldg(&S.perm[b.i]);
 }
 
+// STATS: counts the points within reach (a counter in the plain form cost 6% of
+// a served k = 32 call).
+template <bool STATS>
 __global__ void __launch_bounds__(256) k_knn_single(SingleParams P) {
   __shared__ WalkStack stacks[256 / 32];
   const int lane = threadIdx.x & 31;
@@ -1285,10 +1294,12 @@ __global__ void __launch_bounds__(256) k_knn_single(SingleParams P) {
     set_reach(r);
     SingleEntry e0{INFINITY, kNone}, e1{INFINITY, kNone}, kth{INFINITY, kNone};
     const int last = (int)(P.k < S.n ? P.k : S.n) - 1;
+    uint32_t found = 0;
     walk_single(S, S.trees, q, reach2, stacks[threadIdx.x >> 5], lane, [&](uint32_t i, const float4& p, bool has) {
       const float dx = p.x - q.x, dy = p.y - q.y, dz = p.z - q.z;
       const bool pass = has && fmaf(dz, dz, fmaf(dy, dy, dx * dx)) <= hi2;
       if (!__any_sync(0xffffffffu, pass)) return false;
+      if (STATS) found += __popc(__ballot_sync(0xffffffffu, pass));
       SingleEntry mine{INFINITY, kNone};
       if (pass) mine = SingleEntry{__dsqrt_rn(exact_d2_at(ex, ey, ez, S.pts, S.pts64, scene_inexact, i)), i};
       // only what orders before the list's last entry is inserted, one at a time
@@ -1319,6 +1330,10 @@ __global__ void __launch_bounds__(256) k_knn_single(SingleParams P) {
       }
       return false;
     });
+    if (STATS && lane == 0) {
+      atomicAdd(&P.stats[kStatInRadius], (unsigned long long)found);
+      atomicMax(&P.stats[kStatMaxLeafPoints], (unsigned long long)found);
+    }
     if (P.nearest) {
       if (lane == 0) P.nearest[qin] = e0.i == kNone ? 0u : e0.i;
       continue;
@@ -4034,9 +4049,11 @@ QueryResult run_knn(Scene* sc, const void* queries_dev, uint32_t nq, uint32_t k,
         H.rank_radius = C.rank_radius;
         H.poff = E.poff;
         H.sink = E.sink;
+        H.stats = C.stats;
         if (queries_alone(np, sc->n, sc->dim)) {
           H.nwork = np;
-          k_knn_single<<<div_up(np, 256 / 32), 256, 0, s>>>(H);
+          stats ? k_knn_single<true><<<div_up(np, 256 / 32), 256, 0, s>>>(H)
+                : k_knn_single<false><<<div_up(np, 256 / 32), 256, 0, s>>>(H);
           RTDL_LAUNCHED(1);
           continue;
         }
@@ -4048,7 +4065,8 @@ QueryResult run_knn(Scene* sc, const void* queries_dev, uint32_t nq, uint32_t k,
         RTDL_CUDA_CHECK(cudaStreamWaitEvent(ls, ev_fork, 0));
         H.work = C.single_list;
         H.nwork_dev = small + 6;
-        k_knn_single<<<kSmCount * 4, 256, 0, ls>>>(H);
+        stats ? k_knn_single<true><<<kSmCount * 4, 256, 0, ls>>>(H)
+              : k_knn_single<false><<<kSmCount * 4, 256, 0, ls>>>(H);
         launch_emit_lists(E, C, np, ls);
         RTDL_CUDA_CHECK(cudaEventRecord(ev_join, ls));
         launch_emit(E, np, s);
@@ -4225,7 +4243,7 @@ HausdorffResult run_directed_hausdorff(Scene* sc, const void* queries_dev, uint3
     H.qcodes = P.qcodes;
     H.scodes = P.scodes;
     H.nearest = temp;
-    k_knn_single<<<div_up(nq, 256 / 32), 256, 0, s>>>(H);
+    k_knn_single<false><<<div_up(nq, 256 / 32), 256, 0, s>>>(H);
   } else if (sc->dim == 3)
     k_nearest<3><<<div_up(nq, 128), 128, 0, s>>>(P);
   else
@@ -4363,7 +4381,7 @@ void run_directed_hausdorff_noalloc(Scene* sc, const void* queries_dev, uint32_t
   P.qcodes = codes;
   P.scodes = sc->codes;
   P.nearest = temp;
-  k_knn_single<<<grid_for((uint64_t)nq * 32, 256), 256, 0, s>>>(P);
+  k_knn_single<false><<<grid_for((uint64_t)nq * 32, 256), 256, 0, s>>>(P);
   RTDL_LAUNCHED(1);
   const unsigned int blocks = grid_for(nq, 256) < kNoAllocReduceBlocks ? grid_for(nq, 256) : kNoAllocReduceBlocks;
   k_nearest_reduce<<<blocks, 256, 0, s>>>(sc->view(), qpts, static_cast<const double*>(queries_dev), P.qstride, nq,
