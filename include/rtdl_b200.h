@@ -320,9 +320,9 @@ RTDL_B200_API int rtdl_b200_batch_fixed_radius_neighbors_device(
  * to back, problem p at [query_offsets[p], query_offsets[p + 1]) (host array,
  * total problems + 1 entries), with radius[p] and k_max[p] (1..64).  One
  * replay answers every problem: per batch one persistent collect launch takes
- * 32-query packets from a device work queue, then the scan, the radius
- * refinement and the emit run device-driven (nothing is read back inside the
- * graph).  Rows go to rows_dev (device, capacity rows_capacity rows) problem
+ * packets of up to 32 queries from a device work queue (and narrows the radius
+ * of crowded ones), then the scan and the emit run device-driven (nothing is
+ * read back inside the graph).  Rows go to rows_dev (device, capacity rows_capacity rows) problem
  * by problem, each problem's exactly as rtdl_b200_batch_fixed_radius_neighbors
  * returns them.  The query records, the batches and rows_dev must stay valid
  * until the graph is destroyed. */
@@ -569,9 +569,9 @@ RTDL_B200_API int rtdl_b200_launch_fixed_radius_ranked_summary_aggregate_batch_g
     size_t* query_block_count_out, uint64_t* cuda_stream_ptr_out, char* error_out, size_t error_size);
 
 /* No counterpart in the reference: the device address of the per-request
- * status words of the last replay (0 = the partial is valid; bit 0 traversal
- * stack overflow; bit 1 heavy queries left for the generic path) and how many
- * requests replay has recomputed by the plain call so far. */
+ * status words of the last replay (0 = the partial is valid; bit 1 heavy queries
+ * left for the generic path; bit 0 is not used) and how many requests replay has
+ * recomputed by the plain call so far. */
 RTDL_B200_API int rtdl_b200_fixed_radius_ranked_summary_aggregate_batch_graph_status_device_3d(
     void* graph, uint64_t* status_device_ptr_out, uint64_t* fallback_count_out, char* error_out, size_t error_size);
 

@@ -44,20 +44,14 @@ void check_launch(int n, const char* file, int line) {
 namespace {
 thread_local std::string g_cleanup_error;
 
-std::mutex& tuning_mutex() {
-  static std::mutex m;
-  return m;
-}
-Tuning& tuning_global() {
-  static Tuning t;
-  return t;
-}
-Tuning tuning_copy() {
-  std::lock_guard<std::mutex> g(tuning_mutex());
-  return tuning_global();
-}
-thread_local Tuning g_tuning_snapshot;
-thread_local int g_tuning_depth = 0;
+thread_local int g_entry_depth = 0;
+
+// An entry point that another one calls leaves the thread's errors to it.
+struct EntryScope {
+  EntryScope() : outer(g_entry_depth == 0) { ++g_entry_depth; }
+  ~EntryScope() { --g_entry_depth; }
+  bool outer;
+};
 }  // namespace
 
 void note_cleanup_error(cudaError_t e, const char* what) {
@@ -65,22 +59,6 @@ void note_cleanup_error(cudaError_t e, const char* what) {
   cudaGetLastError();  // consumed here: a later launch check must not report it
   if (g_cleanup_error.empty())
     g_cleanup_error = std::string("CUDA error: ") + cudaGetErrorString(e) + " at " + what;
-}
-
-TuningScope::TuningScope() : outer(g_tuning_depth == 0) {
-  if (outer) g_tuning_snapshot = tuning_copy();
-  ++g_tuning_depth;
-}
-TuningScope::~TuningScope() { --g_tuning_depth; }
-
-const Tuning& tuning() {
-  if (g_tuning_depth == 0) g_tuning_snapshot = tuning_copy();  // outside an entry point: the current setting
-  return g_tuning_snapshot;
-}
-
-void set_tuning(const Tuning& t) {
-  std::lock_guard<std::mutex> g(tuning_mutex());
-  tuning_global() = t;
 }
 
 void ensure_pool_configured(int device) {
@@ -228,11 +206,11 @@ void set_error(const char* msg, char* error_out, size_t error_size) {
 
 // Every entry point runs through here: the thread's last runtime error is
 // cleared first (an error left by earlier, unrelated runtime calls on this
-// thread is not this call's), the call runs with one tuning snapshot, and a
-// cleanup error that nothing else reported fails the call.
+// thread is not this call's), and a cleanup error that nothing else reported
+// fails the call.
 template <typename Fn>
 int guarded(Fn&& fn, char* error_out, size_t error_size) {
-  TuningScope scope;
+  EntryScope scope;
   try {
     if (error_out && error_size) error_out[0] = '\0';
     if (scope.outer) {
@@ -463,12 +441,7 @@ int rtdl_b200_set_tuning(int leaf_size, int block_threads, int traversal) {
   if (leaf_size < 0 || leaf_size > 32) return 1;
   if (block_threads != 64 && block_threads != 128 && block_threads != 256) return 1;
   if (traversal < 0 || traversal > 4) return 1;
-  Tuning t;
-  t.leaf_size = leaf_size;
-  t.block_threads = block_threads;
-  t.traversal = traversal;
-  set_tuning(t);
-  return 0;
+  return 0;  // the walks have one form: there is nothing to set
 }
 
 int rtdl_b200_get_last_phase_timings(const char** names_out, double* values_ms_out, int capacity) {

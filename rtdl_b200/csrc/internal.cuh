@@ -165,25 +165,6 @@ struct Scene {
   }
 };
 
-// ---- tuning ---------------------------------------------------------------
-// Settings of rtdl_b200_set_tuning.  The walks have one form, so every setting
-// runs the same kernels; they stay for callers that set them.
-struct Tuning {
-  int leaf_size = 0;
-  int block_threads = 128;
-  int traversal = 4;
-};
-// The tuning a call runs with: a copy of the process-wide setting taken when
-// the entry point starts (rtdl_b200_set_tuning from another thread changes the
-// next call, never one in progress).
-const Tuning& tuning();
-void set_tuning(const Tuning& t);
-struct TuningScope {  // takes the calling thread's snapshot for one entry point
-  TuningScope();
-  ~TuningScope();
-  bool outer;
-};
-
 // ---- phase timing (CUDA events, read after the call's final sync) ----------
 struct PhaseTimer {
   cudaStream_t stream;

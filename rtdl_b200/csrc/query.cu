@@ -47,7 +47,6 @@ struct DevBands {
   float rho, e_abs, floor2;
   double r2;
   unsigned int ids_sorted;
-  unsigned int any_inexact;
 };
 
 // The bucket test's form of [lo2, hi2].  It computes d2 - top as one fma chain
@@ -78,7 +77,6 @@ __device__ DevBands make_bands(const PointStats* scene, const PointStats* querie
   b.rho = (float)rho;
   b.e_abs = __double2float_ru(e_abs);
   b.floor2 = 1.0e-30f;
-  b.any_inexact = inexact ? 1u : 0u;
   b.ids_sorted = queries->ids_unsorted ? 0u : 1u;
   if (has_radius) {
     const double r_hi = radius * (1.0 + rho) + e_abs + 1.0e-18;
@@ -179,7 +177,9 @@ __device__ __noinline__ bool exact_before(double ex, double ey, double ez, const
   return __ldg(&perm[ia]) < __ldg(&perm[ib]);
 }
 
-// Traversal counters gathered by the STATS instantiation (diagnostics).
+// Counters of RTDL_B200_STATS, by their place in rtdl_b200_get_last_query_stats
+// (the walks gather neither nodes, leaf points, inserts, shifts, band checks nor
+// leaf pairs: those read 0).
 enum Stat { kStatNodes, kStatLeafPoints, kStatInRadius, kStatInserts, kStatShifts, kStatBand, kStatMaxLeafPoints,
             kStatGenericQueries, kStatLargeQueries, kStatLeafPairs, kStatEmitFixups, kStatRefined, kStatCount };
 
@@ -234,7 +234,7 @@ struct CollectParams {
   uint32_t* mid_list;        // processing ranks of the queries with 65..128 candidates
   uint32_t* big_list;        // processing ranks of the queries with 129..kSlab candidates
   uint32_t* single_list;     // processing ranks the packets leave to k_collect_single
-  unsigned int* small;       // [0] generic-path query count, [1] error bits, [2] mid_list length,
+  unsigned int* small;       // [0] generic-path query count, [1] the generic path's error bits, [2] mid_list length,
                              // [3] big_list length, [4] emit fixup queue length, [6] single_list length
   uint8_t* overflow_out;     // optional: 1 per query (input order) when count > kmax
   unsigned long long* stats;
@@ -2095,7 +2095,7 @@ __device__ __forceinline__ Ctx make_ctx(const SceneView& S, const float4* qpts, 
 
 __global__ void __launch_bounds__(kHeavyThreads)
     k_heavy_gather(SceneView S, const float4* qpts, const double* qraw, int qstride, const uint32_t* heavy_list,
-                   const unsigned long long* seg_off, const uint32_t* seg_size, int knn, const DevBands* bands,
+                   const unsigned long long* seg_off, const uint32_t* seg_size, const DevBands* bands,
                    HeavyEntry* scratch, unsigned int* error) {
   __shared__ unsigned int cnt;
   if (threadIdx.x == 0) cnt = 0;
@@ -2107,13 +2107,6 @@ __global__ void __launch_bounds__(kHeavyThreads)
   HeavyEntry* seg = scratch + seg_off[h];
   const uint32_t P2 = seg_size[h];
   for (uint32_t i = threadIdx.x; i < S.n; i += blockDim.x) {
-    if (!knn) {
-      const float4 p = __ldg(&S.pts[i]);
-      const float dx = p.x - c.qx, dy = p.y - c.qy, dz = p.z - c.qz;
-      const float d2 = fmaf(dz, dz, fmaf(dy, dy, dx * dx));
-      if (d2 > B.hi2) continue;
-      if (d2 >= B.lo2 && exact_d2(c, i) > B.r2) continue;
-    }
     const double dist = __dsqrt_rn(exact_d2(c, i));
     const unsigned int pos = atomicAdd(&cnt, 1u);
     if (pos < P2) {
@@ -2706,7 +2699,7 @@ GenericOut run_generic_path(Scene* sc, const QueryPrep& qp, const void* queries_
   RTDL_CUDA_CHECK(cudaMemcpyAsync(d_out_cnt, out_cnt.data(), sizeof(uint32_t) * H, cudaMemcpyHostToDevice, s));
   if (knn)
     k_heavy_gather<<<H, kHeavyThreads, 0, s>>>(sc->view(), qp.qpts, static_cast<const double*>(queries_dev), qstride,
-                                               heavy_list, d_seg_off, d_seg_size, 1, qp.bands, scratch, error);
+                                               heavy_list, d_seg_off, d_seg_size, qp.bands, scratch, error);
   else
     k_heavy_gather_bvh<<<H, 32, 0, s>>>(qp.view, qp.qpts, static_cast<const double*>(queries_dev), qstride,
                                         heavy_list, d_seg_off, d_seg_size, qp.bands, qp.qprob, item_rad, scratch,
@@ -2801,11 +2794,6 @@ void launch_emit_lists(const EmitParams& E, const CollectParams& C, uint32_t np,
   k_emit_mid<<<list_grid(np), kEmitListThreads, 0, s>>>(E, C.mid_list, 0, C.small + 2);
   k_emit_big<<<list_grid(np), kEmitListThreads, 0, s>>>(E, C.big_list, 0, C.small + 3);
   RTDL_LAUNCHED(2);
-}
-
-void check_readback(const Readback& r) {
-  throw_if_bad(r.scene_bad | r.query_bad);
-  if (r.error & 1u) throw std::runtime_error("BVH traversal stack overflow");
 }
 
 // fixed_radius_neighbors / bounded_knn_rows: collect, scan, emit.
@@ -2920,7 +2908,7 @@ QueryResult run_radius_query(Scene* sc, const void* queries_dev, uint32_t nq, in
       reads.add(&rb->query_bad, &qp.qst->bad, sizeof(unsigned int));
       reads.launch(s);
       RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
-      check_readback(*rb);
+      throw_if_bad(rb->scene_bad | rb->query_bad);
       res.rows = rb->rows;
       res.heavy = rb->heavy;
       return *rb;
@@ -3236,7 +3224,7 @@ void count_walk(Scene* sc, const void* queries_dev, uint32_t nq, double radius, 
     if (reached)
       RTDL_CUDA_CHECK(cudaMemcpyAsync(&rb->rows, reached, sizeof(unsigned long long), cudaMemcpyDeviceToHost, s));
     RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
-    check_readback(*rb);
+    throw_if_bad(rb->scene_bad | rb->query_bad);
     if (out.reached_host) *out.reached_host = rb->rows;
   } catch (...) {
     sync_quietly(s);
@@ -3542,16 +3530,13 @@ QueryResult run_build_and_query_chunked(const BuildQueryInputs& in, int predicat
 // ---- captured summary graphs ------------------------------------------------
 namespace {
 
-constexpr unsigned int kGraphStatusOverflow = 1u;  // traversal stack overflow (the plain call raises it)
 constexpr unsigned int kGraphStatusGeneric = 2u;   // heavy queries left for the generic path
 constexpr unsigned int kBatchGraphStatusRows = 4u;  // a batch graph's rows exceed the caller's row buffer
 
 __global__ void k_graph_status(const unsigned int* small, uint32_t requests, unsigned int* status) {
   for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < requests; r += gridDim.x * blockDim.x)
-    status[r] = ((small[8 * (size_t)r + 1] & 1u) ? kGraphStatusOverflow : 0u) |
-                (small[8 * (size_t)r] ? kGraphStatusGeneric : 0u);
+    status[r] = small[8 * (size_t)r] ? kGraphStatusGeneric : 0u;
 }
-
 
 }  // namespace
 
@@ -3818,7 +3803,6 @@ void summary_graph_replay(SummaryGraph* g, RtdlFixedRadiusRankedNeighborAggregat
   RTDL_CUDA_CHECK(cudaMemcpyAsync(g->status_host, g->status, sizeof(unsigned int) * g->R, cudaMemcpyDeviceToHost, s));
   RTDL_CUDA_CHECK(cudaStreamSynchronize(s));
   for (uint32_t r = 0; r < g->R; ++r) {
-    if (g->status_host[r] & kGraphStatusOverflow) throw std::runtime_error("BVH traversal stack overflow");
     if (g->status_host[r] & kGraphStatusGeneric) {
       // the plain call, with its generic path for the queries refinement left
       run_ranked_summaries(g->sc, nullptr, g->nq, g->radius[r], g->kmax[r], nullptr, &out[r], s, nullptr, g->pq);
@@ -4442,8 +4426,7 @@ __global__ void __launch_bounds__(kCollectThreads, 6) k_collect_persistent(const
 __global__ void k_batch_graph_status(const unsigned int* small, uint32_t batches, const unsigned long long* total, unsigned long long capacity,
                                      unsigned int* status) {
   for (uint32_t b = blockIdx.x * blockDim.x + threadIdx.x; b < batches; b += gridDim.x * blockDim.x)
-    status[b] = ((small[8 * (size_t)b + 1] & 1u) ? kGraphStatusOverflow : 0u) |
-                (small[8 * (size_t)b] ? kGraphStatusGeneric : 0u) |
+    status[b] = (small[8 * (size_t)b] ? kGraphStatusGeneric : 0u) |
                 (*total > capacity ? kBatchGraphStatusRows : 0u);
 }
 
@@ -4762,7 +4745,6 @@ void batch_graph_replay(BatchGraph* g, unsigned long long* row_offsets_out, unsi
   for (uint32_t i = 0; i < B; ++i) {
     const unsigned int st = g->status_host[i];
     all |= st;
-    if (st & kGraphStatusOverflow) throw std::runtime_error("LBVH traversal stack overflow");
     if ((st & kGraphStatusGeneric) && g->rows && !(st & kBatchGraphStatusRows)) {
       // heavy queries the refinement did not resolve: this batch's rows by the plain batch call
       BatchGraphPart& b = g->parts[i];
