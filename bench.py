@@ -606,9 +606,6 @@ def batch_workload(args) -> dict:
     d_probe = torch.from_numpy(concat_records(probes).view(np.uint8)).to(dev)
     del probs
     chunks = _plan_chunks(nb, nq, 32 << 20, 8 << 20)
-    from dataclasses import asdict
-
-    from rtdl_b200.autotune import Autotuner
 
     def one_batch(ci, rows_buf, cap):
         a, b = chunks[ci]
@@ -649,12 +646,6 @@ def batch_workload(args) -> dict:
     rows_total = batch_step(None, 0, chunk_sizes)
     max_chunk_rows = max(int(o[-1]) for o in chunk_sizes)
     rows_buf = torch.empty(max_chunk_rows * 16, dtype=torch.uint8, device=dev)
-    # autotune (leaf size, block size; batches always walk in warp packets) on one whole batch, the largest
-    big = int(np.argmax([int(o[-1]) for o in chunk_sizes]))
-    tuner = Autotuner(repeats=2, traversals=("packet_hybrid", "packet"))
-
-    tune_key, tune_cfg = tuner.tune_callable(f"problem batch {big} of {len(chunks)}",
-                                             lambda: one_batch(big, rows_buf, max_chunk_rows), stream=stream)
     assert plain_step(None, 0, plain_sizes) == rows_total
     plain_buf = torch.empty(max(plain_sizes) * 16, dtype=torch.uint8, device=dev)
     for _ in range(args.warmup):
@@ -734,7 +725,6 @@ def batch_workload(args) -> dict:
         "plain_per_call": {"value": rows_total / (plain_ms[0] / 1e3), "unit": "rows/s", "ms": plain_ms[0],
                            "launches": "one scene build + one query per problem"},
         "speedup_vs_plain": plain_ms[0] / ms_step,
-        "autotune": {"shape_class": tune_key, "config": asdict(tune_cfg), "candidates_ms": tuner.cache[tune_key]["ms"]},
         "roofline": {"bound": "hbm", "kernel": "whole batched step (build + collect + emit)",
                      "achieved": alg / (ms_step / 1e3) / 1e9, "peak": hbm_peak, "unit": "GB/s",
                      "frac": alg / (ms_step / 1e3) / 1e9 / hbm_peak, "traffic": None, "algorithmic_bytes": alg},
@@ -1297,13 +1287,11 @@ def main(argv=None) -> int:
         sub = argparse.Namespace(**vars(args))
         sub.steps, sub.warmup = 3, 3
         b = batch_workload(sub)
-        rt.set_tuning()  # the batch leg's autotuner leaves its winner set
         batch2048 = {"metric": b["metric"], "value": b["value"], "unit": b["unit"], "ms_per_step": b["ms_per_step"],
                      "step": "one build + query per batch of problems", "config": b["config"],
                      "plain_per_call": b["plain_per_call"], "speedup_vs_plain": b["speedup_vs_plain"],
                      "graph": b.get("graph"), "speedup_graph_vs_plain": b.get("speedup_graph_vs_plain"),
-                     "exactness": b["exactness"], "roofline": b["roofline"], "gpu_launches": b["gpu_launches"],
-                     "autotune": {"tuned_on": b["autotune"]["shape_class"], "config": b["autotune"]["config"]}}
+                     "exactness": b["exactness"], "roofline": b["roofline"], "gpu_launches": b["gpu_launches"]}
         v = serve_workload(sub)
         serve = {"metric": v["metric"], "value": v["value"], "unit": v["unit"], "config": v["config"],
                  "served": v["served"], "plain_per_call": v["plain_per_call"],
