@@ -269,8 +269,8 @@ RTDL_B200_API int rtdl_b200_scene_directed_hausdorff_device(
 /* ---- problem batches -------------------------------------------------------
  * Many independent fixed-radius problems of uneven sizes answered together:
  * one LBVH build over all problems' points (the sort key carries the problem
- * id, so every problem is a subtree of its own) and one collect / emit launch
- * sequence over all queries, each warp walking its problem's subtree.  No
+ * id, and every problem has a tree of its own) and one collect / emit launch
+ * sequence over all queries, each warp walking its problem's tree.  No
  * reference counterpart: the reference runs one call per problem
  * (rtdl_optix_api.cpp:4076-4150); its batched form only splits one query set
  * into chunks (rtdl_optix_workloads.cpp:14380-14409). */
@@ -278,8 +278,10 @@ RTDL_B200_API int rtdl_b200_scene_directed_hausdorff_device(
 /* Builds the batch.  points: the problems' RtdlPoint / RtdlPoint3D records back
  * to back, problem p at [point_offsets[p], point_offsets[p + 1]) (host array
  * of problems + 1 entries, starting at 0); points_on_device says whether
- * `points` is a device pointer.  At most 67,108,864 points in all.  The
- * handle is released with rtdl_b200_batch_destroy. */
+ * `points` is a device pointer.  At most 67,108,864 points in all.  A problem
+ * owns whole 8-point buckets and a tree node of its own, so one with points takes
+ * at least 0.6 KB, and in a call one with queries whole packets of 32, 34 KB of
+ * scratch.  The handle is released with rtdl_b200_batch_destroy. */
 RTDL_B200_API int rtdl_b200_batch_create(
     const void* points, const unsigned long long* point_offsets, uint32_t problems,
     int dimension, int points_on_device, void* stream, void** batch_out,
@@ -335,7 +337,7 @@ RTDL_B200_API int rtdl_b200_batch_graph_create(
  * entries) receives each problem's first row and the total; status_out
  * (optional) the OR of the batches' status bits (4: the rows exceeded
  * rows_capacity, rows past it were not written).  A batch with heavy queries
- * the refinement did not resolve is recomputed by the plain batch call. */
+ * the collect did not resolve is recomputed by the plain batch call. */
 RTDL_B200_API int rtdl_b200_batch_graph_replay(
     void* graph, unsigned long long* row_offsets_out, uint32_t* status_out, char* error_out, size_t error_size);
 
@@ -540,21 +542,21 @@ RTDL_B200_API void rtdl_b200_destroy_prepared_point_group_nearest_witness_2d(voi
  * Replace the batch-graph entry points of rtdl_optix_api.cpp:4323-4396
  * (prepare / replay / launch-with-device-partials / update / destroy).
  * One CUDA graph holds, for each (radius, k_max) request in order, the whole
- * fixed-radius path over the prepared query set (collect, device-driven
- * heavy-query refinement, emit into an internal row buffer, ranked summary,
+ * fixed-radius path over the prepared query set (collect, which narrows the
+ * radius of crowded queries, emit into an internal row buffer, ranked summary,
  * aggregate); all buffers are allocated at prepare.  The graph runs on its own
  * stream.  update re-captures it with new requests (same request_count).
  * The aggregates are the exact ones of
  * rtdl_b200_aggregate_prepared_query_ranked_fixed_radius_neighbor_summaries_3d.
  * Requests: radius in [0, max_radius], 1 <= k_max <= 64; both handles
- * non-empty.  No query-count cap beyond device memory (nq x 2 KiB of slab plus
+ * non-empty.  No query-count cap beyond device memory (nq x 1 KiB of slab plus
  * nq x k_max rows). */
 RTDL_B200_API int rtdl_b200_prepare_fixed_radius_ranked_summary_aggregate_batch_graph_3d(
     void* prepared, void* prepared_queries, const double* radii, const size_t* k_values, size_t request_count,
     void** graph_out, char* error_out, size_t error_size);
 
 /* Replays the graph and writes request_count aggregates.  A request whose
- * heavy queries the refinement passes left unresolved is recomputed by the
+ * heavy queries the narrowing passes left unresolved is recomputed by the
  * plain call (its generic path) before this returns. */
 RTDL_B200_API int rtdl_b200_replay_fixed_radius_ranked_summary_aggregate_batch_graph_3d(
     void* graph, RtdlFixedRadiusRankedNeighborAggregate* aggregates_out, char* error_out, size_t error_size);

@@ -204,7 +204,7 @@ class B200ProblemBatchGraph:
     (problem p at ``query_offsets[p]:query_offsets[p + 1]``, problems numbered
     batch after batch); rows go to the device buffer at ``rows_address``
     (capacity ``rows_capacity`` rows) problem by problem.  Per batch, one
-    persistent collect launch takes 32-query packets from a device work queue;
+    persistent collect launch takes packets of queries from a device work queue;
     nothing is read back inside the graph.  Mirrors the reference's captured
     batch graph (``rtdl_optix_api.cpp:4323-4396``), for problem batches.
     """

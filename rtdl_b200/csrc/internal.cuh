@@ -373,8 +373,8 @@ QueryResult run_build_and_query_chunked(const BuildQueryInputs& in, int predicat
                                         cudaStream_t s, cudaStream_t copy, PhaseTimer* timer, Scene** scene_out,
                                         void* host_rows, unsigned long long host_capacity_rows, int chunks);
 // Further streams of this thread on the current device: 0 is the query side of
-// run_build_and_query and the row copies, 1 the heavy queries' refinement
-// beside the emit kernels and the query ranges' preparation one range ahead.
+// run_build_and_query, the row copies and the list kernels beside the emit, 1 the
+// query ranges' preparation one range ahead.
 cudaStream_t aux_stream(int which = 0);
 // The events that order this thread's streams on the current device.  A wait
 // holds what its event stood for when it was queued, so an event is recorded
@@ -385,10 +385,9 @@ cudaEvent_t aux_event(AuxEvent which);
 // prepared query set and one plain scene, captured once as a CUDA graph over
 // buffers allocated at creation (worst-case sizes) and replayed on the graph's
 // own stream.  The captured path is the fixed-radius path without host reads:
-// list lengths and refinement counts stay on the device and every pass is
-// launched.  A request whose heavy queries do not resolve in the refinement
-// passes (the plain call takes its generic path for them) is marked in the
-// status words and recomputed by the plain call at replay.
+// list lengths stay on the device.  A request whose heavy queries the collect's
+// narrowing passes do not resolve (the plain call takes its generic path for
+// them) is marked in the status words and recomputed by the plain call at replay.
 struct SummaryGraph;
 SummaryGraph* summary_graph_create(Scene* sc, const PreparedQueries* pq, const double* radii, const uint32_t* kmax,
                                    uint32_t requests);

@@ -13,8 +13,8 @@
 //   5. levels:  the boxes of the upper levels, 32 children per node, until a
 //               level has at most 32 nodes.
 // The tree's shape follows from the number of points, so there are no splits,
-// links or counts to compute: 1M points build in 0.21 ms, of which the sort
-// takes 0.13 (the binary radix tree over the same codes, with its collapse,
+// links or counts to compute: 1M points build in 0.17 ms, of which the sort's
+// passes take 0.07 (the binary radix tree over the same codes, with its collapse,
 // refit and pre-order records, took 0.38 ms).
 #include "internal.cuh"
 

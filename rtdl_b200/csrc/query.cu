@@ -15,9 +15,9 @@
 //     8 * 2^-24 * max|coordinate| (the FP32 rounding of the inputs); see
 //     k_bands.
 //   * A warp walks the wide tree for a packet of 32 neighbouring queries and
-//     keeps every query's candidates (collect); a warp per query then sorts them
-//     by FP32 keys, re-decides near ties exactly (FP64 sqrt(d2), then neighbor
-//     id, then search input index) and writes the rows (emit).  The distance is
+//     keeps every query's candidates (collect); eight lanes or more per query
+//     then sort them by FP32 keys, re-decide near ties exactly (FP64 sqrt(d2),
+//     then neighbor id, then search input index) and write the rows (emit).  The distance is
 //     computed in FP64 without fused multiply-adds, so it is bit-identical to
 //     the reference.
 //   * k nearest (k <= 64) is the same with a radius per query that holds its k
@@ -546,8 +546,9 @@ __device__ __forceinline__ void collect_finish_knn(const CollectParams& P, uint3
 // BATCH: several problems (a problem batch, or several requests on one scene):
 // each warp has one problem, its tree, its bands and its kmax.  OWN: every
 // query has a radius of its own (KNN).
-// A packet of the clustered 1M x 1M sets takes 18 node steps and 87 buckets;
-// what bounds it is instruction issue (about 45 instructions per bucket).
+// A packet of the clustered 1M x 1M sets takes 18 node steps and 87 buckets of
+// about 45 instructions each; what bounds it is the bucket loads (load/store pipe
+// 63% busy, issue 49%, 20 warps per SM to wait on them).
 template <int DIM, bool BATCH, bool OWN>
 __device__ __forceinline__ void collect_packet_body(const CollectParams& P, uint32_t t, CollectWarp& W) {
   const int lane = threadIdx.x & 31;
@@ -659,7 +660,7 @@ __global__ void __launch_bounds__(128) k_collect_single(const __grid_constant__ 
   }
 }
 
-// ---- emit: warp per query -----------------------------------------------------
+// ---- emit ---------------------------------------------------------------------
 // Emitted row writer.
 struct RowSink {
   void* rows;
@@ -1503,18 +1504,6 @@ __global__ void __launch_bounds__(128, 8) k_nearest(const __grid_constant__ Near
   if (valid) P.nearest[qin] = besti == kNone ? 0u : besti;
 }
 
-// ---- ranked summaries ----------------------------------------------------------
-// A query's rows (contiguous, in output order) are reduced to the reference's
-// ranked summary: count, first and last row, and the distances added one by one
-// in row order (so the sum is the one a sequential loop over the rows gives).
-// Every eight consecutive queries also give a partial aggregate, added in query
-// order, which k_summary_final reduces in a fixed order: the aggregate is the
-// same on every run.
-struct SummaryPartial {
-  unsigned long long count, nearest, kth;
-  double sum;
-};
-
 // ---- nearest in-radius witness (k_max 1, one row per query) -------------------
 // offsets[o] = input index of output rank o, offsets[nq] = nq: the emit then
 // writes a query's first row at its input position.
@@ -1795,11 +1784,22 @@ __global__ void k_count_trivial(const float4* qpts, uint32_t nq, uint32_t* ids_o
   }
 }
 
+// ---- ranked summaries ----------------------------------------------------------
+// A query's rows (contiguous, in output order) are reduced to the reference's
+// ranked summary: count, first and last row, and the distances added one by one
+// in row order (so the sum is the one a sequential loop over the rows gives).
+// Every eight consecutive queries also give a partial aggregate, added in query
+// order, which k_summary_final reduces in a fixed order: the aggregate is the
+// same on every run.
+struct SummaryPartial {
+  unsigned long long count, nearest, kth;
+  double sum;
+};
+
 struct SummarySpec {
   RtdlFixedRadiusRankedNeighborSummary* summaries_dev;  // per query, input order (optional)
   RtdlFixedRadiusRankedNeighborAggregate* aggregate_host;
 };
-
 
 constexpr int kSummaryThreads = 128;
 constexpr int kSummaryGroup = 8;  // queries per partial aggregate
@@ -4381,14 +4381,15 @@ void run_directed_hausdorff_noalloc(Scene* sc, const void* queries_dev, uint32_t
 // (build_scene_batch: each problem a tree of its own), answered
 // by one CUDA graph replay with no host read-back inside.  Per batch the graph
 // holds ONE persistent collect launch -- a grid that fills the GPU once, whose
-// warps take 32-query packets (one problem each) from a device work queue
-// until the batch's packets are gone, so small and large problems share the
-// SMs -- then the scan (rows of this batch start where the previous batch's
-// end), the device-driven radius refinement, and the emit kernels striding
-// over device list lengths.  Batches run one after another in the graph and
-// share one set of scratch buffers sized for the largest.  A batch whose heavy
-// queries the refinement passes do not resolve is flagged in its status word
-// and recomputed by the plain batch call at replay, so rows always equal it.
+// warps take packets of 32, 16 or 8 queries (one problem each) from a device
+// work queue until the batch's packets are gone, so small and large problems
+// share the SMs -- then the queries the packets left, the scan (rows of this
+// batch start where the previous batch's end) and the emit kernels striding over
+// device list lengths.  Batches run one after another in the graph and share
+// one set of scratch buffers sized for the largest.  A batch whose heavy
+// queries the narrowing inside the collect does not resolve is flagged in its
+// status word and recomputed by the plain batch call at replay, so rows always
+// equal it.
 namespace {
 
 __global__ void k_add_row_base(unsigned long long* offsets, uint32_t n, const unsigned long long* base,
@@ -4408,7 +4409,7 @@ __global__ void k_empty_batch_rows(const unsigned long long* base, uint32_t prob
   if (blockIdx.x == 0 && threadIdx.x == 0) *next_base = b;
 }
 
-// Persistent collect over one batch: 32-query packets from a work queue.
+// Persistent collect over one batch: packets from a work queue.
 template <int DIM>
 __global__ void __launch_bounds__(kCollectThreads, 6) k_collect_persistent(const __grid_constant__ CollectParams P, unsigned int* queue) {
   __shared__ CollectWarp warps[kCollectThreads / 32];

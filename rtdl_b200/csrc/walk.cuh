@@ -256,7 +256,7 @@ __device__ __forceinline__ uint32_t nodes_met(const SceneView& S, const TreeShap
 // Cuts a packet into runs of neighbouring queries that are worth walking
 // together.  The box around a run may meet far more of the scene than its
 // queries reach: at the edge of a cluster, between clusters, or in a call of
-// few queries over many points.  A walk costs about 50 instructions per bucket
+// few queries over many points.  A walk costs about 45 instructions per bucket
 // its box meets and a query alone 350 and 12 per bucket, so a run of s queries
 // is walked together when its box meets at most 10 s buckets, else its halves
 // are tried, and runs of four that still do not fit go to single() (6 s and

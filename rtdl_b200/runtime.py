@@ -855,10 +855,10 @@ class PreparedB200FixedRadiusRankedSummaryAggregateBatchGraph3D:
     """Captured CUDA graph of prepared-query ranked-summary aggregates; mirrors
     ``PreparedOptixFixedRadiusRankedSummaryAggregateBatchGraph3D`` (``optix_runtime.py:1912-2289``).
 
-    The graph holds the whole fixed-radius path of every request (collect, refinement of heavy
-    queries, emit, summary, aggregate) over buffers allocated once, and runs on its own stream.
+    The graph holds the whole fixed-radius path of every request (collect, emit, summary,
+    aggregate) over buffers allocated once, and runs on its own stream.
     The aggregates are exact (FP64 distances) whatever ``precision`` names; requests whose heavy
-    queries the captured refinement leaves unresolved are recomputed by the plain call."""
+    queries the captured collect leaves unresolved are recomputed by the plain call."""
 
     def __init__(self, owner: PreparedB200FixedRadiusNeighbors3D, prepared_queries: B200Queries, requests, *,
                  precision: str = "float32"):
