@@ -2724,13 +2724,14 @@ constexpr uint32_t kSingleQueries = kSmCount * 32;
 // they are few or lie far apart among its points: the box around a packet then
 // holds little that its queries share.  Time of walking alone over the packets'
 // (fixed radius with 0.5, 32 and 130 in radius; KNN k = 1, 8, 32; uniform and
-// clustered points): 3D, 10k queries 0.70 to 0.95 at any number of points, 40k
-// over 1M points 0.61 to 0.87, 80k over 2M 0.57 to 0.82, 120k over 1M 0.77 to
-// 0.97, 160k 0.93 to 1.16; 2D, 20k over 1M points 0.63 to 0.96, 40k 0.72 to 1.19.
-// With 11,000 in radius 3D packets share more: 40k over 1M points 0.80, 80k 1.35.
-// Nearest points of 40k queries over 1M in 3D: 213 us and 373.
+// clustered points): 3D, 10k queries 0.70 to 0.95 at any number of points, 80k
+// over 1M points 0.68 to 1.05, 120k 0.77 to 0.97, 160k 0.93 to 1.16, over 2M
+// points 160k 0.67 to 0.91, 240k 0.86 to 1.18; 2D, 20k over 1M points 0.63 to
+// 0.96, 40k 0.72 to 1.19.  With 11,000 in radius 3D packets share more: 40k over
+// 1M points 0.80, 80k 1.35.  Nearest points of 40k queries over 1M in 3D: 213 us
+// and 373.
 inline bool queries_alone(uint64_t queries, uint64_t points, int dim) {
-  return dim == 3 ? queries <= 3 * kSingleQueries || 16 * queries <= points
+  return dim == 3 ? queries <= 3 * kSingleQueries || 10 * queries <= points
                   : queries <= kSingleQueries || 50 * queries <= points;
 }
 

@@ -26,9 +26,9 @@ def _first(c, n):
     return {k: v[:n] for k, v in c.items()}
 
 
-# 3D: 14,208 queries, or one per 16 points; 2D: 4,736, or one per 50 points
+# 3D: 14,208 queries, or one per 10 points; 2D: 4,736, or one per 50 points
 @pytest.mark.parametrize("exact", [True, False])
-@pytest.mark.parametrize("dim,ns,line", [(3, 3000, 14208), (3, 240_000, 15_000), (2, 3000, 4736), (2, 300_000, 6000)])
+@pytest.mark.parametrize("dim,ns,line", [(3, 3000, 14208), (3, 240_000, 24_000), (2, 3000, 4736), (2, 300_000, 6000)])
 def test_rows_on_both_sides_of_the_line(gpu, dim, ns, line, exact):
     rng = np.random.default_rng(ns + dim)
     p = np.concatenate([rng.random((ns - 600, dim)), 0.5 + 0.001 * rng.random((600, dim))])  # a spot crowded with 600
