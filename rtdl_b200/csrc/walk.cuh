@@ -257,13 +257,18 @@ __device__ __forceinline__ uint32_t nodes_met(const SceneView& S, const TreeShap
 // together.  The box around a run may meet far more of the scene than its
 // queries reach: at the edge of a cluster, between clusters, or in a call of
 // few queries over many points.  A walk costs about 45 instructions per bucket
-// its box meets and a query alone 350 and 12 per bucket, so a run of s queries
-// is walked together when its box meets at most 10 s buckets, else its halves
-// are tried, and runs of four that still do not fit go to single() (6 s and
-// 16 s: KNN k = 32 of 100k queries 1.26 and 1.12 ms against 1.08).  The
-// buckets are only counted (a step per level-1 node) when the number of level-1
-// nodes, which hold 32 buckets and of which a box meets about 6 each, does not
-// decide (a count of about five steps over the upper levels): up to s / 2 + 4
+// its box meets; a query alone costs 400 and 18 per bucket its own cube meets,
+// which are the cube's share of the run's buckets by volume.  So a run of s
+// queries is walked together when its box meets at most 400 s / (45 - 18 s
+// share) buckets (9 to 20 s), else its halves are tried, and runs of four that
+// still do not fit go to single().  With 10 s whatever the share, rows of 32 in
+// radius for 160k queries over 1M points took 651 us (566), six served requests
+// 1009 (984), a batch of 128 problems 6035 (5918); with 16 and 24 s, 0.5 in radius of
+// 240k queries over 1M clustered points 555 and 636 us (521).  With radii of their
+// own 10 s holds (6 and 16 s: KNN k = 32 of 100k queries 1.26 and 1.12 ms against
+// 1.08).  The buckets are only counted (a step per level-1 node) when the number
+// of level-1 nodes, which hold 32 buckets and of which a box meets about 6 each,
+// does not decide (a count of about five steps over the upper levels): up to s / 2 + 4
 // fit, more than 2 s do not.  Counting the buckets of every hopeless run kept
 // the last packets of a 65k-query shell 25 us longer; with s in place of 2 s too
 // many queries went alone (six served requests 1.03 -> 2.2 ms).  Neither is
@@ -292,19 +297,22 @@ __device__ __forceinline__ void cut_packet(const SceneView& S, const TreeShape* 
       const PacketBox box = packet_box(q, mine);
       PacketBox limit;
       float reach2 = lane_reach2;  // equal in every lane unless own_radii
+      uint32_t most = 10u * (uint32_t)s;  // buckets the run may meet
       bool fits = false;
       if (own_radii) {
         limit = packet_reach_box(q, half, mine);
         reach2 = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(mine ? lane_reach2 : 0.f)));
       } else {
-        const float w = 2.f * sqrtf(reach2);
-        fits = (box.hx - box.lx + w) * (box.hy - box.ly + w) * (box.hz - box.lz + w) <= 8.f * w * w * w;
+        const float w = 2.f * sqrtf(reach2), cube = w * w * w;
+        const float all = (box.hx - box.lx + w) * (box.hy - box.ly + w) * (box.hz - box.lz + w);
+        fits = all <= 8.f * cube;
+        most = (uint32_t)((float)s * fminf(400.f / fmaxf(45.f - 18.f * (float)s * (cube / all), 1.f), 20.f));
       }
       const PacketBox* lim = own_radii ? &limit : nullptr;
       if (!fits) {
         const uint32_t w = (uint32_t)s, met = nodes_met<1>(S, T, box, lim, reach2, stack, lane, 2 * w);
         fits = met <= w / 2 + 4 ||
-               (met <= 2 * w && nodes_met<0>(S, T, box, lim, reach2, stack, lane, 10 * w) <= 10 * w);
+               (met <= 2 * w && nodes_met<0>(S, T, box, lim, reach2, stack, lane, most) <= most);
       }
       if (!fits && s > 4) {
         s >>= 1;
