@@ -2728,11 +2728,16 @@ constexpr uint32_t kSingleQueries = kSmCount * 32;
 // over 1M points 0.68 to 1.05, 120k 0.77 to 0.97, 160k 0.93 to 1.16, over 2M
 // points 160k 0.67 to 0.91, 240k 0.86 to 1.18; 2D, 20k over 1M points 0.63 to
 // 0.96, 40k 0.72 to 1.19.  With 11,000 in radius 3D packets share more: 40k over
-// 1M points 0.80, 80k 1.35.  Nearest points of 40k queries over 1M in 3D: 213 us
-// and 373.
+// 1M points 0.80, 80k 1.35.
 inline bool queries_alone(uint64_t queries, uint64_t points, int dim) {
   return dim == 3 ? queries <= 3 * kSingleQueries || 10 * queries <= points
                   : queries <= kSingleQueries || 50 * queries <= points;
+}
+// Nearest points bound their packets better: 3D, 40k queries over 1M points 0.57
+// (uniform), 0.60 (clustered) and 0.86 (a lattice) of the packets' time, 80k 0.86,
+// 0.81 and 1.39.
+inline bool nearest_alone(uint64_t queries, uint64_t points, int dim) {
+  return queries_alone(dim == 3 && queries > 3 * kSingleQueries ? 2 * queries : queries, points, dim);
 }
 
 // The queries the packets left (their number is on the device).
@@ -4215,7 +4220,7 @@ HausdorffResult run_directed_hausdorff(Scene* sc, const void* queries_dev, uint3
   P.nq = nq;
   P.bands = qp.bands;
   P.nearest = temp;
-  if (queries_alone(nq, sc->n, sc->dim)) {
+  if (nearest_alone(nq, sc->n, sc->dim)) {
     SingleParams H{};
     H.S = P.S;
     H.qpts = P.qpts;
